@@ -1,0 +1,503 @@
+// Exact-slice FP64 products on tcgen05 (see f64_slices.cuh).
+#include "f64_slices.cuh"
+#include "fp_bits.cuh"
+#include "sbe_internal.cuh"
+#include "tc_ptx.cuh"
+
+#include <algorithm>
+
+namespace sbe {
+namespace f64s {
+
+__device__ int g_err;   // a bounded wait gave up
+
+// ---------------------------------------------------------------------------
+// slicing
+
+// Block: 8 rows of one form of one matrix; warps walk the K blocks, a lane takes 8
+// consecutive k of one row (lane = 4 row + chunk), so a warp stores 512 contiguous bytes
+// per plane and the transposed read covers 128-byte segments.  Up to 8 K blocks (Nk <=
+// 256) each value is read once and kept in registers between the row maximum, the norm and
+// the digits; larger rows are read again (from L2).  HBM bound: 16 B read and 32 B written
+// per element.
+__global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ SliceArgs a) {
+  const Form& f = a.f[blockIdx.y];
+  const int kdim = a.kdim, ld = a.ld, b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.x * 8 + (lane >> 2), j = lane & 3;
+  const int nkb = k_blocks(kdim), rows_pad = pad_rows(a.rows);
+  const double2* X = f.src + (long long)b * a.src_batch;
+  const double2* Y = f.add ? f.add + (long long)b * a.src_batch : nullptr;
+  const bool rok = r < a.rows;
+  auto load = [&](int kb, double2* v) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = kb * BK + 8 * j + i;
+      v[i] = make_double2(0.0, 0.0);
+      if (rok && k < kdim) {
+        v[i] = f.transpose ? X[(long long)k * ld + r] : X[(long long)r * ld + k];
+        if (Y) v[i].y += a.add_f * Y[(long long)r * ld + k].x;
+      }
+    }
+  };
+  __shared__ unsigned long long red[8][8];
+  __shared__ float reds[8][8];
+  double2 v[8];
+  unsigned long long m = 0;
+  for (int kb = warp; kb < nkb; kb += 8) {
+    load(kb, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = max(m, max(absbits(v[i].x), absbits(v[i].y)));
+  }
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  if (j == 0) red[warp][lane >> 2] = m;
+  __syncthreads();
+  m = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) m = max(m, red[w][lane >> 2]);
+  const int Em = max_exp(m);
+  float sq = 0.f;
+  for (int kb = warp; kb < nkb; kb += 8) {
+    if (nkb > 8) load(kb, v);
+    if (Em != kBadExp) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sq += scaled_sq(v[i].x, Em) + scaled_sq(v[i].y, Em);
+    }
+  }
+  sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+  sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+  if (j == 0) reds[warp][lane >> 2] = sq;
+  __syncthreads();
+  sq = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) sq += reds[w][lane >> 2];
+  const int E = norm_exp(Em, sq);
+  if (warp == 0 && j == 0 && rok) f.e[(long long)b * a.rows + r] = E;
+  if (!rok) return;
+  __half* dst = f.dst + (long long)b * a.dst_batch;
+  for (int kb = warp; kb < nkb; kb += 8) {
+    if (nkb > 8) load(kb, v);
+    long long q[8];
+    __half* d = dst + chunk_off(rows_pad, r, kb, j);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(v[i].x, E);
+    store_digits(q, d, a.plane);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(v[i].y, E);
+    store_digits(q, d + NS * a.plane, a.plane);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// the product kernel
+
+constexpr int A_SLOT = BM * BK * 2;        // 8 KB: one digit plane of an A tile
+constexpr int B_SLICE = BN * BK * 2;       // 4 KB
+constexpr int B_SLOT = NS * B_SLICE;       // 32 KB: all planes of a B tile
+constexpr int NA = 16, NB = 3;             // ring slots
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
+constexpr int SMEM = 1024 + NA * A_SLOT + NB * B_SLOT + 512;
+
+struct Unit {
+  int job, b, m0, n0, comp, part;
+  int kb0, nkb;     // K blocks of one real product
+  int q0, q1;       // range of this part in the sequence of (product, K block)
+  bool dead;
+};
+
+__device__ __forceinline__ Unit unit_of(const Launch& L, int u) {
+  Unit t;
+  int j = 0;
+  while (j + 1 < L.njobs && L.base[j + 1] <= u) ++j;
+  const Job& d = L.job[j];
+  int r = u - L.base[j];
+  const int tn = (d.N + BN - 1) / BN, tm = (d.M + BM - 1) / BM;
+  t.job = j;
+  t.n0 = (r % tn) * BN;
+  r /= tn;
+  t.m0 = (r % tm) * BM;
+  r /= tm;
+  t.comp = d.cplx ? r & 1 : 0;
+  if (d.cplx) r >>= 1;
+  t.part = r % d.parts;
+  t.b = r / d.parts;
+  t.kb0 = 0;
+  t.nkb = d.nkb;
+  t.dead = false;
+  if (d.band) {
+    // rows 2 dd + c of the sheared operand are zero outside t' in [-d, Nk - 1 - d], d =
+    // dd - (Nk - 1); output (m, dd) is used only if m + dd lies in [Nk - 1, 2 Nk - 2]
+    const int nk = d.band;
+    const int dd_lo = t.n0 / 2, dd_hi = min((t.n0 + BN) / 2, 2 * nk - 1) - 1;
+    const int tlo = max(0, nk - 1 - dd_hi), thi = min(nk - 1, 2 * nk - 2 - dd_lo);
+    t.kb0 = tlo / BK;
+    t.nkb = thi >= tlo ? thi / BK + 1 - t.kb0 : 0;
+    const int m_hi = min(t.m0 + BM, d.M) - 1;
+    t.dead = dd_lo + t.m0 > 2 * nk - 2 || dd_hi + m_hi < nk - 1;
+  }
+  const int n = t.nkb * (d.cplx ? 2 : 1);
+  t.q0 = (int)((long long)t.part * n / d.parts);
+  t.q1 = (int)((long long)(t.part + 1) * n / d.parts);
+  return t;
+}
+
+__device__ __forceinline__ void tmem_ld32_nw(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+
+// v 2^e rounded once to FP64, on the integer pipe while the result is normal
+__device__ __forceinline__ double ll_scaled(long long v, int e) {
+  if (v == 0) return 0.0;
+  const unsigned long long sg = (unsigned long long)v & 0x8000000000000000ull;
+  const unsigned long long a = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int lz = __clzll((long long)a);
+  const unsigned long long n = a << lz;
+  const unsigned long long mant = (n >> 11) + ((n >> 10) & 1ull);   // 53 bits, half up
+  const int ef = 1023 + 63 - lz + e;
+  if (ef <= 0 || ef >= 2046) return ldexp((double)v, e);
+  return __longlong_as_double((long long)(sg | (((unsigned long long)(ef - 1) << 52) + mant)));
+}
+
+__device__ __forceinline__ int f2i(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }
+
+// One accumulator t of a thread's 32 columns into the running sums, in units of 2^6 of
+// sum_t acc_t 2^(8 (7 - t)), modulo 2^64 (the whole sum stays below 2^62).
+template <int T>
+__device__ __forceinline__ void add_acc(long long* run, const uint32_t* r) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    if (T < 3)   // the shift exceeds 32: the high word alone changes
+      run[j] = (long long)((unsigned long long)run[j] +
+                           ((unsigned long long)((unsigned)f2i(r[j]) << (18 - 8 * T)) << 32));
+    else
+      run[j] += (long long)f2i(r[j]) * (1ll << (50 - 8 * T));
+  }
+}
+// accumulators 6 and 7 (rounded to two units at most)
+__device__ __forceinline__ void add_acc67(long long* run, const uint32_t* r6, const uint32_t* r7) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j)
+    run[j] += (long long)__float2int_rn(
+        fmaf(__uint_as_float(r7[j]), 1.f / 64.f, __uint_as_float(r6[j]) * 4.f));
+}
+
+// Persistent, one CTA per SM: warp 0 streams digit planes (bulk copies; A planes through
+// a ring of single planes, B tiles through three slots), warp 1 issues the MMAs, warps 2-9
+// drain the accumulators.  A tile is 128 x 64: its eight accumulators fill the 512 TMEM
+// columns at 64 t, so the plane A_i against the adjacent planes B_0 .. B_{7 - i} (rows
+// adjacent in shared memory) is one or two MMAs of N up to 256 whose result lands on the
+// accumulators i .. 7: 36 plane products per K block in 12 MMAs per 16 k.  Per K block 96 KB
+// of planes feed 2304 clocks of MMA.  The accumulators are drained every 128 k
+// (exactness) with the MMAs waiting.
+__global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__ Launch L) {
+  using namespace tc;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + NA * A_SLOT;
+  uint64_t* fullA = reinterpret_cast<uint64_t*>(sB + NB * B_SLOT);
+  uint64_t* emptyA = fullA + NA;
+  uint64_t* fullB = emptyA + NA;
+  uint64_t* emptyB = fullB + NB;
+  uint64_t* tfull = emptyB + NB;
+  uint64_t* tempty = tfull + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int nunits = L.base[L.njobs];
+  int* err = &g_err;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NA; ++i) {
+      mbar_init(&fullA[i], 1);
+      mbar_init(&emptyA[i], 1);
+    }
+    for (int i = 0; i < NB; ++i) {
+      mbar_init(&fullB[i], 1);
+      mbar_init(&emptyB[i], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, EPI_WARPS);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0 && lane == 0) {
+    // ---------------- producer ----------------
+    int sa = 0, sb = 0;
+    uint32_t pa = 0, pb = 0;   // phases of the ring positions
+    long long na = 0, nb = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
+      const Unit t = unit_of(L, u);
+      if (t.dead) continue;
+      const Job& d = L.job[t.job];
+      for (int q = t.q0; ok && q < t.q1; ++q) {
+        const int p = q >= t.nkb ? 1 : 0, kb = t.kb0 + q - p * t.nkb;
+        // re: Ar Br, Ai Bi; im: Ar Bi, Ai Br
+        const int ca = p, cb = t.comp ? 1 - p : p;
+        const __half* gb = d.B + (long long)cb * NS * d.b_plane + (long long)t.b * d.b_batch +
+                           ((long long)kb * d.b_pad + t.n0) * BK;
+        if (!mbar_wait(&emptyB[sb], pb ^ 1u, err, abort_flag)) {
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&fullB[sb], B_SLOT);
+        for (int i = 0; i < NS; ++i)
+          bulk_load(sB + sb * B_SLOT + i * B_SLICE, gb + i * d.b_plane, B_SLICE, &fullB[sb]);
+        ++nb;
+        if (++sb == NB) {
+          sb = 0;
+          pb ^= 1u;
+        }
+        const __half* ga = d.A + (long long)ca * NS * d.a_plane + (long long)t.b * d.a_batch +
+                           ((long long)kb * d.a_pad + t.m0) * BK;
+        for (int i = 0; i < NS; ++i) {
+          if (!mbar_wait(&emptyA[sa], pa ^ 1u, err, abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&fullA[sa], A_SLOT);
+          bulk_load(sA + sa * A_SLOT, ga + i * d.a_plane, A_SLOT, &fullA[sa]);
+          ++na;
+          if (++sa == NA) {
+            sa = 0;
+            pa ^= 1u;
+          }
+        }
+      }
+    }
+    // no copy may land in shared memory after the CTA has gone: wait (bounded) for the
+    // last ones issued
+    volatile int never = 0;
+    for (long long i = na > NA ? na - NA : 0; i < na; ++i)
+      mbar_wait(&fullA[i % NA], (uint32_t)((i / NA) & 1), err, &never);
+    for (long long i = nb > NB ? nb - NB : 0; i < nb; ++i)
+      mbar_wait(&fullB[i % NB], (uint32_t)((i / NB) & 1), err, &never);
+  } else if (warp == 1 && lane == 0) {
+    // ---------------- MMA issuer ----------------
+    int sa = 0, sb = 0;
+    uint32_t pa = 0, pb = 0, pt = 1;   // tempty: the first wait passes at once
+    bool ok = true;
+    for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
+      const Unit t = unit_of(L, u);
+      if (t.dead) continue;
+      const Job& d = L.job[t.job];
+      // signs of the two real products: re = Ar Br - Ai Bi, im = Ar Bi + Ai Br with the
+      // conjugations' signs on the imaginary planes
+      const int s0 = t.comp ? (d.conj_b ? -1 : 1) : 1;
+      const int s1 = t.comp ? (d.conj_a ? -1 : 1) : -(d.conj_a ? -1 : 1) * (d.conj_b ? -1 : 1);
+      for (int c0 = t.q0; ok && c0 < t.q1; c0 += CHUNK) {
+        const int c1 = min(c0 + CHUNK, t.q1);
+        if (!mbar_wait(tempty, pt, err, abort_flag)) {
+          ok = false;
+          break;
+        }
+        pt ^= 1u;
+        tc_fence_after();
+        for (int q = c0; ok && q < c1; ++q) {
+          const int sg = (q >= t.nkb ? s1 : s0) * (d.neg ? -1 : 1);
+          const uint32_t nega = sg < 0 ? (1u << 13) : 0u;
+          if (!mbar_wait(&fullB[sb], pb, err, abort_flag)) {
+            ok = false;
+            break;
+          }
+          const uint64_t db = sw64_desc(smem_u32(sB + sb * B_SLOT));
+          for (int i = 0; i < NS; ++i) {
+            if (!mbar_wait(&fullA[sa], pa, err, abort_flag)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t da = sw64_desc(smem_u32(sA + sa * A_SLOT));
+            const int nblk = NS - i;                      // accumulators i .. 7
+            const int n1 = nblk > 4 ? (nblk + 1) / 2 : nblk, n2 = nblk - n1;
+            const uint32_t id1 = idesc_f16(BM, BN, 0) - ((uint32_t)(BN >> 3) << 17) +
+                                 ((uint32_t)(n1 * BN >> 3) << 17) + nega;
+            const uint32_t id2 = idesc_f16(BM, BN, 0) - ((uint32_t)(BN >> 3) << 17) +
+                                 ((uint32_t)(n2 * BN >> 3) << 17) + nega;
+#pragma unroll
+            for (int k16 = 0; k16 < 2; ++k16) {
+              const uint32_t acc = (q == c0 && i == 0 && k16 == 0) ? 0u : 1u;
+              const uint64_t ko = 2u * k16;
+              umma_f16(tmem + i * BN, da + ko, db + ko, id1, acc);
+              if (n2 > 0)
+                umma_f16(tmem + (i + n1) * BN, da + ko,
+                         db + ko + (uint64_t)(n1 * (B_SLICE >> 4)), id2, acc);
+            }
+            umma_commit(&emptyA[sa]);
+            if (++sa == NA) {
+              sa = 0;
+              pa ^= 1u;
+            }
+          }
+          umma_commit(&emptyB[sb]);
+          if (++sb == NB) {
+            sb = 0;
+            pb ^= 1u;
+          }
+        }
+        if (ok) umma_commit(tfull);
+      }
+    }
+  } else if (warp >= 2) {
+    // ---------------- epilogue: 32 columns of one row per thread ----------------
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t ta = tmem + ((uint32_t)(32 * quarter) << 16) + half * 32;
+    uint32_t pt = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
+      const Unit t = unit_of(L, u);
+      if (t.dead) continue;
+      const Job& d = L.job[t.job];
+      long long run[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) run[j] = 0;
+      for (int c0 = t.q0; c0 < t.q1; c0 += CHUNK) {
+        if (!mbar_wait(tfull, pt, err, abort_flag)) {
+          ok = false;
+          break;
+        }
+        pt ^= 1u;
+        tc_fence_after();
+        uint32_t a[32], b[32];
+        tmem_ld32_nw(ta, a);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 1 * BN, b);
+        add_acc<0>(run, a);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 2 * BN, a);
+        add_acc<1>(run, b);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 3 * BN, b);
+        add_acc<2>(run, a);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 4 * BN, a);
+        add_acc<3>(run, b);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 5 * BN, b);
+        add_acc<4>(run, a);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 6 * BN, a);
+        add_acc<5>(run, b);
+        tmem_ld_wait();
+        tmem_ld32_nw(ta + 7 * BN, b);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty);
+        add_acc67(run, a, b);
+      }
+      const int m = t.m0 + 32 * quarter + lane;
+      if (!ok || m >= d.M) continue;
+      const int ea = d.ea[(long long)t.b * d.M + m];
+      const int* eb = d.eb + (long long)t.b * d.N;
+      double* o = d.out + t.part * d.o_part + t.comp * d.o_comp + (long long)t.b * d.o_batch;
+      const int n0 = t.n0 + 32 * half;
+      if (d.band) {
+        // column 2 dd + c of row m: component c of element [m][m + dd - (Nk - 1)]
+        const int nk = d.band;
+        o += (long long)m * d.ldo;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int n = n0 + j, k2 = m + (n >> 1) - (nk - 1);
+          if (n < d.N && k2 >= 0 && k2 < nk) {
+            const int e = eb[n];
+            o[2 * k2 + (n & 1)] = (ea == kBadExp || e == kBadExp)
+                                      ? __longlong_as_double(0x7FF8000000000000ll)
+                                      : ll_scaled(run[j], ea + e - 62);
+          }
+        }
+      } else {
+        o += (long long)m * d.ldo + n0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (n0 + j < d.N) {
+            const int e = eb[n0 + j];
+            o[j] = (ea == kBadExp || e == kBadExp) ? __longlong_as_double(0x7FF8000000000000ll)
+                                                   : ll_scaled(run[j], ea + e - 62);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+}  // namespace f64s
+
+void launch_f64_slice(const f64s::SliceArgs& a, int nforms, cudaStream_t s) {
+  f64s::k_f64_slice<<<dim3((a.rows + 7) / 8, nforms, a.batch), 256, 0, s>>>(a);
+}
+
+static int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
+      v = 1;
+    return v;
+  }();
+  return n;
+}
+
+int launch_f64_gemm(const f64s::Job* jobs, int njobs, cudaStream_t s) {
+  if (njobs < 1 || njobs > f64s::MAX_JOBS) return fail(SBE_ERR_ARG, "f64 gemm: 1 to 16 jobs");
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      f64s::k_f64_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, f64s::SMEM);
+  if (attr != cudaSuccess) return fail(SBE_ERR_CUDA, "f64 gemm: cannot raise the shared-memory limit");
+  f64s::Launch L{};
+  L.njobs = njobs;
+  long long nt = 0;
+  for (int j = 0; j < njobs; ++j) {
+    const f64s::Job& d = jobs[j];
+    if (d.M < 1 || d.N < 1 || d.nkb < 1 || d.batch < 1 || d.parts < 1 || d.a_pad % 128 ||
+        d.b_pad % 64 || d.M > d.a_pad || d.N > d.b_pad)
+      return fail(SBE_ERR_ARG, "f64 gemm: bad job");
+    L.job[j] = d;
+    L.base[j] = (int)nt;
+    nt += (long long)((d.N + f64s::BN - 1) / f64s::BN) * ((d.M + f64s::BM - 1) / f64s::BM) *
+          (d.cplx ? 2 : 1) * d.parts * d.batch;
+  }
+  if (nt > 0x7FFFFFFF) return fail(SBE_ERR_ARG, "f64 gemm: too many tiles");
+  L.base[njobs] = (int)nt;
+  const int grid = (int)std::min<long long>(nt, sm_count());
+  f64s::k_f64_gemm<<<grid, f64s::THREADS, f64s::SMEM, s>>>(L);
+  return cuda_check(cudaGetLastError(), "f64 gemm launch");
+}
+
+int f64_gemm_error(int* flag) {
+  *flag = 0;
+  int rc = cuda_check(cudaMemcpyFromSymbol(flag, f64s::g_err, sizeof(int)), "f64 gemm: read flag");
+  if (!rc && *flag) {
+    const int z = 0;
+    rc = cuda_check(cudaMemcpyToSymbol(f64s::g_err, &z, sizeof(int)), "f64 gemm: clear flag");
+  }
+  return rc;
+}
+
+}  // namespace sbe

@@ -294,6 +294,7 @@ int sbe_ctx_destroy(SbeCtx* c) {
   if (c->arena && cudaFree(c->arena) != cudaSuccess) rc = SBE_ERR_CUDA;
   if (c->p2q_coef && cudaFree(c->p2q_coef) != cudaSuccess) rc = SBE_ERR_CUDA;
   sbe::mixed_free(c);
+  sbe::f64_free(c);
   delete c;
   if (rc != SBE_OK) set_error("sbe_ctx_destroy: cudaFree failed");
   return rc;
@@ -363,8 +364,12 @@ static int rhs_single(int which, int nk, const double* C, const double* D, const
   GemmBatch b{};
   const double2 *c2 = (const double2*)C, *d2 = (const double2*)D, *p2 = (const double2*)P;
   const double2 *heh = (const double2*)Heh, *hee = (const double2*)Hee, *hhh = (const double2*)Hhh;
+  if (which == 0 && (!GamE || !GamH)) return fail(SBE_ERR_ARG, "sbe_dpdt: null rates");
+  int rc = SBE_OK;
+  if (f64_rhs_single(which, nk, c2, d2, p2, heh, hee, hhh, GamE, GamH, (const double2*)OffP,
+                     (double2*)out, as_stream(stream), &rc))
+    return rc;
   if (which == 0) {
-    if (!GamE || !GamH) return fail(SBE_ERR_ARG, "sbe_dpdt: null rates");
     b.t[b.nterms++] = T(hhh, OP_N, p2, OP_N, pos);
     b.t[b.nterms++] = T(d2, OP_T, heh, OP_T, neg);
     b.t[b.nterms++] = T(p2, OP_N, hee, OP_T, pos);
@@ -654,11 +659,24 @@ static void prep_frozen(SbeCtx* c, const double2* P, const double2* C, const dou
                         cudaStream_t s) {
   (void)P;
   launch_prep_scalar(c, C, D, s);
+  if (f64_prepare(c, s)) f64_step_operands(c, s);
   launch_gamma(c, -1, s);
   if (c->any_offdiag) {
     launch_offdiag_D(c, -1, nullptr, false, s);
     launch_offdiag_AB(c, -1, s);
   }
+}
+
+// Sources of the state a step has left (occupations in c->ne, c->nh).
+static int step_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D,
+                        double2* src, cudaStream_t s) {
+  if (!c->f64) {
+    launch_sources(c, P, C, D, c->ne, c->nh, src, s);
+    return SBE_OK;
+  }
+  const int rc = sbe::f64_sources(c, P, C, D, src, s);
+  if (!rc) launch_sources_final(c, c->ne, c->nh, src, s);
+  return rc;
 }
 
 int sbe_rhs(SbeCtx* c, const double* P, const double* C, const double* D, const double* Ek,
@@ -668,8 +686,14 @@ int sbe_rhs(SbeCtx* c, const double* P, const double* C, const double* D, const 
   const double2 *p = (const double2*)P, *cc = (const double2*)C, *d = (const double2*)D;
   if (precision == SBE_PREC_FP64) {
     prep_frozen(c, p, cc, d, s);
-    launch_calch_ctx(c, p, cc, d, (const double2*)Ek, s);
-    launch_rhs64_ctx(c, p, cc, d, (double2*)dP, (double2*)dC, (double2*)dD, s);
+    double2* out[3] = {(double2*)dP, (double2*)dC, (double2*)dD};
+    if (c->f64) {
+      const int rc = sbe::f64_rhs(c, p, cc, d, (const double2*)Ek, 0, 0.0, out, nullptr, s);
+      if (rc) return rc;
+    } else {
+      launch_calch_ctx(c, p, cc, d, (const double2*)Ek, s);
+      launch_rhs64_ctx(c, p, cc, d, out[0], out[1], out[2], s);
+    }
   } else if (precision == SBE_PREC_MIXED) {
     int rc = sbe::rhs_mixed(c, p, cc, d, (const double2*)Ek, (double2*)dP, (double2*)dC,
                             (double2*)dD, s);
@@ -690,10 +714,18 @@ int sbe_leapfrog_step(SbeCtx* c, double* const* state9, const double* Ek, double
   for (int i = 0; i < 9; ++i) st[i] = (double2*)state9[i];
   // SBEs.py:5061-5068: p2 = YY3, C2 = CC3, D2 = DD3 (level 3 is "current")
   prep_frozen(c, st[2], st[5], st[8], s);
-  launch_calch_ctx(c, st[2], st[5], st[8], (const double2*)Ek, s);
-  launch_rhs64_ctx(c, st[2], st[5], st[8], c->dP, c->dC, c->dD, s);
+  int rc = SBE_OK;
+  if (c->f64) {
+    double2* out[3] = {c->dP, c->dC, c->dD};
+    rc = sbe::f64_rhs(c, st[2], st[5], st[8], (const double2*)Ek, 0, 0.0, out, nullptr, s);
+    if (rc) return rc;
+  } else {
+    launch_calch_ctx(c, st[2], st[5], st[8], (const double2*)Ek, s);
+    launch_rhs64_ctx(c, st[2], st[5], st[8], c->dP, c->dC, c->dD, s);
+  }
   launch_leapfrog(c, st, (const double2*)Ek, dt, s);
-  launch_sources(c, st[0], st[3], st[6], c->ne, c->nh, (double2*)src_out, s);
+  rc = step_sources(c, st[0], st[3], st[6], (double2*)src_out, s);
+  if (rc) return rc;
   launch_leap_shuffle(c, st, s);
   return cuda_check(cudaGetLastError(), "sbe_leapfrog_step");
 }
@@ -719,12 +751,19 @@ int sbe_rk4_step(SbeCtx* c, double* P, double* C, double* D, const double* Ek0, 
       xd = c->xs + 2 * n;
     }
     launch_stage_field(c, (const double2*)Ek0, (const double2*)dEk, frac[st - 1], s);
+    if (c->f64) {
+      double2* X[3] = {p, cc, d};
+      const int rc = sbe::f64_rhs(c, xp, xc, xd, c->ekst, st, dt, nullptr, X, s);
+      if (rc) return rc;
+      continue;
+    }
     launch_calch_ctx(c, xp, xc, xd, c->ekst, s);
     launch_rhs64_ctx(c, xp, xc, xd, c->dP, c->dC, c->dD, s);
     launch_rk4_axpy(c, st, dt, p, cc, d, s);
   }
   launch_relax_norm(c, p, cc, d, (const double2*)Ek0, dt, s);
-  launch_sources(c, p, cc, d, c->ne, c->nh, (double2*)src_out, s);
+  const int rc = step_sources(c, p, cc, d, (double2*)src_out, s);
+  if (rc) return rc;
   return cuda_check(cudaGetLastError(), "sbe_rk4_step");
 }
 
@@ -776,7 +815,10 @@ int capture_graph(SbeCtx* c, int precision, const std::function<int(cudaStream_t
   if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess)
     return fail(SBE_ERR_CUDA, "graph capture: stream");
   int rc = SBE_OK;
-  if (precision == SBE_PREC_MIXED) rc = mixed_prepare(c, cs);
+  if (precision == SBE_PREC_MIXED)
+    rc = mixed_prepare(c, cs);
+  else
+    f64_prepare(c, cs);
   if (rc == SBE_OK) rc = cuda_check(cudaStreamSynchronize(cs), "graph warm-up");
   cudaGraph_t g = nullptr;
   if (rc == SBE_OK) {

@@ -67,6 +67,8 @@ struct SbeCtx {
 
   int any_offdiag = 0;                   // some wire has OffDiagDph on
   void* mixed = nullptr;                 // mixed-precision workspace (sbe_tc.cu)
+  void* f64 = nullptr;                   // FP64 digit-plane workspace (f64_path.cu)
+  int f64_off = 0;                       // no room for it: the FP64 path stays on SIMT
 
   // kernel timing (sbe_ctx_profile): event pairs per category, and a pool
   int prof = 0;
@@ -153,6 +155,25 @@ void launch_gemm64(const WireDev* d_wires, int nw, int nk_max, const GemmBatch& 
 void launch_sources_gemm64(SbeCtx* c, const GemmBatch& b, cudaStream_t s);
 void launch_rhs64_ctx(SbeCtx* c, const double2* P, const double2* C, const double2* D,
                       double2* dP, double2* dC, double2* dD, cudaStream_t s);
+// f64_path.cu: the FP64 right-hand side and sources on exact-slice tensor-core products.
+// f64_prepare: the context's workspace (false: the SIMT kernels are to be used); the
+// single-wire calls return false likewise, else *rc is their result.
+bool f64_prepare(SbeCtx* c, cudaStream_t s);
+void f64_free(SbeCtx* c);
+void f64_step_operands(SbeCtx* c, cudaStream_t s);
+int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, const double2* Ek,
+            int stage, double dt, double2* const* out, double2* const* X, cudaStream_t s);
+int f64_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D, double2* src,
+                cudaStream_t s);
+bool f64_rhs_single(int which, int nk, const double2* C, const double2* D, const double2* P,
+                    const double2* Heh, const double2* Hee, const double2* Hhh, const double* gamE,
+                    const double* gamH, const double2* offp, double2* out, cudaStream_t s, int* rc);
+bool f64_calch_single(int nk, const double2* Meh, const double2* Wee, const double2* Whh,
+                      const double2* C, const double2* D, const double2* P, const double* VC,
+                      const double* Ee, const double* Eh, double gap, int excitons, int lf,
+                      int freepot, double2* Heh, double2* Hee, double2* Hhh, cudaStream_t s, int* rc);
+void launch_vq_from_vc(int nk, const double* VC, double* vq, cudaStream_t s);
+int f64_gemm_error(int* flag);
 // sbe_step.cu
 void launch_leapfrog(SbeCtx* c, double2* const* st9, const double2* Ek, double dt,
                      cudaStream_t s);

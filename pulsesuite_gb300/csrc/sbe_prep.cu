@@ -867,6 +867,10 @@ __global__ void k_vq_from_vc(int nk, const double* VC, double* vq) {
   for (int n = 0; n < 3; ++n) vq[n * nk + q] = VC[((long long)q * nk + 0) * 3 + n];
 }
 
+void launch_vq_from_vc(int nk, const double* VC, double* vq, cudaStream_t s) {
+  k_vq_from_vc<<<(nk + 127) / 128, 128, 0, s>>>(nk, VC, vq);
+}
+
 __global__ void k_traces_single(int nk, const double2* C, const double2* D, double2* tr) {
   int d = (int)blockIdx.x - (nk - 1);
   int which = blockIdx.y;
@@ -896,6 +900,10 @@ int launch_calch_single(int nk, const double2* Meh, const double2* Wee, const do
                         const double2* C, const double2* D, const double2* P, const double* VC,
                         const double* Ee, const double* Eh, double gap, int excitons, int lf,
                         int freepot, double2* Heh, double2* Hee, double2* Hhh, cudaStream_t s) {
+  int rc = SBE_OK;
+  if (f64_calch_single(nk, Meh, Wee, Whh, C, D, P, VC, Ee, Eh, gap, excitons, lf, freepot, Heh, Hee,
+                       Hhh, s, &rc))
+    return rc;
   double* vq = nullptr;
   double2* tr = nullptr;
   if (cudaMallocAsync(&vq, sizeof(double) * 3 * nk, s) != cudaSuccess ||

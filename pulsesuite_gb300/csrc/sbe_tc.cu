@@ -1935,6 +1935,12 @@ extern "C" int sbe_ctx_check(SbeCtx* c, void* stream) {
   if (!c) return fail(SBE_ERR_ARG, "sbe_ctx_check: null context");
   int rc = cuda_check(cudaStreamSynchronize(as_stream(stream)), "sbe_ctx_check");
   if (rc) return rc;
+  int f = 0;
+  rc = f64_gemm_error(&f);
+  if (rc) return rc;
+  if (f)
+    return fail(SBE_ERR_TIMEOUT, "a pipeline wait of the FP64 products timed out (results of the "
+                                 "affected calls are invalid)");
   MixedAll* A = all_of(c);
   if (!A) return SBE_OK;
   int h = 0;
