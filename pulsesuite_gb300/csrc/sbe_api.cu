@@ -216,6 +216,7 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   add((void**)&c->charge, D8 * 2 * n_wires);
   add((void**)&c->ekst, C16 * 3 * orr);
   add((void**)&c->occf, 4 * 2 * ov);
+  add((void**)&c->occd, D8 * 2 * ov);
   add((void**)&c->dconst, 4 * 16 * (size_t)n_wires);
   add((void**)&c->dpre, 4 * 4 * ov);
   add((void**)&c->dwl, sizeof(int) * (size_t)n_wires);

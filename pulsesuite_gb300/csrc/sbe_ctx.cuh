@@ -56,6 +56,7 @@ struct SbeCtx {
   double* charge = nullptr;              // 2*nw sum |C_kk|, sum |D_kk| before the last normalisation
   double2* ekst = nullptr;               // 3*tot_r stage field
   float* occf = nullptr;                 // 2*tot_vec |ne|, |nh| in FP32
+  double* occd = nullptr;                // 2*tot_vec |ne|, |nh|
   float* dconst = nullptr;               // 16*nw FP32 dephasing constants
   float* dpre = nullptr;                 // 4*tot_vec FP32 dephasing prefactors per |q|
 

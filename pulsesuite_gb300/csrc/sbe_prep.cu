@@ -163,64 +163,194 @@ void launch_gamma(SbeCtx* c, int w_only, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// dephasing.py:227-317 (_CalcOffDiagDeph_E2_jit / _H2_jit): D[q+Nk][k] for one
-// carrier species "a" (electrons for De, holes for Dh) against itself and the
-// other species "b".  FP64, literal energy differences from the Ee/Eh arrays.
-// g3 = [gam_eh, gam_e, gam_h]: De uses (g0, g2), Dh uses (g1, g2) (quirk kept).
-__global__ void k_offdiag_D64(const WireDev* wires, int w_only, const double2* ne,
-                              const double2* nh, const double* Ee, const double* Eh,
-                              const double* vs, double g0, double g1, double g2, int use_g,
-                              double* De, double* Dh) {
-  int wi = (w_only >= 0) ? w_only : blockIdx.z;
-  const WireDev W = wires[wi];
-  const int nk = W.nk;
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  int qi = blockIdx.y >> 1;          // 0 .. 2nk
-  int which = blockIdx.y & 1;        // 0 -> De, 1 -> Dh
-  if (qi > 2 * nk || k >= nk) return;
-  int q = qi - nk;
-  double ga = use_g ? (which == 0 ? g0 : g1) : (which == 0 ? W.gam_eh : W.gam_e);
-  double gab = use_g ? g2 : W.gam_h;
-  const double2* na = (which == 0 ? ne : nh) + W.off_vec;
-  const double2* nb = (which == 0 ? nh : ne) + W.off_vec;
-  const double* Ea = (which == 0 ? Ee : Eh) + W.off_vec;
-  const double* Eb = (which == 0 ? Eh : Ee) + W.off_vec;
-  const double* v = vs + 3 * W.off_vec;
-  int aq = q < 0 ? -q : q;
-  double vaa = 0.0, vab = 0.0;
-  if (aq >= 1 && aq < nk) {
-    double x = v[(which == 0 ? 1 : 2) * nk + aq];
-    double y = v[0 * nk + aq];
-    vaa = x * x;
-    vab = y * y;
+// dephasing.py:227-317 (_CalcOffDiagDeph_E2_jit / _H2_jit) in FP64: D[q+Nk][k] for one
+// carrier species "a" (electrons for De, holes for Dh) against itself and the other
+// species "b".  g3 = [gam_eh, gam_e, gam_h]: De uses (g0, g2), Dh uses (g1, g2) (quirk kept).
+//
+// GB300 runs two FP64 operations per clock and SM, so the kernel is written for their
+// count.  On the reference grid the energy differences are integer forms (see k_offdiag_D32,
+// which also derives row -q from the sums of row q):
+//   a-a: E = 2 c_a dkr^2 q (k - p + q), tabulated per q: two FMAs per (q, k, p);
+//   a-b: E = q dkr^2 [c_a (2k - 2 j0 + q) + c_b (2p - 2 j0 + q)]: one add, one FMA for
+//        x = E^2 + b^2, a reciprocal in three FMAs, two FMAs for the sums.
+// NW wires of equal constants share every reciprocal.  A block takes one q >= 1, one species
+// and 32 k (a lane each); its eight warps split the p and meet in a fixed order.  The rows q
+// = 0, +-Nk and the elements outside the band are zero from the context's creation on.
+// 71.2 -> 2.6 ms at 2 wires x Nk = 512 (38.1 -> 0.6 ms at 8 x 256) against a division and
+// four hypot per (q, k, p) over every q; the energy differences as integers also take the
+// error of Dh at Nk = 128 from 3.9e-14 to 2.9e-15.
+__global__ void k_occd(const WireDev* wires, int w_only, const double2* ne, const double2* nh,
+                       double* occd) {
+  const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= W.nk) return;
+  const double2 e = ne[W.off_vec + k], h = nh[W.off_vec + k];
+  occd[2 * W.off_vec + k] = hypot(e.x, e.y);
+  occd[2 * W.off_vec + W.nk + k] = hypot(h.x, h.y);
+}
+
+// 1 / x from the approximate reciprocal y (2^-20): y (1 + e + e^2), e = 1 - x y, leaves e^3
+__device__ __forceinline__ double rcp64(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+struct Deph64 {
+  const WireDev* wires;
+  const int* wl;        // wire indices of the group
+  int nwl, w_only;      // w_only >= 0: that wire alone
+  const double *occd, *vs;
+  double g0, g1, g2;
+  int use_g;
+  double *De, *Dh;
+};
+
+constexpr int kDephP = 64;   // p per shared-memory chunk
+
+template <int NW>
+__global__ void __launch_bounds__(256) k_offdiag_D64(const Deph64 a) {
+  const int q = blockIdx.y + 1, which = blockIdx.z, k0 = blockIdx.x * 32;
+  const int w0 = a.w_only >= 0 ? a.w_only : a.wl[0];
+  const WireDev& W0 = a.wires[w0];
+  const int nk = W0.nk;
+  if (k0 + q >= nk) return;
+  extern __shared__ __align__(16) double dsh[];
+  double2* ws = reinterpret_cast<double2*>(dsh);     // [kDephP][NW] weight pairs
+  double* eb = dsh + 2 * kDephP * NW;                // [kDephP] b energies (a-b)
+  double* red = eb + kDephP;                         // [8][2 NW][33]
+  double* Ltab = red + 8 * 2 * NW * 33;              // 2 (nk - q): m = i - (nk - 1) + q
+  __shared__ double fa[NW], fb[NW];
+  __shared__ int oa[NW], ob[NW], wi[NW];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, k = k0 + lane;
+  const double ga = a.use_g ? (which == 0 ? a.g0 : a.g1) : (which == 0 ? W0.gam_eh : W0.gam_e);
+  const double gab = a.use_g ? a.g2 : W0.gam_h;
+  const double baa = kHbar * ga, bab = kHbar * gab, dk2 = W0.dkr * W0.dkr;
+  const double ca = kHbar * kHbar / (2.0 * (which == 0 ? W0.me : W0.mh)) * dk2;
+  const double cb = kHbar * kHbar / (2.0 * (which == 0 ? W0.mh : W0.me)) * dk2;
+  if (tid < NW) {
+    double va = 0.0, vb = 0.0;
+    int o1 = 0, o2 = 0, w = 0;
+    if (tid < a.nwl) {
+      w = a.w_only >= 0 ? a.w_only : a.wl[tid];
+      const WireDev& W = a.wires[w];
+      const double* v = a.vs + 3 * W.off_vec;
+      const double x = v[(which == 0 ? 1 : 2) * nk + q], y = v[q];
+      va = x * x * ga;     // V^2 b / hbar
+      vb = y * y * gab;
+      o1 = (int)(2 * W.off_vec + (which == 0 ? 0 : nk));
+      o2 = (int)(2 * W.off_vec + (which == 0 ? nk : 0));
+    }
+    fa[tid] = va;
+    fb[tid] = vb;
+    oa[tid] = o1;
+    ob[tid] = o2;
+    wi[tid] = w;
   }
-  double acc = 0.0;
-  if (k + q >= 0 && k + q < nk) {
-    double nak = hypot(na[k].x, na[k].y);
-    double bb = kHbar * ga, b2 = kHbar * gab;
-    if (vaa != 0.0) {
-      int plo = max(q + 1, 0), phi = min(q + nk - 1, nk - 1);
-      for (int p = plo; p <= phi; ++p) {
-        double Ed = Ea[k + q] + Ea[p - q] - Ea[p] - Ea[k];
-        double npq = hypot(na[p - q].x, na[p - q].y);
-        double np_ = hypot(na[p].x, na[p].y);
-        double lr = (bb / kPi) / (Ed * Ed + bb * bb);
-        acc += vaa * lr * (npq * (1.0 - np_) * (1.0 - nak) + (1.0 - npq) * np_ * nak);
+  for (int i = tid; i < 2 * (nk - q); i += 256) {
+    const double E = 2.0 * ca * (double)((long long)q * (i - (nk - 1) + q));
+    Ltab[i] = rcp64(fma(E, E, baa * baa));
+  }
+  double acc[NW][2];
+#pragma unroll
+  for (int w = 0; w < NW; ++w) acc[w][0] = acc[w][1] = 0.0;
+  __syncthreads();
+  // a-a: p in [q + 1, Nk - 1]
+  for (int p0 = q + 1; p0 < nk; p0 += kDephP) {
+    for (int i = tid; i < kDephP * NW; i += 256) {
+      const int p = p0 + i / NW, w = i % NW;
+      double2 v = make_double2(0.0, 0.0);
+      if (p < nk && w < a.nwl) {
+        const double x = a.occd[oa[w] + p - q], y = a.occd[oa[w] + p];
+        v = make_double2(fa[w] * x * (1.0 - y), fa[w] * (1.0 - x) * y);
+      }
+      ws[i] = v;
+    }
+    __syncthreads();
+    const int pend = min(kDephP, nk - p0);
+    if (k + q < nk) {
+#pragma unroll 4
+      for (int pp = warp; pp < pend; pp += 8) {
+        const double l = Ltab[k - (p0 + pp) + nk - 1];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+          const double2 v = ws[pp * NW + w];
+          acc[w][0] = fma(l, v.x, acc[w][0]);
+          acc[w][1] = fma(l, v.y, acc[w][1]);
+        }
       }
     }
-    if (vab != 0.0) {
-      int plo = max(0, -q), phi = min(nk - 1, nk - 1 - q);
-      for (int p = plo; p <= phi; ++p) {
-        double Ed = Ea[k + q] + Eb[p + q] - Eb[p] - Ea[k];
-        double npq = hypot(nb[p + q].x, nb[p + q].y);
-        double np_ = hypot(nb[p].x, nb[p].y);
-        double lr = (b2 / kPi) / (Ed * Ed + b2 * b2);
-        acc += vab * lr * (npq * (1.0 - np_) * (1.0 - nak) + (1.0 - npq) * np_ * nak);
+    __syncthreads();
+  }
+  // a-b: p in [0, Nk - 1 - q]
+  const int c = -2 * W0.dnk - 1 + q;
+  const double ea = ca * (double)((long long)q * (2 * k + c)), b2 = bab * bab;
+  for (int p0 = 0; p0 < nk - q; p0 += kDephP) {
+    for (int i = tid; i < kDephP * NW; i += 256) {
+      const int p = p0 + i / NW, w = i % NW;
+      double2 v = make_double2(0.0, 0.0);
+      if (p < nk - q && w < a.nwl) {
+        const double x = a.occd[ob[w] + p + q], y = a.occd[ob[w] + p];
+        v = make_double2(fb[w] * x * (1.0 - y), fb[w] * (1.0 - x) * y);
+      }
+      ws[i] = v;
+    }
+    if (tid < kDephP) eb[tid] = cb * (double)((long long)q * (2 * (p0 + tid) + c));
+    __syncthreads();
+    const int pend = min(kDephP, nk - q - p0);
+    if (k + q < nk) {
+#pragma unroll 4
+      for (int pp = warp; pp < pend; pp += 8) {
+        const double E = ea + eb[pp];
+        const double l = rcp64(fma(E, E, b2));
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+          const double2 v = ws[pp * NW + w];
+          acc[w][0] = fma(l, v.x, acc[w][0]);
+          acc[w][1] = fma(l, v.y, acc[w][1]);
+        }
       }
     }
+    __syncthreads();
   }
-  double* D = (which == 0 ? De : Dh) + W.off_dd;
-  D[(long long)qi * nk + k] = acc * kPi / kHbar;
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    red[(warp * 2 * NW + 2 * w) * 33 + lane] = acc[w][0];
+    red[(warp * 2 * NW + 2 * w + 1) * 33 + lane] = acc[w][1];
+  }
+  __syncthreads();
+  // warp w finishes wire w
+  if (warp >= a.nwl || k + q >= nk) return;
+  double X = 0.0, Y = 0.0;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    X += red[(g * 2 * NW + 2 * warp) * 33 + lane];
+    Y += red[(g * 2 * NW + 2 * warp + 1) * 33 + lane];
+  }
+  const WireDev& W = a.wires[wi[warp]];
+  double* D = (which == 0 ? a.De : a.Dh) + W.off_dd;
+  const double* n = a.occd + oa[warp];
+  const double n1 = n[k], n2 = n[k + q], n0 = n[0], nq = n[q];
+  D[(long long)(nk + q) * nk + k] = (1.0 - n1) * X + n1 * Y;
+  // row -q at k + q: the sums swapped, and the a-a term p = q that row q leaves out
+  const double f = fa[warp] * Ltab[k - q + nk - 1];
+  const double xa = Y + f * ((1.0 - n0) * nq), xb = X + f * (n0 * (1.0 - nq));
+  D[(long long)(nk - q) * nk + k + q] = (1.0 - n2) * xa + n2 * xb;
+}
+
+static size_t deph64_smem(int nw, int nk) {
+  return sizeof(double) * ((size_t)2 * kDephP * nw + kDephP + 8 * 2 * nw * 33 + 2 * nk);
+}
+
+template <int NW>
+static void deph64_launch(const Deph64& a, int nk, cudaStream_t s) {
+  static const bool raised = [] {
+    return cudaFuncSetAttribute(k_offdiag_D64<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)deph64_smem(NW, 4096)) == cudaSuccess;
+  }();
+  (void)raised;
+  k_offdiag_D64<NW><<<dim3((nk + 31) / 32, nk - 1, 2), 256, deph64_smem(NW, nk), s>>>(a);
 }
 
 // FP32 version of the off-diagonal dephasing sums for the mixed-precision path.
@@ -668,12 +798,43 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
     }
     return;
   }
-  dim3 g((c->nk_max + 127) / 128, 2 * (2 * c->nk_max + 1), w_only >= 0 ? 1 : c->nw);
-  double g0 = 0, g1 = 0, g2 = 0;
-  int use_g = 0;
-  if (g3) { g0 = g3[0]; g1 = g3[1]; g2 = g3[2]; use_g = 1; }
-  k_offdiag_D64<<<g, 128, 0, s>>>(c->d_wires, w_only, c->ne, c->nh, c->Ee, c->Eh, c->vs, g0, g1,
-                                  g2, use_g, c->De, c->Dh);
+  k_occd<<<dim3((c->nk_max + 127) / 128, w_only >= 0 ? 1 : c->nw), 128, 0, s>>>(
+      c->d_wires, w_only, c->ne, c->nh, c->occd);
+  Deph64 a{};
+  a.wires = c->d_wires;
+  a.w_only = w_only;
+  a.occd = c->occd;
+  a.vs = c->vs;
+  if (g3) {
+    a.g0 = g3[0];
+    a.g1 = g3[1];
+    a.g2 = g3[2];
+    a.use_g = 1;
+  }
+  a.De = c->De;
+  a.Dh = c->Dh;
+  if (w_only >= 0) {
+    a.nwl = 1;
+    deph64_launch<1>(a, c->wires[w_only].nk, s);
+    return;
+  }
+  for (const auto& g : c->dgroups) {
+    const int gk = c->wires[c->dwl_host[g.first]].nk;
+    for (int o = 0; o < g.second;) {
+      const int left = g.second - o;
+      a.wl = c->dwl + g.first + o;
+      a.nwl = std::min(left, 8);
+      if (left > 4)
+        deph64_launch<8>(a, gk, s);
+      else if (left > 2)
+        deph64_launch<4>(a, gk, s);
+      else if (left > 1)
+        deph64_launch<2>(a, gk, s);
+      else
+        deph64_launch<1>(a, gk, s);
+      o += a.nwl;
+    }
+  }
 }
 
 // dephasing.py:320-356: x = i hbar (A p + p B^T) with A[kh,j] = Dh[j-kh+Nk][kh],

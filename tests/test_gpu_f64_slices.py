@@ -108,3 +108,31 @@ def test_non_finite_rows(bad):
     assert bool(torch.isfinite(torch.view_as_real(got)[keep]).all())
     scale = torch.linalg.norm(Hhh) * torch.linalg.norm(D) / HBAR
     assert float((got - ref)[keep].abs().max()) <= 4 * nk * U * float(scale)
+
+
+@pytest.mark.parametrize("nk,nw", ((4, 1), (6, 2), (32, 3), (34, 5), (64, 8), (66, 9), (130, 1)))
+def test_dephasing_sums(nk, nw):
+    """De, Dh of groups of one to nine equal wires, k tiles of 32 and chunks of 64 p with
+    remainders.  The literal sums round four energies of up to 5.1 eV (k = 3e9 1/m, electrons)
+    against hbar gamma = 0.66 meV: 4 u 7750 = 3.5e-12 of a Lorentzian; 1e-11 of the largest."""
+    from oracle import sbe_oracle as O
+    from pulsesuite_gb300.wires import WireContext, WireSpec
+    mat = dict(me=0.067 * O.ME0, mh=0.45 * O.ME0, gap=1.52 * O.E0, HO=100e-3 * O.E0, Delta0=6e-9,
+               gam_e=1e12, gam_h=2e12, gam_eh=1.5e12, epsr=12.9, Oph=36e-3 * O.E0 / O.HBAR,
+               Gph=3e-3 * O.E0 / O.HBAR)
+    L = np.pi / (3e9 / (nk / 2 - 0.5))
+    ctx = WireContext([WireSpec(nk=nk, L=L, wire_index=w + 1, **mat) for w in range(nw)])
+    rng = np.random.default_rng(nk)
+    occ = rng.uniform(0, 0.9, (2, nw, nk))
+    C, D = (ctx.pack([np.diag(o).astype(complex) for o in occ[s]]) for s in range(2))
+    De, Dh = (x.cpu().numpy().reshape(nw, 2 * nk + 1, nk) for x in ctx.deph(C, D))
+    E = O.wire_constants(mat, O.wire_grid(nk, L)["kr"])
+    for w in range(nw):
+        ne, nh = (torch.as_tensor(occ[s][w].astype(complex)).cuda() for s in range(2))
+        VC = ctx.screened_arrays(w, ne, nh)[0].cpu().numpy()
+        for got, ref in ((De[w], O.offdiag_De(occ[0][w], occ[1][w], E["Ee"], E["Eh"], mat["gam_eh"],
+                                              mat["gam_h"], VC)),
+                         (Dh[w], O.offdiag_Dh(occ[0][w], occ[1][w], E["Ee"], E["Eh"], mat["gam_e"],
+                                              mat["gam_h"], VC))):
+            assert np.max(np.abs(got - ref)) <= 1e-11 * np.max(np.abs(ref))
+    ctx.close()
