@@ -9,24 +9,15 @@
 // (SBEs.py:5917).  The polarisation current J = (P^{n+1} - P^n) / dt drives the
 // E update; Ex is the longitudinal field of Rho and Px (rhoPJ.py:703-880).
 //
-// Splines on the GPU.  The FMM spline is a tridiagonal solve whose elimination
-// factors depend on the knots only; they are computed once.  The per-step
-// forward and backward sweeps are first-order linear recurrences whose
-// multipliers have magnitude ~2 - sqrt(3) = 0.268 on a uniform grid, so each
-// thread solves a segment of kSeg points after kWarm warm-up points started from
-// zero (0.268^48 ~ 3e-28 relative); the first and last segments start from the
-// exact boundary values.
+// The splines of a step are one launch for the grid fields and one for the wire sources
+// (spline.cu).
 #include <cmath>
 #include <vector>
 
 #include "fp_bits.cuh"
 #include "pstd.cuh"
 #include "pstd3d.cuh"
-
-namespace {
-constexpr int kSeg = 16;
-constexpr int kWarm = 48;
-}  // namespace
+#include "spline.cuh"
 
 struct SbeCouple {
   SbeCtx* ctx = nullptr;
@@ -39,12 +30,7 @@ struct SbeCouple {
   double* wx = nullptr;       // nw wire positions
   long long* probl = nullptr; // wire spline problems (5 per wire): knot offset, value offset
   int* probn = nullptr;       // knots per problem
-  long long* wfl = nullptr;   // per-wire knot sets (2 per wire: offset, 0)
-  int* wfn = nullptr;         // knots per wire
-  double *g_b = nullptr, *g_t = nullptr;   // grid pivots and multipliers (nx)
-  double *w_b = nullptr, *w_t = nullptr;   // wire-grid pivots and multipliers (tot_r)
-  double2 *g_y = nullptr, *g_c1 = nullptr, *g_c2 = nullptr, *g_coef = nullptr;
-  double2 *w_c1 = nullptr, *w_c2 = nullptr, *w_coef = nullptr;
+  double2 *g_y = nullptr, *g_coef = nullptr, *w_coef = nullptr;
   double2* twr = nullptr;     // tot_r: exp(-2 pi i m / Nr) per wire
   float2* twrf = nullptr;     // the same in FP32
   double2* wv = nullptr;      // 3 tot_r: sampled fields on the wire grids (real parts)
@@ -56,191 +42,6 @@ struct SbeCouple {
 
 namespace sbe {
 namespace {
-
-// ---- spline pieces ----------------------------------------------------------
-struct SplBatch {
-  const double* X;      // knots base
-  const double* B;      // pivots base (indexed like X)
-  const double* T;      // multipliers base
-  const double2* Y;     // values base
-  double2* C1;          // scratch (indexed like Y)
-  double2* C2;
-  double2* coef;        // 3 per value: b, c, d blocks of n
-  const int* n;         // per problem (nullptr: n0 for all)
-  const long long* off; // per problem: ko, vo (nullptr: ko = 0, vo = p * n0)
-  int n0;
-};
-
-__device__ __forceinline__ void prob_of(const SplBatch& s, int p, int& n, long long& ko,
-                                        long long& vo) {
-  if (s.off) {
-    n = s.n[p];
-    ko = s.off[2 * p];
-    vo = s.off[2 * p + 1];
-  } else {
-    n = s.n0;
-    ko = 0;
-    vo = (long long)p * s.n0;
-  }
-}
-
-// numpy complex / complex with a zero imaginary divisor: a * (1 / d).
-__device__ __forceinline__ double2 cdivr(double2 a, double d) {
-  const double s = 1.0 / d;
-  return make_double2(a.x * s, a.y * s);
-}
-
-// Pivots b and multipliers t of the FMM forward elimination (spliner.py:1338-1373).
-__global__ void k_spl_factors(int nprob, const double* X, const int* nv, const long long* off,
-                              int n0, double* B, double* T) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nprob) return;
-  const int n = nv ? nv[p] : n0;
-  const long long ko = off ? off[2 * p] : 0;
-  const double* x = X + ko;
-  double* b = B + ko;
-  double* t = T + ko;
-  for (int i = 1; i < n - 1; ++i) b[i] = 2.0 * ((x[i] - x[i - 1]) + (x[i + 1] - x[i]));
-  b[0] = -(x[1] - x[0]);
-  b[n - 1] = -(x[n - 1] - x[n - 2]);
-  t[0] = 0.0;
-  for (int i = 1; i < n; ++i) {
-    const double d = x[i] - x[i - 1];
-    t[i] = d * (1.0 / b[i - 1]);  // numpy complex division by (b + 0i)
-    b[i] = b[i] - t[i] * d;
-  }
-}
-
-__device__ __forceinline__ double2 delta(const double2* y, const double* x, int i) {
-  return cdivr(csub(y[i + 1], y[i]), x[i + 1] - x[i]);
-}
-
-// Right-hand side: second differences and the FMM end conditions.
-__global__ void k_spl_rhs(SplBatch s) {
-  const int p = blockIdx.y;
-  int n;
-  long long ko, vo;
-  prob_of(s, p, n, ko, vo);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double* x = s.X + ko;
-  const double2* y = s.Y + vo;
-  double2 c;
-  if (i >= 1 && i <= n - 2) {
-    c = csub(delta(y, x, i), delta(y, x, i - 1));
-  } else if (i == 0) {
-    const double2 s1 = csub(delta(y, x, 1), delta(y, x, 0));
-    const double2 s2 = csub(delta(y, x, 2), delta(y, x, 1));
-    c = csub(cdivr(s2, x[3] - x[1]), cdivr(s1, x[2] - x[0]));
-    const double d0 = x[1] - x[0];
-    c = cdivr(cscale(c, d0 * d0), x[3] - x[0]);
-  } else {
-    const double2 sa = csub(delta(y, x, n - 2), delta(y, x, n - 3));
-    const double2 sb = csub(delta(y, x, n - 3), delta(y, x, n - 4));
-    c = csub(cdivr(sa, x[n - 1] - x[n - 3]), cdivr(sb, x[n - 2] - x[n - 4]));
-    const double dl = x[n - 1] - x[n - 2];
-    c = cdivr(cscale(make_double2(-c.x, -c.y), dl * dl), x[n - 1] - x[n - 4]);
-  }
-  s.C1[vo + i] = c;
-}
-
-// Forward sweep c_i -= t_i c_{i-1}, then c_{n-1} /= b_{n-1}.
-__global__ void k_spl_fwd(SplBatch s) {
-  const int p = blockIdx.y;
-  int n;
-  long long ko, vo;
-  prob_of(s, p, n, ko, vo);
-  const int s0 = (blockIdx.x * blockDim.x + threadIdx.x) * kSeg;
-  if (s0 >= n) return;
-  const double* t = s.T + ko;
-  const double2* c1 = s.C1 + vo;
-  double2* c2 = s.C2 + vo;
-  const int e = min(s0 + kSeg, n);
-  int i0 = max(1, s0 - kWarm);
-  double2 v = (i0 == 1) ? c1[0] : make_double2(0.0, 0.0);
-  if (s0 == 0) c2[0] = c1[0];
-  for (int i = i0; i < e; ++i) {
-    const double ti = t[i];
-    const double2 ci = c1[i];
-    v = make_double2(ci.x - ti * v.x, ci.y - ti * v.y);
-    if (i >= s0) c2[i] = v;
-  }
-  if (e == n) c2[n - 1] = cdivr(v, s.B[ko + n - 1]);
-}
-
-// Backward sweep c_i = (c_i - d_i c_{i+1}) / b_i.
-__global__ void k_spl_bwd(SplBatch s) {
-  const int p = blockIdx.y;
-  int n;
-  long long ko, vo;
-  prob_of(s, p, n, ko, vo);
-  const int s0 = (blockIdx.x * blockDim.x + threadIdx.x) * kSeg;
-  if (s0 >= n) return;
-  const double* x = s.X + ko;
-  const double* b = s.B + ko;
-  const double2* c2 = s.C2 + vo;
-  double2* c3 = s.C1 + vo;  // the right-hand side is dead: reuse its buffer
-  const int e = min(s0 + kSeg, n);
-  if (e == n) c3[n - 1] = c2[n - 1];
-  const int i0 = min(n - 2, e - 1 + kWarm);
-  double2 v = (i0 == n - 2) ? c2[n - 1] : make_double2(0.0, 0.0);
-  for (int i = i0; i >= s0; --i) {
-    const double di = x[i + 1] - x[i];
-    const double2 ci = c2[i];
-    v = cdivr(make_double2(ci.x - di * v.x, ci.y - di * v.y), b[i]);
-    if (i < e) c3[i] = v;
-  }
-}
-
-// Final coefficients (spliner.py:1384-1394).
-__global__ void k_spl_final(SplBatch s) {
-  const int p = blockIdx.y;
-  int n;
-  long long ko, vo;
-  prob_of(s, p, n, ko, vo);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double* x = s.X + ko;
-  const double2* y = s.Y + vo;
-  const double2* c = s.C1 + vo;
-  double2* bb = s.coef + 3 * vo;
-  double2* cc = bb + n;
-  double2* dd = bb + 2 * n;
-  if (i < n - 1) {
-    const double di = x[i + 1] - x[i];
-    const double2 t = cadd(c[i + 1], cscale(c[i], 2.0));
-    bb[i] = csub(cdivr(csub(y[i + 1], y[i]), di), cscale(t, di));
-    dd[i] = cdivr(csub(c[i + 1], c[i]), di);
-    cc[i] = cscale(c[i], 3.0);
-  } else {
-    const double dl = x[n - 1] - x[n - 2];
-    const double2 t = cadd(c[n - 2], cscale(c[n - 1], 2.0));
-    bb[i] = cadd(cdivr(csub(y[n - 1], y[n - 2]), dl), cscale(t, dl));
-    cc[i] = cscale(c[n - 1], 3.0);
-    dd[i] = cdivr(csub(c[n - 1], c[n - 2]), dl);
-  }
-}
-
-__device__ __forceinline__ int locate_sorted(const double* xx, int n, double x) {
-  if (x < xx[0]) return 0;
-  if (x >= xx[n - 1]) return n - 1;
-  int jl = 0, ju = n;
-  while (ju - jl > 1) {
-    const int jm = (ju + jl) >> 1;
-    if (x >= xx[jm]) jl = jm;
-    else ju = jm;
-  }
-  return jl;
-}
-
-__device__ __forceinline__ double2 spl_eval(const double2* y, const double2* b, int n, int i,
-                                            double dx) {
-  const double2* c = b + n;
-  const double2* d = b + 2 * n;
-  double2 t = cadd(c[i], cscale(d[i], dx));
-  t = cadd(b[i], cscale(t, dx));
-  return cadd(y[i], cscale(t, dx));
-}
 
 // Grid fields -> wire grids: spline at x_w + r_j, window, real part.
 __global__ void k_couple_eval(const WireDev* wires, int nx, const double* xg, const double2* gy,
@@ -445,41 +246,24 @@ __global__ void k_twr(const WireDev* wires, double2* twr, float2* twrf) {
   twrf[W.off_r + m] = make_float2(f64_to_f32(c), f64_to_f32(s));
 }
 
-void run_splines(const SplBatch& b, int nprob, int nmax, cudaStream_t s) {
-  const int tpb = 128;
-  const dim3 ge((nmax + tpb - 1) / tpb, nprob);
-  const int nseg = (nmax + kSeg - 1) / kSeg;
-  const dim3 gs((nseg + tpb - 1) / tpb, nprob);
-  k_spl_rhs<<<ge, tpb, 0, s>>>(b);
-  k_spl_fwd<<<gs, tpb, 0, s>>>(b);
-  k_spl_bwd<<<gs, tpb, 0, s>>>(b);
-  k_spl_final<<<ge, tpb, 0, s>>>(b);
-}
-
 SplBatch grid_batch(SbeCouple* cp) {
   SplBatch b{};
   b.X = cp->p->x;
-  b.B = cp->g_b;
-  b.T = cp->g_t;
   b.Y = cp->g_y;
-  b.C1 = cp->g_c1;
-  b.C2 = cp->g_c2;
   b.coef = cp->g_coef;
   b.n0 = cp->p->nx;
+  b.nf = 3;
   return b;
 }
 
 SplBatch wire_batch(SbeCouple* cp) {
   SplBatch b{};
   b.X = cp->ctx->r;
-  b.B = cp->w_b;
-  b.T = cp->w_t;
   b.Y = cp->src;
-  b.C1 = cp->w_c1;
-  b.C2 = cp->w_c2;
   b.coef = cp->w_coef;
   b.n = cp->probn;
   b.off = cp->probl;
+  b.nf = 5;
   return b;
 }
 
@@ -636,7 +420,7 @@ int couple_sample(SbeCouple* cp, const double2* Ex, const double2* E, int precis
   SbeCtx* c = cp->ctx;
   const int nx = cp->p->nx;
   k_stage3<<<(nx + 255) / 256, 256, 0, s>>>(nx, Ex, E, cp->g_y);
-  run_splines(grid_batch(cp), 3, nx, s);
+  launch_splines(grid_batch(cp), 1, nx, s);
   k_couple_eval<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(
       c->d_wires, nx, cp->p->x, cp->g_y, cp->g_coef, cp->wx, c->r, c->window, cp->wv, cp->wvf);
   if (precision == SBE_PREC_MIXED)
@@ -651,7 +435,7 @@ int couple_sample(SbeCouple* cp, const double2* Ex, const double2* E, int precis
 int couple_deposit(SbeCouple* cp, cudaStream_t s) {
   SbeCtx* c = cp->ctx;
   const int nx = cp->p->nx;
-  run_splines(wire_batch(cp), cp->nprob_w, c->nr_max, s);
+  launch_splines(wire_batch(cp), c->nw, c->nr_max, s);
   k_couple_deposit<<<(nx + 63) / 64, 64, 0, s>>>(c->d_wires, c->nw, nx, cp->p->x, cp->wx, c->r,
                                                    cp->src, cp->w_coef, cp->Pg, cp->rho);
   return cuda_check(cudaGetLastError(), "couple deposit");
@@ -693,18 +477,8 @@ int sbe_couple_create(SbeCtx* c, SbePstd* p, const double* wire_x, const SbeCoup
       {(void**)&cp->wx, sizeof(double) * c->nw},
       {(void**)&cp->probn, sizeof(int) * cp->nprob_w},
       {(void**)&cp->probl, sizeof(long long) * 2 * cp->nprob_w},
-      {(void**)&cp->wfn, sizeof(int) * c->nw},
-      {(void**)&cp->wfl, sizeof(long long) * 2 * c->nw},
-      {(void**)&cp->g_b, sizeof(double) * nx},
-      {(void**)&cp->g_t, sizeof(double) * nx},
-      {(void**)&cp->w_b, sizeof(double) * R},
-      {(void**)&cp->w_t, sizeof(double) * R},
       {(void**)&cp->g_y, sizeof(double2) * 3 * nx},
-      {(void**)&cp->g_c1, sizeof(double2) * 3 * nx},
-      {(void**)&cp->g_c2, sizeof(double2) * 3 * nx},
       {(void**)&cp->g_coef, sizeof(double2) * 9 * nx},
-      {(void**)&cp->w_c1, sizeof(double2) * 5 * R},
-      {(void**)&cp->w_c2, sizeof(double2) * 5 * R},
       {(void**)&cp->w_coef, sizeof(double2) * 15 * R},
       {(void**)&cp->twr, sizeof(double2) * R},
       {(void**)&cp->twrf, sizeof(float2) * R},
@@ -734,13 +508,8 @@ int sbe_couple_create(SbeCtx* c, SbePstd* p, const double* wire_x, const SbeCoup
   // wire spline problems: wire w, component k -> n = Nr, knots at off_r, values at 5 off_r + k Nr
   std::vector<int> pn(cp->nprob_w);
   std::vector<long long> pl(2 * cp->nprob_w);
-  std::vector<long long> wl(2 * c->nw);
-  std::vector<int> wn(c->nw);
   for (int w = 0; w < c->nw; ++w) {
     const WireDev& W = c->wires[w];
-    wl[2 * w] = W.off_r;
-    wl[2 * w + 1] = 0;
-    wn[w] = W.nr;
     for (int k = 0; k < 5; ++k) {
       const int pi = 5 * w + k;
       pn[pi] = W.nr;
@@ -751,12 +520,7 @@ int sbe_couple_create(SbeCtx* c, SbePstd* p, const double* wire_x, const SbeCoup
   cudaMemcpyAsync(cp->wx, wire_x, sizeof(double) * c->nw, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(cp->probn, pn.data(), sizeof(int) * pn.size(), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(cp->probl, pl.data(), sizeof(long long) * pl.size(), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(cp->wfn, wn.data(), sizeof(int) * wn.size(), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(cp->wfl, wl.data(), sizeof(long long) * wl.size(), cudaMemcpyHostToDevice, s);
   // elimination factors of the grid knots and of each wire's knots (computed once)
-  k_spl_factors<<<1, 32, 0, s>>>(1, p->x, nullptr, nullptr, p->nx, cp->g_b, cp->g_t);
-  k_spl_factors<<<(c->nw + 31) / 32, 32, 0, s>>>(c->nw, c->r, cp->wfn, cp->wfl, 0, cp->w_b,
-                                                 cp->w_t);
   k_twr<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, cp->twr, cp->twrf);
   int rc = cuda_check(cudaGetLastError(), "sbe_couple_create");
   if (rc == SBE_OK) rc = cuda_check(cudaStreamSynchronize(s), "sbe_couple_create: tables");
@@ -886,12 +650,10 @@ struct SbeCouple3 {
   double* wxy = nullptr;        // 2 nw wire positions (x, y)
   int *col_start = nullptr, *col_wire = nullptr;
   double* col_gate = nullptr;
-  int *probn = nullptr, *wfn = nullptr;
-  long long *probl = nullptr, *wfl = nullptr;
-  double *z_b = nullptr, *z_t = nullptr;   // spline factors of the grid z knots
-  double *w_b = nullptr, *w_t = nullptr;   // of the wire knots
-  double2 *lines = nullptr, *l_c1 = nullptr, *l_c2 = nullptr, *l_coef = nullptr;   // 3 nw nz
-  double2 *w_c1 = nullptr, *w_c2 = nullptr, *w_coef = nullptr;
+  int* probn = nullptr;
+  long long* probl = nullptr;
+  double2 *lines = nullptr, *l_coef = nullptr;   // 3 nw nz, 9 nw nz
+  double2* w_coef = nullptr;
   double2* twr = nullptr;
   float2* twrf = nullptr;
   double2* wv = nullptr;
@@ -907,27 +669,21 @@ namespace {
 SplBatch line_batch(SbeCouple3* cp) {
   SplBatch b{};
   b.X = cp->p->x[2];
-  b.B = cp->z_b;
-  b.T = cp->z_t;
   b.Y = cp->lines;
-  b.C1 = cp->l_c1;
-  b.C2 = cp->l_c2;
   b.coef = cp->l_coef;
   b.n0 = cp->p->n[2];
+  b.nf = 3;
   return b;
 }
 
 SplBatch wire_batch3(SbeCouple3* cp) {
   SplBatch b{};
   b.X = cp->ctx->r;
-  b.B = cp->w_b;
-  b.T = cp->w_t;
   b.Y = cp->src;
-  b.C1 = cp->w_c1;
-  b.C2 = cp->w_c2;
   b.coef = cp->w_coef;
   b.n = cp->probn;
   b.off = cp->probl;
+  b.nf = 5;
   return b;
 }
 
@@ -942,7 +698,7 @@ int c3_sample(SbeCouple3* cp, const double2* E, int precision, cudaStream_t s) {
   const int nz = p->n[2];
   k_c3_lines<<<dim3((nz + 127) / 128, c->nw), 128, 0, s>>>(p->n[0], p->n[1], nz, p->x[0],
                                                            p->x[1], cp->wxy, E, cp->lines);
-  run_splines(line_batch(cp), 3 * c->nw, nz, s);
+  launch_splines(line_batch(cp), c->nw, nz, s);
   k_c3_eval<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(
       c->d_wires, nz, p->x[2], cp->lines, cp->l_coef, c->r, c->window, cp->wv, cp->wvf);
   if (precision == SBE_PREC_MIXED)
@@ -958,7 +714,7 @@ int c3_deposit(SbeCouple3* cp, double dt, cudaStream_t s) {
   SbeCtx* c = cp->ctx;
   SbePstd3* p = cp->p;
   const int nz = p->n[2];
-  run_splines(wire_batch3(cp), 5 * c->nw, c->nr_max, s);
+  launch_splines(wire_batch3(cp), c->nw, c->nr_max, s);
   k_c3_wire_lines<<<dim3((nz + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, nz, p->x[2], c->r,
                                                                 cp->src, cp->w_coef, cp->dl);
   C3Dep a{};
@@ -1046,18 +802,8 @@ int sbe_couple3_create(SbeCtx* c, SbePstd3* p, const double* wire_xy, const SbeC
       {(void**)&cp->col_gate, sizeof(double) * std::max<size_t>(cgate.size(), 1)},
       {(void**)&cp->probn, sizeof(int) * np},
       {(void**)&cp->probl, sizeof(long long) * 2 * np},
-      {(void**)&cp->wfn, sizeof(int) * c->nw},
-      {(void**)&cp->wfl, sizeof(long long) * 2 * c->nw},
-      {(void**)&cp->z_b, sizeof(double) * nz},
-      {(void**)&cp->z_t, sizeof(double) * nz},
-      {(void**)&cp->w_b, sizeof(double) * R},
-      {(void**)&cp->w_t, sizeof(double) * R},
       {(void**)&cp->lines, sizeof(double2) * L},
-      {(void**)&cp->l_c1, sizeof(double2) * L},
-      {(void**)&cp->l_c2, sizeof(double2) * L},
       {(void**)&cp->l_coef, sizeof(double2) * 3 * L},
-      {(void**)&cp->w_c1, sizeof(double2) * 5 * R},
-      {(void**)&cp->w_c2, sizeof(double2) * 5 * R},
       {(void**)&cp->w_coef, sizeof(double2) * 15 * R},
       {(void**)&cp->twr, sizeof(double2) * R},
       {(void**)&cp->twrf, sizeof(float2) * R},
@@ -1085,13 +831,9 @@ int sbe_couple3_create(SbeCtx* c, SbePstd3* p, const double* wire_xy, const SbeC
   }
   cudaMemsetAsync(cp->arena, 0, total, s);
   std::vector<int> pn(np);
-  std::vector<long long> pl(2 * np), wl(2 * c->nw);
-  std::vector<int> wn(c->nw);
+  std::vector<long long> pl(2 * np);
   for (int w = 0; w < c->nw; ++w) {
     const WireDev& W = c->wires[w];
-    wl[2 * w] = W.off_r;
-    wl[2 * w + 1] = 0;
-    wn[w] = W.nr;
     for (int k = 0; k < 5; ++k) {
       pn[5 * w + k] = W.nr;
       pl[2 * (5 * w + k)] = W.off_r;
@@ -1108,11 +850,6 @@ int sbe_couple3_create(SbeCtx* c, SbePstd3* p, const double* wire_xy, const SbeC
   }
   cudaMemcpyAsync(cp->probn, pn.data(), sizeof(int) * pn.size(), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(cp->probl, pl.data(), sizeof(long long) * pl.size(), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(cp->wfn, wn.data(), sizeof(int) * wn.size(), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(cp->wfl, wl.data(), sizeof(long long) * wl.size(), cudaMemcpyHostToDevice, s);
-  k_spl_factors<<<1, 32, 0, s>>>(1, p->x[2], nullptr, nullptr, nz, cp->z_b, cp->z_t);
-  k_spl_factors<<<(c->nw + 31) / 32, 32, 0, s>>>(c->nw, c->r, cp->wfn, cp->wfl, 0, cp->w_b,
-                                                 cp->w_t);
   k_twr<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, cp->twr, cp->twrf);
   rc = cuda_check(cudaGetLastError(), "sbe_couple3_create");
   if (!rc) rc = cuda_check(cudaStreamSynchronize(s), "sbe_couple3_create: tables");

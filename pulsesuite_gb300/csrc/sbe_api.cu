@@ -167,6 +167,7 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   add((void**)&c->window, D8 * orr);
   add((void**)&c->expikr, C16 * okr);
   add((void**)&c->wk, C16 * orr);
+  add((void**)&c->twd, C16 * orr);
   add((void**)&c->vcorr, D8 * 3 * (orr + 2 * n_wires));
   add((void**)&c->ne, C16 * ov);
   add((void**)&c->nh, C16 * ov);

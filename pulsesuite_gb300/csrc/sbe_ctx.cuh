@@ -30,6 +30,7 @@ struct SbeCtx {
   double* window = nullptr;   // tot_r
   double2* expikr = nullptr;  // tot_kr  [nk][nr]
   double2* wk = nullptr;      // tot_r: FFTG(window)
+  double2* twd = nullptr;     // tot_r: exp(-2 pi i m / Nr)
   double* vcorr = nullptr;    // 3*(tot_r + 2*nw): Vint correlation scratch
 
   // ---- per-step workspace ----

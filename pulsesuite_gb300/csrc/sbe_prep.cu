@@ -189,14 +189,6 @@ __global__ void k_occd(const WireDev* wires, int w_only, const double2* ne, cons
   occd[2 * W.off_vec + W.nk + k] = hypot(h.x, h.y);
 }
 
-// 1 / x from the approximate reciprocal y (2^-20): y (1 + e + e^2), e = 1 - x y, leaves e^3
-__device__ __forceinline__ double rcp64(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 struct Deph64 {
   const WireDev* wires;
   const int* wl;        // wire indices of the group

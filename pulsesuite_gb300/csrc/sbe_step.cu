@@ -1,7 +1,9 @@
 // Time stepping of every wire: the reference leapfrog update, relaxation and
 // charge normalisation, RK4 stage updates, the polarisation / charge sources and
 // the field resampling between the propagation grid and the wire grid (FP64).
+#include "cluster_sum.cuh"
 #include "sbe_ctx.cuh"
+#include "spline.cuh"
 
 namespace sbe {
 
@@ -418,9 +420,9 @@ void launch_stage_field(SbeCtx* c, const double2* Ek0, const double2* dEk, doubl
 
 // ---------------------------------------------------------------------------
 // Cubic spline resampling, spliner.py:153-189 rescale_1D_dpc with the
-// Forsythe-Malcolm-Moler coefficients of spline_dpc (spliner.py:1329-1394) and
-// the binary search of locate (spliner.py:1137-1167).  The coefficient solve
-// is a sequential tridiagonal sweep: one thread per field.
+// Forsythe-Malcolm-Moler coefficients of spline_dpc (spliner.py:1329-1394, spline.cu) and
+// the binary search of locate (spliner.py:1137-1167).  Two or three knots have their own
+// formulas: one thread per field.
 __device__ void fmm_spline(int n, const double* x, const double2* y, double2* b, double2* c,
                            double2* d) {
   if (n < 3) {
@@ -477,18 +479,6 @@ __device__ void fmm_spline(int n, const double* x, const double2* y, double2* b,
   d[n - 1] = d[n - 2];
 }
 
-__device__ int locate_dev(const double* xx, int n, double x) {
-  if (x < xx[0]) return 0;
-  if (x >= xx[n - 1]) return n - 1;
-  int jl = 0, ju = n;
-  while (ju - jl > 1) {
-    int jm = (ju + jl) / 2;
-    if (x >= xx[jm]) jl = jm;
-    else ju = jm;
-  }
-  return jl;
-}
-
 __global__ void k_spline_coef(int n, const double* x, const double2* y, int nf, double2* coef) {
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
@@ -496,60 +486,102 @@ __global__ void k_spline_coef(int n, const double* x, const double2* y, int nf, 
   fmm_spline(n, x, y + (long long)f * n, b, b + n, b + 2 * n);
 }
 
-// evaluate nf splines (knots x0, n0) at x1 (n1 points); values outside
-// [min x0, max x0] are 0; optional window multiply and real part.
-__global__ void k_spline_eval(int n0, const double* x0, const double2* y0, const double2* coef,
-                              int n1, const double* x1, int nf, const double* win, int real_part,
-                              double2* out) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int f = blockIdx.y;
-  if (j >= n1 || f >= nf) return;
-  double lo = x0[0], hi = x0[0];
-  for (int i = 1; i < n0; ++i) { lo = fmin(lo, x0[i]); hi = fmax(hi, x0[i]); }
-  double u = x1[j];
-  double2 v = make_double2(0, 0);
-  if (u >= lo && u <= hi) {
-    const double2* y = y0 + (long long)f * n0;
-    const double2* b = coef + (long long)f * 3 * n0;
-    const double2* c = b + n0;
-    const double2* d = b + 2 * n0;
-    int i = locate_dev(x0, n0, u);
-    double dx = u - x0[i];
-    double2 t = cadd(c[i], cscale(d[i], dx));
-    t = cadd(b[i], cscale(t, dx));
-    v = cadd(y[i], cscale(t, dx));
+static void spline_coefs(int n, const double* x, const double2* y, int nf, double2* coef,
+                         cudaStream_t s) {
+  if (n < kSplMin) {
+    k_spline_coef<<<1, 32, 0, s>>>(n, x, y, nf, coef);
+    return;
   }
-  if (win) v = cscale(v, win[j]);
-  if (real_part) v.y = 0.0;
-  out[(long long)f * n1 + j] = v;
+  SplBatch b{};
+  b.X = x;
+  b.Y = y;
+  b.coef = coef;
+  b.n0 = n;
+  b.nf = nf;
+  launch_splines(b, 1, n, s);
 }
 
-// FFTG (usefulsubs.py:2245-2268): F[q] = -(1/N) sum_j f[j] e^{-2 pi i q j / N}.
-__global__ void k_fftg(int n, int nf, const double2* in, double2* out) {
-  int q = blockIdx.x;
-  int f = blockIdx.y;
-  const double2* x = in + (long long)f * n;
-  double sr = 0, si = 0;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    long long qj = ((long long)q * j) % n;
-    double s, c;
-    sincospi(-2.0 * (double)qj / (double)n, &s, &c);
-    double2 v = x[j];
-    sr += v.x * c - v.y * s;
-    si += v.x * s + v.y * c;
+// evaluate nf splines (knots x0, n0) at x1 (n1 points); values outside
+// [min x0, max x0] are 0; optional window multiply and real part.  The block finds the
+// knots' range together.
+__global__ void __launch_bounds__(128) k_spline_eval(int n0, const double* x0, const double2* y0,
+                                                     const double2* coef, int n1, const double* x1,
+                                                     int nf, const double* win, int real_part,
+                                                     double2* out) {
+  __shared__ double rlo[4], rhi[4];
+  double lo = x0[0], hi = lo;
+  for (int i = threadIdx.x; i < n0; i += 128) {
+    const double x = x0[i];
+    lo = fmin(lo, x);
+    hi = fmax(hi, x);
   }
-  __shared__ double rr[128], ri[128];
-  rr[threadIdx.x] = sr;
-  ri[threadIdx.x] = si;
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    rlo[threadIdx.x >> 5] = lo;
+    rhi[threadIdx.x >> 5] = hi;
+  }
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      rr[threadIdx.x] += rr[threadIdx.x + o];
-      ri[threadIdx.x] += ri[threadIdx.x + o];
-    }
-    __syncthreads();
+  lo = fmin(fmin(rlo[0], rlo[1]), fmin(rlo[2], rlo[3]));
+  hi = fmax(fmax(rhi[0], rhi[1]), fmax(rhi[2], rhi[3]));
+  const int j = blockIdx.x * 128 + threadIdx.x;
+  if (j >= n1) return;
+  const double u = x1[j];
+  const bool in = u >= lo && u <= hi;
+  const int i = in ? locate_sorted(x0, n0, u) : 0;
+  const double dx = u - x0[i], w = win ? win[j] : 1.0;
+  for (int f = 0; f < nf; ++f) {
+    double2 v = make_double2(0, 0);
+    if (in) v = spl_eval(y0 + (long long)f * n0, coef + (long long)f * 3 * n0, n0, i, dx);
+    if (win) v = cscale(v, w);
+    if (real_part) v.y = 0.0;
+    out[(long long)f * n1 + j] = v;
   }
-  if (threadIdx.x == 0) out[(long long)f * n + q] = make_double2(-rr[0] / n, -ri[0] / n);
+}
+
+// FFTG (usefulsubs.py:2245-2268) of four real fields: F[q] = -(1/N) sum_j f[j] e^{-2 pi i q
+// j / N}, one warp per q = 0 .. N / 2 with the wire's table tw[m] = e^{-2 pi i m / N}; F[N - q]
+// = conj F[q].
+__global__ void __launch_bounds__(64) k_fftg(int n, const double2* tw, const double2* in,
+                                             double2* out) {
+  const int q = blockIdx.x * 2 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (2 * q > n) return;
+  double sr[4] = {0, 0, 0, 0}, si[4] = {0, 0, 0, 0};
+  int m = (int)(((long long)q * lane) % n);
+  const int step = (int)(((long long)q * 32) % n);
+  for (int j = lane; j < n; j += 32) {
+    const double2 t = tw[m];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const double v = in[(long long)f * n + j].x;
+      sr[f] = fma(v, t.x, sr[f]);
+      si[f] = fma(v, t.y, si[f]);
+    }
+    m += step;
+    if (m >= n) m -= n;
+  }
+#pragma unroll
+  for (int f = 0; f < 4; ++f)
+    for (int o = 16; o > 0; o >>= 1) {
+      sr[f] += __shfl_xor_sync(0xffffffffu, sr[f], o);
+      si[f] += __shfl_xor_sync(0xffffffffu, si[f], o);
+    }
+  if (lane < 4) {
+    double re = sr[0], im = si[0];
+#pragma unroll
+    for (int f = 1; f < 4; ++f)
+      if (lane == f) {
+        re = sr[f];
+        im = si[f];
+      }
+    re = -re / n;
+    im = -im / n;
+    double2* o = out + (long long)lane * n;
+    o[q] = make_double2(re, im);
+    if (q > 0 && 2 * q < n) o[n - q] = make_double2(re, -im);
+  }
 }
 
 // Prop2QW on the context's scratch: the wire-grid part lives in the context's arena;
@@ -577,50 +609,38 @@ int launch_prop2qw(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
 int launch_prop2qw_scratch(SbeCtx* c, int w, const double* RR, int n_rr, const double2* fin,
                            double2* out, double2* coef, double2* tmp, cudaStream_t s) {
   const WireDev& W = c->wires[w];
-  k_spline_coef<<<1, 32, 0, s>>>(n_rr, RR, fin, 4, coef);
-  k_spline_eval<<<dim3((W.nr + 127) / 128, 4), 128, 0, s>>>(n_rr, RR, fin, coef, W.nr,
-                                                           c->r + W.off_r, 4,
-                                                           c->window + W.off_r, 1, tmp);
-  k_fftg<<<dim3(W.nr, 4), 128, 0, s>>>(W.nr, 4, tmp, out);
+  spline_coefs(n_rr, RR, fin, 4, coef, s);
+  k_spline_eval<<<(W.nr + 127) / 128, 128, 0, s>>>(n_rr, RR, fin, coef, W.nr, c->r + W.off_r, 4,
+                                                   c->window + W.off_r, 1, tmp);
+  k_fftg<<<(W.nr / 2 + 2) / 2, 64, 0, s>>>(W.nr, c->twd + W.off_r, tmp, out);
   return cuda_check(cudaGetLastError(), "prop2qw (caller scratch)");
 }
 
 // qwoptics.py:760-805 charge renormalisation (Plasmonics).  mode 0: on the wire
-// grid (re, rh -> |.| scaled to total); mode 1: on the propagation grid.
-__global__ void k_plasmonics(int n, const double* grid, double2* a, double2* b, double* total_io,
-                             int mode) {
+// grid (re, rh -> |.| scaled to total); mode 1: on the propagation grid.  One cluster: the
+// magnitudes are bound by the FP64 pipe of the blocks' SMs.
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
+    k_plasmonics(int n, const double* grid, double2* a, double2* b, double* total_io, int mode) {
   const double dx = grid[1] - grid[0];
-  __shared__ double red[2][256];
-  double sa = 0, sb = 0;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double x = hypot(a[j].x, a[j].y), y = hypot(b[j].x, b[j].y);
+  const int i0 = blockIdx.x * 256 + threadIdx.x, st = kCluster * 256;
+  double A = 0, B = 0;
+  for (int j = i0; j < n; j += st) {
+    const double x = cabs_d(a[j]), y = cabs_d(b[j]);
     a[j] = make_double2(x, 0);
     b[j] = make_double2(y, 0);
-    sa += x;
-    sb += y;
+    A += x;
+    B += y;
   }
-  red[0][threadIdx.x] = sa;
-  red[1][threadIdx.x] = sb;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + o];
-      red[1][threadIdx.x] += red[1][threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  double A = red[0][0], B = red[1][0];
-  double total;
+  double total = mode == 0 ? 0.0 : *total_io;
+  cluster_sum2(A, B);
   if (mode == 0) {
     total = (A * dx + B * dx + kQwSmall) / 2.0;
-    if (threadIdx.x == 0) *total_io = total;
-  } else {
-    total = *total_io;
+    if (i0 == 0) *total_io = total;
   }
-  double fa = total / (A * dx + kQwSmall), fb = total / (B * dx + kQwSmall);
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    a[j] = make_double2(a[j].x * fa, 0);
-    b[j] = make_double2(b[j].x * fb, 0);
+  const double fa = total / (A * dx + kQwSmall), fb = total / (B * dx + kQwSmall);
+  for (int j = i0; j < n; j += st) {
+    a[j].x *= fa;
+    b[j].x *= fb;
   }
 }
 
@@ -634,12 +654,11 @@ int launch_qw2prop(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
   cudaMemcpyAsync(tmp, src, sizeof(double2) * 5 * (size_t)W.nr, cudaMemcpyDeviceToDevice, s);
   const double* rw = c->r + W.off_r;
   if (plasmonics)
-    k_plasmonics<<<1, 256, 0, s>>>(W.nr, rw, tmp + 3 * W.nr, tmp + 4 * W.nr, total, 0);
-  k_spline_coef<<<1, 32, 0, s>>>(W.nr, rw, tmp, 5, coef);
-  k_spline_eval<<<dim3((n_rr + 127) / 128, 5), 128, 0, s>>>(W.nr, rw, tmp, coef, n_rr, RR, 5,
-                                                           nullptr, 0, out);
+    k_plasmonics<<<kCluster, 256, 0, s>>>(W.nr, rw, tmp + 3 * W.nr, tmp + 4 * W.nr, total, 0);
+  spline_coefs(W.nr, rw, tmp, 5, coef, s);
+  k_spline_eval<<<(n_rr + 127) / 128, 128, 0, s>>>(W.nr, rw, tmp, coef, n_rr, RR, 5, nullptr, 0, out);
   if (plasmonics)
-    k_plasmonics<<<1, 256, 0, s>>>(n_rr, RR, out + 3 * (size_t)n_rr, out + 4 * (size_t)n_rr,
+    k_plasmonics<<<kCluster, 256, 0, s>>>(n_rr, RR, out + 3 * (size_t)n_rr, out + 4 * (size_t)n_rr,
                                    total, 1);
   return cuda_check(cudaGetLastError(), "qw2prop");
 }

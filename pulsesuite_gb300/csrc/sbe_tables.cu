@@ -265,6 +265,15 @@ __global__ void k_optics(const WireDev* wires, const double* kr, const double* r
   }
 }
 
+__global__ void k_twiddles(const WireDev* wires, double2* tw) {
+  const WireDev& W = wires[blockIdx.y];
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= W.nr) return;
+  double s, c;
+  sincospi(-2.0 * (double)m / (double)W.nr, &s, &c);
+  tw[W.off_r + m] = make_double2(c, s);
+}
+
 __global__ void k_window_fft(const WireDev* wires, const double* win, double2* wk) {
   const WireDev W = wires[blockIdx.y];
   int q = blockIdx.x;
@@ -306,6 +315,7 @@ int build_tables(SbeCtx* c, cudaStream_t s) {
                                                                           c->maps);
   k_optics<<<dim3((c->nr_max + 127) / 128, std::max(c->nk_max, 1), nw), 128, 0, s>>>(
       c->d_wires, c->kr, c->r, c->window, c->expikr);
+  k_twiddles<<<dim3((c->nr_max + 127) / 128, nw), 128, 0, s>>>(c->d_wires, c->twd);
   k_window_fft<<<dim3(c->nr_max, nw), 128, 0, s>>>(c->d_wires, c->window, c->wk);
   return cuda_check(cudaGetLastError(), "table kernels");
 }
