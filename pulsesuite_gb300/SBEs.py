@@ -219,11 +219,14 @@ class SBESolver:
             for i in (3, 4, 5, 6, 7, 8):
                 self._st[w][i].diagonal().copy_(d)
         self.rr_offset = np.asarray(rr) - r0
-        self._rr_dev = None
         # PdotE bookkeeping (SBEs.py:5924-5975): one history of the last two calls'
         # Re P on both grids, shared by all wires as in the reference
         self._pde = None
         self._fld = [None] * Nw
+        # pinned staging of the grid fields and of the resampled sources, for the last
+        # grid size seen
+        self._hin = None
+        self._busy = False
         if self.OffDiagDph and self.write_info:
             # InitializeDephasing opens (truncates) both files (dephasing.py:537-539)
             os.makedirs("dataQW/Wire/info", exist_ok=True)
@@ -269,24 +272,24 @@ class SBESolver:
             self.xxx += 1
             self.jjj += 1
             self.t += dt
-        mag = np.max(np.sqrt(np.abs(Exx) ** 2 + np.abs(Eyy) ** 2 + np.abs(Ezz) ** 2))
-        if self.wireoff and mag < 1e-3 * self.Emax0:
-            return
+        if self.wireoff:
+            mag = np.max(np.sqrt(np.abs(Exx) ** 2 + np.abs(Eyy) ** 2 + np.abs(Ezz) ** 2))
+            if mag < 1e-3 * self.Emax0:
+                return
         self.wireoff = False
         DoQWP[0] = self.Optics
         DoQWDl[0] = self.LF
-        RR = torch.as_tensor(np.asarray(rr, dtype=np.float64), device="cuda")
-        f4 = torch.as_tensor(np.stack([np.asarray(a, dtype=complex) for a in (Exx, Eyy, Ezz, Vrr)]),
-                             dtype=CDTYPE, device="cuda").contiguous()
+        RR, f4 = self._stage(w if self.batch else 1, rr, (Exx, Eyy, Ezz, Vrr))
         if self.batch:
-            self._batched(w, RR, f4, dt, (Pxx, Pyy, Pzz, Rho))
+            self._batched(w, RR, f4, dt, (Pxx, Pyy, Pzz, Rho), (Exx, Eyy, Ezz))
             return
         ctx = self.contexts[w - 1]
         Ek = ctx.prop2qw(0, RR, f4)                       # (4, Nr): Ex, Ey, Ez, Vr in wire k space
         src = torch.empty((5, self.Nr), dtype=CDTYPE, device="cuda")
-        Ek3 = Ek[:3].contiguous()
+        Ek3 = Ek[:3]                                      # the first three rows, contiguous
         ctx.leapfrog_step(self._st[w - 1], Ek3, dt, src)
-        out = ctx.qw2prop(0, RR, src, self.LF).cpu().numpy()
+        ctx.qw2prop(0, RR, src, self.LF, self._dout[0])
+        out = self._fetch(1)[0]
         if self.write_info:
             self._write_info(ctx, w, dt, src, Ek3)
             self._write_maxoffdiag(ctx, 0)
@@ -302,24 +305,53 @@ class SBESolver:
             Pzz[:] = 0.0
             Rho[:] = 0.0
 
-    def _batched(self, w, RR, f4, dt, outs):
+    def _stage(self, w, rr, fields):
+        """Copy a wire's grid and its four fields into pinned host memory and from there, in
+        one transfer on the current stream, to the device: (RR, f4).  The step that reads
+        them is waited for (_fetch) before the buffers are filled again."""
+        n, nslot = len(rr), self.Nw if self.batch else 1
+        if self._hin is None or self._hin.shape[2] != n:
+            self._hin = torch.empty((nslot, 5, n), dtype=CDTYPE).pin_memory()
+            self._din = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
+            self._dout = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
+            self._hout = torch.empty((nslot, 5, n), dtype=CDTYPE).pin_memory()
+            self._hin_np, self._hout_np = self._hin.numpy(), self._hout.numpy()
+        elif self._busy:
+            torch.cuda.current_stream().synchronize()     # an aborted step's transfers
+        h = self._hin_np[w - 1]
+        for i, f in enumerate(fields):
+            h[i] = f
+        h[4].view(np.float64)[:n] = rr
+        d = self._din[w - 1]
+        d.copy_(self._hin[w - 1], non_blocking=True)
+        self._busy = not self.batch or w == self.Nw
+        return torch.view_as_real(d[4]).reshape(-1)[:n], d[:4]
+
+    def _fetch(self, nslot):
+        """The first nslot blocks of the resampled sources on the host (waits for them)."""
+        self._hout[:nslot].copy_(self._dout[:nslot], non_blocking=True)
+        torch.cuda.current_stream().synchronize()
+        self._busy = False
+        return self._hout_np
+
+    def _batched(self, w, RR, f4, dt, outs, E3):
         """Stage wire w's field; on the last wire step them all and fill every wire's
         outputs (Pxx, Pyy, Pzz, Rho = RhoH - RhoE, SBEs.py:5917)."""
         ctx = self.contexts[0]
         Ek = ctx.prop2qw(w - 1, RR, f4)
         ctx.rvec(self._ek, w - 1, 3).copy_(Ek[:3])
         self._outs[w - 1] = outs
-        self._fld[w - 1] = (f4[0].real.cpu().numpy(), f4[1].real.cpu().numpy(),
-                            f4[2].real.cpu().numpy(), RR.cpu().numpy())
+        if self.write_info:
+            self._fld[w - 1] = tuple(np.array(np.real(f)) for f in E3) + (RR.cpu().numpy(),)
         if w != self.Nw:
             return
         ctx.leapfrog_step(self._lev, self._ek, dt, self._src)
-        for wi in range(self.Nw):
-            o = self._outs[wi]
-            if o is None:
-                continue
-            src = ctx.rvec(self._src, wi, 5).contiguous()
-            out = ctx.qw2prop(wi, RR, src, self.LF).cpu().numpy()
+        live = [wi for wi in range(self.Nw) if self._outs[wi] is not None]
+        for wi in live:
+            ctx.qw2prop(wi, RR, ctx.rvec(self._src, wi, 5), self.LF, self._dout[wi])
+        host = self._fetch(self.Nw)
+        for wi in live:
+            o, out = self._outs[wi], host[wi]
             if self.write_info:
                 self._write_info(ctx, wi + 1, dt, None, None)
                 self._write_maxoffdiag(ctx, wi)

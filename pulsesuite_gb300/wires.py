@@ -281,16 +281,18 @@ class WireContext:
                                         _lib.stream_handle()), "sbe_sources")
         return out
 
-    def prop2qw(self, w, RR, fields4):
+    def prop2qw(self, w, RR, fields4, out=None):
         nr = 2 * self.nk[w] + 2
-        out = torch.empty((4, nr), dtype=CDTYPE, device=self.device)
+        if out is None:
+            out = torch.empty((4, nr), dtype=CDTYPE, device=self.device)
         _lib.check(self.lib.sbe_prop2qw(self.handle, w, _lib.ptr(RR), RR.numel(),
                                         _lib.ptr(fields4), _lib.ptr(out), _lib.stream_handle()),
                    "sbe_prop2qw")
         return out
 
-    def qw2prop(self, w, RR, src5, plasmonics):
-        out = torch.empty((5, RR.numel()), dtype=CDTYPE, device=self.device)
+    def qw2prop(self, w, RR, src5, plasmonics, out=None):
+        if out is None:
+            out = torch.empty((5, RR.numel()), dtype=CDTYPE, device=self.device)
         _lib.check(self.lib.sbe_qw2prop(self.handle, w, _lib.ptr(RR), RR.numel(), _lib.ptr(src5),
                                         _lib.ptr(out), int(bool(plasmonics)),
                                         _lib.stream_handle()), "sbe_qw2prop")
