@@ -350,12 +350,22 @@ static const TermDef kTerms[3][4] = {
     // D Hhh^T - Hhh^T D + conj(P) Heh - Heh^H P^T
     {{F_D, F_HH, 0, 0, 0}, {F_HHT, F_DT, 0, 0, 1}, {F_P, F_EHT, 1, 0, 0}, {F_EHT, F_P, 1, 0, 1}}};
 
-// Cuts of a product's K sequence (2 nkb K blocks): enough output tiles for two waves of
-// 152 CTAs, at least two K blocks each.
+// Cuts of a product's K sequence (2 nkb K blocks): the fewest K-block times over the waves of
+// 152 CTAs, a tile's fixed cost being about 1.2 of them and a further part's sums and traffic
+// 0.15 (1 x 512, 768 tiles: 340 us uncut, 322 in two; 8 x 256, 1536 tiles: 326 uncut, 331).
 static int product_parts(long long units, int nkb) {
   const int n = 2 * nkb;
-  int p = (int)std::min<long long>((304 + units - 1) / std::max<long long>(units, 1), n / 2);
-  return std::max(p, 1);
+  int best = 1;
+  double least = 1e300;
+  for (int p = 1; p <= std::min(n / 2, 8); ++p) {
+    const double waves = (double)((units * p + 151) / 152);
+    const double cost = waves * ((n + p - 1) / p + 1.2) + 0.15 * (p - 1);
+    if (cost < least) {
+      least = cost;
+      best = p;
+    }
+  }
+  return best;
 }
 
 // forms planes of Nk x Nk matrices: slab of (form, plane, batch entry)

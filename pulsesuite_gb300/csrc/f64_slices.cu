@@ -92,10 +92,12 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
 // ---------------------------------------------------------------------------
 // the product kernel
 
-constexpr int A_SLOT = BM * BK * 2;        // 8 KB: one digit plane of an A tile
+constexpr int A_SLICE = BM * BK * 2;       // 8 KB: one digit plane of an A tile
+constexpr int A_GROUP = 4;                 // planes of a ring slot
+constexpr int A_SLOT = A_GROUP * A_SLICE;  // 32 KB
 constexpr int B_SLICE = BN * BK * 2;       // 4 KB
 constexpr int B_SLOT = NS * B_SLICE;       // 32 KB: all planes of a B tile
-constexpr int NA = 16, NB = 3;             // ring slots
+constexpr int NA = 4, NB = 3;              // ring slots
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int SMEM = 1024 + NA * A_SLOT + NB * B_SLOT + 512;
@@ -143,19 +145,6 @@ __device__ __forceinline__ Unit unit_of(const Launch& L, int u) {
   return t;
 }
 
-__device__ __forceinline__ void tmem_ld32_nw(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-
 // v 2^e rounded once to FP64, on the integer pipe while the result is normal
 __device__ __forceinline__ double ll_scaled(long long v, int e) {
   if (v == 0) return 0.0;
@@ -169,37 +158,71 @@ __device__ __forceinline__ double ll_scaled(long long v, int e) {
   return __longlong_as_double((long long)(sg | (((unsigned long long)(ef - 1) << 52) + mant)));
 }
 
-__device__ __forceinline__ int f2i(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }
+__device__ __forceinline__ void st_global_v4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
+               : "memory");
+}
 
-// One accumulator t of a thread's 32 columns into the running sums, in units of 2^6 of
-// sum_t acc_t 2^(8 (7 - t)), modulo 2^64 (the whole sum stays below 2^62).
-template <int T>
-__device__ __forceinline__ void add_acc(long long* run, const uint32_t* r) {
+// The accumulators of 16 of a thread's 32 columns into the running sums, in units of 2^6 of
+// sum_t acc_t 2^(8 (7 - t)), modulo 2^64 (the whole sum stays below 2^62).  The conversion
+// float -> int runs at an eighth of the FP32 rate, so every other accumulator takes a cheaper
+// way: adding 1.5 2^25 leaves rint(a / 4) in the mantissa, and the remainder (at most 2, exact)
+// goes to the next accumulator as 256 times itself, which keeps that below 2^24.  The bits are
+// added with their offset; kBias per accumulation is taken off at the end.
+constexpr float kMagic = 50331648.f;
+constexpr uint32_t kMagicBits = 0x4C400000u;
+__host__ __device__ constexpr int sum_shift(int t) { return 50 - 8 * t; }
+constexpr unsigned long long kBias = ((unsigned long long)kMagicBits << (sum_shift(0) + 2)) +
+                                     ((unsigned long long)kMagicBits << (sum_shift(2) + 2)) +
+                                     ((unsigned long long)kMagicBits << (sum_shift(4) + 2));
+
+template <int T>   // a: accumulator T, next: T + 1
+__device__ __forceinline__ void add_magic(unsigned long long* run, const uint32_t* a, uint32_t* next) {
+  constexpr int S = sum_shift(T) + 2;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    if (T < 3)   // the shift exceeds 32: the high word alone changes
-      run[j] = (long long)((unsigned long long)run[j] +
-                           ((unsigned long long)((unsigned)f2i(r[j]) << (18 - 8 * T)) << 32));
+  for (int j = 0; j < 16; ++j) {
+    const float v = __uint_as_float(a[j]), r = __fadd_rn(v, kMagic);
+    const float e = __fsub_rn(v, __fsub_rn(r, kMagic));
+    next[j] = __float_as_uint(__fmaf_rn(e, 256.f, __uint_as_float(next[j])));
+    if constexpr (S >= 32)   // the high word alone changes
+      run[j] += (unsigned long long)(__float_as_uint(r) << (S - 32)) << 32;
     else
-      run[j] += (long long)f2i(r[j]) * (1ll << (50 - 8 * T));
+      run[j] += (unsigned long long)__float_as_uint(r) * (1u << S);
+  }
+}
+template <int T>
+__device__ __forceinline__ void add_acc(unsigned long long* run, const uint32_t* a) {
+  constexpr int S = sum_shift(T);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const int v = __float2int_rn(__uint_as_float(a[j]));
+    if constexpr (S >= 32)
+      run[j] += (unsigned long long)((unsigned)v << (S - 32)) << 32;
+    else
+      run[j] += (unsigned long long)((long long)v * (1 << S));
   }
 }
 // accumulators 6 and 7 (rounded to two units at most)
-__device__ __forceinline__ void add_acc67(long long* run, const uint32_t* r6, const uint32_t* r7) {
+__device__ __forceinline__ void add_acc67(unsigned long long* run, const uint32_t* a6,
+                                          const uint32_t* a7) {
 #pragma unroll
-  for (int j = 0; j < 32; ++j)
-    run[j] += (long long)__float2int_rn(
-        fmaf(__uint_as_float(r7[j]), 1.f / 64.f, __uint_as_float(r6[j]) * 4.f));
+  for (int j = 0; j < 16; ++j)
+    run[j] += (unsigned long long)(long long)__float2int_rn(
+        fmaf(__uint_as_float(a7[j]), 1.f / 64.f, __uint_as_float(a6[j]) * 4.f));
 }
 
-// Persistent, one CTA per SM: warp 0 streams digit planes (bulk copies; A planes through
-// a ring of single planes, B tiles through three slots), warp 1 issues the MMAs, warps 2-9
-// drain the accumulators.  A tile is 128 x 64: its eight accumulators fill the 512 TMEM
-// columns at 64 t, so the plane A_i against the adjacent planes B_0 .. B_{7 - i} (rows
-// adjacent in shared memory) is one or two MMAs of N up to 256 whose result lands on the
-// accumulators i .. 7: 36 plane products per K block in 12 MMAs per 16 k.  Per K block 96 KB
-// of planes feed 2304 clocks of MMA.  The accumulators are drained every 128 k
-// (exactness) with the MMAs waiting.
+// Persistent, one CTA per SM: warp 0 streams digit planes (bulk copies; A planes in groups of
+// four, B tiles whole), warp 1 issues the MMAs, warps 2-9 drain the accumulators.  A tile is
+// 128 x 64: its eight accumulators fill the 512 TMEM columns at 64 t, so the plane A_i against
+// adjacent planes of B (rows adjacent in shared memory) is one MMA of N up to 256 onto adjacent
+// accumulators: 36 plane products per K block in 12 MMAs per 16 k.  The accumulators are
+// drained every 128 k (exactness).  They form two windows, t >= 4 (26 of the 36 products) and
+// t < 4, each with its own barriers: the epilogue drains the upper window while the last MMAs of
+// the lower run, and the lower while the next upper ones do.
+// 1 wire x Nk = 512, the twelve commutator products (464 GFLOP of MMA work): 617 us with a
+// barrier per plane (the issuing thread's waits), 448 with grouped ones, 417 with the windows and
+// fewer conversions, 340 with the drain in 16-column steps (no spills) and 32-byte stores, of
+// which the MMAs alone take 304.
 __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__ Launch L) {
   using namespace tc;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -211,9 +234,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
   uint64_t* emptyA = fullA + NA;
   uint64_t* fullB = emptyA + NA;
   uint64_t* emptyB = fullB + NB;
-  uint64_t* tfull = emptyB + NB;
-  uint64_t* tempty = tfull + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
+  uint64_t* tfull = emptyB + NB;    // per window: 0 lower (t < 4), 1 upper
+  uint64_t* tempty = tfull + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
   const int nunits = L.base[L.njobs];
@@ -227,8 +250,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
       mbar_init(&fullB[i], 1);
       mbar_init(&emptyB[i], 1);
     }
-    mbar_init(tfull, 1);
-    mbar_init(tempty, EPI_WARPS);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], EPI_WARPS);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -271,13 +296,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
         }
         const __half* ga = d.A + (long long)ca * NS * d.a_plane + (long long)t.b * d.a_batch +
                            ((long long)kb * d.a_pad + t.m0) * BK;
-        for (int i = 0; i < NS; ++i) {
+        for (int i = 0; i < NS; i += A_GROUP) {
           if (!mbar_wait(&emptyA[sa], pa ^ 1u, err, abort_flag)) {
             ok = false;
             break;
           }
           mbar_expect_tx(&fullA[sa], A_SLOT);
-          bulk_load(sA + sa * A_SLOT, ga + i * d.a_plane, A_SLOT, &fullA[sa]);
+          for (int j = 0; j < A_GROUP; ++j)
+            bulk_load(sA + sa * A_SLOT + j * A_SLICE, ga + (i + j) * d.a_plane, A_SLICE,
+                      &fullA[sa]);
           ++na;
           if (++sa == NA) {
             sa = 0;
@@ -308,55 +335,62 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
       const int s1 = t.comp ? (d.conj_a ? -1 : 1) : -(d.conj_a ? -1 : 1) * (d.conj_b ? -1 : 1);
       for (int c0 = t.q0; ok && c0 < t.q1; c0 += CHUNK) {
         const int c1 = min(c0 + CHUNK, t.q1);
-        if (!mbar_wait(tempty, pt, err, abort_flag)) {
-          ok = false;
-          break;
-        }
-        pt ^= 1u;
-        tc_fence_after();
-        for (int q = c0; ok && q < c1; ++q) {
+        for (int q = c0; q < c1; ++q) {
           const int sg = (q >= t.nkb ? s1 : s0) * (d.neg ? -1 : 1);
-          const uint32_t nega = sg < 0 ? (1u << 13) : 0u;
-          if (!mbar_wait(&fullB[sb], pb, err, abort_flag)) {
+          const uint32_t id = idesc_f16(BM, 0, sg < 0 ? 1 : 0);
+          const uint32_t first = q == c0 ? 0u : 1u;
+          const int sa1 = sa + 1;   // NA is even: the groups of a K block are adjacent slots
+          if (!mbar_wait(&fullB[sb], pb, err, abort_flag) ||
+              !mbar_wait(&fullA[sa], pa, err, abort_flag) ||
+              !mbar_wait(&fullA[sa1], pa, err, abort_flag) ||
+              (q == c0 && !mbar_wait(&tempty[1], pt, err, abort_flag))) {
             ok = false;
             break;
           }
+          tc_fence_after();
+          const uint64_t da = sw64_desc(smem_u32(sA + sa * A_SLOT));
           const uint64_t db = sw64_desc(smem_u32(sB + sb * B_SLOT));
+          // upper window: A_i with B_{max(0, 4 - i)} .. B_{7 - i} onto accumulators max(4, i) .. 7
+#pragma unroll
           for (int i = 0; i < NS; ++i) {
-            if (!mbar_wait(&fullA[sa], pa, err, abort_flag)) {
+            const int j0 = i < 4 ? 4 - i : 0, t0 = i < 4 ? 4 : i, n = 8 - t0;
+#pragma unroll
+            for (int k16 = 0; k16 < 2; ++k16)
+              umma_f16(tmem + t0 * BN, da + (uint64_t)(i * (A_SLICE >> 4) + 2 * k16),
+                       db + (uint64_t)(j0 * (B_SLICE >> 4) + 2 * k16),
+                       id + ((uint32_t)(n * BN >> 3) << 17), (i == 0 && k16 == 0) ? first : 1u);
+          }
+          umma_commit(&emptyA[sa1]);
+          if (q == c1 - 1) umma_commit(&tfull[1]);
+          if (q == c0) {
+            if (!mbar_wait(&tempty[0], pt, err, abort_flag)) {
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint64_t da = sw64_desc(smem_u32(sA + sa * A_SLOT));
-            const int nblk = NS - i;                      // accumulators i .. 7
-            const int n1 = nblk > 4 ? (nblk + 1) / 2 : nblk, n2 = nblk - n1;
-            const uint32_t id1 = idesc_f16(BM, BN, 0) - ((uint32_t)(BN >> 3) << 17) +
-                                 ((uint32_t)(n1 * BN >> 3) << 17) + nega;
-            const uint32_t id2 = idesc_f16(BM, BN, 0) - ((uint32_t)(BN >> 3) << 17) +
-                                 ((uint32_t)(n2 * BN >> 3) << 17) + nega;
-#pragma unroll
-            for (int k16 = 0; k16 < 2; ++k16) {
-              const uint32_t acc = (q == c0 && i == 0 && k16 == 0) ? 0u : 1u;
-              const uint64_t ko = 2u * k16;
-              umma_f16(tmem + i * BN, da + ko, db + ko, id1, acc);
-              if (n2 > 0)
-                umma_f16(tmem + (i + n1) * BN, da + ko,
-                         db + ko + (uint64_t)(n1 * (B_SLICE >> 4)), id2, acc);
-            }
-            umma_commit(&emptyA[sa]);
-            if (++sa == NA) {
-              sa = 0;
-              pa ^= 1u;
-            }
           }
+          // lower window: A_i with B_0 .. B_{3 - i} onto accumulators i .. 3
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int k16 = 0; k16 < 2; ++k16)
+              umma_f16(tmem + i * BN, da + (uint64_t)(i * (A_SLICE >> 4) + 2 * k16),
+                       db + 2u * k16, id + ((uint32_t)((4 - i) * BN >> 3) << 17),
+                       (i == 0 && k16 == 0) ? first : 1u);
+          umma_commit(&emptyA[sa]);
           umma_commit(&emptyB[sb]);
+          sa += 2;
+          if (sa == NA) {
+            sa = 0;
+            pa ^= 1u;
+          }
           if (++sb == NB) {
             sb = 0;
             pb ^= 1u;
           }
         }
-        if (ok) umma_commit(tfull);
+        pt ^= 1u;
+        if (ok) umma_commit(&tfull[0]);
       }
     }
   } else if (warp >= 2) {
@@ -369,43 +403,59 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
       const Unit t = unit_of(L, u);
       if (t.dead) continue;
       const Job& d = L.job[t.job];
-      long long run[32];
+      unsigned long long run[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) run[j] = 0;
+      unsigned long long bias = 0;
       for (int c0 = t.q0; c0 < t.q1; c0 += CHUNK) {
-        if (!mbar_wait(tfull, pt, err, abort_flag)) {
+        uint32_t a[16], b[16];
+        if (!mbar_wait(&tfull[1], pt, err, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          tmem_ld16_nw(ta + 4 * BN + 16 * h, a);
+          tmem_ld16_nw(ta + 5 * BN + 16 * h, b);
+          tmem_ld_wait();
+          add_magic<4>(run + 16 * h, a, b);
+          add_acc<5>(run + 16 * h, b);
+          tmem_ld16_nw(ta + 6 * BN + 16 * h, a);
+          tmem_ld16_nw(ta + 7 * BN + 16 * h, b);
+          tmem_ld_wait();
+          if (h == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[1]);
+          }
+          add_acc67(run + 16 * h, a, b);
+        }
+        if (!mbar_wait(&tfull[0], pt, err, abort_flag)) {
           ok = false;
           break;
         }
         pt ^= 1u;
         tc_fence_after();
-        uint32_t a[32], b[32];
-        tmem_ld32_nw(ta, a);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 1 * BN, b);
-        add_acc<0>(run, a);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 2 * BN, a);
-        add_acc<1>(run, b);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 3 * BN, b);
-        add_acc<2>(run, a);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 4 * BN, a);
-        add_acc<3>(run, b);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 5 * BN, b);
-        add_acc<4>(run, a);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 6 * BN, a);
-        add_acc<5>(run, b);
-        tmem_ld_wait();
-        tmem_ld32_nw(ta + 7 * BN, b);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty);
-        add_acc67(run, a, b);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          tmem_ld16_nw(ta + 16 * h, a);
+          tmem_ld16_nw(ta + 1 * BN + 16 * h, b);
+          tmem_ld_wait();
+          add_magic<0>(run + 16 * h, a, b);
+          add_acc<1>(run + 16 * h, b);
+          tmem_ld16_nw(ta + 2 * BN + 16 * h, a);
+          tmem_ld16_nw(ta + 3 * BN + 16 * h, b);
+          tmem_ld_wait();
+          if (h == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[0]);
+          }
+          add_magic<2>(run + 16 * h, a, b);
+          add_acc<3>(run + 16 * h, b);
+        }
+        bias += kBias;
       }
       const int m = t.m0 + 32 * quarter + lane;
       if (!ok || m >= d.M) continue;
@@ -424,18 +474,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
             const int e = eb[n];
             o[2 * k2 + (n & 1)] = (ea == kBadExp || e == kBadExp)
                                       ? __longlong_as_double(0x7FF8000000000000ll)
-                                      : ll_scaled(run[j], ea + e - 62);
+                                      : ll_scaled((long long)(run[j] - bias), ea + e - 62);
           }
         }
       } else {
         o += (long long)m * d.ldo + n0;
+        auto value = [&](int j) {
+          const int e = eb[n0 + j];
+          return (ea == kBadExp || e == kBadExp) ? __longlong_as_double(0x7FF8000000000000ll)
+                                                 : ll_scaled((long long)(run[j] - bias), ea + e - 62);
+        };
+        // a thread's 32 columns are 256 contiguous bytes: 32-byte stores where rows allow
+        if ((d.ldo & 3) == 0 && n0 + 32 <= d.N) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (n0 + j < d.N) {
-            const int e = eb[n0 + j];
-            o[j] = (ea == kBadExp || e == kBadExp) ? __longlong_as_double(0x7FF8000000000000ll)
-                                                   : ll_scaled(run[j], ea + e - 62);
-          }
+          for (int j = 0; j < 32; j += 4)
+            st_global_v4(o + j, value(j), value(j + 1), value(j + 2), value(j + 3));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (n0 + j < d.N) o[j] = value(j);
         }
       }
     }
