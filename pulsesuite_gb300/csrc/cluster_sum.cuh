@@ -16,24 +16,24 @@ __device__ __forceinline__ double cabs_d(double2 v) {
   return hypot(v.x, v.y);
 }
 
-// sums of a and b over the block, returned to every thread
-__device__ __forceinline__ void block_sum2(double& a, double& b) {
-  __shared__ double red[2][8];
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    b += __shfl_down_sync(0xffffffffu, b, o);
-  }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = a;
-    red[1][threadIdx.x >> 5] = b;
-  }
-  __syncthreads();
-  a = b = 0.0;
+// sums of the N values over the block (256 threads), returned to every thread; a dependent
+// FP64 addition takes about 130 clocks, so the values go together
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N]) {
+  __shared__ double red[N][8];
 #pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    a += red[0][w];
-    b += red[1][w];
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int i = 0; i < N; ++i) red[i][threadIdx.x >> 5] = v[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const double* r = red[i];
+    v[i] = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
   }
 }
 
@@ -43,18 +43,25 @@ __device__ __forceinline__ void cluster_sum2(double& a, double& b) {
   namespace cg = cooperative_groups;
   __shared__ double part[2];
   cg::cluster_group cl = cg::this_cluster();
-  block_sum2(a, b);
+  double v[2] = {a, b};
+  block_sums(v);
   if (threadIdx.x == 0) {
-    part[0] = a;
-    part[1] = b;
+    part[0] = v[0];
+    part[1] = v[1];
   }
   cl.sync();
-  a = b = 0.0;
+  double p[2][kCluster];
+#pragma unroll
   for (int r = 0; r < kCluster; ++r) {
     const double* q = cl.map_shared_rank(part, r);
-    a += q[0];
-    b += q[1];
+    p[0][r] = q[0];
+    p[1][r] = q[1];
   }
+  auto sum = [](const double* x) {
+    return ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+  };
+  a = sum(p[0]);
+  b = sum(p[1]);
   cl.sync();
 }
 

@@ -300,9 +300,15 @@ __global__ void __launch_bounds__(256) k_f64_finish(const __grid_constant__ Fini
     if (m >= nk || n >= nk) continue;
     const long long o = (long long)m * nk + n;
     double sx = 0.0, sy = 0.0;
-    for (int s = 0; s < a.nsum; ++s) {
-      sx += part[2 * s * cs + o];
-      sy += part[(2 * s + 1) * cs + o];
+    for (int s = 0; s < a.nsum; s += 4) {   // a multiple of four: eight loads in flight
+      double x[4], y[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        x[u] = part[2 * (s + u) * cs + o];
+        y[u] = part[(2 * (s + u) + 1) * cs + o];
+      }
+      sx += (x[0] + x[1]) + (x[2] + x[3]);
+      sy += (y[0] + y[1]) + (y[2] + y[3]);
     }
     double2 v = make_double2(sy * ih, -sx * ih);
     if (which == 0) {
@@ -352,14 +358,14 @@ static const TermDef kTerms[3][4] = {
 
 // Cuts of a product's K sequence (2 nkb K blocks): the fewest K-block times over the waves of
 // 152 CTAs, a tile's fixed cost being about 1.2 of them and a further part's sums and traffic
-// 0.15 (1 x 512, 768 tiles: 340 us uncut, 322 in two; 8 x 256, 1536 tiles: 326 uncut, 331).
-static int product_parts(long long units, int nkb) {
+// 0.15 (sources, whose reduction is as large as the products' output: 2) (1 x 512, 768 tiles: 340 us uncut, 322 in two; 8 x 256, 1536 tiles: 326 uncut, 331).
+static int product_parts(long long units, int nkb, double part_cost = 0.15) {
   const int n = 2 * nkb;
   int best = 1;
   double least = 1e300;
   for (int p = 1; p <= std::min(n / 2, 8); ++p) {
     const double waves = (double)((units * p + 151) / 152);
-    const double cost = waves * ((n + p - 1) / p + 1.2) + 0.15 * (p - 1);
+    const double cost = waves * ((n + p - 1) / p + 1.2) + part_cost * (p - 1);
     if (cost < least) {
       least = cost;
       best = p;
@@ -498,7 +504,7 @@ bool f64_prepare(SbeCtx* c, cudaStream_t s) {
     m.group = 1;
     auto sizes = [&](int g, size_t* out) {
       const int parts = product_parts(24 * tiles * g, k_blocks(nk));
-      const int sparts = product_parts(6 * stiles * g, k_blocks(nk));
+      const int sparts = product_parts(6 * stiles * g, k_blocks(nk), 2.0);
       out[0] = sizeof(__half) * F_N * 2 * NS * g * m.sl_m;                // forms
       out[1] = sizeof(__half) * 3 * NS * g * m.sl_s;                      // sheared
       // partial products, or the source products
@@ -527,7 +533,7 @@ bool f64_prepare(SbeCtx* c, cudaStream_t s) {
     }
     const size_t total = sizes(m.group, sz);
     m.parts = product_parts(24 * tiles * m.group, k_blocks(nk));
-    m.sparts = product_parts(6 * stiles * m.group, k_blocks(nk));
+    m.sparts = product_parts(6 * stiles * m.group, k_blocks(nk), 2.0);
     std::vector<WireDev> hw;
     for (int k = i; k < j; ++k) hw.push_back(c->wires[c->order[k]]);
     ok = cudaMalloc(&m.block, total) == cudaSuccess &&
@@ -688,20 +694,21 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
 // sources
 
 // Column sums of QWPolarization3 / QWRho5 (k_src_reduce) from the planar products
-// G[n][part][re, im][wire][k][r], n = P E, C E, conj(D) E.  Block (32 r) x (16 k groups): thread (x, y) sums
-// k = y, y + 16, ..., the partial sums are added in group order.
+// G[n][part][re, im][wire][k][r], n = P E, C E, conj(D) E.  Block (16 r) x (32 k groups): thread
+// (x, y) sums k = y, y + 32, ..., the partial sums are added in group order.
 __global__ void __launch_bounds__(512) k_f64_src_reduce(const WireDev* wires, int nk, int nr, int nw,
-                                                        int parts, const double2* E, const double* G,
-                                                        const double* win, double2* src) {
-  __shared__ double red[6][16][33];
-  const int b = blockIdx.y, tx = threadIdx.x, ty = threadIdx.y, r = blockIdx.x * 32 + tx;
+                                                        int parts, const double2* E,
+                                                        const double* G, const double* win,
+                                                        double2* src) {
+  __shared__ double red[6][32][17];
+  const int b = blockIdx.y, tx = threadIdx.x, ty = threadIdx.y, r = blockIdx.x * 16 + tx;
   const long long per = (long long)nk * nr, cs = (long long)nw * per;
   double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (r < nr) {
     const double2* e0 = E + (long long)b * per + r;
     const double* g0 = G + (long long)b * per + r;
-#pragma unroll 2
-    for (int k = ty; k < nk; k += 16) {
+#pragma unroll 4
+    for (int k = ty; k < nk; k += 32) {
       const long long o = (long long)k * nr;
       const double2 e = e0[o];   // conj taken below
       double g[6];
@@ -724,10 +731,10 @@ __global__ void __launch_bounds__(512) k_f64_src_reduce(const WireDev* wires, in
   for (int i = 0; i < 6; ++i) red[i][ty][tx] = s[i];
   __syncthreads();
   if (ty >= 6 || r >= nr) return;
-  // row ty sums quantity ty; the outputs below take them from shared memory
+  // row ty sums quantity ty
   double t = 0.0;
 #pragma unroll
-  for (int g = 0; g < 16; ++g) t += red[ty][g][tx];
+  for (int g = 0; g < 32; ++g) t += red[ty][g][tx];
   const WireDev& W = wires[b];
   const bool optics = (W.flags & SBE_F_OPTICS) != 0;
   const double w = win[(long long)b * nr + r], pf = 2 * W.ehint / W.area / W.L;
@@ -785,7 +792,7 @@ int f64_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D,
       launch_f64_slice(a, 3, s);
       const int rc = launch_f64_gemm(jobs, 3, s);
       if (rc) return rc;
-      k_f64_src_reduce<<<dim3((nr + 31) / 32, g), dim3(32, 16), 0, s>>>(
+      k_f64_src_reduce<<<dim3((nr + 15) / 16, g), dim3(16, 32), 0, s>>>(
           m.dw + w0, nk, nr, g, m.sparts, c->expikr + ko, m.part, c->window + ro, src + 5 * ro);
     }
   return cuda_check(cudaGetLastError(), "f64 sources");

@@ -16,10 +16,10 @@ __device__ int g_err;   // a bounded wait gave up
 
 // Block: 8 rows of one form of one matrix; warps walk the K blocks, a lane takes 8
 // consecutive k of one row (lane = 4 row + chunk), so a warp stores 512 contiguous bytes
-// per plane and the transposed read covers 128-byte segments.  Up to 8 K blocks (Nk <=
-// 256) each value is read once and kept in registers between the row maximum, the norm and
-// the digits; larger rows are read again (from L2).  HBM bound: 16 B read and 32 B written
-// per element.
+// per plane and the transposed read covers 128-byte segments.  KB K blocks of a warp stay in
+// registers between the row maximum, the norm and the digits (Nk up to 256 KB); longer rows
+// are read again (from L2).  HBM bound: 16 B read and 32 B written per element.
+template <int KB>
 __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ SliceArgs a) {
   const Form& f = a.f[blockIdx.y];
   const int kdim = a.kdim, ld = a.ld, b = blockIdx.z;
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
   const int nkb = k_blocks(kdim), rows_pad = pad_rows(a.rows);
   const double2* X = f.src + (long long)b * a.src_batch;
   const double2* Y = f.add ? f.add + (long long)b * a.src_batch : nullptr;
-  const bool rok = r < a.rows;
+  const bool rok = r < a.rows, held = nkb <= 8 * KB;
   auto load = [&](int kb, double2* v) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -42,12 +42,22 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
   };
   __shared__ unsigned long long red[8][8];
   __shared__ float reds[8][8];
-  double2 v[8];
+  double2 v[KB][8];
   unsigned long long m = 0;
-  for (int kb = warp; kb < nkb; kb += 8) {
-    load(kb, v);
+  auto maximum = [&](const double2* x) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = max(m, max(absbits(v[i].x), absbits(v[i].y)));
+    for (int i = 0; i < 8; ++i) m = max(m, max(absbits(x[i].x), absbits(x[i].y)));
+  };
+  if (held) {
+#pragma unroll
+    for (int u = 0; u < KB; ++u) load(warp + 8 * u, v[u]);   // zeros past the last K block
+#pragma unroll
+    for (int u = 0; u < KB; ++u) maximum(v[u]);
+  } else {
+    for (int kb = warp; kb < nkb; kb += 8) {
+      load(kb, v[0]);
+      maximum(v[0]);
+    }
   }
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
@@ -58,11 +68,19 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
   for (int w = 0; w < 8; ++w) m = max(m, red[w][lane >> 2]);
   const int Em = max_exp(m);
   float sq = 0.f;
-  for (int kb = warp; kb < nkb; kb += 8) {
-    if (nkb > 8) load(kb, v);
-    if (Em != kBadExp) {
+  auto squares = [&](const double2* x) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sq += scaled_sq(v[i].x, Em) + scaled_sq(v[i].y, Em);
+    for (int i = 0; i < 8; ++i) sq += scaled_sq(x[i].x, Em) + scaled_sq(x[i].y, Em);
+  };
+  if (Em != kBadExp) {
+    if (held) {
+#pragma unroll
+      for (int u = 0; u < KB; ++u) squares(v[u]);
+    } else {
+      for (int kb = warp; kb < nkb; kb += 8) {
+        load(kb, v[0]);
+        squares(v[0]);
+      }
     }
   }
   sq += __shfl_xor_sync(0xffffffffu, sq, 1);
@@ -76,16 +94,25 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
   if (warp == 0 && j == 0 && rok) f.e[(long long)b * a.rows + r] = E;
   if (!rok) return;
   __half* dst = f.dst + (long long)b * a.dst_batch;
-  for (int kb = warp; kb < nkb; kb += 8) {
-    if (nkb > 8) load(kb, v);
+  auto digits = [&](int kb, const double2* x) {
     long long q[8];
     __half* d = dst + chunk_off(rows_pad, r, kb, j);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(v[i].x, E);
+    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(x[i].x, E);
     store_digits(q, d, a.plane);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(v[i].y, E);
+    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(x[i].y, E);
     store_digits(q, d + NS * a.plane, a.plane);
+  };
+  if (held) {
+#pragma unroll
+    for (int u = 0; u < KB; ++u)
+      if (warp + 8 * u < nkb) digits(warp + 8 * u, v[u]);
+  } else {
+    for (int kb = warp; kb < nkb; kb += 8) {
+      load(kb, v[0]);
+      digits(kb, v[0]);
+    }
   }
 }
 
@@ -508,7 +535,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
 }  // namespace f64s
 
 void launch_f64_slice(const f64s::SliceArgs& a, int nforms, cudaStream_t s) {
-  f64s::k_f64_slice<<<dim3((a.rows + 7) / 8, nforms, a.batch), 256, 0, s>>>(a);
+  const dim3 grid((a.rows + 7) / 8, nforms, a.batch);
+  if (f64s::k_blocks(a.kdim) <= 8)
+    f64s::k_f64_slice<1><<<grid, 256, 0, s>>>(a);
+  else
+    f64s::k_f64_slice<2><<<grid, 256, 0, s>>>(a);
 }
 
 static int sm_count() {

@@ -187,6 +187,7 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   add((void**)&c->dC, C16 * om);
   add((void**)&c->dD, C16 * om);
   add((void**)&c->wrate, D8 * 4 * ov);
+  add((void**)&c->vph, D8 * 2 * ov);
   add((void**)&c->rsp, D8 * ov);
   add((void**)&c->dcs, C16 * ov);
   // emission tables (Recomb): InitializeEmission on the host, per wire
@@ -437,17 +438,24 @@ static void copy_in(void* dst, const void* src, size_t bytes, cudaStream_t s) {
   cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s);
 }
 
-__global__ void k_vs_from_vc(int nk, const double* VC, const double* E1D, double* vs, double* eps) {
+__global__ void k_vs_from_vc(int nk, const double* VC, const double* E1D, double vscale, double* vs,
+                             double* eps, double* vph) {
   int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= nk) return;
-  for (int n = 0; n < 3; ++n) vs[n * nk + d] = VC[((long long)d * nk + 0) * 3 + n];
-  if (E1D) eps[d] = E1D[(long long)d * nk + 0];
+  double v[3];
+  for (int n = 0; n < 3; ++n) vs[n * nk + d] = v[n] = VC[((long long)d * nk + 0) * 3 + n];
+  if (E1D) {
+    const double e = E1D[(long long)d * nk + 0];
+    eps[d] = e;
+    vph[d] = v[1] / e * vscale;
+    vph[nk + d] = v[2] / e * vscale;
+  }
 }
 
 static void set_vc(SbeCtx* c, int w, const double* VC, const double* E1D, cudaStream_t s) {
   const WireDev& W = c->wires[w];
-  k_vs_from_vc<<<(W.nk + 127) / 128, 128, 0, s>>>(W.nk, VC, E1D, c->vs + 3 * W.off_vec,
-                                                  c->eps + W.off_vec);
+  k_vs_from_vc<<<(W.nk + 127) / 128, 128, 0, s>>>(W.nk, VC, E1D, W.vscale, c->vs + 3 * W.off_vec,
+                                                  c->eps + W.off_vec, c->vph + 2 * W.off_vec);
 }
 
 int sbe_screened_arrays(SbeCtx* c, int w, const double* ne, const double* nh, double* VC,
@@ -752,14 +760,20 @@ int sbe_rk4_step(SbeCtx* c, double* P, double* C, double* D, const double* Ek0, 
       xc = c->xs + n;
       xd = c->xs + 2 * n;
     }
-    launch_stage_field(c, (const double2*)Ek0, (const double2*)dEk, frac[st - 1], s);
+    // the stage field Ek0 + frac dEk: the caller's own where it does not change
+    const double2* ek = (const double2*)Ek0;
+    if (dEk && st > 1) {
+      if (frac[st - 1] != frac[st - 2])
+        launch_stage_field(c, (const double2*)Ek0, (const double2*)dEk, frac[st - 1], s);
+      ek = c->ekst;
+    }
     if (c->f64) {
       double2* X[3] = {p, cc, d};
-      const int rc = sbe::f64_rhs(c, xp, xc, xd, c->ekst, st, dt, nullptr, X, s);
+      const int rc = sbe::f64_rhs(c, xp, xc, xd, ek, st, dt, nullptr, X, s);
       if (rc) return rc;
       continue;
     }
-    launch_calch_ctx(c, xp, xc, xd, c->ekst, s);
+    launch_calch_ctx(c, xp, xc, xd, ek, s);
     launch_rhs64_ctx(c, xp, xc, xd, c->dP, c->dC, c->dD, s);
     launch_rk4_axpy(c, st, dt, p, cc, d, s);
   }

@@ -44,6 +44,7 @@ struct SbeCtx {
   double2* tr = nullptr;                 // 4*tot_vec diagonal traces (C, D) per wire [2][2nk]
   double2 *dP = nullptr, *dC = nullptr, *dD = nullptr;     // tot_mat
   double* wrate = nullptr;               // 4*tot_vec Win/Wout e/h
+  double* vph = nullptr;                 // 2*tot_vec phonon couplings Vep(d), Vhp(d)
   double* rsp = nullptr;                 // tot_vec spontaneous emission rates (Recomb)
   double2* dcs = nullptr;                // tot_vec DC transport shift kernel s(m) per wire
   double* emis = nullptr;                // emission tables (per wire emis_nw values)
@@ -219,6 +220,7 @@ int launch_wire_pdote(SbeCtx* c, int w, const double2* Ek, const double2* src, c
 int launch_deph_extrema(SbeCtx* c, int w, double* out4, cudaStream_t s);
 // sbe_dc.cu: DC transport (dcfield.py:1154-1236 Transport) of P, C, D
 bool any_dc(const SbeCtx* c);
+bool any_ehs(const SbeCtx* c);
 void launch_dc_transport(SbeCtx* c, double2* P, double2* C, double2* D, const double2* Ek,
                          double dt, cudaStream_t s);
 int rk4_mixed(SbeCtx* c, double2* P, double2* C, double2* D, const double2* Ek0,

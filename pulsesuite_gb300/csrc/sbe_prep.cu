@@ -1,5 +1,6 @@
 // Per-step preparation of every wire: occupations, screening, diagonal and
 // off-diagonal dephasing, and the Hartree-Fock Hamiltonians (FP64).
+#include "cluster_sum.cuh"
 #include "sbe_ctx.cuh"
 #include "fp_bits.cuh"
 
@@ -25,15 +26,42 @@ void launch_extract_diag(SbeCtx* c, const double2* C, const double2* D, cudaStre
   k_extract_diag<<<c->nw, 256, 0, s>>>(c->d_wires, C, D, c->ne, c->nh);
 }
 
-__global__ void k_screen(const WireDev* wires, int w_only, const double* v0, const double* chi,
-                         const double* qeh, const double2* ne, const double2* nh, double* eps,
-                         double* vs) {
-  const WireDev W = wires[w_only >= 0 ? w_only : blockIdx.x];
-  const int nk = W.nk;
+// Blocks (kScreenBlocks per wire) each form n1D in the same order and take every
+// kScreenBlocks-th d: the logarithms are bound by one SM's FP64 pipe.  With C, D given the
+// occupations come from their diagonals and are stored (ne, nh, and |ne|, |nh| in FP64 and
+// FP32 for the dephasing sums).  vph: the phonon couplings V_ee(d) / E1D(d) Vscale, V_hh.
+constexpr int kScreenBlocks = 8;
+
+__global__ void __launch_bounds__(256) k_screen(const WireDev* wires, int w_only, const double2* C,
+                                                const double2* D, const double* v0,
+                                                const double* chi, const double* qeh, double2* ne,
+                                                double2* nh, double* occd, float* occf, double* eps,
+                                                double* vs, double* vph) {
+  const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
+  const int nk = W.nk, bx = blockIdx.x;
   __shared__ double red[256];
   double s = 0.0;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x)
-    s += ne[W.off_vec + k].x + nh[W.off_vec + k].x;
+  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+    double2 e, h;
+    if (C) {
+      const long long o = W.off_mat + (long long)k * nk + k;
+      e = C[o];
+      h = D[o];
+      if (k % kScreenBlocks == bx) {
+        const double ae = cabs_d(e), ah = cabs_d(h);
+        ne[W.off_vec + k] = e;
+        nh[W.off_vec + k] = h;
+        occd[2 * W.off_vec + k] = ae;
+        occd[2 * W.off_vec + nk + k] = ah;
+        occf[2 * W.off_vec + k] = (float)ae;
+        occf[2 * W.off_vec + nk + k] = (float)ah;
+      }
+    } else {
+      e = ne[W.off_vec + k];
+      h = nh[W.off_vec + k];
+    }
+    s += e.x + h.x;
+  }
   red[threadIdx.x] = s;
   __syncthreads();
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
@@ -43,7 +71,7 @@ __global__ void k_screen(const WireDev* wires, int w_only, const double* v0, con
   double n1d = red[0] / 2.0 / W.L;
   n1d = fmin(n1d, W.nmax);
   const bool screened = (W.flags & SBE_F_SCREENED) != 0;
-  for (int d = threadIdx.x; d < nk; d += blockDim.x) {
+  for (int d = bx + kScreenBlocks * threadIdx.x; d < nk; d += kScreenBlocks * blockDim.x) {
     double e = 1.0;
     if (screened) {
       double qe = qeh[2 * W.off_vec + d], qh = qeh[2 * W.off_vec + nk + d];
@@ -52,19 +80,24 @@ __global__ void k_screen(const WireDev* wires, int w_only, const double* v0, con
           chh * 2 * log(fabs((qh - kPi * n1d) / (qh + n1d)));
     }
     eps[W.off_vec + d] = e;
+    double v[3];
     for (int n = 0; n < 3; ++n)
-      vs[3 * W.off_vec + n * nk + d] = v0[3 * W.off_vec + n * nk + d] / e;
+      vs[3 * W.off_vec + n * nk + d] = v[n] = v0[3 * W.off_vec + n * nk + d] / e;
+    vph[2 * W.off_vec + d] = v[1] / e * W.vscale;
+    vph[2 * W.off_vec + nk + d] = v[2] / e * W.vscale;
   }
 }
 
-void launch_screen(SbeCtx* c, int w_only, cudaStream_t s) {
-  k_screen<<<w_only >= 0 ? 1 : c->nw, 256, 0, s>>>(c->d_wires, w_only, c->v0, c->chi, c->qeh,
-                                                   c->ne, c->nh, c->eps, c->vs);
+static void screen(SbeCtx* c, int w_only, const double2* C, const double2* D, cudaStream_t s) {
+  k_screen<<<dim3(kScreenBlocks, w_only >= 0 ? 1 : c->nw), 256, 0, s>>>(
+      c->d_wires, w_only, C, D, c->v0, c->chi, c->qeh, c->ne, c->nh, c->occd, c->occf, c->eps, c->vs,
+      c->vph);
 }
 
+void launch_screen(SbeCtx* c, int w_only, cudaStream_t s) { screen(c, w_only, nullptr, nullptr, s); }
+
 void launch_prep_scalar(SbeCtx* c, const double2* C, const double2* D, cudaStream_t s) {
-  launch_extract_diag(c, C, D, s);
-  launch_screen(c, -1, s);
+  screen(c, -1, C, D, s);
   launch_spont(c, -1, s);   // Recomb: SBEs.py:5203-5226
 }
 
@@ -90,7 +123,7 @@ void launch_expand_vc(SbeCtx* c, int w, double* VC, double* E1D, cudaStream_t s)
 // ---------------------------------------------------------------------------
 // dephasing.py:29-103 (_CalcGammaE_jit/_CalcGammaH_jit) with the index maps of
 // InitializeDephasing and Vxx2 (V[round(|k/dk|), 0]^2, dephasing.py:362-378).
-// One warp per (wire, k), lanes over q.
+// A warp per k, lanes over q.
 __device__ inline double occ_ext(const double2* n, int idx, int nk, bool* ok) {
   // extended array of the reference: index idx+1 in [1, nk] is valid
   if (idx < 0 || idx >= nk) { *ok = false; return 0.0; }
@@ -98,68 +131,83 @@ __device__ inline double occ_ext(const double2* n, int idx, int nk, bool* ok) {
   return n[idx].x;
 }
 
-__global__ void k_gamma(const WireDev* wires, int w_only, const double2* ne, const double2* nh,
-                        const double* vs, const int* iq, const int* maps, const double* xeh,
-                        double* gamE, double* gamH) {
-  int wi = (w_only >= 0) ? w_only : blockIdx.y;
-  const WireDev W = wires[wi];
-  const int nk = W.nk;
-  int k = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  int lane = threadIdx.x & 31;
-  if (k >= nk) return;
+// a warp per k, four per block (the FP64 pipes of all SMs), which form the weights per q once:
+// 2 x 512 50 -> 43 us; 16 per block 67 us
+
+__global__ void __launch_bounds__(128) k_gamma(const WireDev* wires, int w_only, const double2* ne,
+                                               const double2* nh, const double* vs, const int* iq,
+                                               const int* maps, const double* xeh, double* gamE,
+                                               double* gamH) {
+  const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
+  const int nk = W.nk, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = blockIdx.x * 4 + warp;
+  if (blockIdx.x * 4 >= nk) return;
   if (!(W.flags & SBE_F_DIAGDPH)) {
-    if (lane == 0) {
+    if (lane == 0 && k < nk) {
       gamE[W.off_vec + k] = W.gam_e;
       gamH[W.off_vec + k] = W.gam_h;
     }
     return;
   }
+  // per 128 q: (pi / hbar) V^2 |x| of the four terms
+  __shared__ double wt[4][128];
   const double2* pe = ne + W.off_vec;
   const double2* ph = nh + W.off_vec;
   const long long st = (long long)nk * nk;
-  const int* m = maps + 6 * W.off_mat + (long long)k * nk;
   const double* v = vs + 3 * W.off_vec;
   const double* xe = xeh + 2 * W.off_vec;
   const double* xh = xe + nk;
   const double pih = kPi / kHbar;
   double ge = 0.0, gh = 0.0;
-  for (int q = lane; q < nk; q += 32) {
-    int iqq = iq[W.off_vec + q];
-    double veh = v[0 * nk + iqq], vee = v[1 * nk + iqq], vhh = v[2 * nk + iqq];
-    double veh2 = veh * veh, vee2 = vee * vee, vhh2 = vhh * vhh;
-    bool ok, ok1, ok2, ok3;
-    // electrons
-    double a = occ_ext(pe, m[0 * st + q], nk, &ok);
-    if (ok) ge += pih * vee2 * a * (1.0 - a) * fabs(xe[q]);
-    double n1 = occ_ext(ph, m[3 * st + q], nk, &ok1);   // k1p_m_q
-    double n2 = occ_ext(ph, m[2 * st + q], nk, &ok2);   // k1p
-    double n3 = occ_ext(pe, m[1 * st + q], nk, &ok3);   // k_m_q
-    if (ok1 && ok2 && ok3)
-      ge += pih * veh2 * (n1 * (1.0 - n2) * n3 + (1.0 - n1) * n2 * (1.0 - n3)) * fabs(xh[q]);
-    // holes
-    double b = occ_ext(ph, m[0 * st + q], nk, &ok);
-    if (ok) gh += pih * vhh2 * b * (1.0 - b) * fabs(xh[q]);
-    double e1 = occ_ext(pe, m[5 * st + q], nk, &ok1);   // k1_m_q
-    double e2 = occ_ext(pe, m[4 * st + q], nk, &ok2);   // k1
-    double h3 = occ_ext(ph, m[1 * st + q], nk, &ok3);   // k_m_q
-    if (ok1 && ok2 && ok3)
-      gh += pih * veh2 * (e1 * (1.0 - e2) * h3 + (1.0 - e1) * e2 * (1.0 - h3)) * fabs(xe[q]);
+  for (int q0 = 0; q0 < nk; q0 += 128) {
+    __syncthreads();
+    if (q0 + (int)threadIdx.x < nk) {
+      const int q = q0 + threadIdx.x, iqq = iq[W.off_vec + q];
+      const double veh = v[iqq], vee = v[nk + iqq], vhh = v[2 * nk + iqq];
+      const double ae = fabs(xe[q]), ah = fabs(xh[q]);
+      wt[0][threadIdx.x] = pih * (vee * vee) * ae;
+      wt[1][threadIdx.x] = pih * (veh * veh) * ah;
+      wt[2][threadIdx.x] = pih * (vhh * vhh) * ah;
+      wt[3][threadIdx.x] = pih * (veh * veh) * ae;
+    }
+    __syncthreads();
+    const int qe = min(128, nk - q0);
+    if (k < nk) {
+      const int* m = maps + 6 * W.off_mat + (long long)k * nk + q0;
+      for (int q = lane; q < qe; q += 32) {
+        bool ok, ok1, ok2, ok3;
+        // electrons
+        double a = occ_ext(pe, m[0 * st + q], nk, &ok);
+        if (ok) ge += wt[0][q] * (a * (1.0 - a));
+        double n1 = occ_ext(ph, m[3 * st + q], nk, &ok1);   // k1p_m_q
+        double n2 = occ_ext(ph, m[2 * st + q], nk, &ok2);   // k1p
+        double n3 = occ_ext(pe, m[1 * st + q], nk, &ok3);   // k_m_q
+        if (ok1 && ok2 && ok3)
+          ge += wt[1][q] * (n1 * (1.0 - n2) * n3 + (1.0 - n1) * n2 * (1.0 - n3));
+        // holes
+        double b = occ_ext(ph, m[0 * st + q], nk, &ok);
+        if (ok) gh += wt[2][q] * (b * (1.0 - b));
+        double e1 = occ_ext(pe, m[5 * st + q], nk, &ok1);   // k1_m_q
+        double e2 = occ_ext(pe, m[4 * st + q], nk, &ok2);   // k1
+        double h3 = occ_ext(ph, m[1 * st + q], nk, &ok3);   // k_m_q
+        if (ok1 && ok2 && ok3)
+          gh += wt[3][q] * (e1 * (1.0 - e2) * h3 + (1.0 - e1) * e2 * (1.0 - h3));
+      }
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     ge += __shfl_down_sync(0xffffffffu, ge, o);
     gh += __shfl_down_sync(0xffffffffu, gh, o);
   }
-  if (lane == 0) {
+  if (lane == 0 && k < nk) {
     gamE[W.off_vec + k] = ge;
     gamH[W.off_vec + k] = gh;
   }
 }
 
 void launch_gamma(SbeCtx* c, int w_only, cudaStream_t s) {
-  int wpb = 8;
-  dim3 g((c->nk_max + wpb - 1) / wpb, w_only >= 0 ? 1 : c->nw);
-  k_gamma<<<g, 32 * wpb, 0, s>>>(c->d_wires, w_only, c->ne, c->nh, c->vs, c->iq, c->maps,
-                                 c->xeh, c->gamE, c->gamH);
+  k_gamma<<<dim3((c->nk_max + 3) / 4, w_only >= 0 ? 1 : c->nw), 128, 0, s>>>(
+      c->d_wires, w_only, c->ne, c->nh, c->vs, c->iq, c->maps, c->xeh, c->gamE, c->gamH);
 }
 
 // ---------------------------------------------------------------------------
@@ -181,12 +229,11 @@ void launch_gamma(SbeCtx* c, int w_only, cudaStream_t s) {
 // error of Dh at Nk = 128 from 3.9e-14 to 2.9e-15.
 __global__ void k_occd(const WireDev* wires, int w_only, const double2* ne, const double2* nh,
                        double* occd) {
-  const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
+  const WireDev& W = wires[w_only];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= W.nk) return;
-  const double2 e = ne[W.off_vec + k], h = nh[W.off_vec + k];
-  occd[2 * W.off_vec + k] = hypot(e.x, e.y);
-  occd[2 * W.off_vec + W.nk + k] = hypot(h.x, h.y);
+  occd[2 * W.off_vec + k] = cabs_d(ne[W.off_vec + k]);
+  occd[2 * W.off_vec + W.nk + k] = cabs_d(nh[W.off_vec + k]);
 }
 
 struct Deph64 {
@@ -364,14 +411,6 @@ __device__ inline void split12(double v, float* hi, float* lo) {
   *lo = (float)(v - h);
 }
 
-__global__ void k_occf(const WireDev* wires, const double2* ne, const double2* nh, float* occf) {
-  const WireDev& W = wires[blockIdx.y];
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= W.nk) return;
-  occf[2 * W.off_vec + k] = (float)hypot(ne[W.off_vec + k].x, ne[W.off_vec + k].y);
-  occf[2 * W.off_vec + W.nk + k] = (float)hypot(nh[W.off_vec + k].x, nh[W.off_vec + k].y);
-}
-
 // One block per (q >= 0, species, wire) and up to 512 k; each thread sums four
 // consecutive k, so that the per-p shared-memory loads (the Lorentzian window and
 // the paired occupation weights, read as one float2 broadcast) serve four outputs.
@@ -399,7 +438,7 @@ __global__ void __launch_bounds__(128) k_offdiag_D32(const WireDev* wires, const
   float* Ltab = nb + nk;                                 // 2nk entries: m - mlo
   float2* wa = reinterpret_cast<float2*>(Ltab + 2 * nk); // (Aa, Ba) per p (a-a)
   float2* wb = wa + nk;                                  // (Ab, Bb) per p (a-b)
-  // |n_e|, |n_h| as FP32 (formed once per step by k_occf)
+  // |n_e|, |n_h| as FP32 (formed once per step by k_screen)
   const float* pa = occf + 2 * W.off_vec + (which == 0 ? 0 : nk);
   const float* pb = occf + 2 * W.off_vec + (which == 0 ? nk : 0);
   for (int i = threadIdx.x; i < nk; i += blockDim.x) {
@@ -758,8 +797,6 @@ __global__ void k_deph_consts(const WireDev* wires, const double* vs, float* dco
 
 void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaStream_t s) {
   if (fp32 && w_only < 0 && !g3) {
-    k_occf<<<dim3((c->nk_max + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, c->ne, c->nh,
-                                                                 c->occf);
     k_deph_consts<<<dim3((c->nk_max + 127) / 128, 2 * c->nw), 128, 0, s>>>(c->d_wires, c->vs,
                                                                           c->dconst, c->dpre);
     // groups of 4 or more wires share the Lorentzian factors (chunks of up to 16
@@ -790,8 +827,9 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
     }
     return;
   }
-  k_occd<<<dim3((c->nk_max + 127) / 128, w_only >= 0 ? 1 : c->nw), 128, 0, s>>>(
-      c->d_wires, w_only, c->ne, c->nh, c->occd);
+  if (w_only >= 0)   // the caller's occupations; a step's come with the preparation
+    k_occd<<<(c->wires[w_only].nk + 127) / 128, 128, 0, s>>>(c->d_wires, w_only, c->ne, c->nh,
+                                                            c->occd);
   Deph64 a{};
   a.wires = c->d_wires;
   a.w_only = w_only;

@@ -43,13 +43,14 @@ __global__ void k_leap_shuffle(const WireDev* wires, double2* L1, double2* L2, d
   }
 }
 
-// phonons.py:140-268 MBPE / MBPH for row k of every wire, with the screened
-// VC and E1D of the preparation: Vep = VC[:,:,1]/E1D*Vscale (VC already
-// divided by E1D once: the quirk is kept).  ne, nh are Re(diag) of C3, D3.
-__global__ void k_phonon_rates(const WireDev* wires, int w_only, const double2* nev,
-                               const double2* nhv, const double* vs, const double* eps,
-                               const double* EP, const double* HP, double* wrate) {
-  const WireDev W = wires[w_only >= 0 ? w_only : blockIdx.y];
+// phonons.py:140-268 MBPE / MBPH for row k of every wire, with the couplings of the
+// preparation: Vep = VC[:,:,1]/E1D*Vscale (VC already divided by E1D once: the quirk is
+// kept).  ne, nh: Re of the vectors, or (diag) of the diagonals of the matrices C3, D3.
+__global__ void __launch_bounds__(128) k_phonon_rates(const WireDev* wires, int w_only,
+                                                      const double2* nev, const double2* nhv,
+                                                      int diag, const double* vph, const double* EP,
+                                                      const double* HP, double* wrate) {
+  const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int nk = W.nk;
   int k = blockIdx.x;
   if (k >= nk) return;
@@ -58,38 +59,37 @@ __global__ void k_phonon_rates(const WireDev* wires, int w_only, const double2* 
     if (threadIdx.x < 4) wrate[4 * W.off_vec + threadIdx.x * nk + k] = 0.0;
     return;
   }
-  const double* v1 = vs + 3 * W.off_vec + nk;
-  const double* v2 = vs + 3 * W.off_vec + 2 * nk;
-  const double* ep = eps + W.off_vec;
+  const double* ve = vph + 2 * W.off_vec;
+  const double* vh = ve + nk;
+  const double2* pe = nev + (diag ? W.off_mat : W.off_vec);
+  const double2* ph = nhv + (diag ? W.off_mat : W.off_vec);
+  const long long st = diag ? nk + 1 : 1;
   const double* EPw = EP + W.off_mat;
   const double* HPw = HP + W.off_mat;
-  double wie = 0.0, woe = 0.0, wih = 0.0, woh = 0.0;
+  double r[4] = {0.0, 0.0, 0.0, 0.0};
   for (int i = threadIdx.x; i < nk; i += blockDim.x) {
-    double ne_i = nev[W.off_vec + i].x;
-    double nh_i = nhv[W.off_vec + i].x;
-    // electrons: Vep[k, i] (nonzero for k >= i)
-    int d = k - i;
-    double vep = (d >= 0 ? v1[d] : 0.0) / ep[d >= 0 ? d : -d] * W.vscale;
-    wie += vep * ne_i * EPw[(long long)k * nk + i];
-    woe += vep * (1.0 - ne_i) * EPw[(long long)i * nk + k];
-    // holes: Vhp[i, k] (nonzero for i >= k)
-    int e = i - k;
-    double vhp = (e >= 0 ? v2[e] : 0.0) / ep[e >= 0 ? e : -e] * W.vscale;
-    wih += vhp * nh_i * HPw[(long long)k * nk + i];
-    woh += vhp * (1.0 - nh_i) * HPw[(long long)i * nk + k];
+    if (i <= k) {   // electrons: Vep[k, i] (nonzero for k >= i)
+      const double n = pe[i * st].x, v = ve[k - i];
+      r[0] += v * n * EPw[(long long)k * nk + i];
+      r[1] += v * (1.0 - n) * EPw[(long long)i * nk + k];
+    }
+    if (i >= k) {   // holes: Vhp[i, k] (nonzero for i >= k)
+      const double n = ph[i * st].x, v = vh[i - k];
+      r[2] += v * n * HPw[(long long)k * nk + i];
+      r[3] += v * (1.0 - n) * HPw[(long long)i * nk + k];
+    }
   }
-  __shared__ double red[4][128];
-  red[0][threadIdx.x] = wie;
-  red[1][threadIdx.x] = woe;
-  red[2][threadIdx.x] = wih;
-  red[3][threadIdx.x] = woh;
+  __shared__ double red[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    for (int o = 16; o > 0; o >>= 1) r[j] += __shfl_down_sync(0xffffffffu, r[j], o);
+    if ((threadIdx.x & 31) == 0) red[j][threadIdx.x >> 5] = r[j];
+  }
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int j = 0; j < 4; ++j) red[j][threadIdx.x] += red[j][threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x < 4) {
+    const double* q = red[threadIdx.x];
+    wrate[4 * W.off_vec + threadIdx.x * nk + k] = (q[0] + q[1]) + (q[2] + q[3]);
   }
-  if (threadIdx.x < 4) wrate[4 * W.off_vec + threadIdx.x * nk + k] = red[threadIdx.x][0];
 }
 
 // SBEs.py:5677-5702 + 5276-5325: relaxation of the diagonals with the phonon
@@ -104,19 +104,20 @@ __device__ __forceinline__ double2 cexp_d(double2 z) {
 }
 
 // mode 0: relaxation and normalisation; 1: relaxation only (the relaxed complex
-// diagonals back into C3, D3); 2: normalisation only.
-__global__ void k_relax_norm(const WireDev* wires, double2* C3, double2* D3, const double* wrate,
-                             const double* rsp, double dt, double2* ne_out, double2* nh_out,
-                             double* charge, int mode) {
-  const WireDev W = wires[blockIdx.x];
-  const int nk = W.nk;
+// diagonals back into C3, D3); 2: normalisation only.  One cluster per wire: the four
+// exponentials and divisions per k are bound by the FP64 pipes of its SMs.
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
+    k_relax_norm(const WireDev* wires, double2* C3, double2* D3, const double* wrate,
+                 const double* rsp, double dt, double2* ne_out, double2* nh_out, double* charge,
+                 int mode) {
+  const WireDev& W = wires[blockIdx.y];
+  const int nk = W.nk, k0 = blockIdx.x + kCluster * threadIdx.x, kst = kCluster * 256;
   const bool relax = mode != 2 && (W.flags & (SBE_F_PHONON | SBE_F_EHS)) != 0;
   // the decay is part of the relaxation, which runs only with Phonon or EHs
   // (SBEs.py:5677, 5322)
   const bool recomb = relax && (W.flags & SBE_F_RECOMB) != 0;
-  __shared__ double red[2][256];
   double se = 0.0, sh = 0.0;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+  for (int k = k0; k < nk; k += kst) {
     long long o = W.off_mat + (long long)k * nk + k;
     double2 ne = C3[o], nh = D3[o];
     if (relax) {
@@ -143,33 +144,23 @@ __global__ void k_relax_norm(const WireDev* wires, double2* C3, double2* D3, con
       D3[o] = nh;
       continue;
     }
-    double ae = hypot(ne.x, ne.y), ah = hypot(nh.x, nh.y);
+    const double ae = cabs_d(ne), ah = cabs_d(nh);
     ne_out[W.off_vec + k] = make_double2(ae, 0.0);
     nh_out[W.off_vec + k] = make_double2(ah, 0.0);
     se += ae;
     sh += ah;
   }
-  if (mode == 1) return;   // block-uniform
-  red[0][threadIdx.x] = se;
-  red[1][threadIdx.x] = sh;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + o];
-      red[1][threadIdx.x] += red[1][threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  double sum_e = red[0][0], sum_h = red[1][0];
-  if (threadIdx.x == 0) {
+  if (mode == 1) return;   // uniform over the cluster
+  cluster_sum2(se, sh);
+  if (k0 == 0) {
     // the carrier numbers before the normalisation: their difference is what this
     // step's relaxation and rounding left of the electron-hole balance
-    charge[2 * blockIdx.x] = sum_e;
-    charge[2 * blockIdx.x + 1] = sum_h;
+    charge[2 * blockIdx.y] = se;
+    charge[2 * blockIdx.y + 1] = sh;
   }
-  double total = (sum_e + sum_h) / 2.0;
-  double fe = total / (sum_e + kSmall), fh = total / (sum_h + kSmall);
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+  double total = (se + sh) / 2.0;
+  double fe = total / (se + kSmall), fh = total / (sh + kSmall);
+  for (int k = k0; k < nk; k += kst) {
     long long o = W.off_mat + (long long)k * nk + k;
     double ae = ne_out[W.off_vec + k].x * fe, ah = nh_out[W.off_vec + k].x * fh;
     ne_out[W.off_vec + k] = make_double2(ae, 0.0);
@@ -179,11 +170,17 @@ __global__ void k_relax_norm(const WireDev* wires, double2* C3, double2* D3, con
   }
 }
 
+bool any_ehs(const SbeCtx* c) {
+  for (const auto& W : c->wires)
+    if (W.flags & SBE_F_EHS) return true;
+  return false;
+}
+
 void launch_relax_norm(SbeCtx* c, double2* P3, double2* C3, double2* D3, const double2* Ek,
                        double dt, cudaStream_t s) {
-  launch_extract_diag(c, C3, D3, s);
-  k_phonon_rates<<<dim3(c->nk_max, c->nw), 128, 0, s>>>(c->d_wires, -1, c->ne, c->nh, c->vs,
-                                                        c->eps, c->EP, c->HP, c->wrate);
+  if (any_ehs(c)) launch_extract_diag(c, C3, D3, s);   // for the carrier-carrier rates
+  k_phonon_rates<<<dim3(c->nk_max, c->nw), 128, 0, s>>>(c->d_wires, -1, C3, D3, 1, c->vph, c->EP,
+                                                        c->HP, c->wrate);
   launch_mbc_rates(c, -1, s);
   launch_relax_only(c, P3, C3, D3, Ek, dt, s);
 }
@@ -193,20 +190,20 @@ void launch_relax_norm(SbeCtx* c, double2* P3, double2* C3, double2* D3, const d
 void launch_relax_only(SbeCtx* c, double2* P3, double2* C3, double2* D3, const double2* Ek,
                        double dt, cudaStream_t s) {
   if (!any_dc(c)) {
-    k_relax_norm<<<c->nw, 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
+    k_relax_norm<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
                                        c->charge, 0);
     return;
   }
-  k_relax_norm<<<c->nw, 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
+  k_relax_norm<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
                                      c->charge, 1);
   launch_dc_transport(c, P3, C3, D3, Ek, dt, s);
-  k_relax_norm<<<c->nw, 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
+  k_relax_norm<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
                                      c->charge, 2);
 }
 
 void launch_phonon_rates_one(SbeCtx* c, int w, cudaStream_t s) {
-  k_phonon_rates<<<dim3(c->wires[w].nk, 1), 128, 0, s>>>(c->d_wires, w, c->ne, c->nh, c->vs,
-                                                         c->eps, c->EP, c->HP, c->wrate);
+  k_phonon_rates<<<dim3(c->wires[w].nk, 1), 128, 0, s>>>(c->d_wires, w, c->ne, c->nh, 0, c->vph,
+                                                         c->EP, c->HP, c->wrate);
 }
 
 void launch_leapfrog(SbeCtx* c, double2* const* st, const double2* Ek, double dt,
@@ -268,70 +265,50 @@ __global__ void k_src_reduce(const WireDev* wires, int w_only, const double2* ex
 }
 
 // qwoptics.py:1062-1068 boundary-mean subtraction and renormalisation, then
-// SBEs.py:5749-5750 (x 2 e0 ehint / area).  One block per wire.
-__global__ void k_src_final(const WireDev* wires, int w_only, const double* r, const double2* ne,
-                            const double2* nh, double2* src) {
-  const WireDev W = wires[w_only >= 0 ? w_only : blockIdx.x];
-  const int nr = W.nr, nk = W.nk;
+// SBEs.py:5749-5750 (x 2 e0 ehint / area).  One cluster per wire (FP64 square roots); every
+// block forms the carrier sums and boundary means itself, the first cluster barrier keeps
+// the boundary values from being overwritten before all have read them.
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
+    k_src_final(const WireDev* wires, int w_only, const double* r, const double2* ne,
+                const double2* nh, double2* src) {
+  const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
+  const int nr = W.nr, nk = W.nk, j0 = blockIdx.x + kCluster * threadIdx.x, st = kCluster * 256;
   double2* re = src + 5 * W.off_r + 3 * nr;
   double2* rh = re + nr;
-  const bool lf = (W.flags & SBE_F_LF) != 0;
-  if (!lf) {
-    for (int j = threadIdx.x; j < nr; j += blockDim.x) {
+  if (!(W.flags & SBE_F_LF)) {
+    for (int j = j0; j < nr; j += st) {
       re[j] = make_double2(0, 0);
       rh[j] = make_double2(0, 0);
     }
     return;
   }
-  __shared__ double red[4][256];
-  double a = 0, b = 0, c = 0, d = 0;
-  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
-    a += hypot(ne[W.off_vec + k].x, ne[W.off_vec + k].y);
-    b += hypot(nh[W.off_vec + k].x, nh[W.off_vec + k].y);
+  double v[4] = {0, 0, 0, 0};   // carrier sums, boundary sums
+  for (int k = threadIdx.x; k < nk; k += 256) {
+    v[0] += cabs_d(ne[W.off_vec + k]);
+    v[1] += cabs_d(nh[W.off_vec + k]);
   }
   // sum(re[0:10]) + sum(re[Nr-10:Nr]): an index in both slices counts twice
-  for (int j = threadIdx.x; j < nr; j += blockDim.x) {
-    int m = (j < 10 ? 1 : 0) + (j >= nr - 10 ? 1 : 0);
-    c += m * re[j].x;
-    d += m * rh[j].x;
+  if (threadIdx.x < 20) {
+    const int j = threadIdx.x < 10 ? threadIdx.x : nr - 20 + threadIdx.x;
+    v[2] = re[j].x;
+    v[3] = rh[j].x;
   }
-  red[0][threadIdx.x] = a; red[1][threadIdx.x] = b; red[2][threadIdx.x] = c; red[3][threadIdx.x] = d;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int q = 0; q < 4; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + o];
-    __syncthreads();
-  }
-  double NeT = red[0][0] + 1e-50, NhT = red[1][0] + 1e-50;
-  double be = red[2][0] / 20.0, bh = red[3][0] / 20.0;
-  __syncthreads();
+  block_sums(v);
+  const double NeT = v[0] + 1e-50, NhT = v[1] + 1e-50, be = v[2] / 20.0, bh = v[3] / 20.0;
   double ae = 0, ah = 0;
-  for (int j = threadIdx.x; j < nr; j += blockDim.x) {
-    double2 x = re[j], y = rh[j];
-    x.x -= be;
-    y.x -= bh;
-    re[j] = x;
-    rh[j] = y;
-    ae += hypot(x.x, x.y);
-    ah += hypot(y.x, y.y);
+  for (int j = j0; j < nr; j += st) {
+    const double2 x = re[j], y = rh[j];
+    ae += cabs_d(make_double2(x.x - be, x.y));
+    ah += cabs_d(make_double2(y.x - bh, y.y));
   }
-  red[0][threadIdx.x] = ae;
-  red[1][threadIdx.x] = ah;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + o];
-      red[1][threadIdx.x] += red[1][threadIdx.x + o];
-    }
-    __syncthreads();
-  }
+  cluster_sum2(ae, ah);
   const double* rw = r + W.off_r;
-  double dr = rw[1] - rw[0];
-  double fe = NeT / (red[0][0] * dr + kQwSmall), fh = NhT / (red[1][0] * dr + kQwSmall);
-  for (int j = threadIdx.x; j < nr; j += blockDim.x) {
-    double2 x = cscale(re[j], fe), y = cscale(rh[j], fh);
-    re[j] = make_double2(2.0 * kE0 * x.x / W.area * W.ehint, 2.0 * kE0 * x.y / W.area * W.ehint);
-    rh[j] = make_double2(2.0 * kE0 * y.x / W.area * W.ehint, 2.0 * kE0 * y.y / W.area * W.ehint);
+  const double dr = rw[1] - rw[0], f = 2.0 * kE0 / W.area * W.ehint;
+  const double fe = f * (NeT / (ae * dr + kQwSmall)), fh = f * (NhT / (ah * dr + kQwSmall));
+  for (int j = j0; j < nr; j += st) {
+    const double2 x = re[j], y = rh[j];
+    re[j] = make_double2((x.x - be) * fe, x.y * fe);
+    rh[j] = make_double2((y.x - bh) * fh, y.y * fh);
   }
 }
 
@@ -358,7 +335,7 @@ void launch_sources(SbeCtx* c, const double2* P, const double2* C, const double2
   (void)nb;
   k_src_reduce<<<dim3((c->nr_max + 127) / 128, nb), 128, 0, s>>>(c->d_wires, w_only, c->expikr,
                                                                 c->G, c->tot_kr, c->window, src);
-  k_src_final<<<nb, 256, 0, s>>>(c->d_wires, w_only, c->r, ne, nh, src);
+  k_src_final<<<dim3(kCluster, nb), 256, 0, s>>>(c->d_wires, w_only, c->r, ne, nh, src);
 }
 
 // ---------------------------------------------------------------------------
@@ -668,13 +645,13 @@ int launch_qw2prop(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
 namespace sbe {
 void launch_sources_final(SbeCtx* c, const double2* ne, const double2* nh, double2* src,
                           cudaStream_t s) {
-  k_src_final<<<c->nw, 256, 0, s>>>(c->d_wires, -1, c->r, ne, nh, src);
+  k_src_final<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, -1, c->r, ne, nh, src);
 }
 
 void launch_sources_reduce(SbeCtx* c, const double2* ne, const double2* nh, double2* src,
                            cudaStream_t s) {
   k_src_reduce<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, -1, c->expikr,
                                                                    c->G, c->tot_kr, c->window, src);
-  k_src_final<<<c->nw, 256, 0, s>>>(c->d_wires, -1, c->r, ne, nh, src);
+  k_src_final<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, -1, c->r, ne, nh, src);
 }
 }  // namespace sbe

@@ -814,8 +814,9 @@ __global__ void k_phon_tab(const WireDev* wires, const double* vs, const double*
 
 // MBPE / MBPH (phonons.py:157-268) in FP32 from the scaled tables: Win, Wout of
 // electrons and holes at the occupations in ne, nh (real parts) into wrate (FP64).
+// nev, nhv: the vectors, or (diag) the matrices whose diagonals they are.
 __global__ void k_phonon_rates_f(const WireDev* wires, const double2* nev, const double2* nhv,
-                                 const float* phf, const float* epf, const float* eptf,
+                                 int diag, const float* phf, const float* epf, const float* eptf,
                                  const float* hpf, const float* hptf, double* wrate, int nw) {
   extern __shared__ float occ[];
   const WireDev W = wires[blockIdx.y];
@@ -828,8 +829,9 @@ __global__ void k_phonon_rates_f(const WireDev* wires, const double2* nev, const
   float* pe = occ;
   float* ph = occ + nk;
   for (int i = threadIdx.x; i < nk; i += blockDim.x) {
-    pe[i] = f64_to_f32(nev[W.off_vec + i].x);
-    ph[i] = f64_to_f32(nhv[W.off_vec + i].x);
+    const long long o = diag ? W.off_mat + (long long)i * (nk + 1) : W.off_vec + i;
+    pe[i] = f64_to_f32(nev[o].x);
+    ph[i] = f64_to_f32(nhv[o].x);
   }
   __syncthreads();
   const float* ve = phf + (long long)b * nk;
@@ -1670,10 +1672,10 @@ static int mixed_prep(SbeCtx* c, const double2* C, const double2* D, cudaStream_
 static void mixed_relax(SbeCtx* c, double2* P, double2* C, double2* D, const double2* Ek,
                         double dt, cudaStream_t s) {
   MixedAll* A = all_of(c);
-  launch_extract_diag(c, C, D, s);
+  if (any_ehs(c)) launch_extract_diag(c, C, D, s);   // for the carrier-carrier rates
   for (Mixed* m : A->b)
     k_phonon_rates_f<<<dim3(m->nk, m->nw), 128, sizeof(float) * 2 * m->nk, s>>>(
-        m->dw, c->ne, c->nh, m->phf, A->epf, A->eptf, A->hpf, A->hptf, c->wrate, m->nw);
+        m->dw, C, D, 1, m->phf, A->epf, A->eptf, A->hpf, A->hptf, c->wrate, m->nw);
   launch_mbc_rates(c, -1, s, false, true);
   launch_relax_only(c, P, C, D, Ek, dt, s);
   for (Mixed* m : A->b) k_diag_max<<<m->nw, 256, 0, s>>>(m->dw, C, D, m->mxS());
