@@ -47,6 +47,7 @@ namespace {
 __global__ void k_couple_eval(const WireDev* wires, int nx, const double* xg, const double2* gy,
                               const double2* gcoef, const double* wx, const double* r,
                               const double* window, double2* wv, float* wvf) {
+  pdl_enter();
   const int w = blockIdx.y;
   const WireDev W = wires[w];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -73,6 +74,7 @@ __global__ void k_couple_eval(const WireDev* wires, int nx, const double* xg, co
 // even) and store both.
 __global__ void __launch_bounds__(256) k_couple_fftg_f(const WireDev* wires, const float2* twr,
                                                        const float* wv, double2* Ek) {
+  pdl_enter();
   const int w = blockIdx.y;
   const WireDev W = wires[w];
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(256) k_couple_fftg_f(const WireDev* wires, con
 // One warp per q; the twiddle table holds exp(-2 pi i m / Nr).
 __global__ void __launch_bounds__(256) k_couple_fftg(const WireDev* wires, const double2* twr,
                                                      const double2* wv, double2* Ek) {
+  pdl_enter();
   const int w = blockIdx.y;
   const WireDev W = wires[w];
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -161,6 +164,7 @@ __global__ void __launch_bounds__(64) k_couple_deposit(const WireDev* wires, int
                                                        const double* r, const double2* src,
                                                        const double2* wcoef, double2* Pg,
                                                        double2* rho) {
+  pdl_enter();
   __shared__ double s_wx[DEP_CHUNK], s_r0[DEP_CHUNK], s_r1[DEP_CHUNK];
   __shared__ long long s_off[DEP_CHUNK];
   __shared__ int s_nr[DEP_CHUNK];
@@ -207,6 +211,7 @@ __global__ void __launch_bounds__(64) k_couple_deposit(const WireDev* wires, int
 __global__ void k_couple_current(int nx, double dt, const double2* Pg, double2* Pold, double2* J,
                                  const long long* step, double t0, int src_index, double jamp,
                                  double tau, double w0, double tpeak) {
+  pdl_enter();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nx) return;
   for (int c = 0; c < 3; ++c) {
@@ -225,9 +230,11 @@ __global__ void k_couple_current(int nx, double dt, const double2* Pg, double2* 
   }
 }
 
-__global__ void k_tick(long long* step) { *step += 1; }
+__global__ void k_tick(long long* step) {
+  pdl_enter(); *step += 1; }
 
 __global__ void k_stage3(int nx, const double2* Ex, const double2* E, double2* gy) {
+  pdl_enter();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nx) return;
   gy[j] = Ex[j];
@@ -276,6 +283,7 @@ SplBatch wire_batch(SbeCouple* cp) {
 // lines[w][f][k], f the wire's component.
 __global__ void k_c3_lines(int nx, int ny, int nz, const double* xg, const double* yg,
                            const double* wxy, const double2* E, double2* lines) {
+  pdl_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x, w = blockIdx.y;
   if (k >= nz) return;
   const double xw = wxy[2 * w], yw = wxy[2 * w + 1];
@@ -300,6 +308,7 @@ __global__ void k_c3_lines(int nx, int ny, int nz, const double* xg, const doubl
 __global__ void k_c3_eval(const WireDev* wires, int nz, const double* zg, const double2* lines,
                           const double2* lcoef, const double* r, const double* window, double2* wv,
                           float* wvf) {
+  pdl_enter();
   const int w = blockIdx.y;
   const WireDev W = wires[w];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -326,6 +335,7 @@ __global__ void k_c3_eval(const WireDev* wires, int nz, const double* zg, const 
 // c = 0, 1, 2 (Px, Py, Pz of the grid) and 3 (rho = rh - re).
 __global__ void k_c3_wire_lines(const WireDev* wires, int nz, const double* zg, const double* r,
                                 const double2* src, const double2* wcoef, double2* dl) {
+  pdl_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x, w = blockIdx.y;
   if (k >= nz) return;
   const WireDev W = wires[w];
@@ -372,6 +382,7 @@ struct C3Dep {
 };
 
 __global__ void k_c3_deposit(C3Dep a) {
+  pdl_enter();
   const int col = blockIdx.x;
   const int i = col / a.ny, j = col % a.ny;
   const long long N = (long long)a.nx * a.ny * a.nz;
@@ -419,16 +430,16 @@ int couple_sample(SbeCouple* cp, const double2* Ex, const double2* E, int precis
                   cudaStream_t s) {
   SbeCtx* c = cp->ctx;
   const int nx = cp->p->nx;
-  k_stage3<<<(nx + 255) / 256, 256, 0, s>>>(nx, Ex, E, cp->g_y);
+  launch(k_stage3, (nx + 255) / 256, 256, 0, s, nx, Ex, E, cp->g_y);
   launch_splines(grid_batch(cp), 1, nx, s);
-  k_couple_eval<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(
-      c->d_wires, nx, cp->p->x, cp->g_y, cp->g_coef, cp->wx, c->r, c->window, cp->wv, cp->wvf);
+  launch(k_couple_eval, dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s, c->d_wires, nx, cp->p->x,
+         cp->g_y, cp->g_coef, cp->wx, c->r, c->window, cp->wv, cp->wvf);
   if (precision == SBE_PREC_MIXED)
-    k_couple_fftg_f<<<dim3((c->nr_max / 2 + 8) / 8, c->nw), 256, 0, s>>>(c->d_wires, cp->twrf,
-                                                                         cp->wvf, cp->Ek);
+    launch(k_couple_fftg_f, dim3((c->nr_max / 2 + 8) / 8, c->nw), 256, 0, s, c->d_wires, cp->twrf,
+           cp->wvf, cp->Ek);
   else
-    k_couple_fftg<<<dim3((c->nr_max + 7) / 8, c->nw), 256, 0, s>>>(c->d_wires, cp->twr, cp->wv,
-                                                                   cp->Ek);
+    launch(k_couple_fftg, dim3((c->nr_max + 7) / 8, c->nw), 256, 0, s, c->d_wires, cp->twr, cp->wv,
+           cp->Ek);
   return cuda_check(cudaGetLastError(), "couple sample");
 }
 
@@ -436,8 +447,8 @@ int couple_deposit(SbeCouple* cp, cudaStream_t s) {
   SbeCtx* c = cp->ctx;
   const int nx = cp->p->nx;
   launch_splines(wire_batch(cp), c->nw, c->nr_max, s);
-  k_couple_deposit<<<(nx + 63) / 64, 64, 0, s>>>(c->d_wires, c->nw, nx, cp->p->x, cp->wx, c->r,
-                                                   cp->src, cp->w_coef, cp->Pg, cp->rho);
+  launch(k_couple_deposit, (nx + 63) / 64, 64, 0, s, c->d_wires, c->nw, nx, cp->p->x, cp->wx, c->r,
+         cp->src, cp->w_coef, cp->Pg, cp->rho);
   return cuda_check(cudaGetLastError(), "couple deposit");
 }
 
@@ -610,9 +621,9 @@ int sbe_couple_step(SbeCouple* cp, double* P, double* C, double* D, double* E, d
   if ((rc = couple_deposit(cp, s))) return rc;
   const SbeCoupleDesc& d = cp->desc;
   const double jamp = d.src_index >= 0 ? -2.0 * d.E0 / (cp->eta * p->dx) : 0.0;
-  k_couple_current<<<(nx + 255) / 256, 256, 0, s>>>(nx, dt, cp->Pg, cp->Pold, cp->J, cp->step,
-                                                    d.t0, d.src_index, jamp, d.tau, d.w0,
-                                                    d.tpeak);
+  launch(k_couple_current, (nx + 255) / 256, 256, 0, s, nx, dt, cp->Pg, cp->Pold, cp->J, cp->step,
+         d.t0, d.src_index, jamp, d.tau, d.w0,
+         d.tpeak);
   if ((rc = cuda_check(cudaGetLastError(), "couple current"))) return rc;
   if ((rc = sbe_pstd_update_e(p, E, H, reinterpret_cast<double*>(cp->J), dt, stream))) return rc;
   // 5. longitudinal field of the new charge and Px
@@ -621,7 +632,7 @@ int sbe_couple_step(SbeCouple* cp, double* P, double* C, double* D, double* E, d
                              reinterpret_cast<double*>(cp->Pg), Ex, stream)))
       return rc;
   }
-  k_tick<<<1, 1, 0, s>>>(cp->step);
+  launch(k_tick, 1, 1, 0, s, cp->step);
   return cuda_check(cudaGetLastError(), "sbe_couple_step");
 }
 
@@ -696,17 +707,17 @@ int c3_sample(SbeCouple3* cp, const double2* E, int precision, cudaStream_t s) {
   SbeCtx* c = cp->ctx;
   SbePstd3* p = cp->p;
   const int nz = p->n[2];
-  k_c3_lines<<<dim3((nz + 127) / 128, c->nw), 128, 0, s>>>(p->n[0], p->n[1], nz, p->x[0],
-                                                           p->x[1], cp->wxy, E, cp->lines);
+  launch(k_c3_lines, dim3((nz + 127) / 128, c->nw), 128, 0, s, p->n[0], p->n[1], nz, p->x[0],
+         p->x[1], cp->wxy, E, cp->lines);
   launch_splines(line_batch(cp), c->nw, nz, s);
-  k_c3_eval<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(
-      c->d_wires, nz, p->x[2], cp->lines, cp->l_coef, c->r, c->window, cp->wv, cp->wvf);
+  launch(k_c3_eval, dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s, c->d_wires, nz, p->x[2],
+         cp->lines, cp->l_coef, c->r, c->window, cp->wv, cp->wvf);
   if (precision == SBE_PREC_MIXED)
-    k_couple_fftg_f<<<dim3((c->nr_max / 2 + 8) / 8, c->nw), 256, 0, s>>>(c->d_wires, cp->twrf,
-                                                                         cp->wvf, cp->Ek);
+    launch(k_couple_fftg_f, dim3((c->nr_max / 2 + 8) / 8, c->nw), 256, 0, s, c->d_wires, cp->twrf,
+           cp->wvf, cp->Ek);
   else
-    k_couple_fftg<<<dim3((c->nr_max + 7) / 8, c->nw), 256, 0, s>>>(c->d_wires, cp->twr, cp->wv,
-                                                                   cp->Ek);
+    launch(k_couple_fftg, dim3((c->nr_max + 7) / 8, c->nw), 256, 0, s, c->d_wires, cp->twr, cp->wv,
+           cp->Ek);
   return cuda_check(cudaGetLastError(), "couple3 sample");
 }
 
@@ -715,8 +726,8 @@ int c3_deposit(SbeCouple3* cp, double dt, cudaStream_t s) {
   SbePstd3* p = cp->p;
   const int nz = p->n[2];
   launch_splines(wire_batch3(cp), c->nw, c->nr_max, s);
-  k_c3_wire_lines<<<dim3((nz + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, nz, p->x[2], c->r,
-                                                                cp->src, cp->w_coef, cp->dl);
+  launch(k_c3_wire_lines, dim3((nz + 127) / 128, c->nw), 128, 0, s, c->d_wires, nz, p->x[2], c->r,
+         cp->src, cp->w_coef, cp->dl);
   C3Dep a{};
   a.nx = p->n[0];
   a.ny = p->n[1];
@@ -741,7 +752,7 @@ int c3_deposit(SbeCouple3* cp, double dt, cudaStream_t s) {
   a.pol = d.pol;
   a.yg = p->x[1];
   a.zg = p->x[2];
-  k_c3_deposit<<<p->n[0] * p->n[1], 128, 0, s>>>(a);
+  launch(k_c3_deposit, p->n[0] * p->n[1], 128, 0, s, a);
   return cuda_check(cudaGetLastError(), "couple3 deposit");
 }
 
@@ -924,7 +935,7 @@ int sbe_couple3_step(SbeCouple3* cp, double* P, double* C, double* D, double* E,
   if ((rc = pstd3_update_e_from_work(cp->p, reinterpret_cast<double2*>(E),
                                      reinterpret_cast<const double2*>(H), cp->J, dt, s)))
     return rc;
-  k_tick<<<1, 1, 0, s>>>(cp->step);
+  launch(k_tick, 1, 1, 0, s, cp->step);
   return cuda_check(cudaGetLastError(), "sbe_couple3_step");
 }
 

@@ -59,6 +59,7 @@ void f64_free(SbeCtx* c) {
 // of the sheared rows 2 dd, 2 dd + 1 (dd = row - column + Nk - 1).  One warp per diagonal.
 __global__ void __launch_bounds__(128) k_f64_diag(int nk, const double2* P, const double2* C,
                                                   const double2* D, double2* tr, int* es) {
+  pdl_enter();
   const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= 2 * nk - 1) return;
   const int d = i - (nk - 1), which = blockIdx.y, b = blockIdx.z;   // column - row
@@ -111,6 +112,7 @@ __host__ __device__ inline bool shear_live(int nk, int t0, int dd0) {
 __global__ void __launch_bounds__(256) k_f64_shear(int nk, int nw, const double2* P,
                                                    const double2* C, const double2* D,
                                                    const int* es, __half* dst, long long slab) {
+  pdl_enter();
   __shared__ double2 tile[63][33];
   const int n = blockIdx.z / nw, b = blockIdx.z % nw;
   const int t0 = blockIdx.x * 32, dd0 = (shear_first(nk, t0) + blockIdx.y) * 32;
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(256) k_f64_shear(int nk, int nw, const double2
 // ee, hh), with one exponent per wire and n.  vs: 3 x Nk per wire (by |t - t'|).
 __global__ void __launch_bounds__(256) k_f64_toeplitz(int nk, int nw, const double* vs, __half* dst,
                                                       int* et, long long slab) {
+  pdl_enter();
   const int n = blockIdx.y, b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double* v = vs + ((long long)b * 3 + n) * nk;
   __shared__ unsigned long long red[8];
@@ -196,6 +199,7 @@ struct HBuild {
 };
 
 __global__ void __launch_bounds__(128) k_f64_hbuild(const __grid_constant__ HBuild a) {
+  pdl_enter();
   const int nk = a.nk, k2 = blockIdx.x * 128 + threadIdx.x, k1 = blockIdx.y, b = blockIdx.z;
   if (k2 >= nk) return;
   const long long mb = (long long)b * nk * nk, o = (long long)k1 * nk + k2;
@@ -279,6 +283,7 @@ struct Finish {
 };
 
 __global__ void __launch_bounds__(256) k_f64_finish(const __grid_constant__ Finish a) {
+  pdl_enter();
   __shared__ double2 ht[32][33];
   const int nk = a.nk, which = blockIdx.z / a.nw + a.first, b = blockIdx.z % a.nw;
   const int m0 = blockIdx.y * 32, n0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
@@ -434,7 +439,7 @@ static int exchange(int nk, int nw, const double2* P, const double2* C, const do
       if (shear_live(nk, 32 * i, 32 * j)) cnt = j - shear_first(nk, 32 * i) + 1;
     ny = std::max(ny, cnt);
   }
-  k_f64_shear<<<dim3(nb, ny, 3 * nw), 256, 0, s>>>(nk, nw, P, C, D, es, sp, sl_s);
+  launch(k_f64_shear, dim3(nb, ny, 3 * nw), 256, 0, s, nk, nw, P, C, D, es, sp, sl_s);
   f64s::Job jobs[3];
   for (int n = 0; n < 3; ++n) {
     f64s::Job& j = jobs[n];
@@ -589,8 +594,8 @@ bool f64_prepare(SbeCtx* c, cudaStream_t s) {
 // Per-step operands: the Toeplitz planes of the screened interaction.
 void f64_step_operands(SbeCtx* c, cudaStream_t s) {
   for (auto& m : work_of(c)->b)
-    k_f64_toeplitz<<<dim3((m.nk + 7) / 8, 3, m.nw), 256, 0, s>>>(m.nk, m.nw, c->vs + 3 * m.bv, m.tp,
-                                                               m.et, m.sl_m);
+    launch(k_f64_toeplitz, dim3((m.nk + 7) / 8, 3, m.nw), 256, 0, s, m.nk, m.nw, c->vs + 3 * m.bv,
+           m.tp, m.et, m.sl_m);
 }
 
 static void state_forms(f64s::SliceArgs& a, const FormSet& F, const double2* P, const double2* C,
@@ -623,8 +628,8 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       const long long mm = (long long)nk * nk, o = m.bm + w0 * mm, vo = m.bv + (long long)w0 * nk;
       const long long ro = m.br + (long long)w0 * m.nr;
       const FormSet F{m.pl, m.ef, nk, g, m.sl_m};
-      k_f64_diag<<<dim3((2 * nk - 1 + 3) / 4, 3, g), 128, 0, s>>>(nk, P + o, C + o, D + o,
-                                                               c->tr + 4 * vo, m.es);
+      launch(k_f64_diag, dim3((2 * nk - 1 + 3) / 4, 3, g), 128, 0, s, nk, P + o, C + o, D + o,
+             c->tr + 4 * vo, m.es);
       f64s::SliceArgs a = slice_args(F);
       state_forms(a, F, P + o, C + o, D + o);
       launch_f64_slice(a, 6, s);
@@ -650,7 +655,7 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       h.Heh = c->Heh + o;
       h.Hee = c->Hee + o;
       h.Hhh = c->Hhh + o;
-      k_f64_hbuild<<<dim3((nk + 127) / 128, nk, g), 128, 0, s>>>(h);
+      launch(k_f64_hbuild, dim3((nk + 127) / 128, nk, g), 128, 0, s, h);
       const double2* hm[3] = {c->Heh + o, c->Hee + o, c->Hhh + o};
       a = slice_args(F);
       int nf = 0, alias[F_N];
@@ -685,7 +690,7 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
         f.acc[i] = c->kacc + i * n + o;
         f.xs[i] = c->xs + i * n + o;
       }
-      k_f64_finish<<<dim3((nk + 31) / 32, (nk + 31) / 32, 3 * g), dim3(32, 8), 0, s>>>(f);
+      launch(k_f64_finish, dim3((nk + 31) / 32, (nk + 31) / 32, 3 * g), dim3(32, 8), 0, s, f);
     }
   return cuda_check(cudaGetLastError(), "f64 rhs");
 }
@@ -700,6 +705,7 @@ __global__ void __launch_bounds__(512) k_f64_src_reduce(const WireDev* wires, in
                                                         int parts, const double2* E,
                                                         const double* G, const double* win,
                                                         double2* src) {
+  pdl_enter();
   __shared__ double red[6][32][17];
   const int b = blockIdx.y, tx = threadIdx.x, ty = threadIdx.y, r = blockIdx.x * 16 + tx;
   const long long per = (long long)nk * nr, cs = (long long)nw * per;
@@ -792,8 +798,8 @@ int f64_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D,
       launch_f64_slice(a, 3, s);
       const int rc = launch_f64_gemm(jobs, 3, s);
       if (rc) return rc;
-      k_f64_src_reduce<<<dim3((nr + 15) / 16, g), dim3(16, 32), 0, s>>>(
-          m.dw + w0, nk, nr, g, m.sparts, c->expikr + ko, m.part, c->window + ro, src + 5 * ro);
+      launch(k_f64_src_reduce, dim3((nr + 15) / 16, g), dim3(16, 32), 0, s, m.dw + w0, nk, nr, g,
+             m.sparts, c->expikr + ko, m.part, c->window + ro, src + 5 * ro);
     }
   return cuda_check(cudaGetLastError(), "f64 sources");
 }
@@ -906,7 +912,7 @@ bool f64_rhs_single(int which, int nk, const double2* C, const double2* D, const
   f.gamE = gamE;
   f.gamH = gamH;
   f.out[which] = out;
-  k_f64_finish<<<dim3((nk + 31) / 32, (nk + 31) / 32, 1), dim3(32, 8), 0, s>>>(f);
+  launch(k_f64_finish, dim3((nk + 31) / 32, (nk + 31) / 32, 1), dim3(32, 8), 0, s, f);
   *rc = cuda_check(cudaGetLastError(), "f64 rhs single");
   return true;
 }
@@ -927,8 +933,8 @@ bool f64_calch_single(int nk, const double2* Meh, const double2* Wee, const doub
   launch_vq_from_vc(nk, VC, vq, s);
   // blocks of the sheared planes outside the band are not written by the pass
   cudaMemsetAsync(sp, 0, sizeof(__half) * 3 * NS * ss, s);
-  k_f64_diag<<<dim3((2 * nk - 1 + 3) / 4, 3, 1), 128, 0, s>>>(nk, P, C, D, tr, es);
-  k_f64_toeplitz<<<dim3((nk + 7) / 8, 3, 1), 256, 0, s>>>(nk, 1, vq, tp, et, sl);
+  launch(k_f64_diag, dim3((2 * nk - 1 + 3) / 4, 3, 1), 128, 0, s, nk, P, C, D, tr, es);
+  launch(k_f64_toeplitz, dim3((nk + 7) / 8, 3, 1), 256, 0, s, nk, 1, vq, tp, et, sl);
   *rc = exchange(nk, 1, P, C, D, tp, sl, et, nk, sp, es, sl, ss, xsh, s);
   if (*rc) return true;
   HBuild h{};
@@ -952,7 +958,7 @@ bool f64_calch_single(int nk, const double2* Meh, const double2* Wee, const doub
   h.Heh = Heh;
   h.Hee = Hee;
   h.Hhh = Hhh;
-  k_f64_hbuild<<<dim3((nk + 127) / 128, nk, 1), 128, 0, s>>>(h);
+  launch(k_f64_hbuild, dim3((nk + 127) / 128, nk, 1), 128, 0, s, h);
   *rc = cuda_check(cudaGetLastError(), "sbe_calch");
   return true;
 }

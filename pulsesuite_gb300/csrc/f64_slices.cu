@@ -21,6 +21,7 @@ __device__ int g_err;   // a bounded wait gave up
 // are read again (from L2).  HBM bound: 16 B read and 32 B written per element.
 template <int KB>
 __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ SliceArgs a) {
+  pdl_enter();
   const Form& f = a.f[blockIdx.y];
   const int kdim = a.kdim, ld = a.ld, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -251,6 +252,7 @@ __device__ __forceinline__ void add_acc67(unsigned long long* run, const uint32_
 // fewer conversions, 340 with the drain in 16-column steps (no spills) and 32-byte stores, of
 // which the MMAs alone take 304.
 __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__ Launch L) {
+  pdl_enter();
   using namespace tc;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -537,9 +539,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
 void launch_f64_slice(const f64s::SliceArgs& a, int nforms, cudaStream_t s) {
   const dim3 grid((a.rows + 7) / 8, nforms, a.batch);
   if (f64s::k_blocks(a.kdim) <= 8)
-    f64s::k_f64_slice<1><<<grid, 256, 0, s>>>(a);
+    launch(f64s::k_f64_slice<1>, grid, 256, 0, s, a);
   else
-    f64s::k_f64_slice<2><<<grid, 256, 0, s>>>(a);
+    launch(f64s::k_f64_slice<2>, grid, 256, 0, s, a);
 }
 
 static int sm_count() {
@@ -574,7 +576,7 @@ int launch_f64_gemm(const f64s::Job* jobs, int njobs, cudaStream_t s) {
   if (nt > 0x7FFFFFFF) return fail(SBE_ERR_ARG, "f64 gemm: too many tiles");
   L.base[njobs] = (int)nt;
   const int grid = (int)std::min<long long>(nt, sm_count());
-  f64s::k_f64_gemm<<<grid, f64s::THREADS, f64s::SMEM, s>>>(L);
+  launch(f64s::k_f64_gemm, grid, f64s::THREADS, f64s::SMEM, s, L);
   return cuda_check(cudaGetLastError(), "f64 gemm launch");
 }
 

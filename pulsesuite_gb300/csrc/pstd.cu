@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kThreads) k_pstd_cols_fwd(int nx, int n1, int 
                                                             const double2* __restrict__ in1,
                                                             double2* __restrict__ Y,
                                                             const double2* __restrict__ tw) {
+  pdl_enter();
   extern __shared__ double2 sm[];
   double2* a = sm;
   double2* b = sm + n1 * kCols;
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(kThreads) k_pstd_rows(int nx, int n1, int n2, 
                                                         const double* __restrict__ q,
                                                         double small, double inv_eps,
                                                         const double2* __restrict__ tw) {
+  pdl_enter();
   extern __shared__ double2 sm[];
   const int nfl = kind == 1 ? 2 : 1;
   const int f0 = kind == 1 ? 0 : blockIdx.y;
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(kThreads) k_pstd_cols_inv(int nx, int n1, int 
                                                             const double2* __restrict__ tw,
                                                             const double* __restrict__ mask,
                                                             PstdEpiArgs e) {
+  pdl_enter();
   extern __shared__ double2 sm[];
   double2* a = sm;
   double2* b = sm + n1 * kCols;
@@ -228,17 +231,17 @@ int pstd_pipeline(SbePstd* p, int kind, const double2* in0, const double2* in1, 
   const int nx = p->nx, n1 = p->n1, n2 = p->n2;
   const size_t smA = 2 * (size_t)n1 * kCols * sizeof(double2);
   const size_t smB = 2 * (size_t)(kind == 1 ? 2 : 1) * kRows * n2 * sizeof(double2);
-  k_pstd_cols_fwd<<<dim3(n2 / kCols, nf), kThreads, smA, s>>>(nx, n1, n2, in0, in1, p->work,
-                                                              p->tw);
+  launch(k_pstd_cols_fwd, dim3(n2 / kCols, nf), kThreads, smA, s, nx, n1, n2, in0, in1, p->work,
+         p->tw);
   // rhoPJ.py:779: small = (qx[1] - qx[0]) / 1e4, with q[0] = 0 and q[1] = dq
   const double dq = 2.0 * kPi / ((double)nx * p->dx);
   const double sm_q = dq / 1e4;
   const double inv_eps = 1.0 / (kEps0 * p->epsr);
-  k_pstd_rows<<<dim3(n1 / kRows, kind == 1 ? 1 : nf), kThreads, smB, s>>>(
-      nx, n1, n2, kind, p->work, p->q, sm_q, inv_eps, p->tw);
+  launch(k_pstd_rows, dim3(n1 / kRows, kind == 1 ? 1 : nf), kThreads, smB, s, nx, n1, n2, kind,
+         p->work, p->q, sm_q, inv_eps, p->tw);
   const int nout = kind == 1 ? 1 : nf;
-  k_pstd_cols_inv<<<dim3(n2 / kCols, nout), kThreads, smA, s>>>(nx, n1, n2, p->work, p->tw,
-                                                               p->mask, epi);
+  launch(k_pstd_cols_inv, dim3(n2 / kCols, nout), kThreads, smA, s, nx, n1, n2, p->work, p->tw,
+         p->mask, epi);
   return cuda_check(cudaGetLastError(), "pstd pipeline");
 }
 

@@ -146,6 +146,7 @@ struct Upd {
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_line_pass(Pass P, const double2* in64, T* W,
                                                         Upd U) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sa = reinterpret_cast<T*>(smraw);
   const int tl = P.tl, n = P.n;
@@ -236,6 +237,7 @@ __global__ void __launch_bounds__(kThreads) k_line_pass(Pass P, const double2* i
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_x_curl(Pass P, T* W, const double* qy,
                                                      const double* qz, const double* qx, int nz) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sa = reinterpret_cast<T*>(smraw);
   const int tl = P.tl, n = P.n;
@@ -469,6 +471,7 @@ __device__ __forceinline__ void plane_forward(const PlaneArgs& A, float2* a, con
 // (FP64 -> FP32 on the integer pipe: the FP64 pipe is ~1/64 of the FP32 rate here)
 __global__ void __launch_bounds__(kPlaneThreads, 1) k_plane_fwd(PlaneArgs A, const double2* F,
                                                                 float2* W) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* a = reinterpret_cast<float2*>(smraw);
   float2* sty = a + plane_slots(A.P, A.lgz);
@@ -502,6 +505,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) k_plane_fwd(PlaneArgs A, con
 __global__ void __launch_bounds__(kXThreads) k_x_curl_ip(PlaneArgs A, float2* W, int lgx, int tl,
                                                          const float2* twx, const float2* qbx,
                                                          const float2* qby, const float2* qbz) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = 1 << lgx, w3 = 3 * tl;
   float2* a = reinterpret_cast<float2*>(smraw);
@@ -559,6 +563,7 @@ __global__ void __launch_bounds__(kXThreads) k_x_curl_ip(PlaneArgs A, float2* W,
 // only where it is not 1.
 __global__ void __launch_bounds__(kPlaneThreads, 1) k_plane_inv(PlaneArgs A, float2* W, Upd U,
                                                                 int fwd_next) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* a = reinterpret_cast<float2*>(smraw);
   float2* sty = a + plane_slots(A.P, A.lgz);
@@ -643,7 +648,7 @@ int run_line_pass(SbePstd3* p, int axis, int dir, int nf, const double2* in64, T
   P.lgtl = ilog2i(P.tl);
   const size_t smem = 2 * (size_t)P.n * P.tl * sizeof(T);
   const dim3 grid(lines / P.tl, nf);
-  k_line_pass<T><<<grid, kThreads, smem, s>>>(P, in64, W, U);
+  launch(k_line_pass<T>, grid, kThreads, smem, s, P, in64, W, U);
   return cuda_check(cudaGetLastError(), "pstd3 line pass");
 }
 
@@ -660,7 +665,7 @@ int run_x_curl(SbePstd3* p, T* W, cudaStream_t s) {
   P.tl = lines_per_block(P.n, 3, sizeof(T), P.inner);
   P.lgtl = ilog2i(P.tl);
   const size_t smem = 2 * 3 * (size_t)P.n * P.tl * sizeof(T);
-  k_x_curl<T><<<P.s / P.tl, kThreads, smem, s>>>(P, W, p->q[1], p->q[2], p->q[0], p->n[2]);
+  launch(k_x_curl<T>, P.s / P.tl, kThreads, smem, s, P, W, p->q[1], p->q[2], p->q[0], p->n[2]);
   return cuda_check(cudaGetLastError(), "pstd3 curl pass");
 }
 
@@ -737,8 +742,8 @@ int x_lines(const SbePstd3* p) {
 
 int plane_pass_a(SbePstd3* p, const double2* F, cudaStream_t s) {
   const PlaneArgs A = plane_args(p);
-  k_plane_fwd<<<dim3(A.nx, 3), kPlaneThreads, plane_smem(A), s>>>(A, F,
-                                                                  static_cast<float2*>(p->work));
+  launch(k_plane_fwd, dim3(A.nx, 3), kPlaneThreads, plane_smem(A), s, A, F,
+         static_cast<float2*>(p->work));
   return cuda_check(cudaGetLastError(), "pstd3 plane pass");
 }
 
@@ -746,15 +751,15 @@ int plane_pass_b(SbePstd3* p, cudaStream_t s) {
   const PlaneArgs A = plane_args(p);
   const int tl = x_lines(p), nx = p->n[0];
   const size_t smem = sizeof(float2) * ((size_t)3 * nx * tl + (nx >> 1));
-  k_x_curl_ip<<<(unsigned)(A.P / tl), kXThreads, smem, s>>>(
-      A, static_cast<float2*>(p->work), ilog2i(nx), tl, p->twf[0], p->qb[0], p->qb[1], p->qb[2]);
+  launch(k_x_curl_ip, (unsigned)(A.P / tl), kXThreads, smem, s, A, static_cast<float2*>(p->work),
+         ilog2i(nx), tl, p->twf[0], p->qb[0], p->qb[1], p->qb[2]);
   return cuda_check(cudaGetLastError(), "pstd3 x pass");
 }
 
 int plane_pass_c(SbePstd3* p, const Upd& U, int fwd_next, cudaStream_t s) {
   const PlaneArgs A = plane_args(p);
-  k_plane_inv<<<dim3(A.nx, 3), kPlaneThreads, plane_smem(A), s>>>(
-      A, static_cast<float2*>(p->work), U, fwd_next);
+  launch(k_plane_inv, dim3(A.nx, 3), kPlaneThreads, plane_smem(A), s, A,
+         static_cast<float2*>(p->work), U, fwd_next);
   return cuda_check(cudaGetLastError(), "pstd3 plane pass");
 }
 

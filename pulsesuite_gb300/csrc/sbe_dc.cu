@@ -25,6 +25,7 @@ namespace {
 // index 0 of the wire's x component)
 __global__ void __launch_bounds__(256) k_dc_kernel(const WireDev* wires, const double2* Ek,
                                                    double dt, double2* dcs) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   const int n = W.nk, m = blockIdx.x;
   if (m >= n || !(W.flags & SBE_F_DCTRANS)) return;
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(256) k_dc_kernel(const WireDev* wires, const d
 // S of every wire: the circulant for DCTrans with LF, the identity otherwise (the
 // GEMMs then leave the matrix unchanged exactly)
 __global__ void k_dc_smat(const WireDev* wires, const double2* dcs, double2* S) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.z];
   const int n = W.nk;
   const int b = blockIdx.x * blockDim.x + threadIdx.x, a = blockIdx.y;
@@ -74,6 +76,7 @@ __global__ void k_dc_smat(const WireDev* wires, const double2* dcs, double2* S) 
 // LF off: the diagonal alone, d'[a] = sum_c s(a - c) X[c][c] (into tmp)
 __global__ void k_dc_diag(const WireDev* wires, const double2* dcs, const double2* X,
                           double2* tmp) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   const int n = W.nk, a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n || !(W.flags & SBE_F_DCTRANS) || (W.flags & SBE_F_LF)) return;
@@ -85,6 +88,7 @@ __global__ void k_dc_diag(const WireDev* wires, const double2* dcs, const double
 }
 
 __global__ void k_dc_diag_store(const WireDev* wires, const double2* tmp, double2* X) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   const int n = W.nk, a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n || !(W.flags & SBE_F_DCTRANS) || (W.flags & SBE_F_LF)) return;
@@ -97,7 +101,7 @@ void launch_dc_transport(SbeCtx* c, double2* P, double2* C, double2* D, const do
                          double dt, cudaStream_t s) {
   if (!any_dc(c)) return;
   const int nk = c->nk_max;
-  k_dc_kernel<<<dim3(nk, c->nw), 256, 0, s>>>(c->d_wires, Ek, dt, c->dcs);
+  launch(k_dc_kernel, dim3(nk, c->nw), 256, 0, s, c->d_wires, Ek, dt, c->dcs);
   bool lf = false, nolf = false;
   for (const auto& W : c->wires)
     if (W.flags & SBE_F_DCTRANS) (W.flags & SBE_F_LF ? lf : nolf) = true;
@@ -108,7 +112,7 @@ void launch_dc_transport(SbeCtx* c, double2* P, double2* C, double2* D, const do
     // only the wires with DCTrans and LF take part (the others keep X untouched)
     double2* S = c->dA;
     double2* T = c->dP;
-    k_dc_smat<<<dim3((nk + 127) / 128, nk, c->nw), 128, 0, s>>>(c->d_wires, c->dcs, S);
+    launch(k_dc_smat, dim3((nk + 127) / 128, nk, c->nw), 128, 0, s, c->d_wires, c->dcs, S);
     for (int i = 0; i < 3; ++i) {
       GemmBatch b{};
       b.nterms = 1;
@@ -128,8 +132,8 @@ void launch_dc_transport(SbeCtx* c, double2* P, double2* C, double2* D, const do
     double2* tmp[3] = {c->ne, c->nh, reinterpret_cast<double2*>(c->wrate)};
     const dim3 g((nk + 127) / 128, c->nw);
     for (int i = 0; i < 3; ++i) {
-      k_dc_diag<<<g, 128, 0, s>>>(c->d_wires, c->dcs, X[i], tmp[i]);
-      k_dc_diag_store<<<g, 128, 0, s>>>(c->d_wires, tmp[i], X[i]);
+      launch(k_dc_diag, g, 128, 0, s, c->d_wires, c->dcs, X[i], tmp[i]);
+      launch(k_dc_diag_store, g, 128, 0, s, c->d_wires, tmp[i], X[i]);
     }
   }
 }

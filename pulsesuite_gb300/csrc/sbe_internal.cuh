@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/sbe_gb300.h"
+#include "launch.cuh"
 
 namespace sbe {
 

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(256) k_mbc_rates64(const WireDev* wires, int w
                                                      const double* vs, const double* Ee,
                                                      const double* Eh, double* wrate,
                                                      int all) {
+  pdl_enter();
   const WireDev W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int n = W.nk;
   const int row = blockIdx.x + 1;   // 1-based k (electrons) or kp (holes)
@@ -255,6 +256,7 @@ template <bool LZ>
 __global__ void __launch_bounds__(256) k_mbc_rates32(const WireDev* wires, int w_only,
                                                      const double2* nev, const double2* nhv,
                                                      const double* vs, double* wrate, int all) {
+  pdl_enter();
   const WireDev W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int n = W.nk;
   const int row = blockIdx.x + 1;
@@ -501,18 +503,18 @@ void launch_mbc_rates(SbeCtx* c, int w_only, cudaStream_t s, bool all, bool fp32
       if (w_only < 0 || w == w_only) (c->wires[w].flags & SBE_F_LORENTZ ? lor : gauss) = true;
     const dim3 grid(nk, w_only >= 0 ? 1 : c->nw, 2);
     if (gauss)
-      k_mbc_rates32<false><<<grid, 256, smf, s>>>(c->d_wires, w_only, c->ne, c->nh, c->vs,
-                                                   c->wrate, all ? 1 : 0);
+      launch(k_mbc_rates32<false>, grid, 256, smf, s, c->d_wires, w_only, c->ne, c->nh, c->vs,
+             c->wrate, all ? 1 : 0);
     if (lor)
-      k_mbc_rates32<true><<<grid, 256, smf, s>>>(c->d_wires, w_only, c->ne, c->nh, c->vs,
-                                                  c->wrate, all ? 1 : 0);
+      launch(k_mbc_rates32<true>, grid, 256, smf, s, c->d_wires, w_only, c->ne, c->nh, c->vs,
+             c->wrate, all ? 1 : 0);
     return;
   }
   const size_t sm = sizeof(double) * (2 * (size_t)(nk + 1) + 3 * (size_t)nk);
   if (sm > 48 * 1024)
     cudaFuncSetAttribute(k_mbc_rates64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_mbc_rates64<<<dim3(nk, w_only >= 0 ? 1 : c->nw, 2), 256, sm, s>>>(
-      c->d_wires, w_only, c->ne, c->nh, c->vs, c->Ee, c->Eh, c->wrate, all ? 1 : 0);
+  launch(k_mbc_rates64, dim3(nk, w_only >= 0 ? 1 : c->nw, 2), 256, sm, s, c->d_wires, w_only, c->ne,
+         c->nh, c->vs, c->Ee, c->Eh, c->wrate, all ? 1 : 0);
 }
 
 }  // namespace sbe

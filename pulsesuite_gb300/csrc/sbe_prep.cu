@@ -14,6 +14,7 @@ namespace sbe {
 // forms ne, nh, n1D and the screened vs(d) = v0(d)/eps(d).
 __global__ void k_extract_diag(const WireDev* wires, const double2* C, const double2* D,
                                double2* ne, double2* nh) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.x];
   const int nk = W.nk;
   for (int k = threadIdx.x; k < nk; k += blockDim.x) {
@@ -23,7 +24,7 @@ __global__ void k_extract_diag(const WireDev* wires, const double2* C, const dou
 }
 
 void launch_extract_diag(SbeCtx* c, const double2* C, const double2* D, cudaStream_t s) {
-  k_extract_diag<<<c->nw, 256, 0, s>>>(c->d_wires, C, D, c->ne, c->nh);
+  launch(k_extract_diag, c->nw, 256, 0, s, c->d_wires, C, D, c->ne, c->nh);
 }
 
 // Blocks (kScreenBlocks per wire) each form n1D in the same order and take every
@@ -37,6 +38,7 @@ __global__ void __launch_bounds__(256) k_screen(const WireDev* wires, int w_only
                                                 const double* chi, const double* qeh, double2* ne,
                                                 double2* nh, double* occd, float* occf, double* eps,
                                                 double* vs, double* vph) {
+  pdl_enter();
   const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int nk = W.nk, bx = blockIdx.x;
   __shared__ double red[256];
@@ -89,9 +91,8 @@ __global__ void __launch_bounds__(256) k_screen(const WireDev* wires, int w_only
 }
 
 static void screen(SbeCtx* c, int w_only, const double2* C, const double2* D, cudaStream_t s) {
-  k_screen<<<dim3(kScreenBlocks, w_only >= 0 ? 1 : c->nw), 256, 0, s>>>(
-      c->d_wires, w_only, C, D, c->v0, c->chi, c->qeh, c->ne, c->nh, c->occd, c->occf, c->eps, c->vs,
-      c->vph);
+  launch(k_screen, dim3(kScreenBlocks, w_only >= 0 ? 1 : c->nw), 256, 0, s, c->d_wires, w_only, C,
+         D, c->v0, c->chi, c->qeh, c->ne, c->nh, c->occd, c->occf, c->eps, c->vs, c->vph);
 }
 
 void launch_screen(SbeCtx* c, int w_only, cudaStream_t s) { screen(c, w_only, nullptr, nullptr, s); }
@@ -104,6 +105,7 @@ void launch_prep_scalar(SbeCtx* c, const double2* C, const double2* D, cudaStrea
 // Expand to the reference's (Nk, Nk, 3) VC and (Nk, Nk) E1D of wire w.
 __global__ void k_expand_vc(const WireDev* wires, int w, const double* vs, const double* eps,
                             double* VC, double* E1D) {
+  pdl_enter();
   const WireDev W = wires[w];
   int k2 = blockIdx.x * blockDim.x + threadIdx.x;
   int k1 = blockIdx.y;
@@ -117,7 +119,7 @@ __global__ void k_expand_vc(const WireDev* wires, int w, const double* vs, const
 
 void launch_expand_vc(SbeCtx* c, int w, double* VC, double* E1D, cudaStream_t s) {
   int nk = c->wires[w].nk;
-  k_expand_vc<<<dim3((nk + 127) / 128, nk), 128, 0, s>>>(c->d_wires, w, c->vs, c->eps, VC, E1D);
+  launch(k_expand_vc, dim3((nk + 127) / 128, nk), 128, 0, s, c->d_wires, w, c->vs, c->eps, VC, E1D);
 }
 
 // ---------------------------------------------------------------------------
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(128) k_gamma(const WireDev* wires, int w_only,
                                                const double2* nh, const double* vs, const int* iq,
                                                const int* maps, const double* xeh, double* gamE,
                                                double* gamH) {
+  pdl_enter();
   const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int nk = W.nk, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = blockIdx.x * 4 + warp;
@@ -206,8 +209,8 @@ __global__ void __launch_bounds__(128) k_gamma(const WireDev* wires, int w_only,
 }
 
 void launch_gamma(SbeCtx* c, int w_only, cudaStream_t s) {
-  k_gamma<<<dim3((c->nk_max + 3) / 4, w_only >= 0 ? 1 : c->nw), 128, 0, s>>>(
-      c->d_wires, w_only, c->ne, c->nh, c->vs, c->iq, c->maps, c->xeh, c->gamE, c->gamH);
+  launch(k_gamma, dim3((c->nk_max + 3) / 4, w_only >= 0 ? 1 : c->nw), 128, 0, s, c->d_wires, w_only,
+         c->ne, c->nh, c->vs, c->iq, c->maps, c->xeh, c->gamE, c->gamH);
 }
 
 // ---------------------------------------------------------------------------
@@ -229,6 +232,7 @@ void launch_gamma(SbeCtx* c, int w_only, cudaStream_t s) {
 // error of Dh at Nk = 128 from 3.9e-14 to 2.9e-15.
 __global__ void k_occd(const WireDev* wires, int w_only, const double2* ne, const double2* nh,
                        double* occd) {
+  pdl_enter();
   const WireDev& W = wires[w_only];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= W.nk) return;
@@ -250,6 +254,7 @@ constexpr int kDephP = 64;   // p per shared-memory chunk
 
 template <int NW>
 __global__ void __launch_bounds__(256) k_offdiag_D64(const Deph64 a) {
+  pdl_enter();
   const int q = blockIdx.y + 1, which = blockIdx.z, k0 = blockIdx.x * 32;
   const int w0 = a.w_only >= 0 ? a.w_only : a.wl[0];
   const WireDev& W0 = a.wires[w0];
@@ -389,7 +394,7 @@ static void deph64_launch(const Deph64& a, int nk, cudaStream_t s) {
                                 (int)deph64_smem(NW, 4096)) == cudaSuccess;
   }();
   (void)raised;
-  k_offdiag_D64<NW><<<dim3((nk + 31) / 32, nk - 1, 2), 256, deph64_smem(NW, nk), s>>>(a);
+  launch(k_offdiag_D64<NW>, dim3((nk + 31) / 32, nk - 1, 2), 256, deph64_smem(NW, nk), s, a);
 }
 
 // FP32 version of the off-diagonal dephasing sums for the mixed-precision path.
@@ -427,6 +432,7 @@ __global__ void __launch_bounds__(128) k_offdiag_D32(const WireDev* wires, const
                                                      const float* occf,
                                                      const float* dconst, const float* dpre,
                                                      double* De, double* Dh) {
+  pdl_enter();
   const int wi = wl[blockIdx.z >> 1], which = blockIdx.z & 1;   // 0 De, 1 Dh
   const WireDev& W = wires[wi];
   const int nk = W.nk;
@@ -583,6 +589,7 @@ __global__ void __launch_bounds__(128, 2) k_offdiag_D32g(const WireDev* wires, c
                                                       int nwl, const float* occf,
                                                       const float* dconst, const float* dpre,
                                                       double* De, double* Dh) {
+  pdl_enter();
   constexpr int PC = 32;   // p per shared-memory chunk
   const int which = blockIdx.z;
   const WireDev& W0 = wires[wl[0]];
@@ -772,6 +779,7 @@ __global__ void __launch_bounds__(128, 2) k_offdiag_D32g(const WireDev* wires, c
 // and per |q| the prefactors V_aa(q)^2 / (hbar b_aa) and V_ab(q)^2 / (hbar b_ab)
 // (D = (pi/hbar) V^2 Lorentz = V^2 / (hbar b) / (1 + u^2)).
 __global__ void k_deph_consts(const WireDev* wires, const double* vs, float* dconst, float* dpre) {
+  pdl_enter();
   const int wi = blockIdx.y >> 1, which = blockIdx.y & 1;
   const WireDev& W = wires[wi];
   const int nk = W.nk;
@@ -797,8 +805,8 @@ __global__ void k_deph_consts(const WireDev* wires, const double* vs, float* dco
 
 void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaStream_t s) {
   if (fp32 && w_only < 0 && !g3) {
-    k_deph_consts<<<dim3((c->nk_max + 127) / 128, 2 * c->nw), 128, 0, s>>>(c->d_wires, c->vs,
-                                                                          c->dconst, c->dpre);
+    launch(k_deph_consts, dim3((c->nk_max + 127) / 128, 2 * c->nw), 128, 0, s, c->d_wires, c->vs,
+           c->dconst, c->dpre);
     // groups of 4 or more wires share the Lorentzian factors (chunks of up to 16
     // wires); the other wires take the per-wire kernel, one launch each
     for (const auto& g : c->dgroups) {
@@ -806,8 +814,8 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
       if (g.second < 4) {
         const size_t sm1 = sizeof(float) * 8 * (size_t)gk;
         for (int i = 0; i < g.second; ++i)
-          k_offdiag_D32<<<dim3((gk + 511) / 512, gk + 1, 2), 128, sm1, s>>>(
-              c->d_wires, c->dwl + g.first + i, c->occf, c->dconst, c->dpre, c->De, c->Dh);
+          launch(k_offdiag_D32, dim3((gk + 511) / 512, gk + 1, 2), 128, sm1, s, c->d_wires,
+                 c->dwl + g.first + i, c->occf, c->dconst, c->dpre, c->De, c->Dh);
         continue;
       }
       const dim3 grid((gk + 511) / 512, gk + 1, 2);   // 128 threads x 4 k
@@ -816,20 +824,20 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
         const int* wl = c->dwl + g.first + o;
         if (n <= 8) {
           const size_t sm = sizeof(float) * (2 * 32 * 8 + 2 * (size_t)gk);
-          k_offdiag_D32g<8, 4><<<grid, 128, sm, s>>>(c->d_wires, wl, n, c->occf, c->dconst,
-                                                      c->dpre, c->De, c->Dh);
+          launch(k_offdiag_D32g<8, 4>, grid, 128, sm, s, c->d_wires, wl, n, c->occf, c->dconst,
+                 c->dpre, c->De, c->Dh);
         } else {
           const size_t sm = sizeof(float) * (2 * 32 * 16 + 2 * (size_t)gk);
-          k_offdiag_D32g<16, 4><<<grid, 128, sm, s>>>(c->d_wires, wl, n, c->occf, c->dconst,
-                                                       c->dpre, c->De, c->Dh);
+          launch(k_offdiag_D32g<16, 4>, grid, 128, sm, s, c->d_wires, wl, n, c->occf, c->dconst,
+                 c->dpre, c->De, c->Dh);
         }
       }
     }
     return;
   }
   if (w_only >= 0)   // the caller's occupations; a step's come with the preparation
-    k_occd<<<(c->wires[w_only].nk + 127) / 128, 128, 0, s>>>(c->d_wires, w_only, c->ne, c->nh,
-                                                            c->occd);
+    launch(k_occd, (c->wires[w_only].nk + 127) / 128, 128, 0, s, c->d_wires, w_only, c->ne, c->nh,
+           c->occd);
   Deph64 a{};
   a.wires = c->d_wires;
   a.w_only = w_only;
@@ -871,6 +879,7 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
 // B[ke,j] = De[j-ke+Nk][ke] and the j = row entry removed (undel[q=0] = 0).
 __global__ void k_offdiag_AB(const WireDev* wires, int w_only, const double* De,
                              const double* Dh, double2* A, double2* B) {
+  pdl_enter();
   int wi = (w_only >= 0) ? w_only : blockIdx.z;
   const WireDev W = wires[wi];
   int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -886,7 +895,7 @@ __global__ void k_offdiag_AB(const WireDev* wires, int w_only, const double* De,
 
 void launch_offdiag_AB(SbeCtx* c, int w_only, cudaStream_t s) {
   dim3 g((c->nk_max + 127) / 128, c->nk_max, w_only >= 0 ? 1 : c->nw);
-  k_offdiag_AB<<<g, 128, 0, s>>>(c->d_wires, w_only, c->De, c->Dh, c->dA, c->dB);
+  launch(k_offdiag_AB, g, 128, 0, s, c->d_wires, w_only, c->De, c->Dh, c->dA, c->dB);
 }
 
 // ---------------------------------------------------------------------------
@@ -894,6 +903,7 @@ void launch_offdiag_AB(SbeCtx* c, int w_only, cudaStream_t s) {
 // Coulomb terms of CalcH (SBEs.py:1094-1103).  Layout per wire: [2][2Nk] with
 // entry d + Nk (C first, then D).
 __global__ void k_traces(const WireDev* wires, const double2* C, const double2* D, double2* tr) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.z];
   int nk = W.nk;
   int d = blockIdx.x - (nk - 1) + 0;  // blockIdx.x in [0, 2nk-1)
@@ -915,7 +925,7 @@ __global__ void k_traces(const WireDev* wires, const double2* C, const double2* 
 }
 
 void launch_traces(SbeCtx* c, const double2* C, const double2* D, cudaStream_t s) {
-  k_traces<<<dim3(2 * c->nk_max - 1, 2, c->nw), 32, 0, s>>>(c->d_wires, C, D, c->tr);
+  launch(k_traces, dim3(2 * c->nk_max - 1, 2, c->nw), 32, 0, s, c->d_wires, C, D, c->tr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1011,6 +1021,7 @@ __global__ void k_calch_ctx(const WireDev* wires, const double2* P, const double
                             const double2* D, const double2* Ek, const double* vs,
                             const double* Ee, const double* Eh, const double2* tr, double2* Heh,
                             double2* Hee, double2* Hhh) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.z];
   int k1 = blockIdx.x * blockDim.x + threadIdx.x;
   int k2 = blockIdx.y;
@@ -1047,22 +1058,24 @@ void launch_calch_ctx(SbeCtx* c, const double2* P, const double2* C, const doubl
                       const double2* Ek, cudaStream_t s) {
   launch_traces(c, C, D, s);
   dim3 g((c->nk_max + 63) / 64, c->nk_max, c->nw);
-  k_calch_ctx<<<g, 64, 0, s>>>(c->d_wires, P, C, D, Ek, c->vs, c->Ee, c->Eh, c->tr, c->Heh,
-                               c->Hee, c->Hhh);
+  launch(k_calch_ctx, g, 64, 0, s, c->d_wires, P, C, D, Ek, c->vs, c->Ee, c->Eh, c->tr, c->Heh,
+         c->Hee, c->Hhh);
 }
 
 // Single-wire CalcH on explicit arrays (the reference's pure-function call).
 __global__ void k_vq_from_vc(int nk, const double* VC, double* vq) {
+  pdl_enter();
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nk) return;
   for (int n = 0; n < 3; ++n) vq[n * nk + q] = VC[((long long)q * nk + 0) * 3 + n];
 }
 
 void launch_vq_from_vc(int nk, const double* VC, double* vq, cudaStream_t s) {
-  k_vq_from_vc<<<(nk + 127) / 128, 128, 0, s>>>(nk, VC, vq);
+  launch(k_vq_from_vc, (nk + 127) / 128, 128, 0, s, nk, VC, vq);
 }
 
 __global__ void k_traces_single(int nk, const double2* C, const double2* D, double2* tr) {
+  pdl_enter();
   int d = (int)blockIdx.x - (nk - 1);
   int which = blockIdx.y;
   const double2* X = which == 0 ? C : D;
@@ -1081,6 +1094,7 @@ __global__ void k_traces_single(int nk, const double2* C, const double2* D, doub
 }
 
 __global__ void k_calch_single(CalcHArgs a) {
+  pdl_enter();
   int k1 = blockIdx.x * blockDim.x + threadIdx.x;
   int k2 = blockIdx.y;
   if (k1 >= a.nk || k2 >= a.nk) return;
@@ -1100,8 +1114,8 @@ int launch_calch_single(int nk, const double2* Meh, const double2* Wee, const do
   if (cudaMallocAsync(&vq, sizeof(double) * 3 * nk, s) != cudaSuccess ||
       cudaMallocAsync(&tr, sizeof(double2) * 4 * nk, s) != cudaSuccess)
     return fail(SBE_ERR_OOM, "sbe_calch: scratch allocation failed");
-  k_vq_from_vc<<<(nk + 127) / 128, 128, 0, s>>>(nk, VC, vq);
-  k_traces_single<<<dim3(2 * nk - 1, 2), 32, 0, s>>>(nk, C, D, tr);
+  launch(k_vq_from_vc, (nk + 127) / 128, 128, 0, s, nk, VC, vq);
+  launch(k_traces_single, dim3(2 * nk - 1, 2), 32, 0, s, nk, C, D, tr);
   CalcHArgs a;
   a.nk = nk;
   a.nr = 2 * nk + 2;
@@ -1126,7 +1140,7 @@ int launch_calch_single(int nk, const double2* Meh, const double2* Wee, const do
   a.Heh = Heh;
   a.Hee = Hee;
   a.Hhh = Hhh;
-  k_calch_single<<<dim3((nk + 63) / 64, nk), 64, 0, s>>>(a);
+  launch(k_calch_single, dim3((nk + 63) / 64, nk), 64, 0, s, a);
   cudaFreeAsync(vq, s);
   cudaFreeAsync(tr, s);
   return cuda_check(cudaGetLastError(), "sbe_calch");

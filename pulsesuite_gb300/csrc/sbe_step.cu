@@ -14,6 +14,7 @@ __global__ void k_leap_update(const WireDev* wires, double2* L1p, const double2*
                               const double2* dP, double2* L1c, const double2* L2c,
                               const double2* dC, double2* L1d, const double2* L2d,
                               const double2* dD, double dt) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   long long n = (long long)W.nk * W.nk;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -31,6 +32,7 @@ __global__ void k_leap_update(const WireDev* wires, double2* L1p, const double2*
 // SBEs.py:5704-5706 and _checkin (5070-5080): with X3 held in level 1,
 // new level1 = old level2, level2 = (old level2 + X3)/2, level3 = X3.
 __global__ void k_leap_shuffle(const WireDev* wires, double2* L1, double2* L2, double2* L3) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   long long n = (long long)W.nk * W.nk;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -50,6 +52,7 @@ __global__ void __launch_bounds__(128) k_phonon_rates(const WireDev* wires, int 
                                                       const double2* nev, const double2* nhv,
                                                       int diag, const double* vph, const double* EP,
                                                       const double* HP, double* wrate) {
+  pdl_enter();
   const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int nk = W.nk;
   int k = blockIdx.x;
@@ -110,6 +113,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
     k_relax_norm(const WireDev* wires, double2* C3, double2* D3, const double* wrate,
                  const double* rsp, double dt, double2* ne_out, double2* nh_out, double* charge,
                  int mode) {
+  pdl_enter();
   const WireDev& W = wires[blockIdx.y];
   const int nk = W.nk, k0 = blockIdx.x + kCluster * threadIdx.x, kst = kCluster * 256;
   const bool relax = mode != 2 && (W.flags & (SBE_F_PHONON | SBE_F_EHS)) != 0;
@@ -179,8 +183,8 @@ bool any_ehs(const SbeCtx* c) {
 void launch_relax_norm(SbeCtx* c, double2* P3, double2* C3, double2* D3, const double2* Ek,
                        double dt, cudaStream_t s) {
   if (any_ehs(c)) launch_extract_diag(c, C3, D3, s);   // for the carrier-carrier rates
-  k_phonon_rates<<<dim3(c->nk_max, c->nw), 128, 0, s>>>(c->d_wires, -1, C3, D3, 1, c->vph, c->EP,
-                                                        c->HP, c->wrate);
+  launch(k_phonon_rates, dim3(c->nk_max, c->nw), 128, 0, s, c->d_wires, -1, C3, D3, 1, c->vph,
+         c->EP, c->HP, c->wrate);
   launch_mbc_rates(c, -1, s);
   launch_relax_only(c, P3, C3, D3, Ek, dt, s);
 }
@@ -190,20 +194,20 @@ void launch_relax_norm(SbeCtx* c, double2* P3, double2* C3, double2* D3, const d
 void launch_relax_only(SbeCtx* c, double2* P3, double2* C3, double2* D3, const double2* Ek,
                        double dt, cudaStream_t s) {
   if (!any_dc(c)) {
-    k_relax_norm<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
-                                       c->charge, 0);
+    launch(k_relax_norm, dim3(kCluster, c->nw), 256, 0, s, c->d_wires, C3, D3, c->wrate, c->rsp, dt,
+           c->ne, c->nh, c->charge, 0);
     return;
   }
-  k_relax_norm<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
-                                     c->charge, 1);
+  launch(k_relax_norm, dim3(kCluster, c->nw), 256, 0, s, c->d_wires, C3, D3, c->wrate, c->rsp, dt,
+         c->ne, c->nh, c->charge, 1);
   launch_dc_transport(c, P3, C3, D3, Ek, dt, s);
-  k_relax_norm<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, C3, D3, c->wrate, c->rsp, dt, c->ne, c->nh,
-                                     c->charge, 2);
+  launch(k_relax_norm, dim3(kCluster, c->nw), 256, 0, s, c->d_wires, C3, D3, c->wrate, c->rsp, dt,
+         c->ne, c->nh, c->charge, 2);
 }
 
 void launch_phonon_rates_one(SbeCtx* c, int w, cudaStream_t s) {
-  k_phonon_rates<<<dim3(c->wires[w].nk, 1), 128, 0, s>>>(c->d_wires, w, c->ne, c->nh, 0, c->vph,
-                                                         c->EP, c->HP, c->wrate);
+  launch(k_phonon_rates, dim3(c->wires[w].nk, 1), 128, 0, s, c->d_wires, w, c->ne, c->nh, 0, c->vph,
+         c->EP, c->HP, c->wrate);
 }
 
 void launch_leapfrog(SbeCtx* c, double2* const* st, const double2* Ek, double dt,
@@ -211,17 +215,17 @@ void launch_leapfrog(SbeCtx* c, double2* const* st, const double2* Ek, double dt
   // st: YY1, YY2, YY3, CC1, CC2, CC3, DD1, DD2, DD3
   int blocks = (int)std::min<long long>(((long long)c->nk_max * c->nk_max + 255) / 256, 4096);
   dim3 g(blocks, c->nw);
-  k_leap_update<<<g, 256, 0, s>>>(c->d_wires, st[0], st[1], c->dP, st[3], st[4], c->dC, st[6],
-                                  st[7], c->dD, dt);
+  launch(k_leap_update, g, 256, 0, s, c->d_wires, st[0], st[1], c->dP, st[3], st[4], c->dC, st[6],
+         st[7], c->dD, dt);
   launch_relax_norm(c, st[0], st[3], st[6], Ek, dt, s);
 }
 
 void launch_leap_shuffle(SbeCtx* c, double2* const* st, cudaStream_t s) {
   int blocks = (int)std::min<long long>(((long long)c->nk_max * c->nk_max + 255) / 256, 4096);
   dim3 g(blocks, c->nw);
-  k_leap_shuffle<<<g, 256, 0, s>>>(c->d_wires, st[0], st[1], st[2]);
-  k_leap_shuffle<<<g, 256, 0, s>>>(c->d_wires, st[3], st[4], st[5]);
-  k_leap_shuffle<<<g, 256, 0, s>>>(c->d_wires, st[6], st[7], st[8]);
+  launch(k_leap_shuffle, g, 256, 0, s, c->d_wires, st[0], st[1], st[2]);
+  launch(k_leap_shuffle, g, 256, 0, s, c->d_wires, st[3], st[4], st[5]);
+  launch(k_leap_shuffle, g, 256, 0, s, c->d_wires, st[6], st[7], st[8]);
 }
 
 // ---------------------------------------------------------------------------
@@ -232,6 +236,7 @@ void launch_leap_shuffle(SbeCtx* c, double2* const* st, cudaStream_t s) {
 // reference's FFTG here is undone by the iFFTG of QW2Prop).
 __global__ void k_src_reduce(const WireDev* wires, int w_only, const double2* expikr,
                              const double2* G, long long tot_kr, const double* win, double2* src) {
+  pdl_enter();
   const WireDev W = wires[w_only >= 0 ? w_only : blockIdx.y];
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= W.nr) return;
@@ -271,6 +276,7 @@ __global__ void k_src_reduce(const WireDev* wires, int w_only, const double2* ex
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
     k_src_final(const WireDev* wires, int w_only, const double* r, const double2* ne,
                 const double2* nh, double2* src) {
+  pdl_enter();
   const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
   const int nr = W.nr, nk = W.nk, j0 = blockIdx.x + kCluster * threadIdx.x, st = kCluster * 256;
   double2* re = src + 5 * W.off_r + 3 * nr;
@@ -333,9 +339,9 @@ void launch_sources(SbeCtx* c, const double2* P, const double2* C, const double2
   }
   int nb = w_only >= 0 ? 1 : c->nw;
   (void)nb;
-  k_src_reduce<<<dim3((c->nr_max + 127) / 128, nb), 128, 0, s>>>(c->d_wires, w_only, c->expikr,
-                                                                c->G, c->tot_kr, c->window, src);
-  k_src_final<<<dim3(kCluster, nb), 256, 0, s>>>(c->d_wires, w_only, c->r, ne, nh, src);
+  launch(k_src_reduce, dim3((c->nr_max + 127) / 128, nb), 128, 0, s, c->d_wires, w_only, c->expikr,
+         c->G, c->tot_kr, c->window, src);
+  launch(k_src_final, dim3(kCluster, nb), 256, 0, s, c->d_wires, w_only, c->r, ne, nh, src);
 }
 
 // ---------------------------------------------------------------------------
@@ -346,6 +352,7 @@ void launch_sources(SbeCtx* c, const double2* P, const double2* C, const double2
 //                      s=4: X += dt/6 (acc + k)
 __global__ void k_rk4_axpy(long long n, int stage, double dt, double2* X, double2* acc,
                            double2* xs, const double2* k) {
+  pdl_enter();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     double2 kv = k[i];
@@ -373,11 +380,12 @@ void launch_rk4_axpy(SbeCtx* c, int stage, double dt, double2* P, double2* C, do
   double2* X[3] = {P, C, D};
   double2* K[3] = {c->dP, c->dC, c->dD};
   for (int i = 0; i < 3; ++i)
-    k_rk4_axpy<<<blocks, 256, 0, s>>>(n, stage, dt, X[i], c->kacc + i * n, c->xs + i * n, K[i]);
+    launch(k_rk4_axpy, blocks, 256, 0, s, n, stage, dt, X[i], c->kacc + i * n, c->xs + i * n, K[i]);
 }
 
 __global__ void k_stage_field(long long n, const double2* Ek0, const double2* dEk, double frac,
                               double2* out) {
+  pdl_enter();
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double2 a = Ek0[i];
@@ -392,7 +400,7 @@ __global__ void k_stage_field(long long n, const double2* Ek0, const double2* dE
 void launch_stage_field(SbeCtx* c, const double2* Ek0, const double2* dEk, double frac,
                         cudaStream_t s) {
   long long n = 3 * c->tot_r;
-  k_stage_field<<<(int)((n + 255) / 256), 256, 0, s>>>(n, Ek0, dEk, frac, c->ekst);
+  launch(k_stage_field, (int)((n + 255) / 256), 256, 0, s, n, Ek0, dEk, frac, c->ekst);
 }
 
 // ---------------------------------------------------------------------------
@@ -457,6 +465,7 @@ __device__ void fmm_spline(int n, const double* x, const double2* y, double2* b,
 }
 
 __global__ void k_spline_coef(int n, const double* x, const double2* y, int nf, double2* coef) {
+  pdl_enter();
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
   double2* b = coef + (long long)f * 3 * n;
@@ -466,7 +475,7 @@ __global__ void k_spline_coef(int n, const double* x, const double2* y, int nf, 
 static void spline_coefs(int n, const double* x, const double2* y, int nf, double2* coef,
                          cudaStream_t s) {
   if (n < kSplMin) {
-    k_spline_coef<<<1, 32, 0, s>>>(n, x, y, nf, coef);
+    launch(k_spline_coef, 1, 32, 0, s, n, x, y, nf, coef);
     return;
   }
   SplBatch b{};
@@ -485,6 +494,7 @@ __global__ void __launch_bounds__(128) k_spline_eval(int n0, const double* x0, c
                                                      const double2* coef, int n1, const double* x1,
                                                      int nf, const double* win, int real_part,
                                                      double2* out) {
+  pdl_enter();
   __shared__ double rlo[4], rhi[4];
   double lo = x0[0], hi = lo;
   for (int i = threadIdx.x; i < n0; i += 128) {
@@ -523,6 +533,7 @@ __global__ void __launch_bounds__(128) k_spline_eval(int n0, const double* x0, c
 // = conj F[q].
 __global__ void __launch_bounds__(64) k_fftg(int n, const double2* tw, const double2* in,
                                              double2* out) {
+  pdl_enter();
   const int q = blockIdx.x * 2 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (2 * q > n) return;
   double sr[4] = {0, 0, 0, 0}, si[4] = {0, 0, 0, 0};
@@ -587,9 +598,9 @@ int launch_prop2qw_scratch(SbeCtx* c, int w, const double* RR, int n_rr, const d
                            double2* out, double2* coef, double2* tmp, cudaStream_t s) {
   const WireDev& W = c->wires[w];
   spline_coefs(n_rr, RR, fin, 4, coef, s);
-  k_spline_eval<<<(W.nr + 127) / 128, 128, 0, s>>>(n_rr, RR, fin, coef, W.nr, c->r + W.off_r, 4,
-                                                   c->window + W.off_r, 1, tmp);
-  k_fftg<<<(W.nr / 2 + 2) / 2, 64, 0, s>>>(W.nr, c->twd + W.off_r, tmp, out);
+  launch(k_spline_eval, (W.nr + 127) / 128, 128, 0, s, n_rr, RR, fin, coef, W.nr, c->r + W.off_r, 4,
+         c->window + W.off_r, 1, tmp);
+  launch(k_fftg, (W.nr / 2 + 2) / 2, 64, 0, s, W.nr, c->twd + W.off_r, tmp, out);
   return cuda_check(cudaGetLastError(), "prop2qw (caller scratch)");
 }
 
@@ -598,6 +609,7 @@ int launch_prop2qw_scratch(SbeCtx* c, int w, const double* RR, int n_rr, const d
 // magnitudes are bound by the FP64 pipe of the blocks' SMs.
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
     k_plasmonics(int n, const double* grid, double2* a, double2* b, double* total_io, int mode) {
+  pdl_enter();
   const double dx = grid[1] - grid[0];
   const int i0 = blockIdx.x * 256 + threadIdx.x, st = kCluster * 256;
   double A = 0, B = 0;
@@ -631,12 +643,13 @@ int launch_qw2prop(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
   cudaMemcpyAsync(tmp, src, sizeof(double2) * 5 * (size_t)W.nr, cudaMemcpyDeviceToDevice, s);
   const double* rw = c->r + W.off_r;
   if (plasmonics)
-    k_plasmonics<<<kCluster, 256, 0, s>>>(W.nr, rw, tmp + 3 * W.nr, tmp + 4 * W.nr, total, 0);
+    launch(k_plasmonics, kCluster, 256, 0, s, W.nr, rw, tmp + 3 * W.nr, tmp + 4 * W.nr, total, 0);
   spline_coefs(W.nr, rw, tmp, 5, coef, s);
-  k_spline_eval<<<(n_rr + 127) / 128, 128, 0, s>>>(W.nr, rw, tmp, coef, n_rr, RR, 5, nullptr, 0, out);
+  launch(k_spline_eval, (n_rr + 127) / 128, 128, 0, s, W.nr, rw, tmp, coef, n_rr, RR, 5, nullptr, 0,
+         out);
   if (plasmonics)
-    k_plasmonics<<<kCluster, 256, 0, s>>>(n_rr, RR, out + 3 * (size_t)n_rr, out + 4 * (size_t)n_rr,
-                                   total, 1);
+    launch(k_plasmonics, kCluster, 256, 0, s, n_rr, RR, out + 3 * (size_t)n_rr,
+           out + 4 * (size_t)n_rr, total, 1);
   return cuda_check(cudaGetLastError(), "qw2prop");
 }
 
@@ -645,13 +658,13 @@ int launch_qw2prop(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
 namespace sbe {
 void launch_sources_final(SbeCtx* c, const double2* ne, const double2* nh, double2* src,
                           cudaStream_t s) {
-  k_src_final<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, -1, c->r, ne, nh, src);
+  launch(k_src_final, dim3(kCluster, c->nw), 256, 0, s, c->d_wires, -1, c->r, ne, nh, src);
 }
 
 void launch_sources_reduce(SbeCtx* c, const double2* ne, const double2* nh, double2* src,
                            cudaStream_t s) {
-  k_src_reduce<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, -1, c->expikr,
-                                                                   c->G, c->tot_kr, c->window, src);
-  k_src_final<<<dim3(kCluster, c->nw), 256, 0, s>>>(c->d_wires, -1, c->r, ne, nh, src);
+  launch(k_src_reduce, dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s, c->d_wires, -1, c->expikr,
+         c->G, c->tot_kr, c->window, src);
+  launch(k_src_final, dim3(kCluster, c->nw), 256, 0, s, c->d_wires, -1, c->r, ne, nh, src);
 }
 }  // namespace sbe

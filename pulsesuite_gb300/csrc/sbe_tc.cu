@@ -23,6 +23,7 @@ namespace sbe {
 // max(|re|, |im|) of each batch entry of a packed complex array (integer compare
 // of the magnitudes' bit patterns; atomicMax on the pattern of the FP32 value).
 __global__ void k_absmax(const double2* X, long long per_batch, long long bstride, unsigned* out) {
+  pdl_enter();
   const int b = blockIdx.y;
   const double2* x = X + (long long)b * bstride;
   unsigned long long m = 0;
@@ -37,6 +38,7 @@ __global__ void k_absmax(const double2* X, long long per_batch, long long bstrid
 
 // e[b] = 14 - ceil(log2(max)): scaled magnitudes stay <= 2^14 (FP16 max 65504).
 __global__ void k_exponents(int nb, const unsigned* mx, int* e, const int* add, int* sum) {
+  pdl_enter();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   float m = __uint_as_float(mx[b]) * 1.0001f;
@@ -52,6 +54,7 @@ __global__ void k_exponents(int nb, const unsigned* mx, int* e, const int* add, 
 // the stage's Hamiltonian.
 __global__ void k_stage_exponents(int nb, unsigned* mxS, unsigned* mxO, unsigned* mxH, int* eS,
                                   int* eO, const int* eT, int* esx, int reset) {
+  pdl_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   const float ms = __uint_as_float(mxS[b]) * 1.0001f, mo = __uint_as_float(mxO[b]) * 1.0001f;
@@ -69,6 +72,7 @@ __global__ void k_stage_exponents(int nb, unsigned* mxS, unsigned* mxO, unsigned
 // e[b] from the larger of two maxima (rule of k_exponents) and sum[b] = e[b] + add[b]
 __global__ void k_exponents2_sum(int nb, const unsigned* mx1, const unsigned* mx2, int* e,
                                  const int* add, int* sum) {
+  pdl_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   const float m = fmaxf(__uint_as_float(mx1[b]), __uint_as_float(mx2[b])) * 1.0001f;
@@ -88,6 +92,7 @@ __device__ __forceinline__ void put_hilo(__half* base, long long plane, float v)
 // re_hi, re_lo, im_hi, im_lo (complex) or hi, lo of the real part.
 __global__ void k_planes(const double2* X, long long bstride, int nk, int transpose,
                          const int* e, tc::PlaneSet dst, int mat, int real_only) {
+  pdl_enter();
   __shared__ double2 tile[32][33];
   const int b = blockIdx.z;
   const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
@@ -116,7 +121,7 @@ void launch_planes(const double2* X, long long bstride, int nk, int nbatch, int 
                    const int* e, const tc::PlaneSet& dst, int mat, int real_only,
                    cudaStream_t s) {
   dim3 blk(32, 8), grid((nk + 31) / 32, (nk + 31) / 32, nbatch);
-  k_planes<<<grid, blk, 0, s>>>(X, bstride, nk, transpose, e, dst, mat, real_only);
+  launch(k_planes, grid, blk, 0, s, X, bstride, nk, transpose, e, dst, mat, real_only);
 }
 
 // a complex value scaled by 2^e and rounded once to FP32
@@ -181,6 +186,7 @@ __device__ __forceinline__ void store_tiles_t(const __half (*hs)[32][40], int np
 template <typename T>
 __global__ void k_planes_nt(const T* X, int nk, const int* e, tc::PlaneSet dst, int matN, int matT,
                             int nbatch, float* cdf = nullptr, const double* dg = nullptr) {
+  pdl_enter();
   __shared__ T tile[32][33];
   __shared__ __align__(16) __half hs[4][32][40];
   const int b = blockIdx.z;
@@ -239,6 +245,7 @@ __host__ __device__ inline bool shear_block_live(int nk, int t0, int dd0) {
 // of X (row k1, column k2) is trace index d + Nk with d = k2 - k1, summed over the
 // nb column blocks in a fixed order into trf[b][which][d + Nk] (SBEs.py:1094-1103).
 __global__ void k_trace_from_shear(int nk, int nb, int ndd, const float2* dpart, float2* trf) {
+  pdl_enter();
   const int b = blockIdx.z, which = blockIdx.y;
   const int dd = blockIdx.x * blockDim.x + threadIdx.x;
   if (dd >= 2 * nk - 1) return;
@@ -257,8 +264,8 @@ void launch_exponents(const double2* X, long long per_batch, long long bstride, 
                       unsigned* mx, int* e, const int* add, int* sum, cudaStream_t s) {
   cudaMemsetAsync(mx, 0, sizeof(unsigned) * nbatch, s);
   int blocks = (int)std::min<long long>((per_batch + 255) / 256, 256);
-  k_absmax<<<dim3(blocks, nbatch), 256, 0, s>>>(X, per_batch, bstride, mx);
-  k_exponents<<<(nbatch + 127) / 128, 128, 0, s>>>(nbatch, mx, e, add, sum);
+  launch(k_absmax, dim3(blocks, nbatch), 256, 0, s, X, per_batch, bstride, mx);
+  launch(k_exponents, (nbatch + 127) / 128, 128, 0, s, nbatch, mx, e, add, sum);
 }
 
 // ---------------------------------------------------------------------------
@@ -299,6 +306,7 @@ void mixed_free(SbeCtx* c) {
 
 // E^T planes: Y[r][k] = Expikr[k][r] (|E| = 1, exponent 13).
 __global__ void k_eplanes(const WireDev* wires, const double2* expikr, tc::PlaneSet dst, int nw) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.z];
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   int r = blockIdx.y;
@@ -311,6 +319,7 @@ __global__ void k_eplanes(const WireDev* wires, const double2* expikr, tc::Plane
 }
 
 __global__ void k_fill_int(int* p, int n, int v) {
+  pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
@@ -318,6 +327,7 @@ __global__ void k_fill_int(int* p, int n, int v) {
 // real absmax per wire of a packed Nk x Nk real table, as the FP64 bit pattern
 // (the phonon tables exceed the FP32 range)
 __global__ void k_absmax_r(const double* X, long long per, unsigned long long* out) {
+  pdl_enter();
   const int b = blockIdx.y;
   const double* x = X + (long long)b * per;
   unsigned long long m = 0;
@@ -331,6 +341,7 @@ __global__ void k_absmax_r(const double* X, long long per, unsigned long long* o
 // sP[b] = -(E + 1) for max |EP|, |HP| in [2^E, 2^(E+1)): the scaled tables lie
 // in [0, 1)
 __global__ void k_phon_exp(int nb, const unsigned long long* mx, int* sP) {
+  pdl_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   const unsigned long long m = mx[b];
@@ -341,6 +352,7 @@ __global__ void k_phon_exp(int nb, const unsigned long long* mx, int* sP) {
 // EP, EP^T, HP, HP^T of every wire as scaled FP32 (coalesced transposes via tiles)
 __global__ void k_phon_tables(int nk, const double* EP, const double* HP, const int* sP,
                               float* epf, float* eptf, float* hpf, float* hptf) {
+  pdl_enter();
   __shared__ double te[32][33], th[32][33];
   const int b = blockIdx.z;
   const long long mb = (long long)b * nk * nk;
@@ -369,12 +381,14 @@ __global__ void k_phon_tables(int nk, const double* EP, const double* HP, const 
 }
 
 __global__ void k_ekrf(long long n, const double2* expikr, float2* ekrf) {
+  pdl_enter();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < n) ekrf[i] = f64_to_f32(expikr[i]);
 }
 
 // |xe|, |xh| of a bucket's wires in FP32: xef[b][j], j < 2 nk
 __global__ void k_xef(const WireDev* wires, int nk, const double* xeh, float* xef) {
+  pdl_enter();
   const int j = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
   if (j < 2 * nk) xef[(long long)b * 2 * nk + j] = fabsf(f64_to_f32(xeh[2 * wires[b].off_vec + j]));
 }
@@ -503,7 +517,7 @@ static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
   ka = Carver{0, static_cast<char*>(A->block)};
   carve_all(A, ka, c);
   cudaMemsetAsync(A->block, 0, ka.off, s);
-  k_ekrf<<<(unsigned)((c->tot_kr + 255) / 256), 256, 0, s>>>(c->tot_kr, c->expikr, A->ekrf);
+  launch(k_ekrf, (unsigned)((c->tot_kr + 255) / 256), 256, 0, s, c->tot_kr, c->expikr, A->ekrf);
   for (Mixed* m : A->b) {
     const int nk = m->nk, nw = m->nw;
     const long long mm = (long long)nk * nk;
@@ -516,16 +530,15 @@ static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
     cudaMemsetAsync(m->tp.ptr, 0, tc::planeset_bytes(m->tp), s);
     cudaMemsetAsync(m->sp.ptr, 0, tc::planeset_bytes(m->sp), s);
     cudaMemsetAsync(m->ep.ptr, 0, tc::planeset_bytes(m->ep), s);
-    k_eplanes<<<dim3((nk + 127) / 128, m->nr, nw), 128, 0, s>>>(m->dw, c->expikr, m->ep, nw);
-    k_fill_int<<<(nw + 127) / 128, 128, 0, s>>>(m->eE(), nw, 13);
+    launch(k_eplanes, dim3((nk + 127) / 128, m->nr, nw), 128, 0, s, m->dw, c->expikr, m->ep, nw);
+    launch(k_fill_int, (nw + 127) / 128, 128, 0, s, m->eE(), nw, 13);
     cudaMemsetAsync(m->mx64, 0, sizeof(unsigned long long) * nw, s);
-    k_absmax_r<<<dim3(64, nw), 256, 0, s>>>(c->EP + m->bm, mm, m->mx64);
-    k_absmax_r<<<dim3(64, nw), 256, 0, s>>>(c->HP + m->bm, mm, m->mx64);
-    k_phon_exp<<<(nw + 127) / 128, 128, 0, s>>>(nw, m->mx64, m->sP);
-    k_phon_tables<<<dim3(T, T, nw), dim3(32, 8), 0, s>>>(nk, c->EP + m->bm, c->HP + m->bm, m->sP,
-                                                        A->epf + m->bm, A->eptf + m->bm,
-                                                        A->hpf + m->bm, A->hptf + m->bm);
-    k_xef<<<dim3((2 * nk + 127) / 128, nw), 128, 0, s>>>(m->dw, nk, c->xeh, m->xef);
+    launch(k_absmax_r, dim3(64, nw), 256, 0, s, c->EP + m->bm, mm, m->mx64);
+    launch(k_absmax_r, dim3(64, nw), 256, 0, s, c->HP + m->bm, mm, m->mx64);
+    launch(k_phon_exp, (nw + 127) / 128, 128, 0, s, nw, m->mx64, m->sP);
+    launch(k_phon_tables, dim3(T, T, nw), dim3(32, 8), 0, s, nk, c->EP + m->bm, c->HP + m->bm,
+           m->sP, A->epf + m->bm, A->eptf + m->bm, A->hpf + m->bm, A->hptf + m->bm);
+    launch(k_xef, dim3((2 * nk + 127) / 128, nw), 128, 0, s, m->dw, nk, c->xeh, m->xef);
   }
   return cuda_check(cudaGetLastError(), "mixed workspace");
 }
@@ -542,6 +555,7 @@ __global__ void __launch_bounds__(256) k_state_in(const double2* __restrict__ X,
                                                   unsigned* __restrict__ mx,
                                                   unsigned* __restrict__ mo,
                                                   float2* __restrict__ xf, double* __restrict__ dg) {
+  pdl_enter();
   const int b = blockIdx.y;
   const int per = nk * nk;   // < 2^31
   const double2* x = X + (long long)b * per;
@@ -604,7 +618,7 @@ __global__ void __launch_bounds__(256) k_state_in(const double2* __restrict__ X,
 
 static void absmax_into(const double2* X, long long per, int nw, unsigned* mx, cudaStream_t s) {
   int blocks = (int)std::min<long long>((per + 255) / 256, 128);
-  k_absmax<<<dim3(blocks, nw), 256, 0, s>>>(X, per, per, mx);
+  launch(k_absmax, dim3(blocks, nw), 256, 0, s, X, per, per, mx);
 }
 
 // ---------------------------------------------------------------------------
@@ -614,6 +628,7 @@ static void absmax_into(const double2* X, long long per, int nw, unsigned* mx, c
 // FP32 copy of vs for the direct terms.
 __global__ void k_toeplitz_planes(const WireDev* wires, const double* vs, const int* e,
                                   tc::PlaneSet dst, int nw, float* vsf) {
+  pdl_enter();
   // block (32, 8) over a 32 x 32 tile (rows t, columns t')
   __shared__ __align__(16) __half hs[2][32][40];
   const int b = blockIdx.z / 3, n = blockIdx.z % 3;
@@ -649,6 +664,7 @@ __global__ void k_toeplitz_planes(const WireDev* wires, const double* vs, const 
 }
 
 __global__ void k_vs_max(const WireDev* wires, const double* vs, unsigned* mx) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.x];
   unsigned long long m = 0;
   for (int i = threadIdx.x; i < 3 * W.nk; i += blockDim.x) m = max(m, absbits(vs[3 * W.off_vec + i]));
@@ -662,6 +678,7 @@ __global__ void k_vs_max(const WireDev* wires, const double* vs, unsigned* mx) {
 // rows, are read row by row (coalesced) into shared memory.
 __global__ void k_hab(const WireDev* wires, const double* De, const double* Dh, float* habf,
                       long long tot_mat, unsigned* mx) {
+  pdl_enter();
   __shared__ double ta[63][33], tb[63][33];
   const WireDev W = wires[blockIdx.z];
   const int nk = W.nk;
@@ -720,6 +737,7 @@ __global__ void k_hab(const WireDev* wires, const double* De, const double* Dh, 
 // with V = Vxx2 at iq[q]: [0] vee^2 |xe|, [1] veh^2 |xh|, [2] vhh^2 |xh|, [3] veh^2 |xe|.
 __global__ void k_gamma_tab(const WireDev* wires, const double* vs, const int* iq,
                             const double* xeh, float* gtab, int nw) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   const int nk = W.nk, b = blockIdx.y;
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -740,6 +758,7 @@ __global__ void k_gamma_tab(const WireDev* wires, const double* vs, const int* i
 // k), lanes over q; occupations (real parts) staged in shared memory.
 __global__ void k_gamma_f(const WireDev* wires, const double2* ne, const double2* nh,
                           const int* maps, const float* gtab, float* gamf, int nw) {
+  pdl_enter();
   extern __shared__ float occ[];
   const WireDev W = wires[blockIdx.y];
   const int nk = W.nk, b = blockIdx.y;
@@ -802,6 +821,7 @@ __global__ void k_gamma_f(const WireDev* wires, const double2* ne, const double2
 // E1D(d) Vscale and Vhp for holes, scaled by 2^-sP to pair with the FP32 tables.
 __global__ void k_phon_tab(const WireDev* wires, const double* vs, const double* eps,
                            const int* sP, float* phf, int nw) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.y];
   const int nk = W.nk, b = blockIdx.y;
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
@@ -818,6 +838,7 @@ __global__ void k_phon_tab(const WireDev* wires, const double* vs, const double*
 __global__ void k_phonon_rates_f(const WireDev* wires, const double2* nev, const double2* nhv,
                                  int diag, const float* phf, const float* epf, const float* eptf,
                                  const float* hpf, const float* hptf, double* wrate, int nw) {
+  pdl_enter();
   extern __shared__ float occ[];
   const WireDev W = wires[blockIdx.y];
   const int nk = W.nk, b = blockIdx.y, k = blockIdx.x;
@@ -869,6 +890,7 @@ __global__ void k_phonon_rates_f(const WireDev* wires, const double2* nev, const
 // step has rewritten them)
 __global__ void k_diag_max(const WireDev* wires, const double2* C, const double2* D,
                            unsigned* mx) {
+  pdl_enter();
   const WireDev W = wires[blockIdx.x];
   unsigned long long m = 0;
   for (int k = threadIdx.x; k < W.nk; k += blockDim.x) {
@@ -886,6 +908,7 @@ __global__ void k_diag_max(const WireDev* wires, const double2* C, const double2
 // sums k = y, y + 8, ... of point r, the eight partial sums meet in shared memory.
 __global__ void k_src_reduce_f(const WireDev* wires, const float2* ekrf, const float2* G,
                                long long tot_kr, const double* win, double2* src) {
+  pdl_enter();
   __shared__ float part[6][8][33];
   const WireDev W = wires[blockIdx.y];
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -975,6 +998,7 @@ __global__ void k_src_reduce_f(const WireDev* wires, const float2* ekrf, const f
 // direct Coulomb terms are their sums over the blocks that exist.
 __global__ void k_shear_tiles(int nk, int nw, int ndd, const float2* X0, const float2* X1,
                               const float2* X2, const int* e, tc::PlaneSet dst, float2* dpart) {
+  pdl_enter();
   __shared__ float2 tile[63][32];
   __shared__ __align__(16) __half hs[2][64][40];   // hi, lo of rows 2 dd0 .. 2 dd0 + 63
   const int n = blockIdx.z / nw, b = blockIdx.z % nw;
@@ -1047,6 +1071,7 @@ __global__ void k_shear_tiles(int nk, int nw, int ndd, const float2* X0, const f
 
 __global__ void k_field_f(long long n, const double2* ek, const double2* dek, double frac,
                           float2* ekf) {
+  pdl_enter();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double2 a = ek[i];
@@ -1073,6 +1098,7 @@ __global__ void k_h_build(const WireDev* __restrict__ wires, const float2* __res
                           const float2* __restrict__ xsh, int have_x, float2* __restrict__ hf,
                           long long tot_mat, double2* __restrict__ dgE, double2* __restrict__ dgH,
                           float2* __restrict__ dgf, unsigned* __restrict__ mx) {
+  pdl_enter();
   const WireDev& W = wires[blockIdx.z];
   const int nk = W.nk, b = blockIdx.z, nw = gridDim.z;
   float hmax = 0.f;
@@ -1163,6 +1189,7 @@ __global__ void k_h_build(const WireDev* __restrict__ wires, const float2* __res
 // (slots M_EEX, M_HHX) from the FP32 values.
 __global__ void k_hplanes(const float2* hee, const float2* hhh, const float* hA, const float* hB,
                           int nk, const int* e, tc::PlaneSet dst, int nw) {
+  pdl_enter();
   // block (32, 8) over a 32 x 32 tile; each slot's planes go through shared memory
   __shared__ __align__(16) __half hs[4][32][40];
   const int b = blockIdx.z;
@@ -1303,6 +1330,7 @@ __global__ void __launch_bounds__(256) k_antiherm(
     int nk, const float2* __restrict__ W, const float2* __restrict__ Hp, const float2* X,
     const float2* __restrict__ ghi, const float2* __restrict__ glo, const float* __restrict__ chi,
     const float* __restrict__ clo, float2* out, Rk4Ctl rk) {
+  pdl_enter();
   // tb / hb: W and H' of the mirror tile (rows j0.., columns i0..); vt: results;
   // gv / cv: g (hi, lo) and c (hi, lo) at the tile's rows i0.. (0) and columns j0.. (1)
   __shared__ float2 tb[32][33], hb[32][33], vt[32][33];
@@ -1421,6 +1449,7 @@ __global__ void __launch_bounds__(256) k_rhs_p(
     int nk, int nw, const float2* __restrict__ G, const float2* __restrict__ hehf,
     const float2* X, const float2* __restrict__ dgf, const float* __restrict__ gamf,
     const float* __restrict__ cdf, float2* out, Rk4Ctl rk) {
+  pdl_enter();
   __shared__ float2 ht[32][33];
   // per-row (kh = m0 + r) values: hh hi, lo; GamH; d hi, lo
   __shared__ float2 rg[2][32];
@@ -1496,11 +1525,13 @@ __global__ void __launch_bounds__(256) k_rhs_p(
 }
 
 __global__ void k_f32_to_f64(long long n, const float2* a, double2* out) {
+  pdl_enter();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < n) out[i] = f32_to_f64(a[i]);
 }
 
 __global__ void k_add_int(int n, const int* a, const int* b, int* out) {
+  pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = a[i] + b[i];
 }
@@ -1632,7 +1663,7 @@ static std::vector<tc::GemmJob> all_jobs(SbeCtx* c, int kind) {
 }
 
 static void exponents_from(Mixed* m, const unsigned* mx, int* e, cudaStream_t s) {
-  k_exponents<<<(m->nw + 127) / 128, 128, 0, s>>>(m->nw, mx, e, nullptr, nullptr);
+  launch(k_exponents, (m->nw + 127) / 128, 128, 0, s, m->nw, mx, e, nullptr, nullptr);
 }
 
 // Per-step set-up of the mixed path: the frozen preparation (screening, rates,
@@ -1643,16 +1674,16 @@ static int mixed_prep(SbeCtx* c, const double2* C, const double2* D, cudaStream_
   for (Mixed* m : A->b) {
     const int nk = m->nk, nw = m->nw;
     cudaMemsetAsync(m->mxH(), 0, sizeof(unsigned) * nw, s);
-    k_vs_max<<<nw, 256, 0, s>>>(m->dw, c->vs, m->mxH());
+    launch(k_vs_max, nw, 256, 0, s, m->dw, c->vs, m->mxH());
     exponents_from(m, m->mxH(), m->eT(), s);
-    k_toeplitz_planes<<<dim3((nk + 31) / 32, (nk + 31) / 32, 3 * nw), dim3(32, 8), 0, s>>>(
-        m->dw, c->vs, m->eT(), m->tp, nw, m->vsf);
-    k_gamma_tab<<<dim3((nk + 127) / 128, nw), 128, 0, s>>>(m->dw, c->vs, c->iq, c->xeh, m->gtab,
-                                                           nw);
-    k_gamma_f<<<dim3((nk + 7) / 8, nw), 256, sizeof(float) * 2 * nk, s>>>(
-        m->dw, c->ne, c->nh, c->maps, m->gtab, m->gamf, nw);
-    k_phon_tab<<<dim3((nk + 127) / 128, nw), 128, 0, s>>>(m->dw, c->vs, c->eps, m->sP, m->phf,
-                                                          nw);
+    launch(k_toeplitz_planes, dim3((nk + 31) / 32, (nk + 31) / 32, 3 * nw), dim3(32, 8), 0, s,
+           m->dw, c->vs, m->eT(), m->tp, nw, m->vsf);
+    launch(k_gamma_tab, dim3((nk + 127) / 128, nw), 128, 0, s, m->dw, c->vs, c->iq, c->xeh, m->gtab,
+           nw);
+    launch(k_gamma_f, dim3((nk + 7) / 8, nw), 256, sizeof(float) * 2 * nk, s, m->dw, c->ne, c->nh,
+           c->maps, m->gtab, m->gamf, nw);
+    launch(k_phon_tab, dim3((nk + 127) / 128, nw), 128, 0, s, m->dw, c->vs, c->eps, m->sP, m->phf,
+           nw);
     cudaMemsetAsync(m->mxAB(), 0, sizeof(unsigned) * nw, s);
   }
   if (c->any_offdiag) {
@@ -1661,8 +1692,8 @@ static int mixed_prep(SbeCtx* c, const double2* C, const double2* D, cudaStream_
   }
   for (Mixed* m : A->b) {
     const int T = (m->nk + 31) / 32;
-    k_hab<<<dim3(T, T, m->nw), dim3(32, 8), 0, s>>>(m->dw, c->De, c->Dh, A->habf, c->tot_mat,
-                                                    m->mxAB());
+    launch(k_hab, dim3(T, T, m->nw), dim3(32, 8), 0, s, m->dw, c->De, c->Dh, A->habf, c->tot_mat,
+           m->mxAB());
   }
   return cuda_check(cudaGetLastError(), "mixed prep");
 }
@@ -1674,11 +1705,11 @@ static void mixed_relax(SbeCtx* c, double2* P, double2* C, double2* D, const dou
   MixedAll* A = all_of(c);
   if (any_ehs(c)) launch_extract_diag(c, C, D, s);   // for the carrier-carrier rates
   for (Mixed* m : A->b)
-    k_phonon_rates_f<<<dim3(m->nk, m->nw), 128, sizeof(float) * 2 * m->nk, s>>>(
-        m->dw, C, D, 1, m->phf, A->epf, A->eptf, A->hpf, A->hptf, c->wrate, m->nw);
+    launch(k_phonon_rates_f, dim3(m->nk, m->nw), 128, sizeof(float) * 2 * m->nk, s, m->dw, C, D, 1,
+           m->phf, A->epf, A->eptf, A->hpf, A->hptf, c->wrate, m->nw);
   launch_mbc_rates(c, -1, s, false, true);
   launch_relax_only(c, P, C, D, Ek, dt, s);
-  for (Mixed* m : A->b) k_diag_max<<<m->nw, 256, 0, s>>>(m->dw, C, D, m->mxS());
+  for (Mixed* m : A->b) launch(k_diag_max, m->nw, 256, 0, s, m->dw, C, D, m->mxS());
 }
 
 // Stage-1 state of the mixed path from the FP64 state: FP32 copies (the first
@@ -1695,11 +1726,12 @@ static void mixed_state_in(SbeCtx* c, const double2* P, const double2* C, const 
     cudaMemsetAsync(m->mxS(), 0, sizeof(unsigned) * nw, s);
     cudaMemsetAsync(m->mxO(), 0, sizeof(unsigned) * nw, s);
     const int blocks = (int)std::min<long long>((mm + 255) / 256, 128);
-    k_state_in<<<dim3(blocks, nw), 256, 0, s>>>(P + o, nk, 0, m->mxS(), m->mxO(), xf + o, nullptr);
-    k_state_in<<<dim3(blocks, nw), 256, 0, s>>>(C + o, nk, 1, m->mxS(), m->mxO(), xf + tm + o,
-                                                m->xdg);
-    k_state_in<<<dim3(blocks, nw), 256, 0, s>>>(D + o, nk, 1, m->mxS(), m->mxO(),
-                                                xf + 2 * tm + o, m->xdg + vn);
+    launch(k_state_in, dim3(blocks, nw), 256, 0, s, P + o, nk, 0, m->mxS(), m->mxO(), xf + o,
+           nullptr);
+    launch(k_state_in, dim3(blocks, nw), 256, 0, s, C + o, nk, 1, m->mxS(), m->mxO(), xf + tm + o,
+           m->xdg);
+    launch(k_state_in, dim3(blocks, nw), 256, 0, s, D + o, nk, 1, m->mxS(), m->mxO(),
+           xf + 2 * tm + o, m->xdg + vn);
   }
 }
 
@@ -1715,7 +1747,8 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
   const long long tm = c->tot_mat;
   const int have_x = (c->wires[0].flags & SBE_F_EXCITONS) ? 1 : 0;
   // stage field in FP32 (all wires)
-  k_field_f<<<(int)((3 * c->tot_r + 255) / 256), 256, 0, s>>>(3 * c->tot_r, Ek, dEk, frac, A->ekf);
+  launch(k_field_f, (int)((3 * c->tot_r + 255) / 256), 256, 0, s, 3 * c->tot_r, Ek, dEk, frac,
+         A->ekf);
   // state exponents and planes: P and P^T from one read; C and D need only their own
   // layout (C^T = conj C and D^T = conj D for the Hermitian C and D).  eS: full state
   // maximum (sheared exchange operands); eO: maximum over P and the off-diagonal C, D
@@ -1725,14 +1758,15 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
     const int nk = m->nk, nw = m->nw;
     const long long vn = (long long)nw * nk;
     const float2 *P = xs + m->bm, *C = xs + tm + m->bm, *D = xs + 2 * tm + m->bm;
-    k_stage_exponents<<<(nw + 127) / 128, 128, 0, s>>>(nw, m->mxS(), m->mxO(), m->mxH(),
-                                                       m->eS(), m->eO(), m->eT(), m->esx(),
-                                                       stage > 0);
+    launch(k_stage_exponents, (nw + 127) / 128, 128, 0, s, nw, m->mxS(), m->mxO(), m->mxH(),
+           m->eS(), m->eO(), m->eT(), m->esx(),
+           stage > 0);
     const dim3 tb(32, 8), tg((nk + 31) / 32, (nk + 31) / 32, nw);
-    k_planes_nt<float2><<<tg, tb, 0, s>>>(P, nk, m->eO(), m->pl, M_P, M_PT, nw);
-    k_planes_nt<float2><<<tg, tb, 0, s>>>(C, nk, m->eO(), m->pl, M_C, -1, nw, m->cdf, m->xdg);
-    k_planes_nt<float2><<<tg, tb, 0, s>>>(D, nk, m->eO(), m->pl, M_D, -1, nw, m->cdf + 2 * vn,
-                                          m->xdg + vn);
+    launch(k_planes_nt<float2>, tg, tb, 0, s, P, nk, m->eO(), m->pl, M_P, M_PT, nw,
+           nullptr, nullptr);
+    launch(k_planes_nt<float2>, tg, tb, 0, s, C, nk, m->eO(), m->pl, M_C, -1, nw, m->cdf, m->xdg);
+    launch(k_planes_nt<float2>, tg, tb, 0, s, D, nk, m->eO(), m->pl, M_D, -1, nw, m->cdf + 2 * vn,
+           m->xdg + vn);
     if (have_x) {
       // the traces of C and D (direct terms) come from the shear's diagonal partials
       const int nbk = (nk + 31) / 32, ndd = 32 * ((2 * nk + 31) / 32);
@@ -1743,10 +1777,10 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
           if (shear_block_live(nk, 32 * i, 32 * j)) cnt = j - shear_first_block(nk, 32 * i) + 1;
         ny = std::max(ny, cnt);
       }
-      k_shear_tiles<<<dim3(nbk, ny, 3 * nw), dim3(32, 8), 0, s>>>(nk, nw, ndd, P, C, D, m->eS(),
-                                                                 m->sp, m->tpart);
-      k_trace_from_shear<<<dim3((2 * nk - 1 + 127) / 128, 2, nw), 128, 0, s>>>(nk, nbk, ndd,
-                                                                               m->tpart, m->trf);
+      launch(k_shear_tiles, dim3(nbk, ny, 3 * nw), dim3(32, 8), 0, s, nk, nw, ndd, P, C, D, m->eS(),
+             m->sp, m->tpart);
+      launch(k_trace_from_shear, dim3((2 * nk - 1 + 127) / 128, 2, nw), 128, 0, s, nk, nbk, ndd,
+             m->tpart, m->trf);
     }
   }
   int rc = SBE_OK;
@@ -1759,16 +1793,17 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
   // the Hamiltonians: Meh + diagonal + direct + exchange, diagonal peeled; their planes
   for (Mixed* m : A->b) {
     const int nk = m->nk, nw = m->nw;
-    k_h_build<<<dim3((nk + 511) / 512, (nk + HB_ROWS - 1) / HB_ROWS, nw), 128, 0, s>>>(
-        m->dw, A->ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh),
-        have_x, A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH());
+    launch(k_h_build, dim3((nk + 511) / 512, (nk + HB_ROWS - 1) / HB_ROWS, nw), 128, 0, s, m->dw,
+           A->ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh), have_x,
+           A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH());
     // H exponent: max over the operands and the step's 2 hbar |A|, |B|
-    k_exponents2_sum<<<(nw + 127) / 128, 128, 0, s>>>(nw, m->mxH(), m->mxAB(), m->eH(), m->eO(),
-                                                      m->esc());
+    launch(k_exponents2_sum, (nw + 127) / 128, 128, 0, s, nw, m->mxH(), m->mxAB(), m->eH(), m->eO(),
+           m->esc());
     const dim3 tb(32, 8), tg((nk + 31) / 32, (nk + 31) / 32, nw);
-    k_planes_nt<float2><<<tg, tb, 0, s>>>(A->hf + m->bm, nk, m->eH(), m->pl, M_EH, M_EHT, nw);
-    k_hplanes<<<tg, tb, 0, s>>>(A->hf + tm + m->bm, A->hf + 2 * tm + m->bm, A->habf + m->bm,
-                                A->habf + tm + m->bm, nk, m->eH(), m->pl, nw);
+    launch(k_planes_nt<float2>, tg, tb, 0, s, A->hf + m->bm, nk, m->eH(), m->pl, M_EH, M_EHT, nw,
+           nullptr, nullptr);
+    launch(k_hplanes, tg, tb, 0, s, A->hf + tm + m->bm, A->hf + 2 * tm + m->bm, A->habf + m->bm,
+           A->habf + tm + m->bm, nk, m->eH(), m->pl, nw);
   }
   // commutator GEMMs: dP and the cross terms of W and V, then the hi*hi products of
   // W and V (the partials of W and V meet in the anti-Hermitian pass)
@@ -1810,13 +1845,13 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
       rk[i].mo = m->mxO();
     }
     const dim3 ag((nk + 31) / 32, (nk + 31) / 32, nw), ab(32, 8);
-    k_rhs_p<<<ag, ab, 0, s>>>(nk, nw, gp + o, A->hf + o, P, m->dgf, m->gamf, m->cdf, A->kf + o,
-                              rk[0]);
-    k_antiherm<<<ag, ab, 0, s>>>(nk, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf,
-                                 m->dgf + vn, m->cdf, m->cdf + vn, A->kf + tm + o, rk[1]);
-    k_antiherm<<<ag, ab, 0, s>>>(nk, wf + G_V * tm + o, A->hf + 2 * tm + o, D,
-                                 m->dgf + 2 * vn, m->dgf + 3 * vn, m->cdf + 2 * vn,
-                                 m->cdf + 3 * vn, A->kf + 2 * tm + o, rk[2]);
+    launch(k_rhs_p, ag, ab, 0, s, nk, nw, gp + o, A->hf + o, P, m->dgf, m->gamf, m->cdf, A->kf + o,
+           rk[0]);
+    launch(k_antiherm, ag, ab, 0, s, nk, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf,
+           m->dgf + vn, m->cdf, m->cdf + vn, A->kf + tm + o, rk[1]);
+    launch(k_antiherm, ag, ab, 0, s, nk, wf + G_V * tm + o, A->hf + 2 * tm + o, D,
+           m->dgf + 2 * vn, m->dgf + 3 * vn, m->cdf + 2 * vn,
+           m->cdf + 3 * vn, A->kf + 2 * tm + o, rk[2]);
   }
   return cuda_check(cudaGetLastError(), "mixed stage");
 }
@@ -1840,8 +1875,9 @@ static int mixed_sources(SbeCtx* c, const double2* P, const double2* C, const do
     const double2* st[3] = {P + o, C + o, D + o};
     const dim3 tb(32, 8), tg((nk + 31) / 32, (nk + 31) / 32, nw);
     for (int i = 0; i < 3; ++i)
-      k_planes_nt<double2><<<tg, tb, 0, s>>>(st[i], nk, m->eS(), m->pl, 2 * i, -1, nw);
-    k_add_int<<<(nw + 127) / 128, 128, 0, s>>>(nw, m->eS(), m->eE(), m->ess());
+      launch(k_planes_nt<double2>, tg, tb, 0, s, st[i], nk, m->eS(), m->pl, 2 * i, -1, nw,
+             nullptr, nullptr);
+    launch(k_add_int, (nw + 127) / 128, 128, 0, s, nw, m->eS(), m->eE(), m->ess());
   }
   float2* gf = reinterpret_cast<float2*>(c->G);
   {
@@ -1850,8 +1886,8 @@ static int mixed_sources(SbeCtx* c, const double2* P, const double2* C, const do
     if (rc) return rc;
   }
   for (Mixed* m : A->b)
-    k_src_reduce_f<<<dim3((m->nr + 31) / 32, m->nw), dim3(32, 8), 0, s>>>(
-        m->dw, A->ekrf, gf, c->tot_kr, c->window, src);
+    launch(k_src_reduce_f, dim3((m->nr + 31) / 32, m->nw), dim3(32, 8), 0, s, m->dw, A->ekrf, gf,
+           c->tot_kr, c->window, src);
   launch_sources_final(c, c->ne, c->nh, src, s);
   return cuda_check(cudaGetLastError(), "mixed sources");
 }
@@ -1877,9 +1913,9 @@ int rhs_mixed(SbeCtx* c, const double2* P, const double2* C, const double2* D, c
                    s);
   if (rc) return rc;
   const int g = (int)((n + 255) / 256);
-  k_f32_to_f64<<<g, 256, 0, s>>>(n, A->kf, dP);
-  k_f32_to_f64<<<g, 256, 0, s>>>(n, A->kf + n, dC);
-  k_f32_to_f64<<<g, 256, 0, s>>>(n, A->kf + 2 * n, dD);
+  launch(k_f32_to_f64, g, 256, 0, s, n, A->kf, dP);
+  launch(k_f32_to_f64, g, 256, 0, s, n, A->kf + n, dC);
+  launch(k_f32_to_f64, g, 256, 0, s, n, A->kf + 2 * n, dD);
   return cuda_check(cudaGetLastError(), "rhs_mixed");
 }
 

@@ -28,6 +28,7 @@ constexpr int kThreads = 256;
 __device__ __forceinline__ double2 cdivr(double2 a, double d) { return cscale(a, 1.0 / d); }
 
 __global__ void __launch_bounds__(kThreads) k_spline(SplBatch s) {
+  pdl_enter();
   __shared__ double2 c1[kFields][kCap], c2[kFields][kCap];
   __shared__ double x[kCap], ip[kCap], id[kCap], tt[kCap], mm[kCap];
   __shared__ double red[2][kThreads / 32];
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(kThreads) k_spline(SplBatch s) {
 }  // namespace
 
 void launch_splines(const SplBatch& b, int ngroups, int nmax, cudaStream_t s) {
-  k_spline<<<dim3((nmax + kTile - 1) / kTile, ngroups), kThreads, 0, s>>>(b);
+  launch(k_spline, dim3((nmax + kTile - 1) / kTile, ngroups), kThreads, 0, s, b);
 }
 
 }  // namespace sbe

@@ -189,6 +189,7 @@ constexpr int STAGE_AREA = 192 * 1024;
 template <int BNT, int MODE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     k_tc_gemm(const __grid_constant__ GemmLaunch L) {
+  pdl_enter();
   constexpr int BTB = BNT * BK * 2;   // B tile bytes per plane
   constexpr bool HH = (MODE == MODE_HH);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -518,6 +519,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  // the last CTA leaves the slot zeroed for its next launch: every CTA has drawn its last
+  // tile by now (a memset ahead of the launch costs a launch of its own and the overlap with
+  // the kernel before)
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(L.sched + 1, 1) == (int)gridDim.x - 1) {
+      L.sched[0] = 0;
+      L.sched[1] = 0;
+    }
+  }
 }
 
 }  // namespace tc
@@ -527,16 +538,24 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
 static const int kTcSmem = 1024 + tc::STAGE_AREA + tc::SCR_BYTES + 512;
 
-// per-launch tile counters of the dynamic scheduler (cycled; each launch zeroes its own)
+// per-launch tile and exit counters of the dynamic scheduler (cycled; a launch leaves its
+// pair zeroed)
 static int* g_sched = nullptr;
 static unsigned g_sched_seq = 0;
 constexpr int kSchedSlots = 1024;
 
 int tc_gemm_init() {
   static bool attr = false;
-  if (!g_sched && cudaMalloc(&g_sched, sizeof(int) * kSchedSlots) != cudaSuccess) {
-    g_sched = nullptr;
-    return fail(SBE_ERR_OOM, "tc_gemm: scheduler counters");
+  if (!g_sched) {
+    int* p = nullptr;
+    if (cudaMalloc(&p, sizeof(int) * 2 * kSchedSlots) != cudaSuccess)
+      return fail(SBE_ERR_OOM, "tc_gemm: scheduler counters");
+    if (cudaMemset(p, 0, sizeof(int) * 2 * kSchedSlots) != cudaSuccess ||
+        cudaStreamSynchronize(0) != cudaSuccess) {
+      cudaFree(p);
+      return cuda_check(cudaGetLastError(), "tc_gemm: scheduler counters");
+    }
+    g_sched = p;
   }
   if (!attr) {
     if (cudaFuncSetAttribute(tc::k_tc_gemm<tc::BN, tc::MODE_FULL>,
@@ -615,16 +634,14 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   }
   L.tile_base[njobs] = nt;
   if (nt == 0) return SBE_OK;
-  L.sched = g_sched + (g_sched_seq++ % kSchedSlots);
-  if (cudaMemsetAsync(L.sched, 0, sizeof(int), s) != cudaSuccess)
-    return cuda_check(cudaGetLastError(), "tc_gemm scheduler reset");
+  L.sched = g_sched + 2 * (g_sched_seq++ % kSchedSlots);
   const int grid = (int)std::min<long long>(nt, num_sms());
   if (mode == tc::MODE_HH)
-    tc::k_tc_gemm<tc::BN_HH, tc::MODE_HH><<<grid, tc::NUM_THREADS, kTcSmem, s>>>(L);
+    launch(tc::k_tc_gemm<tc::BN_HH, tc::MODE_HH>, grid, tc::NUM_THREADS, kTcSmem, s, L);
   else if (bnt == 128)
-    tc::k_tc_gemm<128, tc::MODE_FULL><<<grid, tc::NUM_THREADS, kTcSmem, s>>>(L);
+    launch(tc::k_tc_gemm<128, tc::MODE_FULL>, grid, tc::NUM_THREADS, kTcSmem, s, L);
   else
-    tc::k_tc_gemm<tc::BN, tc::MODE_FULL><<<grid, tc::NUM_THREADS, kTcSmem, s>>>(L);
+    launch(tc::k_tc_gemm<tc::BN, tc::MODE_FULL>, grid, tc::NUM_THREADS, kTcSmem, s, L);
   return cuda_check(cudaGetLastError(), "tc_gemm launch");
 }
 
