@@ -9,12 +9,27 @@
 
 namespace sbe {
 
+// round-to-nearest-even of x to FP32: results below the normal range become signed zero (see
+// the scaled form below), overflow infinity, NaN stays NaN.  The common case is a funnel shift,
+// one 64-bit add for the rounding and a select for zeros; what the branch takes is the last
+// value below 2^-126 and everything from 2^126.
+__device__ __forceinline__ float f64_to_f32(double x, int e);
+__device__ __forceinline__ float f64_to_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned sign = hi & 0x80000000u, a = hi & 0x7FFFFFFFu;
+  if (a >= 0x47E00000u || a == 0x380FFFFFu) return f64_to_f32(x, 0);
+  const unsigned t = __funnelshift_l(lo, a, 3);   // exponent and 23 bits, modulo 2^32
+  const unsigned long long r =
+      (((unsigned long long)(t + 0x40000000u) << 32) | (lo << 3)) + (0x7FFFFFFFu + (t & 1u));
+  return __uint_as_float(sign | (a < 0x380FFFFFu ? 0u : (unsigned)(r >> 32)));
+}
+
 // round-to-nearest-even of x * 2^e to FP32 (e is added to the exponent, so the
 // scaling is exact).  Results below the FP32 normal range (|x 2^e| < 2^-126)
 // become signed zero; overflow gives infinity; NaN stays NaN.  The 52-bit
 // mantissa is rounded to 23 bits with one 64-bit integer add (ties to even); a
 // carry out of the mantissa runs into the exponent field.
-__device__ __forceinline__ float f64_to_f32(double x, int e = 0) {
+__device__ __forceinline__ float f64_to_f32(double x, int e) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
   const unsigned long long a = u & 0x7FFFFFFFFFFFFFFFull;
@@ -34,24 +49,21 @@ __device__ __forceinline__ float f32_ldexp(float x, int e) {
   return x * __int_as_float((127 + e1) << 23) * __int_as_float((127 + e2) << 23);
 }
 
-// exact widening of an FP32 value to FP64
+// exact widening of an FP32 value to FP64 (normal values and zeros without a branch)
 __device__ __forceinline__ double f32_to_f64(float f) {
   const unsigned u = __float_as_uint(f);
-  const unsigned sign = u & 0x80000000u;
-  unsigned ex = (u >> 23) & 0xFFu;
-  unsigned m = u & 0x7FFFFFu;
-  if (ex == 0xFFu) {
-    return __hiloint2double((int)(sign | 0x7FF00000u | (m ? 0x80000u : 0u)), 0);
-  }
-  if (ex == 0) {
-    if (m == 0) return __hiloint2double((int)sign, 0);
+  const unsigned sign = u & 0x80000000u, a = u & 0x7FFFFFFFu;
+  if (a - 0x00800000u >= 0x7F000000u && a != 0) {
+    unsigned m = u & 0x7FFFFFu;
+    if (a >= 0x7F800000u)   // infinity or NaN
+      return __hiloint2double((int)(sign | 0x7FF00000u | (m ? 0x80000u : 0u)), 0);
     // FP32 subnormal m 2^-149: normalise the leading bit to bit 23
     const int sh = __clz((int)m) - 8;
     m = (m << sh) & 0x7FFFFFu;
     const unsigned e64 = (unsigned)(1 - 127 + 1023 - sh);
     return __hiloint2double((int)(sign | (e64 << 20) | (m >> 3)), (int)(m << 29));
   }
-  return __hiloint2double((int)(sign | ((ex - 127u + 1023u) << 20) | (m >> 3)), (int)(m << 29));
+  return __hiloint2double((int)(sign | (a ? (a >> 3) + 0x38000000u : 0u)), (int)(u << 29));
 }
 
 // f * 2^e exactly in FP64 (f finite; the result is assumed to stay normal)
@@ -61,7 +73,11 @@ __device__ __forceinline__ double f32_to_f64_scaled(float f, int e) {
   return __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
 }
 
-__device__ __forceinline__ float2 f64_to_f32(double2 v, int e = 0) {
+__device__ __forceinline__ float2 f64_to_f32(double2 v) {
+  return make_float2(f64_to_f32(v.x), f64_to_f32(v.y));
+}
+
+__device__ __forceinline__ float2 f64_to_f32(double2 v, int e) {
   return make_float2(f64_to_f32(v.x, e), f64_to_f32(v.y, e));
 }
 

@@ -22,6 +22,7 @@
 // Every transform is a radix-2 Stockham sequence in shared memory.  The work array
 // W is FP64 or FP32 complex (chosen at creation): with FP32 work the three middle
 // passes move half the bytes and the FP64 field is touched only by passes 1 and 5.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -349,96 +350,162 @@ __global__ void k_tables3(int n, double d, double* x, double* q, double2* tw, fl
 //      i q x F, inverse along x
 //   C  per plane: inverse along y and z, out (+)= a curl / N (- ja J), mask; in the
 //      field step C of the H update continues with pass A of the E update on the new
-//      H it has just written (the plane is still in shared memory)
-// The transforms run in place: radix-2 decimation in frequency (natural order in,
-// bit-reversed order out, exp(-i ...)) and its exact inverse, decimation in time
-// (bit-reversed in, natural out, unnormalised), two radix-2 stages fused per sweep
-// over shared memory.  The spectrum is never reordered: the curl is pointwise in k
-// space and reads the wavenumber of position p as q[bitrev(p)].
+//      H it has just written (the elements are still in registers)
+// The transforms are radix-2 decimation in frequency (natural order in, bit-reversed
+// order out, exp(-i ...)) and its exact inverse, decimation in time (bit-reversed in,
+// natural out, unnormalised).  The spectrum is never reordered: the curl is pointwise
+// in k space and reads the wavenumber of position p as q[bitrev(p)].
+//
+// A thread takes up to four radix-2 stages of 16 elements in registers, so a line of
+// 128 or 256 goes through shared memory once between its two groups of stages instead
+// of before and after every pair of them, and the first and last group of a pass work
+// straight from and to global memory.  The radix-4 sweeps over shared memory that this
+// replaces bound all three passes (one plane per SM, 9 round trips of 128 KB forward):
+// 256 x 128 x 128 step 1.14 -> 0.77 ms (per launch: A 157 -> 95 us, B 155 -> 81, C 339 -> 256;
+// 2.7 TB/s in A and C, whose single block per SM alternates between memory and transforms;
+// 1024 threads with groups of at most 8 elements 0.82 ms).
 constexpr int kPlaneMax = 16384;   // FP32 complex elements of one plane (128 KB)
-constexpr int kPlaneThreads = 1024;
-constexpr int kXThreads = 512;
+constexpr int kPlaneThreads = 512;
+constexpr int kXThreads = 256;
 constexpr int kXSmem = 96 * 1024;  // shared memory of one x-pass block's lines
 
+// Complex arithmetic with one fixed rounding per product wherever the compiler puts it, on the
+// two-wide FP32 instructions.
 __device__ __forceinline__ float2 c_mul(float2 a, float2 w) {
-  return make_float2(a.x * w.x - a.y * w.y, a.x * w.y + a.y * w.x);
+  return __ffma2_rn(a, make_float2(w.x, w.x), make_float2(-__fmul_rn(a.y, w.y), __fmul_rn(a.x, w.y)));
+}
+__device__ __forceinline__ float2 c_mul2(float2 a, float2 w) {   // the imaginary sum turned round
+  return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)),
+                     __fmaf_rn(a.x, w.y, __fmul_rn(a.y, w.x)));
 }
 __device__ __forceinline__ float2 c_mulc(float2 a, float2 w) {   // a conj(w)
-  return make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
+  return __ffma2_rn(a, make_float2(w.x, w.x), make_float2(__fmul_rn(a.y, w.y), -__fmul_rn(a.x, w.y)));
 }
-__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ int brev(int p, int lg) { return lg ? (int)(__brev((unsigned)p) >> (32 - lg)) : 0; }
+__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 c_sub(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
 
-// nl lines of n = 2^lg elements in shared memory, element p of line l at logical
-// index i = l * ls + p * es, stored at a[i + (i >> psh)] (psh > 0: one padding slot
-// after every 2^psh elements; the planes pad each row of nz, so that rows start on
-// successive banks); tw[j] = exp(-2 pi i j / n), j < n / 2.  line_fast: consecutive
-// threads take consecutive lines, else consecutive positions of one line.  Ends with
-// __syncthreads.
-__device__ __forceinline__ int smi(int i, int psh) { return psh ? i + (i >> psh) : i; }
-
-template <bool INV>
-__device__ void fft_inplace(float2* a, int lg, int nl, int ls, int es, bool line_fast,
-                            const float2* tw, int psh) {
-  const int n = 1 << lg, npair = lg >> 1, q4 = n >> 2;
-  if ((lg & 1) && INV) {
-    // the radix-2 stage of span 1 (twiddle 1): first for DIT, last for DIF
-    for (int u = threadIdx.x; u < nl * (n >> 1); u += blockDim.x) {
-      const int l = line_fast ? u % nl : u / (n >> 1), b = line_fast ? u / nl : u % (n >> 1);
-      const int i0 = l * ls + 2 * b * es;
-      const float2 x0 = a[smi(i0, psh)], x1 = a[smi(i0 + es, psh)];
-      a[smi(i0, psh)] = c_add(x0, x1);
-      a[smi(i0 + es, psh)] = c_sub(x0, x1);
-    }
-    __syncthreads();
+// Two radix-2 stages on x[0], x[ST], x[2 ST], x[3 ST] (positions m apart).
+template <bool INV, int ST>
+__device__ __forceinline__ void pair_stage(float2* x, float2 w1a, float2 w1b, float2 w2) {
+  const float2 x0 = x[0], x1 = x[ST], x2 = x[2 * ST], x3 = x[3 * ST];
+  if (!INV) {
+    const float2 a0 = c_add(x0, x2), a2 = c_mul(c_sub(x0, x2), w1a);
+    const float2 a1 = c_add(x1, x3), a3 = c_mul(c_sub(x1, x3), w1b);
+    x[0] = c_add(a0, a1);
+    x[ST] = c_mul(c_sub(a0, a1), w2);
+    x[2 * ST] = c_add(a2, a3);
+    x[3 * ST] = c_mul2(c_sub(a2, a3), w2);
+  } else {
+    const float2 t1 = c_mulc(x1, w2), t3 = c_mulc(x3, w2);
+    const float2 a0 = c_add(x0, t1), a1 = c_sub(x0, t1);
+    const float2 a2 = c_add(x2, t3), a3 = c_sub(x2, t3);
+    const float2 t2 = c_mulc(a2, w1a), t4 = c_mulc(a3, w1b);
+    x[0] = c_add(a0, t2);
+    x[2 * ST] = c_sub(a0, t2);
+    x[ST] = c_add(a1, t4);
+    x[3 * ST] = c_sub(a1, t4);
   }
-  for (int t = 0; t < npair; ++t) {
-    const int pi = INV ? npair - 1 - t : t;
-    const int m = n >> (2 * pi + 2), lgm = lg - 2 * pi - 2;
-    const int tws = q4 / m;     // n / (4 m): w_{4m}^j = tw[j tws]
-    for (int u = threadIdx.x; u < nl * q4; u += blockDim.x) {
-      const int l = line_fast ? u % nl : u / q4, r = line_fast ? u / nl : u % q4;
-      const int j = r & (m - 1), p0 = ((r >> lgm) << (lgm + 2)) + j;
-      const int sm = m * es, i0 = l * ls + p0 * es;
-      const int k0 = smi(i0, psh), k1 = smi(i0 + sm, psh), k2 = smi(i0 + 2 * sm, psh),
-                k3 = smi(i0 + 3 * sm, psh);
-      const float2 x0 = a[k0], x1 = a[k1], x2 = a[k2], x3 = a[k3];
-      const float2 w1a = tw[j * tws], w1b = tw[(j + m) * tws], w2 = tw[2 * j * tws];
-      float2 y0, y1, y2, y3;
-      if (!INV) {
-        const float2 a0 = c_add(x0, x2), a2 = c_mul(c_sub(x0, x2), w1a);
-        const float2 a1 = c_add(x1, x3), a3 = c_mul(c_sub(x1, x3), w1b);
-        y0 = c_add(a0, a1);
-        y1 = c_mul(c_sub(a0, a1), w2);
-        y2 = c_add(a2, a3);
-        y3 = c_mul(c_sub(a2, a3), w2);
-      } else {
-        const float2 t1 = c_mulc(x1, w2), t3 = c_mulc(x3, w2);
-        const float2 a0 = c_add(x0, t1), a1 = c_sub(x0, t1);
-        const float2 a2 = c_add(x2, t3), a3 = c_sub(x2, t3);
-        const float2 t2 = c_mulc(a2, w1a), t4 = c_mulc(a3, w1b);
-        y0 = c_add(a0, t2);
-        y2 = c_sub(a0, t2);
-        y1 = c_add(a1, t4);
-        y3 = c_sub(a1, t4);
+}
+
+// The radix-2 stage of span 1 (twiddle 1).
+__device__ __forceinline__ void last_stage(float2* x) {
+  const float2 x0 = x[0], x1 = x[1];
+  x[0] = c_add(x0, x1);
+  x[1] = c_sub(x0, x1);
+}
+
+// G radix-2 stages (the lowest of them of span 2^(top - G)) on the 2^G elements of a
+// thread, positions ... + i 2^(top - G) + j of a line of 2^lgn; tw[j] = exp(-2 pi i j / n)
+template <int G, bool INV>
+__device__ __forceinline__ void stages(float2 (&x)[1 << G], const float2* tw, int j, int lgn,
+                                       int top) {
+  constexpr int R = 1 << G;
+  if constexpr (G == 1) {
+    last_stage(x);
+  } else {
+    const int m = 1 << (top - 2), lgs = lgn - top;   // the upper pair: spans 2 m and m
+    auto upper = [&] {
+#pragma unroll
+      for (int i = 0; i < R / 4; ++i) {
+        const int jj = j + (i << (top - G));
+        pair_stage<INV, R / 4>(x + i, tw[jj << lgs], tw[(jj + m) << lgs], tw[(2 * jj) << lgs]);
       }
-      a[k0] = y0;
-      a[k1] = y1;
-      a[k2] = y2;
-      a[k3] = y3;
+    };
+    auto lower = [&] {
+      if constexpr (G == 4) {
+        const int l2 = lgs + 2, m2 = m >> 2;
+        const float2 w1a = tw[j << l2], w1b = tw[(j + m2) << l2], w2 = tw[(2 * j) << l2];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) pair_stage<INV, 1>(x + 4 * g, w1a, w1b, w2);
+      }
+      if constexpr (G == 3) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) last_stage(x + 2 * g);
+      }
+    };
+    if (INV) {
+      lower();
+      upper();
+    } else {
+      upper();
+      lower();
     }
-    __syncthreads();
   }
-  if ((lg & 1) && !INV) {
-    for (int u = threadIdx.x; u < nl * (n >> 1); u += blockDim.x) {
-      const int l = line_fast ? u % nl : u / (n >> 1), b = line_fast ? u / nl : u % (n >> 1);
-      const int i0 = l * ls + 2 * b * es;
-      const float2 x0 = a[smi(i0, psh)], x1 = a[smi(i0 + es, psh)];
-      a[smi(i0, psh)] = c_add(x0, x1);
-      a[smi(i0 + es, psh)] = c_sub(x0, x1);
-    }
-    __syncthreads();
+}
+
+// Stages of the group that starts at span 2^(top - 1): the pairs of stages from the top,
+// a last single one (odd lg) in a group with the pair above it.
+// The x lines end in a group of at most 8, since the curl holds it of all three components.
+enum Axis { YZ, X };
+template <Axis AX>
+__host__ __device__ constexpr int group(int top) {
+  return top >= 6 ? 4 : (top == 5 || (AX == X && top == 4) ? 2 : top);
+}
+
+// x[i] = ld(l, p0 + i 2^lgm); FP64 values are all loaded before the first conversion (its rare
+// branch would keep the later loads behind it)
+template <int R, class Ld>
+__device__ __forceinline__ void load_all(float2 (&x)[R], Ld ld, int l, int p0, int lgm) {
+  if constexpr (sizeof(ld(0, 0)) == sizeof(double2)) {
+    double2 v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = ld(l, p0 + (i << lgm));
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = f64_to_f32(v[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = ld(l, p0 + (i << lgm));
+  }
+}
+
+// One group of stages of every line: item u -> (line l, position base p0, twiddle index j)
+// by map, element i at position p0 + i 2^(top - G); ld and sv move them.
+template <int G, bool INV, class Map, class Ld, class Sv>
+__device__ __forceinline__ void group_pass(int items, int lgn, int top, const float2* tw, Map map,
+                                           Ld ld, Sv sv) {
+  const int lgm = top - G;
+  for (int u = threadIdx.x; u < items; u += blockDim.x) {
+    int l, r;
+    map(u, G, l, r);
+    const int j = r & ((1 << lgm) - 1), p0 = ((r >> lgm) << top) + j;
+    float2 x[1 << G];
+    load_all<1 << G>(x, ld, l, p0, lgm);
+    stages<G, INV>(x, tw, j, lgn, top);
+#pragma unroll
+    for (int i = 0; i < (1 << G); ++i) sv(l, p0 + (i << lgm), x[i]);
+  }
+}
+
+template <bool INV, Axis AX = YZ, class Map, class Ld, class Sv>
+__device__ __forceinline__ void any_group(int points, int lgn, int top, const float2* tw, Map map,
+                                          Ld ld, Sv sv) {
+  switch (group<AX>(top)) {
+    case 4: group_pass<4, INV>(points >> 4, lgn, top, tw, map, ld, sv); break;
+    case 3: group_pass<3, INV>(points >> 3, lgn, top, tw, map, ld, sv); break;
+    case 2: group_pass<2, INV>(points >> 2, lgn, top, tw, map, ld, sv); break;
+    default: group_pass<1, INV>(points >> 1, lgn, top, tw, map, ld, sv); break;
   }
 }
 
@@ -449,23 +516,73 @@ struct PlaneArgs {
   const float2* twz;
 };
 
-// padded plane of P elements in shared memory
+// padded plane of P elements in shared memory: one slot after each row of nz, so that
+// rows start on successive banks
 __host__ __device__ inline long long plane_slots(long long P, int lgz) { return P + (P >> lgz); }
 
-// shared memory of a plane block: the padded plane, then the y and z twiddles (half each)
-__device__ __forceinline__ void plane_tables(const PlaneArgs& A, float2* sty, float2* stz) {
-  for (int j = threadIdx.x; j < (A.ny >> 1); j += blockDim.x) sty[j] = A.twy[j];
-  for (int j = threadIdx.x; j < (A.nz >> 1); j += blockDim.x) stz[j] = A.twz[j];
-}
-
-// forward along z (rows of the plane) then y (columns)
-__device__ __forceinline__ void plane_forward(const PlaneArgs& A, float2* a, const float2* sty,
-                                              const float2* stz) {
-  // both directions with consecutive threads on consecutive lines: along z the lines
-  // are the padded rows (successive banks), along y the adjacent columns
-  fft_inplace<false>(a, A.lgz, A.ny, A.nz, 1, true, stz, A.lgz);
-  fft_inplace<false>(a, A.lgy, A.nz, 1, A.nz, true, sty, A.lgz);
-}
+// The plane in shared memory with its twiddles, and how items of its passes lie on threads.
+struct Plane {
+  float2 *a, *sty, *stz;
+  int lgy, lgz, row;              // slots per row
+  __device__ explicit Plane(const PlaneArgs& A, unsigned char* sm)
+      : a(reinterpret_cast<float2*>(sm)), lgy(A.lgy), lgz(A.lgz), row(A.nz + 1) {
+    sty = a + plane_slots(A.P, A.lgz);
+    stz = sty + (A.ny >> 1);
+    for (int j = threadIdx.x; j < (A.ny >> 1); j += blockDim.x) sty[j] = A.twy[j];
+    for (int j = threadIdx.x; j < (A.nz >> 1); j += blockDim.x) stz[j] = A.twz[j];
+  }
+  // along y: consecutive threads on consecutive columns
+  __device__ auto ymap() const {
+    return [lgz = lgz](int u, int, int& l, int& r) {
+      l = u & ((1 << lgz) - 1);
+      r = u >> lgz;
+    };
+  }
+  // along z within shared memory: consecutive threads on consecutive rows
+  __device__ auto zmap() const {
+    return [lgy = lgy](int u, int, int& l, int& r) {
+      l = u & ((1 << lgy) - 1);
+      r = u >> lgy;
+    };
+  }
+  // along z with a global side: consecutive threads on the 2^(lgz - G) consecutive points
+  // of a row, then (half a warp) on rows as far apart as that, for successive banks
+  __device__ auto zmap_global() const {
+    return [lgy = lgy, lgz = lgz](int u, int G, int& l, int& r) {
+      const int lgj = lgz - G;
+      r = u & ((1 << lgj) - 1);
+      l = u >> lgj;
+      if (lgj < 4 && lgy >= 4) {
+        const int h = 4 - lgj, q = l & 15;
+        l = (l & ~15) | ((q & ((1 << h) - 1)) << lgj) | (q >> h);
+      }
+    };
+  }
+  __device__ auto yat() const {
+    return [a = a, row = row](int l, int p) -> float2& { return a[p * row + l]; };
+  }
+  __device__ auto zat() const {
+    return [a = a, row = row](int l, int p) -> float2& { return a[l * row + p]; };
+  }
+  // forward: the groups of z after the first, then y; the last one to W
+  __device__ void forward_rest(const PlaneArgs& A, float2* W) const {
+    const auto z = zat();
+    const auto y = yat();
+    const int P = (int)A.P;
+    for (int top = lgz - group<YZ>(lgz); top > 0; top -= group<YZ>(top)) {
+      __syncthreads();
+      any_group<false>(P, lgz, top, stz, zmap(), z, [&](int l, int p, float2 v) { z(l, p) = v; });
+    }
+    for (int top = lgy; top > 0; top -= group<YZ>(top)) {
+      __syncthreads();
+      if (top > group<YZ>(top))
+        any_group<false>(P, lgy, top, sty, ymap(), y, [&](int l, int p, float2 v) { y(l, p) = v; });
+      else
+        any_group<false>(P, lgy, top, sty, ymap(), y,
+                         [&](int l, int p, float2 v) { W[(p << lgz) + l] = v; });
+    }
+  }
+};
 
 // pass A: plane (x = blockIdx.x, component blockIdx.y) of the FP64 field F -> W
 // (FP64 -> FP32 on the integer pipe: the FP64 pipe is ~1/64 of the FP32 rate here)
@@ -473,38 +590,65 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) k_plane_fwd(PlaneArgs A, con
                                                                 float2* W) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
-  float2* a = reinterpret_cast<float2*>(smraw);
-  float2* sty = a + plane_slots(A.P, A.lgz);
-  float2* stz = sty + (A.ny >> 1);
+  const Plane S(A, smraw);
   const long long base = blockIdx.y * A.N + blockIdx.x * A.P;
-  plane_tables(A, sty, stz);
-  // all loads of a thread before the stores to shared memory (4 per round)
-  for (int i0 = threadIdx.x; i0 < A.P; i0 += 4 * kPlaneThreads) {
-    double2 v[4];
+  F += base;
+  __syncthreads();   // twiddles
+  const auto z = S.zat();
+  any_group<false>((int)A.P, A.lgz, A.lgz, S.stz, S.zmap_global(),
+                   [&](int l, int p) { return F[(l << A.lgz) + p]; },
+                   [&](int l, int p, float2 v) { z(l, p) = v; });
+  S.forward_rest(A, W + base);
+}
+
+// The middle of pass B on the 2^G bottom positions of an x line of all three components:
+// the last forward stages, the curl, the first inverse stages.  qb*: the wavenumbers of the
+// bit-reversed positions as FP32 pairs (hi, lo): k f = fmaf(hi, f, lo f), one rounding per
+// product (an FP32 wavenumber alone is up to 6e-8 off, a fixed phase-velocity error of its
+// mode)
+template <int G, class Ld, class Sv>
+__device__ __forceinline__ void curl_group(const PlaneArgs& A, int lgx, int tl, long long b0,
+                                           const float2* tw, const float2* qbx, const float2* qby,
+                                           const float2* qbz, Ld ld, Sv sv) {
+  constexpr int R = 1 << G;
+  for (int u = threadIdx.x; u < (tl << lgx) >> G; u += blockDim.x) {
+    const int c = u & (tl - 1), p0 = (u / tl) << G;   // tl is a power of two
+    const long long col = b0 + c;
+    const float2 ky = qby[(int)(col >> A.lgz)], kz = qbz[(int)(col & (A.nz - 1))];
+    float2 x[3][R];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * kPlaneThreads;
-      v[u] = i < A.P ? F[base + i] : make_double2(0.0, 0.0);
+    for (int f = 0; f < 3; ++f) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[f][i] = ld(f, c, p0 + i);
+      stages<G, false>(x[f], tw, 0, lgx, G);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * kPlaneThreads;
-      if (i < A.P) a[smi(i, A.lgz)] = f64_to_f32(v[u]);
+    for (int i = 0; i < R; ++i) {
+      const float2 kx = qbx[p0 + i];
+      const float2 fx = x[0][i], fy = x[1][i], fz = x[2][i];
+      auto km = [](float2 k, float f) { return fmaf(k.x, f, k.y * f); };
+      // i (k x F)
+      const float cxr = km(ky, fz.x) - km(kz, fy.x), cxi = km(ky, fz.y) - km(kz, fy.y);
+      const float cyr = km(kz, fx.x) - km(kx, fz.x), cyi = km(kz, fx.y) - km(kx, fz.y);
+      const float czr = km(kx, fy.x) - km(ky, fx.x), czi = km(kx, fy.y) - km(ky, fx.y);
+      x[0][i] = make_float2(-cxi, cxr);
+      x[1][i] = make_float2(-cyi, cyr);
+      x[2][i] = make_float2(-czi, czr);
+    }
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      stages<G, true>(x[f], tw, 0, lgx, G);
+#pragma unroll
+      for (int i = 0; i < R; ++i) sv(f, c, p0 + i, x[f][i]);
     }
   }
-  __syncthreads();
-  plane_forward(A, a, sty, stz);
-  for (int i = threadIdx.x; i < A.P; i += kPlaneThreads) W[base + i] = a[smi(i, A.lgz)];
 }
 
 // pass B: the x lines of tl consecutive (y, z) columns of all three components;
-// shared memory [x][component][column].  qb*: the wavenumbers of the bit-reversed
-// positions as FP32 pairs (hi, lo): k f = fmaf(hi, f, lo f), one rounding per
-// product (an FP32 wavenumber alone is up to 6e-8 off, a fixed phase-velocity error
-// of its mode)
-__global__ void __launch_bounds__(kXThreads) k_x_curl_ip(PlaneArgs A, float2* W, int lgx, int tl,
-                                                         const float2* twx, const float2* qbx,
-                                                         const float2* qby, const float2* qbz) {
+// shared memory [x][component][column]
+__global__ void __launch_bounds__(kXThreads, 2) k_x_curl_ip(PlaneArgs A, float2* W, int lgx, int tl,
+                                                            const float2* twx, const float2* qbx,
+                                                            const float2* qby, const float2* qbz) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int nx = 1 << lgx, w3 = 3 * tl;
@@ -512,110 +656,161 @@ __global__ void __launch_bounds__(kXThreads) k_x_curl_ip(PlaneArgs A, float2* W,
   float2* stx = a + (size_t)nx * w3;
   for (int j = threadIdx.x; j < (nx >> 1); j += blockDim.x) stx[j] = twx[j];
   const long long b0 = (long long)blockIdx.x * tl;
-  const int total = nx * w3;
-  // four loads of a thread in flight before their stores to shared memory
-  for (int i0 = threadIdx.x; i0 < total; i0 += 4 * kXThreads) {
-    float2 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int idx = i0 + u * kXThreads;
-      if (idx < total) {
-        const int px = idx / w3, r = idx - px * w3, f = r / tl, c = r - f * tl;
-        v[u] = W[f * A.N + px * A.P + b0 + c];
-      }
+  W += b0;
+  const auto wat = [&](int f, int c, int p) -> float2& { return W[f * A.N + p * A.P + c]; };
+  const auto sat = [&](int f, int c, int p) -> float2& { return a[p * w3 + f * tl + c]; };
+  // lines of one component: consecutive threads on consecutive columns
+  const auto map = [&](int u, int, int& l, int& r) {
+    l = u & (tl - 1);
+    r = u / tl;
+  };
+  __syncthreads();   // twiddles
+  int top = lgx;
+  for (; top > group<X>(top); top -= group<X>(top)) {
+    for (int f = 0; f < 3; ++f)
+      if (top == lgx)
+        any_group<false, X>(tl << lgx, lgx, top, stx, map, [&](int l, int p) { return wat(f, l, p); },
+                         [&](int l, int p, float2 v) { sat(f, l, p) = v; });
+      else
+        any_group<false, X>(tl << lgx, lgx, top, stx, map, [&](int l, int p) { return sat(f, l, p); },
+                         [&](int l, int p, float2 v) { sat(f, l, p) = v; });
+    __syncthreads();
+  }
+  const auto ws = [&](int f, int c, int p, float2 v) { wat(f, c, p) = v; };
+  const auto ss = [&](int f, int c, int p, float2 v) { sat(f, c, p) = v; };
+  if (top == lgx) {   // at most 8 points: nothing goes through shared memory
+    switch (top) {
+      case 3: curl_group<3>(A, lgx, tl, b0, stx, qbx, qby, qbz, wat, ws); break;
+      case 2: curl_group<2>(A, lgx, tl, b0, stx, qbx, qby, qbz, wat, ws); break;
+      default: curl_group<1>(A, lgx, tl, b0, stx, qbx, qby, qbz, wat, ws); break;
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (i0 + u * kXThreads < total) a[i0 + u * kXThreads] = v[u];
+    return;
   }
-  __syncthreads();
-  fft_inplace<false>(a, lgx, w3, 1, w3, true, stx, 0);
-  for (int idx = threadIdx.x; idx < nx * tl; idx += blockDim.x) {
-    const int px = idx / tl, c = idx - px * tl;
-    const long long col = b0 + c;
-    const int py = (int)(col >> A.lgz), pz = (int)(col & (A.nz - 1));
-    const float2 kx = qbx[px], ky = qby[py], kz = qbz[pz];
-    float2* e = a + (size_t)px * w3 + c;
-    const float2 fx = e[0], fy = e[tl], fz = e[2 * tl];
-    auto km = [](float2 k, float f) { return fmaf(k.x, f, k.y * f); };
-    // i (k x F)
-    const float cxr = km(ky, fz.x) - km(kz, fy.x), cxi = km(ky, fz.y) - km(kz, fy.y);
-    const float cyr = km(kz, fx.x) - km(kx, fz.x), cyi = km(kz, fx.y) - km(kx, fz.y);
-    const float czr = km(kx, fy.x) - km(ky, fx.x), czi = km(kx, fy.y) - km(ky, fx.y);
-    e[0] = make_float2(-cxi, cxr);
-    e[tl] = make_float2(-cyi, cyr);
-    e[2 * tl] = make_float2(-czi, czr);
+  switch (top) {   // 2 or 3 below a group of its own
+    case 3: curl_group<3>(A, lgx, tl, b0, stx, qbx, qby, qbz, sat, ss); break;
+    default: curl_group<2>(A, lgx, tl, b0, stx, qbx, qby, qbz, sat, ss); break;
   }
-  __syncthreads();
-  fft_inplace<true>(a, lgx, w3, 1, w3, true, stx, 0);
-  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    const int px = idx / w3, r = idx - px * w3, f = r / tl, c = r - f * tl;
-    W[f * A.N + px * A.P + b0 + c] = a[idx];
+  // the inverse groups above, in the order of the forward ones turned round
+  while (top < lgx) {
+    int up = lgx;
+    while (up - group<X>(up) > top) up -= group<X>(up);
+    __syncthreads();
+    for (int f = 0; f < 3; ++f)
+      if (up == lgx)
+        any_group<true, X>(tl << lgx, lgx, up, stx, map, [&](int l, int p) { return sat(f, l, p); },
+                        [&](int l, int p, float2 v) { wat(f, l, p) = v; });
+      else
+        any_group<true, X>(tl << lgx, lgx, up, stx, map, [&](int l, int p) { return sat(f, l, p); },
+                        [&](int l, int p, float2 v) { sat(f, l, p) = v; });
+    top = up;
   }
 }
 
-// pass C: inverse along y and z of plane (x, component), then out (+)= ...: the
-// update of Upd (the masks per axis); with fwd_next the plane of the updated FP64
-// field continues as pass A of the next curl (W overwritten with its transform: the
-// block owns its plane of W).  The increment a v / N - ja J is formed in FP32 (v is
-// the FP32 transform; a / N and ja as FP32 pairs, J rounded to FP32 on the integer
-// pipe) and added to the FP64 field: one FP64 add per component; the mask multiplies
-// only where it is not 1.
+// The end of pass C on one thread's 2^G points of a z line: the last inverse stages, then
+// out (+)= ...: the update of Upd (the masks per axis); with fwd_next the updated values
+// continue as the first stages of the next curl.  The increment a v / N - ja J is formed in
+// FP32 (v is the FP32 transform; a / N and ja as FP32 pairs, J rounded to FP32 on the integer
+// pipe) and added to the FP64 field: one FP64 add per component; the mask multiplies only
+// where it is not 1.
+template <int G>
+__device__ __forceinline__ void update_group(const PlaneArgs& A, const Plane& S, const Upd& U,
+                                             long long base, int x, int fwd_next) {
+  constexpr int R = 1 << G;
+  const auto z = S.zat();
+  const auto map = S.zmap_global();
+  const double mx = U.m0 ? U.m0[x] : 1.0;
+  const bool xin = min(x, A.nx - 1 - x) >= U.nabc[0];
+  const int lgm = A.lgz - G;
+  double2* out = U.out + base;
+  const double2* J = U.J ? U.J + base : nullptr;
+  for (int u = threadIdx.x; u < (int)A.P >> G; u += blockDim.x) {
+    int y, j;
+    map(u, G, y, j);
+    float2 v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = z(y, j + (i << lgm));
+    stages<G, true>(v, S.stz, j, A.lgz, A.lgz);
+    const bool yin = xin && min(y, A.ny - 1 - y) >= U.nabc[1];
+    constexpr int B = R < 4 ? R : 4;   // FP64 loads of B points before their updates
+#pragma unroll
+    for (int i0 = 0; i0 < R; i0 += B) {
+      double2 o[B], jv[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int i = (y << A.lgz) + j + ((i0 + q) << lgm);
+        o[q] = U.store ? make_double2(0.0, 0.0) : out[i];
+        jv[q] = J ? J[i] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int zi = j + ((i0 + q) << lgm);
+        const float2 w = v[i0 + q];
+        float ix = fmaf(w.x, U.af[0], w.x * U.af[1]), iy = fmaf(w.y, U.af[0], w.y * U.af[1]);
+        if (J) {
+          const float2 jf = f64_to_f32(jv[q]);
+          ix -= fmaf(jf.x, U.jf[0], jf.x * U.jf[1]);
+          iy -= fmaf(jf.y, U.jf[0], jf.y * U.jf[1]);
+        }
+        double2 r = make_double2(o[q].x + f32_to_f64(ix), o[q].y + f32_to_f64(iy));
+        // FP64 only inside the absorbing layers (integer test of the position)
+        if (U.m0 && (!yin || min(zi, A.nz - 1 - zi) < U.nabc[2])) {
+          const double m = mx * U.m1[y] * U.m2[zi];
+          r.x *= m;
+          r.y *= m;
+        }
+        out[(y << A.lgz) + zi] = r;
+        v[i0 + q] = f64_to_f32(r);
+      }
+    }
+    if (fwd_next) {
+      stages<G, false>(v, S.stz, j, A.lgz, A.lgz);
+#pragma unroll
+      for (int i = 0; i < R; ++i) z(y, j + (i << lgm)) = v[i];
+    }
+  }
+}
+
+// pass C: inverse along y and z of plane (x, component), the update, and with fwd_next pass A
+// of the next curl (W overwritten with its transform: the block owns its plane of W)
 __global__ void __launch_bounds__(kPlaneThreads, 1) k_plane_inv(PlaneArgs A, float2* W, Upd U,
                                                                 int fwd_next) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
-  float2* a = reinterpret_cast<float2*>(smraw);
-  float2* sty = a + plane_slots(A.P, A.lgz);
-  float2* stz = sty + (A.ny >> 1);
-  const int x = blockIdx.x;
+  const Plane S(A, smraw);
+  const int x = blockIdx.x, P = (int)A.P;
   const long long base = blockIdx.y * A.N + x * A.P;
-  plane_tables(A, sty, stz);
-  for (int i = threadIdx.x; i < A.P; i += kPlaneThreads) a[smi(i, A.lgz)] = W[base + i];
-  __syncthreads();
-  fft_inplace<true>(a, A.lgy, A.nz, 1, A.nz, true, sty, A.lgz);
-  fft_inplace<true>(a, A.lgz, A.ny, A.nz, 1, true, stz, A.lgz);
-  const double mx = U.m0 ? U.m0[x] : 1.0;
-  const bool xin = min(x, A.nx - 1 - x) >= U.nabc[0];
-  for (int i0 = threadIdx.x; i0 < A.P; i0 += 2 * kPlaneThreads) {
-    // both elements' FP64 loads before their updates
-    double2 o[2], jv[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = i0 + u * kPlaneThreads;
-      const bool in = i < A.P;
-      o[u] = (in && !U.store) ? U.out[base + i] : make_double2(0.0, 0.0);
-      jv[u] = (in && U.J) ? U.J[base + i] : make_double2(0.0, 0.0);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = i0 + u * kPlaneThreads;
-      if (i >= A.P) continue;
-      const float2 v = a[smi(i, A.lgz)];
-      float ix = fmaf(v.x, U.af[0], v.x * U.af[1]), iy = fmaf(v.y, U.af[0], v.y * U.af[1]);
-      if (U.J) {
-        const float2 jf = f64_to_f32(jv[u]);
-        ix -= fmaf(jf.x, U.jf[0], jf.x * U.jf[1]);
-        iy -= fmaf(jf.y, U.jf[0], jf.y * U.jf[1]);
-      }
-      double2 r = make_double2(o[u].x + f32_to_f64(ix), o[u].y + f32_to_f64(iy));
-      if (U.m0) {
-        // FP64 only inside the absorbing layers (integer test of the position)
-        const int y = i >> A.lgz, z = i & (A.nz - 1);
-        if (!xin || min(y, A.ny - 1 - y) < U.nabc[1] || min(z, A.nz - 1 - z) < U.nabc[2]) {
-          const double m = mx * U.m1[y] * U.m2[z];
-          r.x *= m;
-          r.y *= m;
-        }
-      }
-      U.out[base + i] = r;
-      if (fwd_next) a[smi(i, A.lgz)] = f64_to_f32(r);
-    }
+  float2* w = W + base;
+  const auto z = S.zat();
+  const auto y = S.yat();
+  // y from the lowest group up, the first one from W
+  for (int top = 0; top < A.lgy;) {
+    int up = A.lgy;
+    while (up - group<YZ>(up) > top) up -= group<YZ>(up);
+    __syncthreads();
+    if (top == 0)
+      any_group<true>(P, A.lgy, up, S.sty, S.ymap(),
+                      [&](int l, int p) { return w[(p << A.lgz) + l]; },
+                      [&](int l, int p, float2 v) { y(l, p) = v; });
+    else
+      any_group<true>(P, A.lgy, up, S.sty, S.ymap(), y,
+                      [&](int l, int p, float2 v) { y(l, p) = v; });
+    top = up;
   }
-  if (!fwd_next) return;   // block-uniform
+  for (int top = 0; top < A.lgz - group<YZ>(A.lgz);) {
+    int up = A.lgz;
+    while (up - group<YZ>(up) > top) up -= group<YZ>(up);
+    __syncthreads();
+    any_group<true>(P, A.lgz, up, S.stz, S.zmap(), z, [&](int l, int p, float2 v) { z(l, p) = v; });
+    top = up;
+  }
   __syncthreads();
-  plane_forward(A, a, sty, stz);
-  for (int i = threadIdx.x; i < A.P; i += kPlaneThreads) W[base + i] = a[smi(i, A.lgz)];
+  switch (group<YZ>(A.lgz)) {
+    case 4: update_group<4>(A, S, U, base, x, fwd_next); break;
+    case 3: update_group<3>(A, S, U, base, x, fwd_next); break;
+    case 2: update_group<2>(A, S, U, base, x, fwd_next); break;
+    default: update_group<1>(A, S, U, base, x, fwd_next); break;
+  }
+  if (fwd_next) S.forward_rest(A, w);   // block-uniform
 }
 
 bool pow2(int v) { return v >= 2 && v <= 1024 && (v & (v - 1)) == 0; }
@@ -731,6 +926,11 @@ size_t plane_smem(const PlaneArgs& A) {
   return sizeof(float2) * ((size_t)plane_slots(A.P, A.lgz) + (A.ny >> 1) + (A.nz >> 1));
 }
 
+// 16 points per thread, so that small planes share an SM
+int plane_threads(const PlaneArgs& A) {
+  return (int)std::min<long long>(kPlaneThreads, std::max<long long>(32, A.P / 16));
+}
+
 // x-pass columns per block: the three components' x lines of tl columns within
 // kXSmem, tl <= 16 and dividing the plane
 int x_lines(const SbePstd3* p) {
@@ -742,7 +942,7 @@ int x_lines(const SbePstd3* p) {
 
 int plane_pass_a(SbePstd3* p, const double2* F, cudaStream_t s) {
   const PlaneArgs A = plane_args(p);
-  launch(k_plane_fwd, dim3(A.nx, 3), kPlaneThreads, plane_smem(A), s, A, F,
+  launch(k_plane_fwd, dim3(A.nx, 3), plane_threads(A), plane_smem(A), s, A, F,
          static_cast<float2*>(p->work));
   return cuda_check(cudaGetLastError(), "pstd3 plane pass");
 }
@@ -758,7 +958,7 @@ int plane_pass_b(SbePstd3* p, cudaStream_t s) {
 
 int plane_pass_c(SbePstd3* p, const Upd& U, int fwd_next, cudaStream_t s) {
   const PlaneArgs A = plane_args(p);
-  launch(k_plane_inv, dim3(A.nx, 3), kPlaneThreads, plane_smem(A), s, A,
+  launch(k_plane_inv, dim3(A.nx, 3), plane_threads(A), plane_smem(A), s, A,
          static_cast<float2*>(p->work), U, fwd_next);
   return cuda_check(cudaGetLastError(), "pstd3 plane pass");
 }
