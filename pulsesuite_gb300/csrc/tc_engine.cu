@@ -269,8 +269,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       // a last N tile narrower than BNT (MODE_FULL) loads only the B rows its
       // MMAs read, rounded up to the 64-row tile granule
       const int nrem = d.N - ti.n0;
-      const int bbytes = (HH || nrem >= BNT) ? BTB : ((nrem + 63) & ~63) * BK * 2;
-      const uint32_t tx_bytes = (uint32_t)(npl * (A_TILE_BYTES + bbytes));
+      const int bbytes = (HH || BNT <= 64 || nrem >= BNT) ? BTB : ((nrem + 63) & ~63) * BK * 2;
+      // so does a last M tile of A (the MMAs' rows beyond it are never read back)
+      const int abytes = d.M - ti.m0 > 64 ? A_TILE_BYTES : A_TILE_BYTES / 2;
+      const uint32_t tx_bytes = (uint32_t)(npl * (abytes + bbytes));
       int s = (int)(g % nstage);
       uint32_t ph = (uint32_t)((g / nstage) & 1);
       for (int part = 0; ok && part < ti.nparts; ++part) {
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           const __half* ga = ga0 + kk * kstepA;
           const __half* gb = gb0 + kk * kstepB;
           for (int p = 0; p < npl; ++p) {
-            bulk_load(sa + p * A_TILE_BYTES, ga + p * pA, A_TILE_BYTES, &full[s]);
+            bulk_load(sa + p * A_TILE_BYTES, ga + p * pA, abytes, &full[s]);
             bulk_load(sb + p * BTB, gb + p * pB, bbytes, &full[s]);
           }
           if (++s == nstage) {
@@ -558,13 +560,15 @@ int tc_gemm_init() {
     g_sched = p;
   }
   if (!attr) {
-    if (cudaFuncSetAttribute(tc::k_tc_gemm<tc::BN, tc::MODE_FULL>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(tc::k_tc_gemm<128, tc::MODE_FULL>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(tc::k_tc_gemm<tc::BN_HH, tc::MODE_HH>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
-      return fail(SBE_ERR_CUDA, "tc_gemm: cannot raise the shared-memory limit");
+    using Kernel = void (*)(const tc::GemmLaunch);
+    const Kernel kernels[] = {
+        tc::k_tc_gemm<256, tc::MODE_FULL>, tc::k_tc_gemm<128, tc::MODE_FULL>,
+        tc::k_tc_gemm<64, tc::MODE_FULL>,  tc::k_tc_gemm<128, tc::MODE_HH>,
+        tc::k_tc_gemm<64, tc::MODE_HH>};
+    for (Kernel k : kernels)
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) !=
+          cudaSuccess)
+        return fail(SBE_ERR_CUDA, "tc_gemm: cannot raise the shared-memory limit");
     attr = true;
   }
   return SBE_OK;
@@ -597,6 +601,68 @@ static bool job_ok(const tc::GemmDesc& d) {
   return ok;
 }
 
+// Time of a launch at N tile bnt in units of one K block of one product on a 256-wide tile: the
+// larger of the longest tile and an even share of all tiles.  A product's time falls with the
+// tile's width to 0.55 at 64 and below (the 128 rows of A bound it there), the epilogue costs
+// 0.17 a column; the band of an exchange tile shortens its K range, tiles outside it are dead.
+static double launch_cost(const tc::GemmJob* jobs, int njobs, int bnt) {
+  double total = 0.0, longest = 0.0;
+  for (int j = 0; j < njobs; ++j) {
+    const tc::GemmDesc& d = jobs[j].d;
+    const int products = d.complex_mode ? (d.xonly ? 8 : 12) : 3;
+    const int ks = d.ksplit > 1 && !d.kseq ? d.ksplit : 1;
+    for (int n0 = 0; n0 < d.N; n0 += bnt) {
+      const int w = std::min(bnt, d.N - n0);
+      int kb = (d.K + tc::BK - 1) / tc::BK, rows = (d.M + tc::BM - 1) / tc::BM;
+      if (d.kskip) {
+        const int nk = d.nk_shear, lo = n0 / 2, hi = std::min((n0 + bnt) / 2, 2 * nk - 1) - 1;
+        const int tlo = std::max(0, nk - 1 - hi), thi = std::min(nk - 1, 2 * nk - 2 - lo);
+        kb = thi >= tlo ? thi / tc::BK + 1 - tlo / tc::BK : 0;
+        int live = 0;
+        for (int m0 = 0; m0 < d.M; m0 += tc::BM)
+          live += lo + m0 <= 2 * nk - 2 && hi + std::min(m0 + tc::BM, d.M) - 1 >= nk - 1;
+        rows = live;
+      }
+      const double t = std::max(0.55, 0.2 + w / 320.0) * products * d.nterms * kb / ks + 0.17 * w;
+      if (rows) longest = std::max(longest, t);
+      total += t * rows * d.batch * ks;
+    }
+  }
+  return std::max(longest, total / num_sms());
+}
+
+// The N tile of a launch: the jobs' own (256, or 128 where chosen), narrowed where that brings
+// the launch at least a fifth closer to an even load of the SMs.  The products of an element and
+// their order are the same at every width.  1 x 256 (commutators, exchange, sources): 256-wide
+// 62, 16, 25 us, 128-wide 41, 12, 17, 64-wide 39, 11, 16; 4 x 512: 115, 32, 71 / 75, 35, 64 /
+// 123, 51, 112; 16 x 512: 217, 79, 209 / 226, 105, 229 / 410, 170, 393.  hi*hi launches take
+// 64-wide tiles while those fit the SMs in one wave: 1 x 256 29 -> 18 us, 8 x 256 30 -> 19,
+// 4 x 512 (two waves) 37 -> 40.
+static int n_tile(const tc::GemmJob* jobs, int njobs, int mode, int widest) {
+  int nmax = 0;
+  for (int j = 0; j < njobs; ++j) nmax = std::max(nmax, jobs[j].d.N);
+  // no wider than the matrix: a narrower stage leaves room for more of them
+  while (widest > 64 && nmax <= widest / 2) widest /= 2;
+  long long tiles = 0;   // of the widest, an upper bound of the CTAs at work
+  for (int j = 0; j < njobs; ++j) {
+    const tc::GemmDesc& d = jobs[j].d;
+    const int n = mode == tc::MODE_HH ? 64 : widest;
+    tiles += (long long)((d.N + n - 1) / n) * ((d.M + tc::BM - 1) / tc::BM) * d.batch;
+  }
+  if (mode == tc::MODE_HH) return tiles <= num_sms() ? 64 : tc::BN_HH;
+  if (tiles > 4LL * num_sms()) return widest;
+  int best = widest;
+  double cost = launch_cost(jobs, njobs, widest);
+  for (int n = widest / 2; n >= 64; n /= 2) {
+    const double c = launch_cost(jobs, njobs, n);
+    if (c < 0.8 * cost) {
+      best = n;
+      cost = c;
+    }
+  }
+  return best;
+}
+
 int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   int rc = tc_gemm_init();
   if (rc) return rc;
@@ -609,7 +675,7 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   if (mode != tc::MODE_FULL && mode != tc::MODE_HH) return fail(SBE_ERR_ARG, "tc_gemm: bad mode");
   const int bn = jobs[0].d.bn;
   if (bn != 0 && bn != 128 && bn != 256) return fail(SBE_ERR_ARG, "tc_gemm: N tile 128 or 256");
-  const int bnt = mode == tc::MODE_HH ? tc::BN_HH : (bn == 128 ? 128 : tc::BN);
+  const int bnt = n_tile(jobs, njobs, mode, bn == 128 ? 128 : tc::BN);
   long long nt = 0;
   for (int j = 0; j < njobs; ++j) {
     const tc::GemmDesc& d = jobs[j].d;
@@ -636,12 +702,13 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   if (nt == 0) return SBE_OK;
   L.sched = g_sched + 2 * (g_sched_seq++ % kSchedSlots);
   const int grid = (int)std::min<long long>(nt, num_sms());
-  if (mode == tc::MODE_HH)
-    launch(tc::k_tc_gemm<tc::BN_HH, tc::MODE_HH>, grid, tc::NUM_THREADS, kTcSmem, s, L);
-  else if (bnt == 128)
-    launch(tc::k_tc_gemm<128, tc::MODE_FULL>, grid, tc::NUM_THREADS, kTcSmem, s, L);
-  else
-    launch(tc::k_tc_gemm<tc::BN, tc::MODE_FULL>, grid, tc::NUM_THREADS, kTcSmem, s, L);
+  void (*const kernel)(const tc::GemmLaunch) =
+      mode == tc::MODE_HH ? (bnt == 64 ? tc::k_tc_gemm<64, tc::MODE_HH>
+                                       : tc::k_tc_gemm<tc::BN_HH, tc::MODE_HH>)
+      : bnt == 64  ? tc::k_tc_gemm<64, tc::MODE_FULL>
+      : bnt == 128 ? tc::k_tc_gemm<128, tc::MODE_FULL>
+                   : tc::k_tc_gemm<tc::BN, tc::MODE_FULL>;
+  launch(kernel, grid, tc::NUM_THREADS, kTcSmem, s, L);
   return cuda_check(cudaGetLastError(), "tc_gemm launch");
 }
 

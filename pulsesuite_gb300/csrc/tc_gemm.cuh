@@ -8,7 +8,7 @@
 // textbook formula (conjugation and sign by the MMA's operand-negate bit), all
 // accumulated in FP32 in tensor memory.
 //
-// Tiles: BM = 128 rows, BN = 256 or 128 columns, BK = 32 (64-byte rows,
+// Tiles: BM = 128 rows, BN = 256, 128 or 64 columns, BK = 32 (64-byte rows,
 // K-major on both operands, 64-byte swizzle).  The planes live in global memory
 // in the tile layout of PlaneSet: every operand tile is one contiguous chunk,
 // moved to shared memory with a single cp.async.bulk.
@@ -30,7 +30,7 @@ namespace tc {
 
 constexpr int BM = 128;
 constexpr int BN = 256;
-constexpr int BN_HH = 128;     // N tile of the hi*hi mode (MMA N = 256 over re and im of B)
+constexpr int BN_HH = 128;     // widest N tile of the hi*hi mode (MMA N = 256 over re and im of B)
 constexpr int BK = 32;
 constexpr int A_TILE_BYTES = BM * BK * 2;   // 8 KB
 constexpr int B_TILE_BYTES = BN * BK * 2;   // 16 KB
@@ -146,7 +146,8 @@ struct GemmDesc {
   int kacc;
   // N tile of MODE_FULL: 256 (0 = the default) or 128; with 128 a complex tile's
   // accumulators take 256 TMEM columns, so two tiles are in flight (the epilogue of
-  // one overlaps the MMAs of the next) at twice the operand loads per output
+  // one overlaps the MMAs of the next) at twice the operand loads per output.  The
+  // widest the launch takes: with few tiles it narrows them (n_tile, tc_engine.cu)
   int bn;
   PlaneSet A, B;              // operand planes (A: M rows, B: N rows, both K-major)
 };
