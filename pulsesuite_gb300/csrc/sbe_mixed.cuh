@@ -65,6 +65,7 @@ struct MixedAll {
   float2* ekf = nullptr;     // 3 x tot_r stage field
   float2* ekrf = nullptr;    // tot_kr Expikr
   int* err = nullptr;        // engine error flag (bounded waits that gave up)
+  unsigned* mx = nullptr;    // the buckets' maxima (4 x nw in all)
 };
 
 // matrix slots of the commutator plane sets

@@ -16,6 +16,7 @@
 #include "sbe_ctx.cuh"
 #include "tc_gemm.cuh"
 #include "sbe_mixed.cuh"
+#include "batch.cuh"
 
 namespace sbe {
 
@@ -36,31 +37,36 @@ __global__ void k_absmax(const double2* X, long long per_batch, long long bstrid
   if ((threadIdx.x & 31) == 0) atomicMax(out + b, bits_to_fmax(m));
 }
 
-// e[b] = 14 - ceil(log2(max)): scaled magnitudes stay <= 2^14 (FP16 max 65504).
-__global__ void k_exponents(int nb, const unsigned* mx, int* e, const int* add, int* sum) {
-  pdl_enter();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+// 14 - ceil(log2(max)): scaled magnitudes stay <= 2^14 (FP16 max 65504).
+__device__ __forceinline__ int exponent_of(float mx) {
+  const float m = mx * 1.0001f;
+  return (m > 0.f) ? 14 - (int)ceilf(log2f(m)) : 0;
+}
+
+// e[b] of the maximum mx[b]; sum[b] = e[b] + add[b]
+__device__ __forceinline__ void exponents(Blk blk, int nb, const unsigned* mx, int* e,
+                                          const int* add, int* sum) {
+  int b = blk.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
-  float m = __uint_as_float(mx[b]) * 1.0001f;
-  int v = (m > 0.f) ? 14 - (int)ceilf(log2f(m)) : 0;
+  const int v = exponent_of(__uint_as_float(mx[b]));
   e[b] = v;
   if (sum) sum[b] = v + (add ? add[b] : 0);
 }
+SBE_PASS(ExponentsPass, 128, exponents);
 
 // The exponents of one stage in one launch (one thread per wire): eS from the
 // full state maximum, eO from the off-diagonal one, esx = eT + eS (exchange
 // products); with reset set the maxima are cleared for the fused RK4 update of
 // the stage, which collects the next state's maxima in them; mxH is cleared for
 // the stage's Hamiltonian.
-__global__ void k_stage_exponents(int nb, unsigned* mxS, unsigned* mxO, unsigned* mxH, int* eS,
-                                  int* eO, const int* eT, int* esx, int reset) {
-  pdl_enter();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void stage_exponents(Blk blk, int nb, unsigned* mxS, unsigned* mxO,
+                                                unsigned* mxH, int* eS, int* eO, const int* eT,
+                                                int* esx, int reset) {
+  const int b = blk.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
-  const float ms = __uint_as_float(mxS[b]) * 1.0001f, mo = __uint_as_float(mxO[b]) * 1.0001f;
-  const int vs = (ms > 0.f) ? 14 - (int)ceilf(log2f(ms)) : 0;
+  const int vs = exponent_of(__uint_as_float(mxS[b]));
   eS[b] = vs;
-  eO[b] = (mo > 0.f) ? 14 - (int)ceilf(log2f(mo)) : 0;
+  eO[b] = exponent_of(__uint_as_float(mxO[b]));
   esx[b] = eT[b] + vs;
   mxH[b] = 0u;
   if (reset) {
@@ -68,18 +74,19 @@ __global__ void k_stage_exponents(int nb, unsigned* mxS, unsigned* mxO, unsigned
     mxO[b] = 0u;
   }
 }
+SBE_PASS(StageExponentsPass, 128, stage_exponents);
 
 // e[b] from the larger of two maxima (rule of k_exponents) and sum[b] = e[b] + add[b]
-__global__ void k_exponents2_sum(int nb, const unsigned* mx1, const unsigned* mx2, int* e,
-                                 const int* add, int* sum) {
-  pdl_enter();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void exponents2_sum(Blk blk, int nb, const unsigned* mx1,
+                                               const unsigned* mx2, int* e, const int* add,
+                                               int* sum) {
+  const int b = blk.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
-  const float m = fmaxf(__uint_as_float(mx1[b]), __uint_as_float(mx2[b])) * 1.0001f;
-  const int v = (m > 0.f) ? 14 - (int)ceilf(log2f(m)) : 0;
+  const int v = exponent_of(fmaxf(__uint_as_float(mx1[b]), __uint_as_float(mx2[b])));
   e[b] = v;
   sum[b] = v + add[b];
 }
+SBE_PASS(HamExponentsPass, 128, exponents2_sum);
 
 __device__ __forceinline__ void put_hilo(__half* base, long long plane, float v) {
   const __half h = __float2half_rn(v);
@@ -184,13 +191,13 @@ __device__ __forceinline__ void store_tiles_t(const __half (*hs)[32][40], int np
 // The block (32 x 8 threads) converts its 32 x 32 tile once into shared-memory
 // plane tiles and writes both layouts with 16-byte stores.
 template <typename T>
-__global__ void k_planes_nt(const T* X, int nk, const int* e, tc::PlaneSet dst, int matN, int matT,
-                            int nbatch, float* cdf = nullptr, const double* dg = nullptr) {
-  pdl_enter();
+__device__ __forceinline__ void planes_nt(Blk blk, const T* X, int nk, const int* e,
+                                          tc::PlaneSet dst, int matN, int matT, int nbatch,
+                                          float* cdf, const double* dg) {
   __shared__ T tile[32][33];
   __shared__ __align__(16) __half hs[4][32][40];
-  const int b = blockIdx.z;
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  const int b = blk.z;
+  const int r0 = blk.y * 32, c0 = blk.x * 32;
   const T* x = X + (long long)b * nk * nk;
   {
     // block (32, 8): four rows per thread, all loads issued before the stores
@@ -228,6 +235,8 @@ __global__ void k_planes_nt(const T* X, int nk, const int* e, tc::PlaneSet dst, 
   store_tiles(hs, 4, dst, matN, b, r0, c0 >> 5, tid, nth);
   if (matT >= 0) store_tiles_t(hs, 4, dst, matT, b, c0, r0 >> 5, tid, nth);
 }
+SBE_PASS(PlanesPass, 256, planes_nt<float2>);
+SBE_PASS(Planes64Pass, 256, planes_nt<double2>);
 
 // Band of the sheared state planes (k_shear_tiles): the first dd block of the
 // t' block at t0 whose source rows can reach the matrix, and whether the block
@@ -244,10 +253,10 @@ __host__ __device__ inline bool shear_block_live(int nk, int t0, int dd0) {
 // Traces from the diagonal partials of k_shear_tiles: diagonal dd = k1 - k2 + Nk - 1
 // of X (row k1, column k2) is trace index d + Nk with d = k2 - k1, summed over the
 // nb column blocks in a fixed order into trf[b][which][d + Nk] (SBEs.py:1094-1103).
-__global__ void k_trace_from_shear(int nk, int nb, int ndd, const float2* dpart, float2* trf) {
-  pdl_enter();
-  const int b = blockIdx.z, which = blockIdx.y;
-  const int dd = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void trace_from_shear(Blk blk, int nk, int nb, int ndd,
+                                                 const float2* dpart, float2* trf) {
+  const int b = blk.z, which = blk.y;
+  const int dd = blk.x * blockDim.x + threadIdx.x;
   if (dd >= 2 * nk - 1) return;
   const float2* part = dpart + (((long long)b * 2 + which) * ndd + dd) * nb;
   float sr = 0.f, si = 0.f;
@@ -259,21 +268,24 @@ __global__ void k_trace_from_shear(int nk, int nb, int ndd, const float2* dpart,
   }
   trf[(long long)b * 4 * nk + which * 2 * nk + (2 * nk - 1 - dd)] = make_float2(sr, si);
 }
+SBE_PASS(TracesPass, 128, trace_from_shear);
 
 void launch_exponents(const double2* X, long long per_batch, long long bstride, int nbatch,
                       unsigned* mx, int* e, const int* add, int* sum, cudaStream_t s) {
   cudaMemsetAsync(mx, 0, sizeof(unsigned) * nbatch, s);
   int blocks = (int)std::min<long long>((per_batch + 255) / 256, 256);
   launch(k_absmax, dim3(blocks, nbatch), 256, 0, s, X, per_batch, bstride, mx);
-  launch(k_exponents, (nbatch + 127) / 128, 128, 0, s, nbatch, mx, e, add, sum);
+  Batch<ExponentsPass> pass(128, s);
+  pass.add((nbatch + 127) / 128, nbatch, mx, e, add, sum);
 }
 
 // ---------------------------------------------------------------------------
 // Mixed-precision workspace of a context.  The layout groups the wires by Nk, so
 // the wires of one Nk form a bucket whose matrices are one contiguous block of
-// every packed buffer: the per-element kernels run once per bucket (uniform Nk,
-// grid z = the bucket's wires) on pointers offset to the bucket's block, and each
-// GEMM kind runs as one persistent launch over the jobs of all buckets.
+// every packed buffer: a per-element pass is one launch whose parts are the buckets
+// (uniform Nk, grid z = the bucket's wires, pointers offset to the bucket's block;
+// batch.cuh), and each GEMM kind runs as one persistent launch over the jobs of all
+// buckets.
 //
 // Per bucket, commutator planes: 14 matrix slots x 4 planes x Nw x Nk x Nk (FP16):
 //   0 P, 1 P^T, 2 C, 4 D                            (state, exponent eS)
@@ -409,7 +421,6 @@ static void carve_bucket(Mixed* m, Carver& k) {
   const size_t v = (size_t)m->nw * m->nk;
   const int T = (m->nk + 31) / 32;
   m->ints = k.take<int>(9 * (size_t)m->nw);
-  m->mx = k.take<unsigned>(4 * (size_t)m->nw);
   m->mx64 = k.take<unsigned long long>((size_t)m->nw);
   m->sP = k.take<int>((size_t)m->nw);
   m->vsf = k.take<float>(3 * v);
@@ -439,6 +450,7 @@ static void carve_all(MixedAll* A, Carver& k, const SbeCtx* c) {
   A->ekf = k.take<float2>(3 * (size_t)c->tot_r);
   A->ekrf = k.take<float2>((size_t)c->tot_kr);
   A->err = k.take<int>(1);
+  A->mx = k.take<unsigned>(4 * (size_t)c->nw);
 }
 
 static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
@@ -523,7 +535,7 @@ static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
     const long long mm = (long long)nk * nk;
     const int T = (nk + 31) / 32;
     cudaMemsetAsync(m->ints, 0, sizeof(int) * 9 * nw, s);
-    cudaMemsetAsync(m->mx, 0, sizeof(unsigned) * 4 * nw, s);
+    m->mx = A->mx + 4 * (size_t)m->first;
     // the padding of every plane set stays zero: producers write only inside; the
     // sheared planes are zeroed once, stages write only the in-band part
     cudaMemsetAsync(m->pl.ptr, 0, tc::planeset_bytes(m->pl), s);
@@ -551,12 +563,10 @@ static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
 // set the FP64 real diagonal (the occupations of C and D, which the peeled terms
 // use beyond FP32).  The diagonal is tracked by a row / column counter stepped
 // with the grid stride (no division per element).
-__global__ void __launch_bounds__(256) k_state_in(const double2* __restrict__ X, int nk, int peel,
-                                                  unsigned* __restrict__ mx,
-                                                  unsigned* __restrict__ mo,
-                                                  float2* __restrict__ xf, double* __restrict__ dg) {
-  pdl_enter();
-  const int b = blockIdx.y;
+__device__ __forceinline__ void state_in(Blk blk, const double2* __restrict__ X, int nk, int peel,
+                                         unsigned* __restrict__ mx, unsigned* __restrict__ mo,
+                                         float2* __restrict__ xf, double* __restrict__ dg) {
+  const int b = blk.y;
   const int per = nk * nk;   // < 2^31
   const double2* x = X + (long long)b * per;
   float2* y = xf + (long long)b * per;
@@ -564,9 +574,9 @@ __global__ void __launch_bounds__(256) k_state_in(const double2* __restrict__ X,
   // four elements per thread and pass (stride S), loads issued together; the
   // diagonal is tracked by row / column counters stepped with S (no division per
   // element)
-  const int S = gridDim.x * blockDim.x;
+  const int S = blk.gx * blockDim.x;
   const int srow = S / nk, scol = S % nk;
-  const int i00 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i00 = blk.x * blockDim.x + threadIdx.x;
   int row = i00 / nk, col = i00 % nk;
   for (int i0 = i00; i0 < per; i0 += 4 * S) {
     double2 v[4];
@@ -615,26 +625,21 @@ __global__ void __launch_bounds__(256) k_state_in(const double2* __restrict__ X,
     atomicMax(mo + b, o);
   }
 }
-
-static void absmax_into(const double2* X, long long per, int nw, unsigned* mx, cudaStream_t s) {
-  int blocks = (int)std::min<long long>((per + 255) / 256, 128);
-  launch(k_absmax, dim3(blocks, nw), 256, 0, s, X, per, per, mx);
-}
+SBE_PASS(StateInPass, 256, state_in);
 
 // ---------------------------------------------------------------------------
 // Per-step tables of the mixed path (coefficients frozen over the step).
 
 // Toeplitz exchange planes T_n[t][t'] = vs_n(|t - t'|) (t != t'), real; and the
 // FP32 copy of vs for the direct terms.
-__global__ void k_toeplitz_planes(const WireDev* wires, const double* vs, const int* e,
-                                  tc::PlaneSet dst, int nw, float* vsf) {
-  pdl_enter();
+__device__ __forceinline__ void toeplitz_planes(Blk blk, const WireDev* wires, const double* vs,
+                                                const int* e, tc::PlaneSet dst, int nw, float* vsf) {
   // block (32, 8) over a 32 x 32 tile (rows t, columns t')
   __shared__ __align__(16) __half hs[2][32][40];
-  const int b = blockIdx.z / 3, n = blockIdx.z % 3;
+  const int b = blk.z / 3, n = blk.z % 3;
   const WireDev W = wires[b];
   const int nk = W.nk;
-  const int t0 = blockIdx.y * 32, c0 = blockIdx.x * 32, tx = threadIdx.x;
+  const int t0 = blk.y * 32, c0 = blk.x * 32, tx = threadIdx.x;
   if (t0 >= nk || c0 >= nk) return;
   __shared__ __half th[2][64];   // hi, lo of the tile's 63 diagonals t - t' - (t0 - c0) + 31
   const int eb = e[b];
@@ -662,27 +667,35 @@ __global__ void k_toeplitz_planes(const WireDev* wires, const double* vs, const 
   __syncthreads();
   store_tiles(hs, 2, dst, n, b, t0, c0 >> 5, threadIdx.y * 32 + tx, 32 * blockDim.y);
 }
+SBE_PASS(ToeplitzPass, 256, toeplitz_planes);
 
-__global__ void k_vs_max(const WireDev* wires, const double* vs, unsigned* mx) {
-  pdl_enter();
-  const WireDev W = wires[blockIdx.x];
+// Exponent of the screened interactions of wire blk.x (one block per wire).
+__device__ __forceinline__ void vs_exponent(Blk blk, const WireDev* wires, const double* vs, int* e) {
+  __shared__ unsigned red[8];
+  const WireDev W = wires[blk.x];
   unsigned long long m = 0;
   for (int i = threadIdx.x; i < 3 * W.nk; i += blockDim.x) m = max(m, absbits(vs[3 * W.off_vec + i]));
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(mx + blockIdx.x, bits_to_fmax(m));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = bits_to_fmax(m);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned v = red[0];
+    for (int w = 1; w < 8; ++w) v = max(v, red[w]);
+    e[blk.x] = exponent_of(__uint_as_float(v));
+  }
 }
+SBE_PASS(VsExponentPass, 256, vs_exponent);
 
 // hbar A and hbar B in FP32 (dephasing.py:714-743 contraction matrices A[k][j] =
 // Dh[j - k][k], B[k][j] = De[j - k][k], j != k) and max(2 hbar |A|, 2 hbar |B|).
 // The block's sources Dh[q][k], q = j - k + Nk in a 63-wide band, k in its 32
 // rows, are read row by row (coalesced) into shared memory.
-__global__ void k_hab(const WireDev* wires, const double* De, const double* Dh, float* habf,
-                      long long tot_mat, unsigned* mx) {
-  pdl_enter();
+__device__ __forceinline__ void hab(Blk blk, const WireDev* wires, const double* De,
+                                    const double* Dh, float* habf, long long tot_mat, unsigned* mx) {
   __shared__ double ta[63][33], tb[63][33];
-  const WireDev W = wires[blockIdx.z];
+  const WireDev W = wires[blk.z];
   const int nk = W.nk;
-  const int j0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+  const int j0 = blk.x * 32, k0 = blk.y * 32;
   const int qbase = j0 - k0 - 31 + nk;
   const bool on_w = (W.flags & SBE_F_OFFDIAGDPH) != 0;
   {
@@ -729,18 +742,18 @@ __global__ void k_hab(const WireDev* wires, const double* De, const double* Dh, 
   __syncthreads();
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
-    atomicMax(mx + blockIdx.z, __float_as_uint(m));
+    atomicMax(mx + blk.z, __float_as_uint(m));
   }
 }
+SBE_PASS(DephasingPass, 256, hab);
 
 // Per-step weights of CalcGammaE/H (dephasing.py:29-103) per q: (pi/hbar) V^2 |x|
 // with V = Vxx2 at iq[q]: [0] vee^2 |xe|, [1] veh^2 |xh|, [2] vhh^2 |xh|, [3] veh^2 |xe|.
-__global__ void k_gamma_tab(const WireDev* wires, const double* vs, const int* iq,
-                            const double* xeh, float* gtab, int nw) {
-  pdl_enter();
-  const WireDev W = wires[blockIdx.y];
-  const int nk = W.nk, b = blockIdx.y;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void gamma_tab(Blk blk, const WireDev* wires, const double* vs,
+                                          const int* iq, const double* xeh, float* gtab, int nw) {
+  const WireDev W = wires[blk.y];
+  const int nk = W.nk, b = blk.y;
+  const int q = blk.x * blockDim.x + threadIdx.x;
   if (q >= nk) return;
   const double* v = vs + 3 * W.off_vec;
   const int i = iq[W.off_vec + q];
@@ -753,15 +766,16 @@ __global__ void k_gamma_tab(const WireDev* wires, const double* vs, const int* i
   gtab[2 * st + o] = f64_to_f32(pih * vhh * vhh * xh);
   gtab[3 * st + o] = f64_to_f32(pih * veh * veh * xe);
 }
+SBE_PASS(GammaTabPass, 128, gamma_tab);
 
 // CalcGammaE/H in FP32 (same sums and index maps as k_gamma); one warp per (wire,
 // k), lanes over q; occupations (real parts) staged in shared memory.
-__global__ void k_gamma_f(const WireDev* wires, const double2* ne, const double2* nh,
-                          const int* maps, const float* gtab, float* gamf, int nw) {
-  pdl_enter();
+__device__ __forceinline__ void gamma_f(Blk blk, const WireDev* wires, const double2* ne,
+                                        const double2* nh, const int* maps, const float* gtab,
+                                        float* gamf, int nw) {
   extern __shared__ float occ[];
-  const WireDev W = wires[blockIdx.y];
-  const int nk = W.nk, b = blockIdx.y;
+  const WireDev W = wires[blk.y];
+  const int nk = W.nk, b = blk.y;
   float* pe = occ;
   float* ph = occ + nk;
   for (int i = threadIdx.x; i < nk; i += blockDim.x) {
@@ -769,7 +783,7 @@ __global__ void k_gamma_f(const WireDev* wires, const double2* ne, const double2
     ph[i] = f64_to_f32(nh[W.off_vec + i].x);
   }
   __syncthreads();
-  const int k = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  const int k = blk.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (k >= nk) return;
   const long long vo = (long long)b * nk, st1 = (long long)nw * nk;
@@ -816,32 +830,34 @@ __global__ void k_gamma_f(const WireDev* wires, const double2* ne, const double2
     gamf[st1 + vo + k] = gh;
   }
 }
+SBE_PASS(GammaPass, 256, gamma_f);
 
 // Per-step phonon coupling per |k - k'| (phonons.py:140-268): Vep(d) = VC_ee(d) /
 // E1D(d) Vscale and Vhp for holes, scaled by 2^-sP to pair with the FP32 tables.
-__global__ void k_phon_tab(const WireDev* wires, const double* vs, const double* eps,
-                           const int* sP, float* phf, int nw) {
-  pdl_enter();
-  const WireDev W = wires[blockIdx.y];
-  const int nk = W.nk, b = blockIdx.y;
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void phon_tab(Blk blk, const WireDev* wires, const double* vs,
+                                         const double* eps, const int* sP, float* phf, int nw) {
+  const WireDev W = wires[blk.y];
+  const int nk = W.nk, b = blk.y;
+  const int d = blk.x * blockDim.x + threadIdx.x;
   if (d >= nk) return;
   const double* v = vs + 3 * W.off_vec;
   const double ep = eps[W.off_vec + d];
   phf[(long long)b * nk + d] = f64_to_f32(v[nk + d] / ep * W.vscale, -sP[b]);
   phf[((long long)nw + b) * nk + d] = f64_to_f32(v[2 * nk + d] / ep * W.vscale, -sP[b]);
 }
+SBE_PASS(PhononTabPass, 128, phon_tab);
 
 // MBPE / MBPH (phonons.py:157-268) in FP32 from the scaled tables: Win, Wout of
 // electrons and holes at the occupations in ne, nh (real parts) into wrate (FP64).
 // nev, nhv: the vectors, or (diag) the matrices whose diagonals they are.
-__global__ void k_phonon_rates_f(const WireDev* wires, const double2* nev, const double2* nhv,
-                                 int diag, const float* phf, const float* epf, const float* eptf,
-                                 const float* hpf, const float* hptf, double* wrate, int nw) {
-  pdl_enter();
+__device__ __forceinline__ void phonon_rates_f(Blk blk, const WireDev* wires, const double2* nev,
+                                               const double2* nhv, int diag, const float* phf,
+                                               const float* epf, const float* eptf,
+                                               const float* hpf, const float* hptf, double* wrate,
+                                               int nw) {
   extern __shared__ float occ[];
-  const WireDev W = wires[blockIdx.y];
-  const int nk = W.nk, b = blockIdx.y, k = blockIdx.x;
+  const WireDev W = wires[blk.y];
+  const int nk = W.nk, b = blk.y, k = blk.x;
   if (!(W.flags & SBE_F_PHONON)) {
     // no phonon rates: the carrier-carrier rates (EHs) are added to zeros
     if (threadIdx.x < 4) wrate[4 * W.off_vec + threadIdx.x * nk + k] = 0.0;
@@ -885,13 +901,13 @@ __global__ void k_phonon_rates_f(const WireDev* wires, const double2* nev, const
     wrate[4 * W.off_vec + threadIdx.x * nk + k] = f32_to_f64(t);
   }
 }
+SBE_PASS(PhononRatesPass, 128, phonon_rates_f);
 
 // max(|re|, |im|) of the diagonals of C and D into mx[b] (after the relaxation
 // step has rewritten them)
-__global__ void k_diag_max(const WireDev* wires, const double2* C, const double2* D,
-                           unsigned* mx) {
-  pdl_enter();
-  const WireDev W = wires[blockIdx.x];
+__device__ __forceinline__ void diag_max(Blk blk, const WireDev* wires, const double2* C,
+                                         const double2* D, unsigned* mx) {
+  const WireDev W = wires[blk.x];
   unsigned long long m = 0;
   for (int k = threadIdx.x; k < W.nk; k += blockDim.x) {
     const long long o = W.off_mat + (long long)k * W.nk + k;
@@ -899,20 +915,21 @@ __global__ void k_diag_max(const WireDev* wires, const double2* C, const double2
     m = max(m, max(max(absbits(a.x), absbits(a.y)), max(absbits(d.x), absbits(d.y))));
   }
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(mx + blockIdx.x, bits_to_fmax(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(mx + blk.x, bits_to_fmax(m));
 }
+SBE_PASS(DiagMaxPass, 256, diag_max);
 
 // QWPolarization3 / QWRho5 reduction (qwoptics.py:809-1071) from the FP32 source
 // GEMM outputs G[k][r] = sum_k' X[k][k'] e^{i k' r}: sums over k in FP32, the
 // physical prefactors in FP64 per r.  Block (32 r) x (8 k-groups): thread (x, y)
 // sums k = y, y + 8, ... of point r, the eight partial sums meet in shared memory.
-__global__ void k_src_reduce_f(const WireDev* wires, const float2* ekrf, const float2* G,
-                               long long tot_kr, const double* win, double2* src) {
-  pdl_enter();
+__device__ __forceinline__ void src_reduce_f(Blk blk, const WireDev* wires, const float2* ekrf,
+                                             const float2* G, long long tot_kr, const double* win,
+                                             double2* src) {
   __shared__ float part[6][8][33];
-  const WireDev W = wires[blockIdx.y];
+  const WireDev W = wires[blk.y];
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int r = blockIdx.x * 32 + tx;
+  const int r = blk.x * 32 + tx;
   const int nk = W.nk, nr = W.nr;
   float sx = 0.f, sy = 0.f, ser = 0.f, sei = 0.f, shr = 0.f, shi = 0.f;
   if (r < nr) {
@@ -977,6 +994,7 @@ __global__ void k_src_reduce_f(const WireDev* wires, const float2* ekrf, const f
   out[3 * nr + r] = make_double2(f32_to_f64(v[2]) * f, f32_to_f64(v[3]) * f);
   out[4 * nr + r] = make_double2(f32_to_f64(v[4]) * f, f32_to_f64(v[5]) * f);
 }
+SBE_PASS(SrcReducePass, 256, src_reduce_f);
 
 // ---------------------------------------------------------------------------
 // Per-stage kernels.
@@ -988,22 +1006,22 @@ __global__ void k_src_reduce_f(const WireDev* wires, const float2* ekrf, const f
 // lie in rows t0 + dd0 - (Nk - 1) ... + 62 of columns t0 ... t0 + 31, which are
 // read row by row (coalesced) into shared memory and then read along diagonals
 // (row stride 32 float2: diagonal reads are free of bank conflicts).
-// The grid covers only the band: blockIdx.y counts the dd blocks from
+// The grid covers only the band: y counts the dd blocks from
 // shear_first_block(t0) on (the other blocks hold zeros, which the buffer keeps
-// from its initialisation); blockIdx.z = matrix n (0 P, 1 C, 2 D) * Nw + wire;
+// from its initialisation); z = matrix n (0 P, 1 C, 2 D) * Nw + wire;
 // block (32, 8).
 // For C and D the block also writes the sum of its 32 values of every diagonal
 // (unscaled FP32, in the fixed order t' = ddl, ddl + 1, ... cyclically) to
-// dpart[((b * 2 + n - 1) * ndd + dd) * gridDim.x + blockIdx.x]; the traces of the
+// dpart[((b * 2 + n - 1) * ndd + dd) * grid x + block x]; the traces of the
 // direct Coulomb terms are their sums over the blocks that exist.
-__global__ void k_shear_tiles(int nk, int nw, int ndd, const float2* X0, const float2* X1,
-                              const float2* X2, const int* e, tc::PlaneSet dst, float2* dpart) {
-  pdl_enter();
+__device__ __forceinline__ void shear_tiles(Blk blk, int nk, int nw, int ndd, const float2* X0,
+                                            const float2* X1, const float2* X2, const int* e,
+                                            tc::PlaneSet dst, float2* dpart) {
   __shared__ float2 tile[63][32];
   __shared__ __align__(16) __half hs[2][64][40];   // hi, lo of rows 2 dd0 .. 2 dd0 + 63
-  const int n = blockIdx.z / nw, b = blockIdx.z % nw;
-  const int t0 = blockIdx.x * 32;
-  const int dd0 = (shear_first_block(nk, t0) + blockIdx.y) * 32;
+  const int n = blk.z / nw, b = blk.z % nw;
+  const int t0 = blk.x * 32;
+  const int dd0 = (shear_first_block(nk, t0) + blk.y) * 32;
   if (dd0 >= ndd || !shear_block_live(nk, t0, dd0)) return;
   const float2* X = (n == 0 ? X0 : n == 1 ? X1 : X2) + (long long)b * nk * nk;
   const int rbase = t0 + dd0 - (nk - 1);
@@ -1034,7 +1052,7 @@ __global__ void k_shear_tiles(int nk, int nw, int ndd, const float2* X0, const f
       sr += v.x;
       si += v.y;
     }
-    dpart[(((long long)b * 2 + n - 1) * ndd + dd0 + tx) * gridDim.x + blockIdx.x] =
+    dpart[(((long long)b * 2 + n - 1) * ndd + dd0 + tx) * blk.gx + blk.x] =
         make_float2(sr, si);
   }
   const int eb = e[b];
@@ -1066,6 +1084,7 @@ __global__ void k_shear_tiles(int nk, int nw, int ndd, const float2* X0, const f
         v;
   }
 }
+SBE_PASS(ShearPass, 256, shear_tiles);
 
 // The stage field in FP32.
 
@@ -1092,21 +1111,24 @@ __global__ void k_field_f(long long n, const double2* ek, const double2* dek, do
 // FP32 hi / lo parts (dgf).  The block maximum of the operands goes to mx[b].
 constexpr int HB_ROWS = 1;
 
-__global__ void k_h_build(const WireDev* __restrict__ wires, const float2* __restrict__ ekf,
-                          const float* __restrict__ vsf, const double* __restrict__ Ee,
-                          const double* __restrict__ Eh, const float2* __restrict__ trf,
-                          const float2* __restrict__ xsh, int have_x, float2* __restrict__ hf,
-                          long long tot_mat, double2* __restrict__ dgE, double2* __restrict__ dgH,
-                          float2* __restrict__ dgf, unsigned* __restrict__ mx) {
-  pdl_enter();
-  const WireDev& W = wires[blockIdx.z];
-  const int nk = W.nk, b = blockIdx.z, nw = gridDim.z;
+__device__ __forceinline__ void h_build(Blk blk, const WireDev* __restrict__ wires, int nw,
+                                        const float2* __restrict__ ekf,
+                                        const float* __restrict__ vsf,
+                                        const double* __restrict__ Ee,
+                                        const double* __restrict__ Eh,
+                                        const float2* __restrict__ trf,
+                                        const float2* __restrict__ xsh, int have_x,
+                                        float2* __restrict__ hf, long long tot_mat,
+                                        double2* __restrict__ dgE, double2* __restrict__ dgH,
+                                        float2* __restrict__ dgf, unsigned* __restrict__ mx) {
+  const WireDev& W = wires[blk.z];
+  const int nk = W.nk, b = blk.z;
   float hmax = 0.f;
   // HB_ROWS rows per block
   for (int rr = 0; rr < HB_ROWS; ++rr) {
-  const int k1 = blockIdx.y * HB_ROWS + rr;
+  const int k1 = blk.y * HB_ROWS + rr;
   for (int it = 0; it < 4; ++it) {
-  const int k2 = blockIdx.x * blockDim.x * 4 + it * blockDim.x + threadIdx.x;
+  const int k2 = blk.x * blockDim.x * 4 + it * blockDim.x + threadIdx.x;
   if (k1 < nk && k2 < nk) {
     float2 heh = make_float2(0.f, 0.f), hee = heh, hhh = heh;
     if (W.flags & SBE_F_OPTICS) {
@@ -1184,16 +1206,17 @@ __global__ void k_h_build(const WireDev* __restrict__ wires, const float2* __res
     atomicMax(mx + b, __float_as_uint(hmax));
   }
 }
+SBE_PASS(HBuildPass, 128, h_build);
 
 // Planes of Hee', Hhh' (slots M_EE, M_HH) and of Hee' + i hbar B, Hhh' + i hbar A
 // (slots M_EEX, M_HHX) from the FP32 values.
-__global__ void k_hplanes(const float2* hee, const float2* hhh, const float* hA, const float* hB,
-                          int nk, const int* e, tc::PlaneSet dst, int nw) {
-  pdl_enter();
+__device__ __forceinline__ void hplanes(Blk blk, const float2* hee, const float2* hhh,
+                                        const float* hA, const float* hB, int nk, const int* e,
+                                        tc::PlaneSet dst, int nw) {
   // block (32, 8) over a 32 x 32 tile; each slot's planes go through shared memory
   __shared__ __align__(16) __half hs[4][32][40];
-  const int b = blockIdx.z;
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
+  const int b = blk.z;
+  const int r0 = blk.y * 32, c0 = blk.x * 32, tx = threadIdx.x, ty = threadIdx.y;
   const long long mm = (long long)nk * nk;
   const int eb = e[b];
   float2 a[4], h[4];
@@ -1226,6 +1249,7 @@ __global__ void k_hplanes(const float2* hee, const float2* hhh, const float* hA,
     __syncthreads();
   }
 }
+SBE_PASS(HPlanesPass, 256, hplanes);
 
 // s + e = a + b exactly (Knuth's two-sum in round-to-nearest FP32).  The peeled
 // diagonal energies enter as products with the state every stage; a rounded FP32
@@ -1326,19 +1350,20 @@ __device__ __forceinline__ void rk4_block_max(const Rk4Ctl& r, int b, unsigned m
 // once.  W arrives in FP32 from the GEMMs (the hi*lo + lo*hi products, to
 // which the hi*hi launch adds its K parts in order); g[j] - g[i] comes from the hi /
 // lo FP32 parts of g.
-__global__ void __launch_bounds__(256) k_antiherm(
-    int nk, const float2* __restrict__ W, const float2* __restrict__ Hp, const float2* X,
-    const float2* __restrict__ ghi, const float2* __restrict__ glo, const float* __restrict__ chi,
-    const float* __restrict__ clo, float2* out, Rk4Ctl rk) {
-  pdl_enter();
+__device__ __forceinline__ void antiherm(Blk blk, int nk, const float2* __restrict__ W,
+                                         const float2* __restrict__ Hp, const float2* X,
+                                         const float2* __restrict__ ghi,
+                                         const float2* __restrict__ glo,
+                                         const float* __restrict__ chi,
+                                         const float* __restrict__ clo, float2* out, Rk4Ctl rk) {
   // tb / hb: W and H' of the mirror tile (rows j0.., columns i0..); vt: results;
   // gv / cv: g (hi, lo) and c (hi, lo) at the tile's rows i0.. (0) and columns j0.. (1)
   __shared__ float2 tb[32][33], hb[32][33], vt[32][33];
   __shared__ float2 gv[2][2][32];
   __shared__ float cv[2][2][32];
-  const int bi = blockIdx.y, bj = blockIdx.x;
+  const int bi = blk.y, bj = blk.x;
   if (bi > bj) return;
-  const int b = blockIdx.z, tx = threadIdx.x, ty = threadIdx.y;
+  const int b = blk.z, tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = bi * 32, j0 = bj * 32;
   const long long mb = (long long)b * nk * nk;
   if (ty < 2) {
@@ -1436,6 +1461,7 @@ __global__ void __launch_bounds__(256) k_antiherm(
   }
   if (rk.stage != 0) rk4_block_max(rk, b, mxv, mov);
 }
+SBE_PASS(AntihermPass, 256, antiherm);
 
 // dP of a stage from the FP32 commutator sums G (the engine's scaled products with
 // the off-diagonal C', D'), following dpdt (SBEs.py:1942-1965):
@@ -1445,17 +1471,17 @@ __global__ void __launch_bounds__(256) k_antiherm(
 // occupations c, d enter through the Pauli-blocking factor of the driving term and
 // the peeled energy diagonals ee, hh as hi + lo FP32 parts.  32 x 32 tiles; Heh^T
 // goes through shared memory so that every global access runs along rows.
-__global__ void __launch_bounds__(256) k_rhs_p(
-    int nk, int nw, const float2* __restrict__ G, const float2* __restrict__ hehf,
-    const float2* X, const float2* __restrict__ dgf, const float* __restrict__ gamf,
-    const float* __restrict__ cdf, float2* out, Rk4Ctl rk) {
-  pdl_enter();
+__device__ __forceinline__ void rhs_p(Blk blk, int nk, int nw, const float2* __restrict__ G,
+                                      const float2* __restrict__ hehf, const float2* X,
+                                      const float2* __restrict__ dgf,
+                                      const float* __restrict__ gamf,
+                                      const float* __restrict__ cdf, float2* out, Rk4Ctl rk) {
   __shared__ float2 ht[32][33];
   // per-row (kh = m0 + r) values: hh hi, lo; GamH; d hi, lo
   __shared__ float2 rg[2][32];
   __shared__ float rv[3][32];
-  const int b = blockIdx.z;
-  const int m0 = blockIdx.y * 32, n0 = blockIdx.x * 32;
+  const int b = blk.z;
+  const int m0 = blk.y * 32, n0 = blk.x * 32;
   const long long mb = (long long)b * nk * nk, vb = (long long)b * nk, vn = (long long)nw * nk;
   const int tx = threadIdx.x, ty = threadIdx.y;
   {
@@ -1523,17 +1549,12 @@ __global__ void __launch_bounds__(256) k_rhs_p(
   }
   if (rk.stage != 0) rk4_block_max(rk, b, mxv, mov);
 }
+SBE_PASS(RhsPPass, 256, rhs_p);
 
 __global__ void k_f32_to_f64(long long n, const float2* a, double2* out) {
   pdl_enter();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < n) out[i] = f32_to_f64(a[i]);
-}
-
-__global__ void k_add_int(int n, const int* a, const int* b, int* out) {
-  pdl_enter();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = a[i] + b[i];
 }
 
 static tc::GemmJob job(Mixed* m, const tc::PlaneSet& A, const tc::PlaneSet& B, int M, int N,
@@ -1662,38 +1683,52 @@ static std::vector<tc::GemmJob> all_jobs(SbeCtx* c, int kind) {
   return jobs;
 }
 
-static void exponents_from(Mixed* m, const unsigned* mx, int* e, cudaStream_t s) {
-  launch(k_exponents, (m->nw + 127) / 128, 128, 0, s, m->nw, mx, e, nullptr, nullptr);
-}
+// The buckets, largest Nk first.
+static std::vector<Mixed*> by_size(const MixedAll* A) { return {A->b.rbegin(), A->b.rend()}; }
 
 // Per-step set-up of the mixed path: the frozen preparation (screening, rates,
 // dephasing matrices with the FP32 Lorentzian sums) and its FP32 tables.
 static int mixed_prep(SbeCtx* c, const double2* C, const double2* D, cudaStream_t s) {
   MixedAll* A = all_of(c);
+  // the maxima that this step's passes collect
+  cudaMemsetAsync(A->mx, 0, sizeof(unsigned) * 4 * c->nw, s);
   launch_prep_scalar(c, C, D, s);   // occupations, screening (FP64, O(Nk) per wire)
-  for (Mixed* m : A->b) {
-    const int nk = m->nk, nw = m->nw;
-    cudaMemsetAsync(m->mxH(), 0, sizeof(unsigned) * nw, s);
-    launch(k_vs_max, nw, 256, 0, s, m->dw, c->vs, m->mxH());
-    exponents_from(m, m->mxH(), m->eT(), s);
-    launch(k_toeplitz_planes, dim3((nk + 31) / 32, (nk + 31) / 32, 3 * nw), dim3(32, 8), 0, s,
-           m->dw, c->vs, m->eT(), m->tp, nw, m->vsf);
-    launch(k_gamma_tab, dim3((nk + 127) / 128, nw), 128, 0, s, m->dw, c->vs, c->iq, c->xeh, m->gtab,
-           nw);
-    launch(k_gamma_f, dim3((nk + 7) / 8, nw), 256, sizeof(float) * 2 * nk, s, m->dw, c->ne, c->nh,
-           c->maps, m->gtab, m->gamf, nw);
-    launch(k_phon_tab, dim3((nk + 127) / 128, nw), 128, 0, s, m->dw, c->vs, c->eps, m->sP, m->phf,
-           nw);
-    cudaMemsetAsync(m->mxAB(), 0, sizeof(unsigned) * nw, s);
+  const std::vector<Mixed*> buckets = by_size(A);
+  {
+    Batch<VsExponentPass> pass(256, s);
+    for (Mixed* m : buckets) pass.add(m->nw, m->dw, c->vs, m->eT());
+  }
+  {
+    Batch<ToeplitzPass> pass(dim3(32, 8), s);
+    for (Mixed* m : buckets)
+      pass.add(dim3((m->nk + 31) / 32, (m->nk + 31) / 32, 3 * m->nw), m->dw, c->vs, m->eT(), m->tp,
+               m->nw, m->vsf);
+  }
+  {
+    Batch<GammaTabPass> pass(128, s);
+    for (Mixed* m : buckets)
+      pass.add(dim3((m->nk + 127) / 128, m->nw), m->dw, c->vs, c->iq, c->xeh, m->gtab, m->nw);
+  }
+  {
+    Batch<GammaPass> pass(256, s, sizeof(float) * 2 * buckets[0]->nk);
+    for (Mixed* m : buckets)
+      pass.add(dim3((m->nk + 7) / 8, m->nw), m->dw, c->ne, c->nh, c->maps, m->gtab, m->gamf, m->nw);
+  }
+  {
+    Batch<PhononTabPass> pass(128, s);
+    for (Mixed* m : buckets)
+      pass.add(dim3((m->nk + 127) / 128, m->nw), m->dw, c->vs, c->eps, m->sP, m->phf, m->nw);
   }
   if (c->any_offdiag) {
     ProfScope ps(c, 3, s);
     launch_offdiag_D(c, -1, nullptr, true, s);
   }
-  for (Mixed* m : A->b) {
-    const int T = (m->nk + 31) / 32;
-    launch(k_hab, dim3(T, T, m->nw), dim3(32, 8), 0, s, m->dw, c->De, c->Dh, A->habf, c->tot_mat,
-           m->mxAB());
+  {
+    Batch<DephasingPass> pass(dim3(32, 8), s);
+    for (Mixed* m : buckets) {
+      const int T = (m->nk + 31) / 32;
+      pass.add(dim3(T, T, m->nw), m->dw, c->De, c->Dh, A->habf, c->tot_mat, m->mxAB());
+    }
   }
   return cuda_check(cudaGetLastError(), "mixed prep");
 }
@@ -1704,12 +1739,17 @@ static void mixed_relax(SbeCtx* c, double2* P, double2* C, double2* D, const dou
                         double dt, cudaStream_t s) {
   MixedAll* A = all_of(c);
   if (any_ehs(c)) launch_extract_diag(c, C, D, s);   // for the carrier-carrier rates
-  for (Mixed* m : A->b)
-    launch(k_phonon_rates_f, dim3(m->nk, m->nw), 128, sizeof(float) * 2 * m->nk, s, m->dw, C, D, 1,
-           m->phf, A->epf, A->eptf, A->hpf, A->hptf, c->wrate, m->nw);
+  const std::vector<Mixed*> buckets = by_size(A);
+  {
+    Batch<PhononRatesPass> pass(128, s, sizeof(float) * 2 * buckets[0]->nk);
+    for (Mixed* m : buckets)
+      pass.add(dim3(m->nk, m->nw), m->dw, C, D, 1, m->phf, A->epf, A->eptf, A->hpf, A->hptf,
+               c->wrate, m->nw);
+  }
   launch_mbc_rates(c, -1, s, false, true);
   launch_relax_only(c, P, C, D, Ek, dt, s);
-  for (Mixed* m : A->b) launch(k_diag_max, m->nw, 256, 0, s, m->dw, C, D, m->mxS());
+  Batch<DiagMaxPass> pass(256, s);
+  for (Mixed* m : buckets) pass.add(m->nw, m->dw, C, D, m->mxS());
 }
 
 // Stage-1 state of the mixed path from the FP64 state: FP32 copies (the first
@@ -1720,18 +1760,14 @@ static void mixed_state_in(SbeCtx* c, const double2* P, const double2* C, const 
   MixedAll* A = all_of(c);
   const long long tm = c->tot_mat;
   float2* xf = reinterpret_cast<float2*>(c->xs);
-  for (Mixed* m : A->b) {
+  Batch<StateInPass> pass(256, s);
+  for (Mixed* m : by_size(A)) {
     const int nk = m->nk, nw = m->nw;
     const long long mm = (long long)nk * nk, vn = (long long)nw * nk, o = m->bm;
-    cudaMemsetAsync(m->mxS(), 0, sizeof(unsigned) * nw, s);
-    cudaMemsetAsync(m->mxO(), 0, sizeof(unsigned) * nw, s);
-    const int blocks = (int)std::min<long long>((mm + 255) / 256, 128);
-    launch(k_state_in, dim3(blocks, nw), 256, 0, s, P + o, nk, 0, m->mxS(), m->mxO(), xf + o,
-           nullptr);
-    launch(k_state_in, dim3(blocks, nw), 256, 0, s, C + o, nk, 1, m->mxS(), m->mxO(), xf + tm + o,
-           m->xdg);
-    launch(k_state_in, dim3(blocks, nw), 256, 0, s, D + o, nk, 1, m->mxS(), m->mxO(),
-           xf + 2 * tm + o, m->xdg + vn);
+    const dim3 grid((unsigned)std::min<long long>((mm + 255) / 256, 128), nw);
+    pass.add(grid, P + o, nk, 0, m->mxS(), m->mxO(), xf + o, nullptr);
+    pass.add(grid, C + o, nk, 1, m->mxS(), m->mxO(), xf + tm + o, m->xdg);
+    pass.add(grid, D + o, nk, 1, m->mxS(), m->mxO(), xf + 2 * tm + o, m->xdg + vn);
   }
 }
 
@@ -1754,21 +1790,34 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
   // maximum (sheared exchange operands); eO: maximum over P and the off-diagonal C, D
   // (commutator operands; the diagonals of C and D are peeled off and applied exactly
   // in the element-wise passes)
-  for (Mixed* m : A->b) {
-    const int nk = m->nk, nw = m->nw;
-    const long long vn = (long long)nw * nk;
-    const float2 *P = xs + m->bm, *C = xs + tm + m->bm, *D = xs + 2 * tm + m->bm;
-    launch(k_stage_exponents, (nw + 127) / 128, 128, 0, s, nw, m->mxS(), m->mxO(), m->mxH(),
-           m->eS(), m->eO(), m->eT(), m->esx(),
-           stage > 0);
-    const dim3 tb(32, 8), tg((nk + 31) / 32, (nk + 31) / 32, nw);
-    launch(k_planes_nt<float2>, tg, tb, 0, s, P, nk, m->eO(), m->pl, M_P, M_PT, nw,
-           nullptr, nullptr);
-    launch(k_planes_nt<float2>, tg, tb, 0, s, C, nk, m->eO(), m->pl, M_C, -1, nw, m->cdf, m->xdg);
-    launch(k_planes_nt<float2>, tg, tb, 0, s, D, nk, m->eO(), m->pl, M_D, -1, nw, m->cdf + 2 * vn,
-           m->xdg + vn);
-    if (have_x) {
-      // the traces of C and D (direct terms) come from the shear's diagonal partials
+  const std::vector<Mixed*> buckets = by_size(A);
+  const dim3 tile(32, 8);
+  const auto tiles = [](const Mixed* m) {
+    return dim3((m->nk + 31) / 32, (m->nk + 31) / 32, m->nw);
+  };
+  {
+    Batch<StageExponentsPass> pass(128, s);
+    for (Mixed* m : buckets)
+      pass.add((m->nw + 127) / 128, m->nw, m->mxS(), m->mxO(), m->mxH(), m->eS(), m->eO(), m->eT(),
+               m->esx(), stage > 0);
+  }
+  {
+    Batch<PlanesPass> pass(tile, s);
+    for (Mixed* m : buckets) {
+      const int nk = m->nk, nw = m->nw;
+      const long long vn = (long long)nw * nk;
+      const float2 *P = xs + m->bm, *C = xs + tm + m->bm, *D = xs + 2 * tm + m->bm;
+      pass.add(tiles(m), P, nk, m->eO(), m->pl, M_P, M_PT, nw, nullptr, nullptr);
+      pass.add(tiles(m), C, nk, m->eO(), m->pl, M_C, -1, nw, m->cdf, m->xdg);
+      pass.add(tiles(m), D, nk, m->eO(), m->pl, M_D, -1, nw, m->cdf + 2 * vn, m->xdg + vn);
+    }
+  }
+  if (have_x) {
+    // the traces of C and D (direct terms) come from the shear's diagonal partials
+    Batch<ShearPass> shear(tile, s);
+    Batch<TracesPass> traces(128, s);
+    for (Mixed* m : buckets) {
+      const int nk = m->nk, nw = m->nw;
       const int nbk = (nk + 31) / 32, ndd = 32 * ((2 * nk + 31) / 32);
       int ny = 0;   // dd blocks of the band per t' block
       for (int i = 0; i < nbk; ++i) {
@@ -1777,11 +1826,13 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
           if (shear_block_live(nk, 32 * i, 32 * j)) cnt = j - shear_first_block(nk, 32 * i) + 1;
         ny = std::max(ny, cnt);
       }
-      launch(k_shear_tiles, dim3(nbk, ny, 3 * nw), dim3(32, 8), 0, s, nk, nw, ndd, P, C, D, m->eS(),
-             m->sp, m->tpart);
-      launch(k_trace_from_shear, dim3((2 * nk - 1 + 127) / 128, 2, nw), 128, 0, s, nk, nbk, ndd,
-             m->tpart, m->trf);
+      shear.add(dim3(nbk, ny, 3 * nw), nk, nw, ndd, xs + m->bm, xs + tm + m->bm,
+                xs + 2 * tm + m->bm, m->eS(), m->sp, m->tpart);
     }
+    shear.flush();
+    for (Mixed* m : buckets)
+      traces.add(dim3((2 * m->nk - 1 + 127) / 128, 2, m->nw), m->nk, (m->nk + 31) / 32,
+                 32 * ((2 * m->nk + 31) / 32), m->tpart, m->trf);
   }
   int rc = SBE_OK;
   if (have_x) {
@@ -1791,19 +1842,30 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
     if (rc) return rc;
   }
   // the Hamiltonians: Meh + diagonal + direct + exchange, diagonal peeled; their planes
-  for (Mixed* m : A->b) {
-    const int nk = m->nk, nw = m->nw;
-    launch(k_h_build, dim3((nk + 511) / 512, (nk + HB_ROWS - 1) / HB_ROWS, nw), 128, 0, s, m->dw,
-           A->ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh), have_x,
-           A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH());
+  {
+    Batch<HBuildPass> pass(128, s);
+    for (Mixed* m : buckets)
+      pass.add(dim3((m->nk + 511) / 512, (m->nk + HB_ROWS - 1) / HB_ROWS, m->nw), m->dw, m->nw,
+               A->ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh),
+               have_x, A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH());
+  }
+  {
     // H exponent: max over the operands and the step's 2 hbar |A|, |B|
-    launch(k_exponents2_sum, (nw + 127) / 128, 128, 0, s, nw, m->mxH(), m->mxAB(), m->eH(), m->eO(),
-           m->esc());
-    const dim3 tb(32, 8), tg((nk + 31) / 32, (nk + 31) / 32, nw);
-    launch(k_planes_nt<float2>, tg, tb, 0, s, A->hf + m->bm, nk, m->eH(), m->pl, M_EH, M_EHT, nw,
-           nullptr, nullptr);
-    launch(k_hplanes, tg, tb, 0, s, A->hf + tm + m->bm, A->hf + 2 * tm + m->bm, A->habf + m->bm,
-           A->habf + tm + m->bm, nk, m->eH(), m->pl, nw);
+    Batch<HamExponentsPass> pass(128, s);
+    for (Mixed* m : buckets)
+      pass.add((m->nw + 127) / 128, m->nw, m->mxH(), m->mxAB(), m->eH(), m->eO(), m->esc());
+  }
+  {
+    Batch<PlanesPass> pass(tile, s);
+    for (Mixed* m : buckets)
+      pass.add(tiles(m), A->hf + m->bm, m->nk, m->eH(), m->pl, M_EH, M_EHT, m->nw, nullptr,
+               nullptr);
+  }
+  {
+    Batch<HPlanesPass> pass(tile, s);
+    for (Mixed* m : buckets)
+      pass.add(tiles(m), A->hf + tm + m->bm, A->hf + 2 * tm + m->bm, A->habf + m->bm,
+               A->habf + tm + m->bm, m->nk, m->eH(), m->pl, m->nw);
   }
   // commutator GEMMs: dP and the cross terms of W and V, then the hi*hi products of
   // W and V (the partials of W and V meet in the anti-Hermitian pass)
@@ -1821,7 +1883,9 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
   // stage buffers (FP32, 3 tot_mat each): the step-start state, then the stage states
   float2* x0 = reinterpret_cast<float2*>(c->xs);
   float2* xn = x0 + 3 * tm;
-  for (Mixed* m : A->b) {
+  Batch<RhsPPass> dp(tile, s);
+  Batch<AntihermPass> dcd(tile, s);
+  for (Mixed* m : buckets) {
     const int nk = m->nk, nw = m->nw;
     const long long vn = (long long)nw * nk, o = m->bm;
     const float2 *P = xs + o, *C = xs + tm + o, *D = xs + 2 * tm + o;
@@ -1844,40 +1908,35 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
       rk[i].mx = m->mxS();
       rk[i].mo = m->mxO();
     }
-    const dim3 ag((nk + 31) / 32, (nk + 31) / 32, nw), ab(32, 8);
-    launch(k_rhs_p, ag, ab, 0, s, nk, nw, gp + o, A->hf + o, P, m->dgf, m->gamf, m->cdf, A->kf + o,
-           rk[0]);
-    launch(k_antiherm, ag, ab, 0, s, nk, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf,
-           m->dgf + vn, m->cdf, m->cdf + vn, A->kf + tm + o, rk[1]);
-    launch(k_antiherm, ag, ab, 0, s, nk, wf + G_V * tm + o, A->hf + 2 * tm + o, D,
-           m->dgf + 2 * vn, m->dgf + 3 * vn, m->cdf + 2 * vn,
-           m->cdf + 3 * vn, A->kf + 2 * tm + o, rk[2]);
+    dp.add(tiles(m), nk, nw, gp + o, A->hf + o, P, m->dgf, m->gamf, m->cdf, A->kf + o, rk[0]);
+    dcd.add(tiles(m), nk, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf, m->dgf + vn, m->cdf,
+            m->cdf + vn, A->kf + tm + o, rk[1]);
+    dcd.add(tiles(m), nk, wf + G_V * tm + o, A->hf + 2 * tm + o, D, m->dgf + 2 * vn,
+            m->dgf + 3 * vn, m->cdf + 2 * vn, m->cdf + 3 * vn, A->kf + 2 * tm + o, rk[2]);
   }
+  dp.flush();
+  dcd.flush();
   return cuda_check(cudaGetLastError(), "mixed stage");
 }
 
 // Sources of the new state through the engine: G = [P; C; conj(D)] E (FP32
-// outputs), then the per-r reductions.  mxS holds the state maximum when
-// state_max_ready is set.
+// outputs), then the per-r reductions.  mxS holds the state maximum.
 static int mixed_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D,
-                         double2* src, int state_max_ready, cudaStream_t s) {
+                         double2* src, cudaStream_t s) {
   MixedAll* A = all_of(c);
-  for (Mixed* m : A->b) {
-    const int nk = m->nk, nw = m->nw;
-    const long long mm = (long long)nk * nk, o = m->bm;
-    if (!state_max_ready) {
-      cudaMemsetAsync(m->mxS(), 0, sizeof(unsigned) * nw, s);
-      absmax_into(P + o, mm, nw, m->mxS(), s);
-      absmax_into(C + o, mm, nw, m->mxS(), s);
-      absmax_into(D + o, mm, nw, m->mxS(), s);
-    }
-    exponents_from(m, m->mxS(), m->eS(), s);
-    const double2* st[3] = {P + o, C + o, D + o};
-    const dim3 tb(32, 8), tg((nk + 31) / 32, (nk + 31) / 32, nw);
-    for (int i = 0; i < 3; ++i)
-      launch(k_planes_nt<double2>, tg, tb, 0, s, st[i], nk, m->eS(), m->pl, 2 * i, -1, nw,
-             nullptr, nullptr);
-    launch(k_add_int, (nw + 127) / 128, 128, 0, s, nw, m->eS(), m->eE(), m->ess());
+  const std::vector<Mixed*> buckets = by_size(A);
+  {
+    Batch<ExponentsPass> pass(128, s);
+    for (Mixed* m : buckets)
+      pass.add((m->nw + 127) / 128, m->nw, m->mxS(), m->eS(), m->eE(), m->ess());
+  }
+  {
+    Batch<Planes64Pass> pass(dim3(32, 8), s);
+    const double2* st[3] = {P, C, D};
+    for (Mixed* m : buckets)
+      for (int i = 0; i < 3; ++i)
+        pass.add(dim3((m->nk + 31) / 32, (m->nk + 31) / 32, m->nw), st[i] + m->bm, m->nk, m->eS(),
+                 m->pl, 2 * i, -1, m->nw, nullptr, nullptr);
   }
   float2* gf = reinterpret_cast<float2*>(c->G);
   {
@@ -1885,9 +1944,11 @@ static int mixed_sources(SbeCtx* c, const double2* P, const double2* C, const do
     const int rc = launch_jobs(all_jobs(c, JK_SRC), s);
     if (rc) return rc;
   }
-  for (Mixed* m : A->b)
-    launch(k_src_reduce_f, dim3((m->nr + 31) / 32, m->nw), dim3(32, 8), 0, s, m->dw, A->ekrf, gf,
-           c->tot_kr, c->window, src);
+  {
+    Batch<SrcReducePass> pass(dim3(32, 8), s);
+    for (Mixed* m : buckets)
+      pass.add(dim3((m->nr + 31) / 32, m->nw), m->dw, A->ekrf, gf, c->tot_kr, c->window, src);
+  }
   launch_sources_final(c, c->ne, c->nh, src, s);
   return cuda_check(cudaGetLastError(), "mixed sources");
 }
@@ -1939,8 +2000,7 @@ int rk4_mixed(SbeCtx* c, double2* P, double2* C, double2* D, const double2* Ek0,
     if (rc) return rc;
   }
   mixed_relax(c, P, C, D, Ek0, dt, s);   // the new diagonals join the maximum
-  // DC transport moves every element: the sources then measure the maximum themselves
-  return mixed_sources(c, P, C, D, src, any_dc(c) ? 0 : 1, s);
+  return mixed_sources(c, P, C, D, src, s);
 }
 
 }  // namespace sbe
