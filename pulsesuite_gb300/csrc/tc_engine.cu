@@ -15,13 +15,14 @@ namespace tc {
 // dependent load into every chunk).  Output pointers are offset to the tile's
 // batch entry and K part.
 struct EpiTile {
-  int kind, M, N, ld, cplx, es, unshear;
+  int kind, M, N, ld, cplx, es, unshear, comp;
   float* of;      // EPI_F32
   float2* of2;    // EPI_RAWF
   double2* od;    // EPI_RAW
 };
 
-__device__ __forceinline__ EpiTile epi_tile(const GemmDesc& d, const EpiArgs& e, int b, int ks) {
+__device__ __forceinline__ EpiTile epi_tile(const GemmDesc& d, const EpiArgs& e, int b, int ks,
+                                            int comp) {
   EpiTile t;
   t.kind = e.kind;
   t.M = d.M;
@@ -30,6 +31,7 @@ __device__ __forceinline__ EpiTile epi_tile(const GemmDesc& d, const EpiArgs& e,
   t.cplx = d.complex_mode;
   t.es = -e.escale[b];
   t.unshear = e.unshear;
+  t.comp = comp;
   const long long off = (long long)ks * e.ks_stride + (long long)b * e.out_bstride;
   t.of = e.outf ? e.outf + off : nullptr;
   t.of2 = e.outf2 ? e.outf2 + off : nullptr;
@@ -77,7 +79,12 @@ __device__ __forceinline__ void epilogue_chunk(const EpiTile& t, int mrow0, int 
   const long long rs = 2 * (long long)t.ld;
   if (t.kind == EPI_RAWF) {
     float2* o = t.of2 + base;
-    if (accumulate) {
+    if (t.comp) {
+      float* oc = reinterpret_cast<float*>(o) + (t.comp - 1);
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (2 * i + rh < rmax) oc[2 * i * rs] = t.comp == 1 ? v[i].x : v[i].y;
+    } else if (accumulate) {
       // a later K part of a kseq tile: add to the running sum this thread stored
       float2 pv[16];
 #pragma unroll
@@ -125,6 +132,7 @@ __device__ __forceinline__ void epilogue_chunk(const EpiTile& t, int mrow0, int 
 struct TileInfo {
   int job, b, m0, n0, ks, kb_begin, nkb, n_iters;
   int nparts;  // K parts run in sequence in this tile (kseq), else 1
+  int comp;    // 0: the complex product; 1, 2: its real, imaginary part alone
   bool dead;   // exchange tile whose outputs all lie outside the un-sheared matrix
 };
 
@@ -148,6 +156,11 @@ __device__ __forceinline__ TileInfo tile_info(const GemmLaunch& L, long long t) 
   }
   const GemmDesc& d = L.job[j].d;
   long long r = t - L.tile_base[j];
+  ti.comp = 0;
+  if (L.csplit) {
+    ti.comp = 1 + (int)(r & 1);
+    r >>= 1;
+  }
   const int tn = (d.N + BNT - 1) / BNT, tm = (d.M + BM - 1) / BM;
   ti.job = j;
   ti.n0 = (int)(r % tn) * BNT;
@@ -395,22 +408,40 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
               umma_f16(acc_re + 2 * BNT, A(1), B(0), iir, acc);
             } else {
               // planes 0 re_hi, 1 re_lo, 2 im_hi, 3 im_lo
-              uint32_t ar = acc, ai = acc;
-              if (hh) {
-                umma_f16(acc_re, A(0), B(0), irr, ar);
-                umma_f16(acc_re, A(2), B(2), iii, 1u);
-                umma_f16(acc_im, A(0), B(2), iri, ai);
-                umma_f16(acc_im, A(2), B(0), iir, 1u);
-                ar = ai = 1u;
+              if (ti.comp == 0) {
+                uint32_t ar = acc, ai = acc;
+                if (hh) {
+                  umma_f16(acc_re, A(0), B(0), irr, ar);
+                  umma_f16(acc_re, A(2), B(2), iii, 1u);
+                  umma_f16(acc_im, A(0), B(2), iri, ai);
+                  umma_f16(acc_im, A(2), B(0), iir, 1u);
+                  ar = ai = 1u;
+                }
+                umma_f16(acc_re, A(0), B(1), irr, ar);
+                umma_f16(acc_re, A(1), B(0), irr, 1u);
+                umma_f16(acc_re, A(2), B(3), iii, 1u);
+                umma_f16(acc_re, A(3), B(2), iii, 1u);
+                umma_f16(acc_im, A(0), B(3), iri, ai);
+                umma_f16(acc_im, A(1), B(2), iri, 1u);
+                umma_f16(acc_im, A(2), B(1), iir, 1u);
+                umma_f16(acc_im, A(3), B(0), iir, 1u);
+              } else {
+                // one part alone: the same products in the same order
+                const bool im = ti.comp == 2;
+                const uint32_t d = im ? acc_im : acc_re;
+                const uint32_t i0 = im ? iri : irr, i1 = im ? iir : iii;
+                const int b0 = im ? 2 : 0, b1 = im ? 0 : 2;   // B planes (hi) beside A re, A im
+                uint32_t ac = acc;
+                if (hh) {
+                  umma_f16(d, A(0), B(b0), i0, ac);
+                  umma_f16(d, A(2), B(b1), i1, 1u);
+                  ac = 1u;
+                }
+                umma_f16(d, A(0), B(b0 + 1), i0, ac);
+                umma_f16(d, A(1), B(b0), i0, 1u);
+                umma_f16(d, A(2), B(b1 + 1), i1, 1u);
+                umma_f16(d, A(3), B(b1), i1, 1u);
               }
-              umma_f16(acc_re, A(0), B(1), irr, ar);
-              umma_f16(acc_re, A(1), B(0), irr, 1u);
-              umma_f16(acc_re, A(2), B(3), iii, 1u);
-              umma_f16(acc_re, A(3), B(2), iii, 1u);
-              umma_f16(acc_im, A(0), B(3), iri, ai);
-              umma_f16(acc_im, A(1), B(2), iri, 1u);
-              umma_f16(acc_im, A(2), B(1), iir, 1u);
-              umma_f16(acc_im, A(3), B(0), iir, 1u);
             }
             first = false;
           }
@@ -448,7 +479,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       const GemmDesc& d = L.job[ti.job].d;
       const EpiArgs& e = L.job[ti.job].e;
       const int mrow0 = ti.m0 + 32 * q;
-      const EpiTile et = epi_tile(d, e, ti.b, ti.ks);   // before the wait
+      const EpiTile et = epi_tile(d, e, ti.b, ti.ks, ti.comp);   // before the wait
 #pragma unroll 1
       for (int part = 0; part < ti.nparts; ++part, ++st) {
       int nkb = ti.nkb;
@@ -493,6 +524,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             im[j] = __uint_as_float(a1[j]) + __uint_as_float(a2[j]);
           }
         } else if (have) {
+          // (a part that was not formed is not stored either)
           tmem_ld16(lane_addr + c * 16, re);
           if (cplx) {
             tmem_ld16(lane_addr + BNT + c * 16, im);
@@ -634,7 +666,8 @@ static double launch_cost(const tc::GemmJob* jobs, int njobs, int bnt) {
 // The N tile of a launch: the jobs' own (256, or 128 where chosen), narrowed where that brings
 // the launch at least a fifth closer to an even load of the SMs.  The products of an element and
 // their order are the same at every width.  1 x 256 (commutators, exchange, sources): 256-wide
-// 62, 16, 25 us, 128-wide 41, 12, 17, 64-wide 39, 11, 16; 4 x 512: 115, 32, 71 / 75, 35, 64 /
+// 62, 16, 25 us, 128-wide 41, 12, 17, 64-wide 39, 11, 16 (before the parts of a tile were
+// split, below); 4 x 512: 115, 32, 71 / 75, 35, 64 /
 // 123, 51, 112; 16 x 512: 217, 79, 209 / 226, 105, 229 / 410, 170, 393.  hi*hi launches take
 // 64-wide tiles while those fit the SMs in one wave: 1 x 256 29 -> 18 us, 8 x 256 30 -> 19,
 // 4 x 512 (two waves) 37 -> 40.
@@ -663,6 +696,24 @@ static int n_tile(const tc::GemmJob* jobs, int njobs, int mode, int widest) {
   return best;
 }
 
+// Whether the real and imaginary parts of the tiles go to CTAs of their own: with all of them in
+// one wave a tile's chain of products is the launch's time, and the parts' chains are
+// independent: commutators of 1 x 64 15.2 -> 12.8 us, 1 x 256 40.6 -> 32.2, 1 x 512 72 -> 55.
+// One-term products (sources) gain less than their half-filled stores cost (1 x 512 26 -> 28).
+static bool splits_parts(const tc::GemmJob* jobs, int njobs, int bnt) {
+  long long tiles = 0;
+  int terms = 0;
+  for (int j = 0; j < njobs; ++j) {
+    const tc::GemmDesc& d = jobs[j].d;
+    terms = std::max(terms, d.nterms);
+    if (!d.complex_mode || d.mode != tc::MODE_FULL || jobs[j].e.kind != tc::EPI_RAWF || d.kacc ||
+        d.ksplit > 1)
+      return false;
+    tiles += (long long)((d.N + bnt - 1) / bnt) * ((d.M + tc::BM - 1) / tc::BM) * d.batch;
+  }
+  return terms > 1 && 2 * tiles <= num_sms();
+}
+
 int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   int rc = tc_gemm_init();
   if (rc) return rc;
@@ -676,6 +727,7 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   const int bn = jobs[0].d.bn;
   if (bn != 0 && bn != 128 && bn != 256) return fail(SBE_ERR_ARG, "tc_gemm: N tile 128 or 256");
   const int bnt = n_tile(jobs, njobs, mode, bn == 128 ? 128 : tc::BN);
+  L.csplit = splits_parts(jobs, njobs, bnt) ? 1 : 0;
   long long nt = 0;
   for (int j = 0; j < njobs; ++j) {
     const tc::GemmDesc& d = jobs[j].d;
@@ -695,7 +747,7 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
     if (d.kacc && (jobs[j].e.kind != tc::EPI_RAWF || (d.ksplit > 1 && !d.kseq)))
       return fail(SBE_ERR_ARG, "tc_gemm: accumulating output needs FP32 complex output and one "
                                "tile per output");
-    nt += (long long)((d.N + bnt - 1) / bnt) * ((d.M + tc::BM - 1) / tc::BM) * d.batch *
+    nt += (L.csplit ? 2 : 1) * (long long)((d.N + bnt - 1) / bnt) * ((d.M + tc::BM - 1) / tc::BM) * d.batch *
           (d.ksplit > 1 && !d.kseq ? d.ksplit : 1);
   }
   L.tile_base[njobs] = nt;

@@ -163,6 +163,7 @@ struct GemmLaunch {
   GemmJob job[MAX_JOBS];
   long long tile_base[MAX_JOBS + 1];
   int njobs;
+  int csplit;                 // 1: two tiles per complex output tile, real and imaginary part
   int* sched;                 // tile and exit counters of this launch (zero; left zero)
 };
 static_assert(sizeof(GemmLaunch) <= 32000, "kernel parameter space (32 KB) exceeded");
