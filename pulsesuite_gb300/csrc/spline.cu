@@ -13,7 +13,8 @@
 // dependent FMA a point, p_i = theta_i / theta_{i-1} beside it), and a block holds few points
 // (64, all fields of one set of knots) so that the grid spreads them over the SMs.
 // Mean of the solves of a step (4 fields on 4096 points, 5 on Nr = 230): 17.5 ms with one
-// thread per field, 32 us here.
+// thread per field, 32 us here; with the pivots' coefficients and reciprocals formed by all
+// threads (3 fields on 8192, 5 on 514: 31 -> 22 us) 22 us.
 #include "spline.cuh"
 #include "fp_bits.cuh"
 
@@ -79,28 +80,45 @@ __global__ void __launch_bounds__(kThreads) k_spline(SplBatch s) {
   const int fe = min(n, e + warm);                // forward sweep up to here
   const int l0 = max(0, sb - warm - 1);           // first right-hand side
   // reciprocal pivots over [l0, fe), with t_{i+1} and d_i / p_i
-  for (int a = l0 + tid * kSeg; a < fe; a += kThreads * kSeg) {
-    const int b = min(a + kSeg, fe);
-    if (det) {
-      int i = max(0, a - warm / 2);
-      double t1 = 1.0, t2 = 0.0;   // theta_{i-1}, theta_{i-2}, spacings in units of hi
-      double dm = i > 0 ? (x[i - x0] - x[i - 1 - x0]) * is : 0.0;
+  if (det) {
+    double *bb = reinterpret_cast<double*>(c1[0]), *th = reinterpret_cast<double*>(c1[1]);
+    // b_i and d_{i-1}^2 (in mm), spacings in units of hi: a warp's FP64 instruction holds its
+    // scheduler for 64 clocks however few its lanes, so only the recurrence itself stays with
+    // the few threads of the segments
+    for (int i = max(0, l0 - warm / 2) + tid; i < fe; i += kThreads) {
+      const int j = i - x0;
+      const double dm = i > 0 ? (x[j] - x[j - 1]) * is : 0.0;
+      const double dp = i < n - 1 ? (x[j + 1] - x[j]) * is : 0.0;
+      bb[j] = i == 0 ? -dp : i == n - 1 ? -dm : 2.0 * (dm + dp);
+      mm[j] = -(dm * dm);
+    }
+    __syncthreads();
+    for (int a = l0 + tid * kSeg; a < fe; a += kThreads * kSeg) {
+      const int b = min(a + kSeg, fe);
+      double t1 = 1.0, t2 = 0.0;   // theta_{i-1}, theta_{i-2}
 #pragma unroll 4
-      for (; i < b; ++i) {
+      for (int i = max(0, a - warm / 2); i < b; ++i) {
         const int j = i - x0;
-        const double dp = i < n - 1 ? (x[j + 1] - x[j]) * is : 0.0;
-        const double bi = i == 0 ? -dp : i == n - 1 ? -dm : 2.0 * (dm + dp);
-        const double t0 = fma(bi, t1, -(dm * dm) * t2);
+        const double t0 = fma(bb[j], t1, mm[j] * t2);
         if (i >= a) {
-          const double r = t1 * rcp64(t0);   // hi / p_i
-          ip[j] = r * is;
-          mm[j] = tt[j + 1] = dp * r;
+          ip[j] = t1;
+          th[j] = t0;
         }
         t2 = t1;
         t1 = t0;
-        dm = dp;
       }
-    } else {
+    }
+    __syncthreads();
+    for (int i = l0 + tid; i < fe; i += kThreads) {
+      const int j = i - x0;
+      const double dp = i < n - 1 ? (x[j + 1] - x[j]) * is : 0.0;
+      const double r = ip[j] * rcp64(th[j]);   // hi / p_i
+      ip[j] = r * is;
+      mm[j] = tt[j + 1] = dp * r;
+    }
+  } else {
+    for (int a = l0 + tid * kSeg; a < fe; a += kThreads * kSeg) {
+      const int b = min(a + kSeg, fe);
       double r = 0.0;   // 1 / p of the point before
       for (int i = max(0, a - kWarmP); i < b; ++i) {
         const int j = i - x0;
