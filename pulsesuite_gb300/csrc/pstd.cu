@@ -18,6 +18,7 @@
 //   pass C  inverse column FFTs, 1/nx, and the field update.
 // Each transform is a radix-2 Stockham sequence in shared memory; the field data
 // crosses HBM/L2 three times per derivative.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -27,8 +28,12 @@ namespace sbe {
 namespace {
 
 constexpr double kMu0 = 1.25663706127e-6;  // CODATA 2022 (scipy.constants.mu_0)
-constexpr int kCols = 8;                   // columns per CTA, passes A and C
-constexpr int kRows = 8;                   // rows per CTA, pass B
+// Columns per CTA of passes A and C and rows per CTA of pass B: eight (128-byte segments), fewer
+// while the CTAs do not cover the SMs; a row or column of 64 to 256 FP64 points holds an SM's
+// two FMA a clock and its stages' latency for some us, so the SMs have to share them.  One step
+// of 8192 points: A 8.0 -> 5.5, B 32 -> 9.9, C 8.9 -> 6.0 us (16 CTAs before); 16384 points
+// 16, 33, 16 -> 6.8, 10.4, 7.2.
+constexpr int kMaxLines = 8;
 constexpr int kThreads = 256;
 
 __device__ __forceinline__ double2 ld(const double2* p) { return __ldg(p); }
@@ -36,14 +41,15 @@ __device__ __forceinline__ double2 ld(const double2* p) { return __ldg(p); }
 // Radix-2 Stockham over shared memory.  ntr transforms of length L = 2^lg; element
 // p of transform c lives at a[p * ps + c * cs].  rows_fast: consecutive threads walk
 // p (transforms stored contiguously) instead of c.  dir -1: exp(-i ...), +1: exp(+i ...).
-// Returns the buffer that holds the result (natural order).
+// tw[j] = exp(-2 pi i j / L), j < L / 2, in shared memory.  Returns the buffer that holds the
+// result (natural order).
 __device__ double2* smem_fft(double2* a, double2* b, int lg, int lgtr, int ps, int cs,
-                             bool rows_fast, int dir, const double2* __restrict__ tw, int nx) {
+                             bool rows_fast, int dir, const double2* tw) {
   const int L = 1 << lg;
   const int half = L >> 1;
   const int total = half << lgtr;
   for (int ns = 1; ns < L; ns <<= 1) {
-    const int tws = nx / (2 * ns);
+    const int tws = half / ns;
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
       int j, c;
       if (rows_fast) {
@@ -56,7 +62,7 @@ __device__ double2* smem_fft(double2* a, double2* b, int lg, int lgtr, int ps, i
       const int k = j & (ns - 1);
       const double2 u = a[j * ps + c * cs];
       double2 v = a[(j + half) * ps + c * cs];
-      double2 w = ld(&tw[k * tws]);
+      double2 w = tw[k * tws];
       if (dir > 0) w.y = -w.y;
       v = cmul(v, w);
       const int o = ((j - k) << 1) + k;
@@ -71,6 +77,11 @@ __device__ double2* smem_fft(double2* a, double2* b, int lg, int lgtr, int ps, i
   return a;
 }
 
+// the twiddles of length L from the table of nx
+__device__ __forceinline__ void load_twiddles(double2* st, const double2* tw, int L, int nx) {
+  for (int j = threadIdx.x; j < (L >> 1); j += blockDim.x) st[j] = ld(&tw[j * (nx / L)]);
+}
+
 __host__ __device__ inline int ilog2(int v) {
   int l = 0;
   while ((1 << l) < v) ++l;
@@ -78,34 +89,37 @@ __host__ __device__ inline int ilog2(int v) {
 }
 
 // Pass A: forward column FFTs (length n1) of field blockIdx.y, times the four-step twiddle.
-__global__ void __launch_bounds__(kThreads) k_pstd_cols_fwd(int nx, int n1, int n2,
+__global__ void __launch_bounds__(kThreads) k_pstd_cols_fwd(int nx, int n1, int n2, int lgc,
                                                             const double2* __restrict__ in0,
                                                             const double2* __restrict__ in1,
                                                             double2* __restrict__ Y,
                                                             const double2* __restrict__ tw) {
   pdl_enter();
   extern __shared__ double2 sm[];
+  const int cols = 1 << lgc;
   double2* a = sm;
-  double2* b = sm + n1 * kCols;
+  double2* b = sm + n1 * cols;
+  double2* st = b + n1 * cols;
   const double2* x = blockIdx.y == 0 ? in0 : in1;
-  const int c0 = blockIdx.x * kCols;
-  for (int idx = threadIdx.x; idx < n1 * kCols; idx += blockDim.x) {
-    const int c = idx & (kCols - 1), p = idx >> 3;
-    a[p * kCols + c] = ld(&x[(long long)p * n2 + c0 + c]);
+  const int c0 = blockIdx.x * cols;
+  load_twiddles(st, tw, n1, nx);
+  for (int idx = threadIdx.x; idx < n1 * cols; idx += blockDim.x) {
+    const int c = idx & (cols - 1), p = idx >> lgc;
+    a[idx] = ld(&x[(long long)p * n2 + c0 + c]);
   }
   __syncthreads();
-  const double2* r = smem_fft(a, b, ilog2(n1), 3, kCols, 1, false, -1, tw, nx);
+  const double2* r = smem_fft(a, b, ilog2(n1), lgc, cols, 1, false, -1, st);
   double2* y = Y + (long long)blockIdx.y * nx;
-  for (int idx = threadIdx.x; idx < n1 * kCols; idx += blockDim.x) {
-    const int c = idx & (kCols - 1), k1 = idx >> 3;
-    y[(long long)k1 * n2 + c0 + c] = cmul(r[k1 * kCols + c], ld(&tw[(c0 + c) * k1]));
+  for (int idx = threadIdx.x; idx < n1 * cols; idx += blockDim.x) {
+    const int c = idx & (cols - 1), k1 = idx >> lgc;
+    y[(long long)k1 * n2 + c0 + c] = cmul(r[idx], ld(&tw[(c0 + c) * k1]));
   }
 }
 
-// Pass B: rows k1 in [blockIdx.x kRows, +kRows).  kind 0: each field (blockIdx.y)
+// Pass B: rows k1 in [blockIdx.x 2^lgr, + 2^lgr).  kind 0: each field (blockIdx.y)
 // times i q;  kind 1: (rho, Px) -> (-i rho - q Px) q / (eps (q^2 + small)) into
 // field 0 (rhoPJ.py:836-866 restricted to x).
-__global__ void __launch_bounds__(kThreads) k_pstd_rows(int nx, int n1, int n2, int kind,
+__global__ void __launch_bounds__(kThreads) k_pstd_rows(int nx, int n1, int n2, int kind, int lgr,
                                                         double2* __restrict__ Y,
                                                         const double* __restrict__ q,
                                                         double small, double inv_eps,
@@ -114,30 +128,32 @@ __global__ void __launch_bounds__(kThreads) k_pstd_rows(int nx, int n1, int n2, 
   extern __shared__ double2 sm[];
   const int nfl = kind == 1 ? 2 : 1;
   const int f0 = kind == 1 ? 0 : blockIdx.y;
-  const int ntr = nfl * kRows;
+  const int rows = 1 << lgr, ntr = nfl * rows;
   const int lg2 = ilog2(n2);
   double2* a = sm;
   double2* b = sm + ntr * n2;
-  const int r0 = blockIdx.x * kRows;
+  double2* st = b + ntr * n2;
+  const int r0 = blockIdx.x * rows;
+  load_twiddles(st, tw, n2, nx);
   for (int idx = threadIdx.x; idx < ntr * n2; idx += blockDim.x) {
     const int t = idx >> lg2, p = idx & (n2 - 1);
-    const int f = f0 + t / kRows, row = r0 + (t & (kRows - 1));
+    const int f = f0 + (t >> lgr), row = r0 + (t & (rows - 1));
     a[t * n2 + p] = Y[(long long)f * nx + (long long)row * n2 + p];
   }
   __syncthreads();
-  double2* r = smem_fft(a, b, lg2, ilog2(ntr), 1, n2, true, -1, tw, nx);
-  for (int idx = threadIdx.x; idx < kRows * n2; idx += blockDim.x) {
+  double2* r = smem_fft(a, b, lg2, ilog2(ntr), 1, n2, true, -1, st);
+  for (int idx = threadIdx.x; idx < rows * n2; idx += blockDim.x) {
     const int t = idx >> lg2, k2 = idx & (n2 - 1);
     const int k = r0 + t + n1 * k2;
     const double qk = q[k];
     if (kind == 0) {
       for (int g = 0; g < nfl; ++g) {
-        const double2 v = r[(t + g * kRows) * n2 + k2];
-        r[(t + g * kRows) * n2 + k2] = make_double2(-qk * v.y, qk * v.x);
+        const double2 v = r[(t + g * rows) * n2 + k2];
+        r[(t + g * rows) * n2 + k2] = make_double2(-qk * v.y, qk * v.x);
       }
     } else {
       const double2 rho = r[t * n2 + k2];
-      const double2 px = r[(t + kRows) * n2 + k2];
+      const double2 px = r[(t + rows) * n2 + k2];
       const double qs = qk * qk + small;
       // rho_term = -i rho inv_eps / qs ; P_term = -(q Px) inv_eps / qs ; out = (rho_term + P_term) q
       const double2 rt = make_double2(rho.y * inv_eps / qs, -rho.x * inv_eps / qs);
@@ -146,43 +162,46 @@ __global__ void __launch_bounds__(kThreads) k_pstd_rows(int nx, int n1, int n2, 
     }
   }
   __syncthreads();
-  const int ntr_out = kind == 1 ? kRows : ntr;
+  const int ntr_out = kind == 1 ? rows : ntr;
   double2* o = (r == a) ? b : a;
-  const double2* s = smem_fft(r, o, lg2, ilog2(ntr_out), 1, n2, true, +1, tw, nx);
+  const double2* s = smem_fft(r, o, lg2, ilog2(ntr_out), 1, n2, true, +1, st);
   for (int idx = threadIdx.x; idx < ntr_out * n2; idx += blockDim.x) {
     const int t = idx >> lg2, p = idx & (n2 - 1);
-    const int f = f0 + t / kRows, k1 = r0 + (t & (kRows - 1));
+    const int f = f0 + (t >> lgr), k1 = r0 + (t & (rows - 1));
     const double2 w = cconj(ld(&tw[p * k1]));
     Y[(long long)f * nx + (long long)k1 * n2 + p] = cmul(s[t * n2 + p], w);
   }
 }
 
 // Pass C: inverse column FFTs (length n1), 1/nx, epilogue.
-__global__ void __launch_bounds__(kThreads) k_pstd_cols_inv(int nx, int n1, int n2,
+__global__ void __launch_bounds__(kThreads) k_pstd_cols_inv(int nx, int n1, int n2, int lgc,
                                                             const double2* __restrict__ Y,
                                                             const double2* __restrict__ tw,
                                                             const double* __restrict__ mask,
                                                             PstdEpiArgs e) {
   pdl_enter();
   extern __shared__ double2 sm[];
+  const int cols = 1 << lgc;
   double2* a = sm;
-  double2* b = sm + n1 * kCols;
+  double2* b = sm + n1 * cols;
+  double2* st = b + n1 * cols;
   const int f = blockIdx.y;
   const double2* y = Y + (long long)f * nx;
-  const int c0 = blockIdx.x * kCols;
-  for (int idx = threadIdx.x; idx < n1 * kCols; idx += blockDim.x) {
-    const int c = idx & (kCols - 1), k1 = idx >> 3;
-    a[k1 * kCols + c] = y[(long long)k1 * n2 + c0 + c];
+  const int c0 = blockIdx.x * cols;
+  load_twiddles(st, tw, n1, nx);
+  for (int idx = threadIdx.x; idx < n1 * cols; idx += blockDim.x) {
+    const int c = idx & (cols - 1), k1 = idx >> lgc;
+    a[idx] = y[(long long)k1 * n2 + c0 + c];
   }
   __syncthreads();
-  const double2* r = smem_fft(a, b, ilog2(n1), 3, kCols, 1, false, +1, tw, nx);
+  const double2* r = smem_fft(a, b, ilog2(n1), lgc, cols, 1, false, +1, st);
   const double inv_n = 1.0 / (double)nx;
   double2* out = e.out[f];
   const double2* js = e.jsrc[f];
-  for (int idx = threadIdx.x; idx < n1 * kCols; idx += blockDim.x) {
-    const int c = idx & (kCols - 1), p = idx >> 3;
+  for (int idx = threadIdx.x; idx < n1 * cols; idx += blockDim.x) {
+    const int c = idx & (cols - 1), p = idx >> lgc;
     const long long n = (long long)p * n2 + c0 + c;
-    const double2 d = cscale(r[p * kCols + c], inv_n);
+    const double2 d = cscale(r[idx], inv_n);
     if (e.mode == PSTD_STORE) {
       out[n] = d;
     } else {
@@ -229,19 +248,29 @@ bool g_attr_done[64] = {};
 int pstd_pipeline(SbePstd* p, int kind, const double2* in0, const double2* in1, int nf,
                   const PstdEpiArgs& epi, cudaStream_t s) {
   const int nx = p->nx, n1 = p->n1, n2 = p->n2;
-  const size_t smA = 2 * (size_t)n1 * kCols * sizeof(double2);
-  const size_t smB = 2 * (size_t)(kind == 1 ? 2 : 1) * kRows * n2 * sizeof(double2);
-  launch(k_pstd_cols_fwd, dim3(n2 / kCols, nf), kThreads, smA, s, nx, n1, n2, in0, in1, p->work,
-         p->tw);
+  // lines per CTA (see kMaxLines) of n lines in f fields, at least least
+  const auto lines = [](int n, int f, int least) {
+    int l = kMaxLines;
+    while (l > least && (long long)(n / l) * f < 152) l /= 2;
+    return l;
+  };
+  // threads: one per butterfly of a stage
+  const auto threads = [](int len, int tr) { return std::min(kThreads, std::max(32, len / 2 * tr)); };
+  const int nout = kind == 1 ? 1 : nf, nrow = kind == 1 ? 2 : 1;   // fields of pass C, of a CTA of B
+  const int ca = lines(n2, nf, 2), cb = lines(n1, kind == 1 ? 1 : nf, 1), cc = lines(n2, nout, 2);
+  const auto smem = [](int len, int tr) {
+    return (2 * (size_t)len * tr + len / 2) * sizeof(double2);
+  };
+  launch(k_pstd_cols_fwd, dim3(n2 / ca, nf), threads(n1, ca), smem(n1, ca), s, nx, n1, n2,
+         ilog2(ca), in0, in1, p->work, p->tw);
   // rhoPJ.py:779: small = (qx[1] - qx[0]) / 1e4, with q[0] = 0 and q[1] = dq
   const double dq = 2.0 * kPi / ((double)nx * p->dx);
   const double sm_q = dq / 1e4;
   const double inv_eps = 1.0 / (kEps0 * p->epsr);
-  launch(k_pstd_rows, dim3(n1 / kRows, kind == 1 ? 1 : nf), kThreads, smB, s, nx, n1, n2, kind,
-         p->work, p->q, sm_q, inv_eps, p->tw);
-  const int nout = kind == 1 ? 1 : nf;
-  launch(k_pstd_cols_inv, dim3(n2 / kCols, nout), kThreads, smA, s, nx, n1, n2, p->work, p->tw,
-         p->mask, epi);
+  launch(k_pstd_rows, dim3(n1 / cb, kind == 1 ? 1 : nf), threads(n2, nrow * cb),
+         smem(n2, nrow * cb), s, nx, n1, n2, kind, ilog2(cb), p->work, p->q, sm_q, inv_eps, p->tw);
+  launch(k_pstd_cols_inv, dim3(n2 / cc, nout), threads(n1, cc), smem(n1, cc), s, nx, n1, n2,
+         ilog2(cc), p->work, p->tw, p->mask, epi);
   return cuda_check(cudaGetLastError(), "pstd pipeline");
 }
 
@@ -297,8 +326,8 @@ int sbe_pstd_create(const SbePstdDesc* d, void* stream, SbePstd** out) {
     return fail(SBE_ERR_OOM, "sbe_pstd_create: device allocation");
   }
   if (p->dev >= 0 && p->dev < 64 && !g_attr_done[p->dev]) {
-    const int maxA = 2 * 256 * kCols * (int)sizeof(double2);
-    const int maxB = 2 * 2 * kRows * 256 * (int)sizeof(double2);
+    const int maxA = (2 * 256 * kMaxLines + 128) * (int)sizeof(double2);
+    const int maxB = (2 * 2 * kMaxLines * 256 + 128) * (int)sizeof(double2);
     cudaFuncSetAttribute(k_pstd_cols_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, maxA);
     cudaFuncSetAttribute(k_pstd_cols_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, maxA);
     cudaFuncSetAttribute(k_pstd_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, maxB);
