@@ -267,8 +267,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     for (int k = 0; ok; ++k) {
       const int qs = k & 3;
       if (!mbar_wait(&qempty[qs], (uint32_t)(((k >> 2) & 1) ^ 1), err, abort_flag)) break;
-      long long t = atomicAdd(L.sched, 1);
-      while (t < ntiles && tile_info<BNT>(L, t).dead) t = atomicAdd(L.sched, 1);
+      // the first tile is the CTA's own, the others come from the counter
+      long long t = k == 0 ? (long long)blockIdx.x : gridDim.x + atomicAdd(L.sched, 1);
+      while (t < ntiles && tile_info<BNT>(L, t).dead) t = gridDim.x + atomicAdd(L.sched, 1);
       tq[qs] = t < ntiles ? (int)t : -1;
       mbar_arrive(&qfull[qs]);   // release: the entry is visible to the waiters
       if (t >= ntiles) break;
@@ -324,6 +325,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         }
       }
       }
+    }
+    // the last CTA to have drawn its last tile leaves the slot zeroed for its next launch (a
+    // memset ahead of the launch costs a launch of its own and the overlap with the kernel
+    // before)
+    if (atomicAdd(L.sched + 1, 1) == (int)gridDim.x - 1) {
+      L.sched[0] = 0;
+      L.sched[1] = 0;
     }
     // no copy may still be landing in shared memory when the CTA exits: wait
     // (bounded) for the last stages issued
@@ -552,16 +560,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
-  }
-  // the last CTA leaves the slot zeroed for its next launch: every CTA has drawn its last
-  // tile by now (a memset ahead of the launch costs a launch of its own and the overlap with
-  // the kernel before)
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(L.sched + 1, 1) == (int)gridDim.x - 1) {
-      L.sched[0] = 0;
-      L.sched[1] = 0;
-    }
   }
 }
 
