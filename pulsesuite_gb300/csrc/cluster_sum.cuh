@@ -16,53 +16,59 @@ __device__ __forceinline__ double cabs_d(double2 v) {
   return hypot(v.x, v.y);
 }
 
-// sums of the N values over the block (256 threads), returned to every thread; a dependent
-// FP64 addition takes about 130 clocks, so the values go together
+// Sums of the N values over the block (256 threads), returned to every thread.  An FP64
+// instruction holds its scheduler for 64 clocks in every warp that issues it, so the warps that
+// hold nothing (live false, the same over a warp) leave out the first sums and one warp per value
+// forms the last ones.
 template <int N>
-__device__ __forceinline__ void block_sums(double (&v)[N]) {
-  __shared__ double red[N][8];
+__device__ __forceinline__ void block_sums(double (&v)[N], bool live) {
+  __shared__ double red[N][8], tot[N];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (live) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-    for (int i = 0; i < N; ++i) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int i = 0; i < N; ++i) red[i][threadIdx.x >> 5] = v[i];
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const double* r = red[i];
-    v[i] = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
+      for (int i = 0; i < N; ++i) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
   }
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < N; ++i) red[i][warp] = live ? v[i] : 0.0;
+  __syncthreads();
+  if (warp < N) {
+    double x = lane < 8 ? red[warp][lane] : 0.0;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) tot[warp] = x;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = tot[i];
 }
 
 // ... and over the cluster (also a cluster barrier: what every block read before it may be
 // overwritten after it); no block leaves before the others have read its sums
-__device__ __forceinline__ void cluster_sum2(double& a, double& b) {
+__device__ __forceinline__ void cluster_sum2(double& a, double& b, bool live) {
   namespace cg = cooperative_groups;
-  __shared__ double part[2];
+  __shared__ double part[2], all[2];
   cg::cluster_group cl = cg::this_cluster();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v[2] = {a, b};
-  block_sums(v);
+  block_sums(v, live);
   if (threadIdx.x == 0) {
     part[0] = v[0];
     part[1] = v[1];
   }
   cl.sync();
-  double p[2][kCluster];
+  if (warp < 2) {
+    double x = lane < kCluster ? cl.map_shared_rank(part, lane)[warp] : 0.0;
 #pragma unroll
-  for (int r = 0; r < kCluster; ++r) {
-    const double* q = cl.map_shared_rank(part, r);
-    p[0][r] = q[0];
-    p[1][r] = q[1];
+    for (int o = 1; o < kCluster; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) all[warp] = x;
   }
-  auto sum = [](const double* x) {
-    return ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
-  };
-  a = sum(p[0]);
-  b = sum(p[1]);
   cl.sync();
+  a = all[0];
+  b = all[1];
 }
 
 }  // namespace sbe

@@ -207,14 +207,6 @@ __global__ void __launch_bounds__(64) k_couple_deposit(const WireDev* wires, int
   rho[j] = rh;
 }
 
-// x / d from r = 1 / d (rounded): the quotient's remainder corrects it to the division's own
-// rounding, in three instructions of the two-wide FP64 pipe instead of a dozen.
-__device__ __forceinline__ double div_by(double x, double d, double r) {
-  const double q = x * r;
-  if ((__double2hiint(q) & 0x7FF00000) == 0x7FF00000) return q;   // infinite or NaN
-  return fma(fma(-q, d, x), r, q);
-}
-
 // J = (P^{n+1} - P^n)/dt (y, z) plus the soft source; P^n <- P^{n+1}.
 __global__ void k_couple_current(int nx, double dt, double rdt, const double2* Pg, double2* Pold, double2* J,
                                  const long long* step, double t0, int src_index, double jamp,

@@ -272,10 +272,12 @@ __global__ void __launch_bounds__(128) k_f64_hbuild(const __grid_constant__ HBui
 
 // dP, dC, dD from the partial products (SBEs.py:1942-1965, 2309-2327, 2607-2625): the sum
 // of each output's partials over i hbar, for dP also Heh^T / (i hbar), the rates and OffP;
-// with stage 1-4 the RK4 update of k_rk4_axpy.
+// with stage 1-4 the RK4 update of k_rk4_axpy.  Bound by the FP64 pipes (some 30 operations an
+// element); one element a thread, so that a few small wires reach all SMs (four elements a thread: 1 x 64
+// 13.3 us, 2 x 512 93; here 2 x 512 81).
 struct Finish {
   int nk, nw, nsum, stage, first;   // first: output of blockIdx.z / nw = 0 (single calls)
-  double dt;
+  double dt, dt6;                   // the step, and a sixth of it
   const double* part;               // [output][nsum][re, im][wire][Nk x Nk]
   const double2 *Heh, *P, *offp;
   const double *gamE, *gamH;
@@ -284,65 +286,60 @@ struct Finish {
 
 __global__ void __launch_bounds__(256) k_f64_finish(const __grid_constant__ Finish a) {
   pdl_enter();
-  __shared__ double2 ht[32][33];
+  __shared__ double2 ht[32][9];
   const int nk = a.nk, which = blockIdx.z / a.nw + a.first, b = blockIdx.z % a.nw;
-  const int m0 = blockIdx.y * 32, n0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
+  const int m0 = blockIdx.y * 8, n0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
   const long long mm = (long long)nk * nk, mb = (long long)b * mm;
   if (which == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int n = n0 + ty + 8 * q, m = m0 + tx;
-      if (n < nk && m < nk) ht[ty + 8 * q][tx] = a.Heh[mb + (long long)n * nk + m];
-    }
+    const int t = ty * 32 + tx, n = n0 + (t >> 3), m = m0 + (t & 7);
+    if (n < nk && m < nk) ht[t >> 3][t & 7] = a.Heh[mb + (long long)n * nk + m];
     __syncthreads();
   }
   const double ih = 1.0 / kHbar;
   const long long cs = (long long)a.nw * mm;
   const double* part = a.part + (long long)(which - a.first) * a.nsum * 2 * cs + mb;
+  const int m = m0 + ty, n = n0 + tx;
+  if (m >= nk || n >= nk) return;
+  const long long o = (long long)m * nk + n;
+  const long long i = mb + o;
+  double2 x0 = make_double2(0.0, 0.0), s0 = x0;
+  if (a.stage > 0) x0 = a.X[which][i];
+  if (a.stage > 1) s0 = a.acc[which][i];
+  double sx = 0.0, sy = 0.0;
+  for (int s = 0; s < a.nsum; s += 4) {   // a multiple of four: eight loads in flight
+    double x[4], y[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int m = m0 + ty + 8 * q, n = n0 + tx;
-    if (m >= nk || n >= nk) continue;
-    const long long o = (long long)m * nk + n;
-    double sx = 0.0, sy = 0.0;
-    for (int s = 0; s < a.nsum; s += 4) {   // a multiple of four: eight loads in flight
-      double x[4], y[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        x[u] = part[2 * (s + u) * cs + o];
-        y[u] = part[(2 * (s + u) + 1) * cs + o];
-      }
-      sx += (x[0] + x[1]) + (x[2] + x[3]);
-      sy += (y[0] + y[1]) + (y[2] + y[3]);
+    for (int u = 0; u < 4; ++u) {
+      x[u] = part[2 * (s + u) * cs + o];
+      y[u] = part[(2 * (s + u) + 1) * cs + o];
     }
-    double2 v = make_double2(sy * ih, -sx * ih);
-    if (which == 0) {
-      const double2 h = ht[tx][ty + 8 * q], p = a.P[mb + o];
-      const double gam = a.gamE[(long long)b * nk + n] + a.gamH[(long long)b * nk + m];
-      v.x += h.y * ih - gam * p.x;
-      v.y += -h.x * ih - gam * p.y;
-      if (a.offp) {
-        const double2 f = a.offp[mb + o];
-        v.x += f.y * ih;
-        v.y += -f.x * ih;
-      }
+    const double tx4 = (x[0] + x[1]) + (x[2] + x[3]), ty4 = (y[0] + y[1]) + (y[2] + y[3]);
+    sx = s ? sx + tx4 : tx4;
+    sy = s ? sy + ty4 : ty4;
+  }
+  double2 v = make_double2(sy * ih, -sx * ih);
+  if (which == 0) {
+    const double2 h = ht[tx][ty], p = a.P[mb + o];
+    const double gam = a.gamE[(long long)b * nk + n] + a.gamH[(long long)b * nk + m];
+    v.x += h.y * ih - gam * p.x;
+    v.y += -h.x * ih - gam * p.y;
+    if (a.offp) {
+      const double2 f = a.offp[mb + o];
+      v.x += f.y * ih;
+      v.y += -f.x * ih;
     }
-    const long long i = mb + o;
-    if (a.stage == 0) {
-      a.out[which][i] = v;
-    } else if (a.stage == 1) {
-      a.acc[which][i] = v;
-      const double2 x = a.X[which][i];
-      a.xs[which][i] = make_double2(x.x + 0.5 * a.dt * v.x, x.y + 0.5 * a.dt * v.y);
-    } else if (a.stage < 4) {
-      const double2 s = a.acc[which][i], x = a.X[which][i];
-      a.acc[which][i] = make_double2(s.x + 2.0 * v.x, s.y + 2.0 * v.y);
-      const double f = a.stage == 2 ? 0.5 * a.dt : a.dt;
-      a.xs[which][i] = make_double2(x.x + f * v.x, x.y + f * v.y);
-    } else {
-      const double2 s = a.acc[which][i], x = a.X[which][i];
-      a.X[which][i] = make_double2(x.x + a.dt / 6.0 * (s.x + v.x), x.y + a.dt / 6.0 * (s.y + v.y));
-    }
+  }
+  if (a.stage == 0) {
+    a.out[which][i] = v;
+  } else if (a.stage == 1) {
+    a.acc[which][i] = v;
+    a.xs[which][i] = make_double2(x0.x + 0.5 * a.dt * v.x, x0.y + 0.5 * a.dt * v.y);
+  } else if (a.stage < 4) {
+    a.acc[which][i] = make_double2(s0.x + 2.0 * v.x, s0.y + 2.0 * v.y);
+    const double f = a.stage == 2 ? 0.5 * a.dt : a.dt;
+    a.xs[which][i] = make_double2(x0.x + f * v.x, x0.y + f * v.y);
+  } else {
+    a.X[which][i] = make_double2(x0.x + a.dt6 * (s0.x + v.x), x0.y + a.dt6 * (s0.y + v.y));
   }
 }
 
@@ -678,6 +675,7 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       f.nsum = 4 * m.parts;
       f.stage = stage;
       f.dt = dt;
+      f.dt6 = dt / 6.0;
       f.part = m.part;
       f.Heh = c->Heh + o;
       f.P = P + o;
@@ -690,7 +688,7 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
         f.acc[i] = c->kacc + i * n + o;
         f.xs[i] = c->xs + i * n + o;
       }
-      launch(k_f64_finish, dim3((nk + 31) / 32, (nk + 31) / 32, 3 * g), dim3(32, 8), 0, s, f);
+      launch(k_f64_finish, dim3((nk + 31) / 32, (nk + 7) / 8, 3 * g), dim3(32, 8), 0, s, f);
     }
   return cuda_check(cudaGetLastError(), "f64 rhs");
 }
@@ -912,7 +910,7 @@ bool f64_rhs_single(int which, int nk, const double2* C, const double2* D, const
   f.gamE = gamE;
   f.gamH = gamH;
   f.out[which] = out;
-  launch(k_f64_finish, dim3((nk + 31) / 32, (nk + 31) / 32, 1), dim3(32, 8), 0, s, f);
+  launch(k_f64_finish, dim3((nk + 31) / 32, (nk + 7) / 8, 1), dim3(32, 8), 0, s, f);
   *rc = cuda_check(cudaGetLastError(), "f64 rhs single");
   return true;
 }

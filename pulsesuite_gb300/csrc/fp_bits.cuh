@@ -94,6 +94,14 @@ __device__ __forceinline__ double rcp64(double x) {
   return fma(y, fma(e, e, e), y);
 }
 
+// x / d from r = 1 / d (rounded): the quotient's remainder corrects it to the division's own
+// rounding, in three instructions of the two-wide FP64 pipe instead of a dozen.
+__device__ __forceinline__ double div_by(double x, double d, double r) {
+  const double q = x * r;
+  if ((__double2hiint(q) & 0x7FF00000) == 0x7FF00000) return q;   // infinite or NaN
+  return fma(fma(-q, d, x), r, q);
+}
+
 // |x| as an ordered integer (the bit pattern of a non-negative double grows with
 // its value), for maxima without floating-point instructions
 __device__ __forceinline__ unsigned long long absbits(double x) {

@@ -2,6 +2,7 @@
 // charge normalisation, RK4 stage updates, the polarisation / charge sources and
 // the field resampling between the propagation grid and the wire grid (FP64).
 #include "cluster_sum.cuh"
+#include "fp_bits.cuh"
 #include "sbe_ctx.cuh"
 #include "spline.cuh"
 
@@ -108,69 +109,75 @@ __device__ __forceinline__ double2 cexp_d(double2 z) {
 
 // mode 0: relaxation and normalisation; 1: relaxation only (the relaxed complex
 // diagonals back into C3, D3); 2: normalisation only.  One cluster per wire: the four
-// exponentials and divisions per k are bound by the FP64 pipes of its SMs.
+// exponentials and divisions per k are bound by the FP64 pipes of its SMs, a warp's
+// instruction by its 64 clocks, so they run side by side in a warp's lanes (1 x 64: 12.6 -> 6.7 us).
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
     k_relax_norm(const WireDev* wires, double2* C3, double2* D3, const double* wrate,
                  const double* rsp, double dt, double2* ne_out, double2* nh_out, double* charge,
                  int mode) {
   pdl_enter();
   const WireDev& W = wires[blockIdx.y];
-  const int nk = W.nk, k0 = blockIdx.x + kCluster * threadIdx.x, kst = kCluster * 256;
+  // four lanes per k: electrons and holes, the two exponentials and then the two components
+  const int nk = W.nk, sub = threadIdx.x & 3, kst = kCluster * 64;
+  const int k0 = blockIdx.x + kCluster * (threadIdx.x >> 2);
+  const unsigned quad = 0xFu << (threadIdx.x & 28);
+  const bool hole = sub >= 2, im = sub & 1;
+  double2* X3 = hole ? D3 : C3;
+  double2* x_out = hole ? nh_out : ne_out;
   const bool relax = mode != 2 && (W.flags & (SBE_F_PHONON | SBE_F_EHS)) != 0;
   // the decay is part of the relaxation, which runs only with Phonon or EHs
   // (SBEs.py:5677, 5322)
   const bool recomb = relax && (W.flags & SBE_F_RECOMB) != 0;
-  double se = 0.0, sh = 0.0;
+  double sum = 0.0;
   for (int k = k0; k < nk; k += kst) {
-    long long o = W.off_mat + (long long)k * nk + k;
-    double2 ne = C3[o], nh = D3[o];
+    const long long o = W.off_mat + (long long)k * nk + k;
+    double2 n = X3[o];
     if (relax) {
-      const double* wr = wrate + 4 * W.off_vec;
-      double wie = wr[k], woe = wr[nk + k], wih = wr[2 * nk + k], woh = wr[3 * nk + k];
-      double We = wie + woe, Wh = wih + woh;
-      double ee = exp(-We * dt), ep = exp(We * dt);
-      double he = exp(-Wh * dt), hp = exp(Wh * dt);
-      double den_e = We + kSmall, den_h = Wh + kSmall;
-      ne = make_double2(ee * ((-1 + ep + ne.x) * wie + ne.x * woe) / den_e,
-                        ee * (ne.y * wie + ne.y * woe) / den_e);
-      nh = make_double2(he * ((-1 + hp + nh.x) * wih + nh.x * woh) / den_h,
-                        he * (nh.y * wih + nh.y * woh) / den_h);
+      const double* wr = wrate + 4 * W.off_vec + (hole ? 2 * nk : 0);
+      const double wi = wr[k], wo = wr[nk + k], w = wi + wo;
+      const double mine = exp(im ? w * dt : -w * dt);
+      const double other = __shfl_xor_sync(quad, mine, 1);
+      const double em = im ? other : mine, ep = im ? mine : other;
+      const double first = im ? n.y : -1 + ep + n.x, x = im ? n.y : n.x;
+      const double y = em * (first * wi + x * wo) / (w + kSmall);
+      const double z = __shfl_xor_sync(quad, y, 1);
+      n = im ? make_double2(z, y) : make_double2(y, z);
     }
     if (recomb) {
       // SBEs.py:5322-5325: ne exp(-Rsp nh dt), then nh exp(-Rsp ne dt) with the new ne
       // (complex occupations, complex exponential)
       const double r = rsp[W.off_vec + k];
-      ne = cmul(ne, cexp_d(make_double2(-r * nh.x * dt, -r * nh.y * dt)));
-      nh = cmul(nh, cexp_d(make_double2(-r * ne.x * dt, -r * ne.y * dt)));
+      for (int turn = 0; turn < 2; ++turn) {
+        const double2 u = make_double2(__shfl_xor_sync(quad, n.x, 2), __shfl_xor_sync(quad, n.y, 2));
+        if (hole == (turn == 1)) n = cmul(n, cexp_d(make_double2(-r * u.x * dt, -r * u.y * dt)));
+      }
     }
     if (mode == 1) {
-      C3[o] = ne;
-      D3[o] = nh;
+      __syncwarp(quad);
+      if (!im) X3[o] = n;
       continue;
     }
-    const double ae = cabs_d(ne), ah = cabs_d(nh);
-    ne_out[W.off_vec + k] = make_double2(ae, 0.0);
-    nh_out[W.off_vec + k] = make_double2(ah, 0.0);
-    se += ae;
-    sh += ah;
+    const double a = cabs_d(n);
+    if (!im) {
+      x_out[W.off_vec + k] = make_double2(a, 0.0);
+      sum += a;
+    }
   }
   if (mode == 1) return;   // uniform over the cluster
-  cluster_sum2(se, sh);
-  if (k0 == 0) {
+  double se = hole ? 0.0 : sum, sh = hole ? sum : 0.0;
+  cluster_sum2(se, sh, blockIdx.x + kCluster * ((threadIdx.x & ~31) >> 2) < nk);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     // the carrier numbers before the normalisation: their difference is what this
     // step's relaxation and rounding left of the electron-hole balance
     charge[2 * blockIdx.y] = se;
     charge[2 * blockIdx.y + 1] = sh;
   }
-  double total = (se + sh) / 2.0;
-  double fe = total / (se + kSmall), fh = total / (sh + kSmall);
+  if (im || k0 >= nk) return;
+  const double f = (se + sh) / 2.0 / ((hole ? sh : se) + kSmall);
   for (int k = k0; k < nk; k += kst) {
-    long long o = W.off_mat + (long long)k * nk + k;
-    double ae = ne_out[W.off_vec + k].x * fe, ah = nh_out[W.off_vec + k].x * fh;
-    ne_out[W.off_vec + k] = make_double2(ae, 0.0);
-    nh_out[W.off_vec + k] = make_double2(ah, 0.0);
-    C3[o] = make_double2(ae, 0.0);
-    D3[o] = make_double2(ah, 0.0);
+    const double2 a = make_double2(x_out[W.off_vec + k].x * f, 0.0);
+    x_out[W.off_vec + k] = a;
+    X3[W.off_mat + (long long)k * nk + k] = a;
   }
 }
 
@@ -278,14 +285,15 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
                 const double2* nh, double2* src) {
   pdl_enter();
   const WireDev& W = wires[w_only >= 0 ? w_only : blockIdx.y];
-  const int nr = W.nr, nk = W.nk, j0 = blockIdx.x + kCluster * threadIdx.x, st = kCluster * 256;
+  // two lanes per point: electron and hole density
+  const int nr = W.nr, nk = W.nk, st = kCluster * 128;
+  const int j0 = blockIdx.x + kCluster * (threadIdx.x >> 1);
+  const bool hole = threadIdx.x & 1;
   double2* re = src + 5 * W.off_r + 3 * nr;
   double2* rh = re + nr;
+  double2* rho = hole ? rh : re;
   if (!(W.flags & SBE_F_LF)) {
-    for (int j = j0; j < nr; j += st) {
-      re[j] = make_double2(0, 0);
-      rh[j] = make_double2(0, 0);
-    }
+    for (int j = j0; j < nr; j += st) rho[j] = make_double2(0, 0);
     return;
   }
   double v[4] = {0, 0, 0, 0};   // carrier sums, boundary sums
@@ -299,22 +307,25 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
     v[2] = re[j].x;
     v[3] = rh[j].x;
   }
-  block_sums(v);
-  const double NeT = v[0] + 1e-50, NhT = v[1] + 1e-50, be = v[2] / 20.0, bh = v[3] / 20.0;
-  double ae = 0, ah = 0;
-  for (int j = j0; j < nr; j += st) {
-    const double2 x = re[j], y = rh[j];
-    ae += cabs_d(make_double2(x.x - be, x.y));
-    ah += cabs_d(make_double2(y.x - bh, y.y));
+  block_sums(v, (threadIdx.x & ~31) < nk || threadIdx.x < 32);
+  const bool live = blockIdx.x + kCluster * ((threadIdx.x & ~31) >> 1) < nr;
+  double sum = 0.0, bnd = 0.0;
+  if (live) {
+    bnd = div_by(hole ? v[3] : v[2], 20.0, 0.05);
+    for (int j = j0; j < nr; j += st) {
+      const double2 x = rho[j];
+      sum += cabs_d(make_double2(x.x - bnd, x.y));
+    }
   }
-  cluster_sum2(ae, ah);
+  double ae = hole ? 0.0 : sum, ah = hole ? sum : 0.0;
+  cluster_sum2(ae, ah, live);
+  if (j0 >= nr) return;
   const double* rw = r + W.off_r;
-  const double dr = rw[1] - rw[0], f = 2.0 * kE0 / W.area * W.ehint;
-  const double fe = f * (NeT / (ae * dr + kQwSmall)), fh = f * (NhT / (ah * dr + kQwSmall));
+  const double dr = rw[1] - rw[0], N = (hole ? v[1] : v[0]) + 1e-50;
+  const double f = W.rho_scale * (N / ((hole ? ah : ae) * dr + kQwSmall));
   for (int j = j0; j < nr; j += st) {
-    const double2 x = re[j], y = rh[j];
-    re[j] = make_double2((x.x - be) * fe, x.y * fe);
-    rh[j] = make_double2((y.x - bh) * fh, y.y * fh);
+    const double2 x = rho[j];
+    rho[j] = make_double2((x.x - bnd) * f, x.y * f);
   }
 }
 
@@ -621,7 +632,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(256)
     B += y;
   }
   double total = mode == 0 ? 0.0 : *total_io;
-  cluster_sum2(A, B);
+  cluster_sum2(A, B, blockIdx.x * 256 + (threadIdx.x & ~31) < n);
   if (mode == 0) {
     total = (A * dx + B * dx + kQwSmall) / 2.0;
     if (i0 == 0) *total_io = total;
