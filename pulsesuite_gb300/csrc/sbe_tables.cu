@@ -124,13 +124,19 @@ __global__ void k_grid(const WireDev* wires, double* kr, double* r, double* Ee, 
 // exp(-(a1 y_i)^2) exp(-(a2 y_j)^2) K0t(dk sqrt((y_i-y_j)^2 + D0^2)) depends on
 // i-j through K0t only, so corr[m] = sum_{i-j=m} ea_i eb_j is formed once and
 // each V(Q) is a sum over m.
+// A wire's 3 (Nr + 2) scratch values, in the layout order of its tables: off_r + 2 per wire
+// before it there, off_r being the sum of their Nr = 2 Nk + 2 and off_vec that of their Nk.
+__device__ __forceinline__ long long vcorr_offset(const WireDev& W) {
+  return 6 * (W.off_r - W.off_vec);
+}
+
 __global__ void k_vcorr(const WireDev* wires, const double* r, double* vcorr) {
   const WireDev W = wires[blockIdx.y];
   int n = blockIdx.z;  // 0 eh, 1 ee, 2 hh
   double a1 = (n == 2) ? W.alphah : W.alphae;
   double a2 = (n == 1) ? W.alphae : W.alphah;
   int N1 = W.nr / 4, N2 = 3 * W.nr / 4, N = N2 - N1 + 1;
-  double* out = vcorr + 3 * (W.off_r + 2 * blockIdx.y) + (long long)n * (W.nr + 2);
+  double* out = vcorr + vcorr_offset(W) + (long long)n * (W.nr + 2);
   const double* y = r + W.off_r + N1;
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < 2 * N - 1; m += gridDim.x * blockDim.x) {
     int dm = m - (N - 1);  // i - j
@@ -154,7 +160,7 @@ __global__ void k_vtab(const WireDev* wires, const double* r, const double* vcor
   double a1 = (n == 2) ? W.alphah : W.alphae;
   double a2 = (n == 1) ? W.alphae : W.alphah;
   int N1 = W.nr / 4, N2 = 3 * W.nr / 4, N = N2 - N1 + 1;
-  const double* cor = vcorr + 3 * (W.off_r + 2 * blockIdx.z) + (long long)n * (W.nr + 2);
+  const double* cor = vcorr + vcorr_offset(W) + (long long)n * (W.nr + 2);
   const double* y = r + W.off_r;
   double dyy = y[1] - y[0];
   // Qr (GetKArray rolled): ((d + Nr/2) dk) - ((Nr/2) dk) with dk = 2 pi / (2 L)
