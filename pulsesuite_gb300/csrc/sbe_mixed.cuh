@@ -8,6 +8,8 @@
 
 namespace sbe {
 
+constexpr int kMaxima = 15;   // maxima of a wire's step (see Mixed)
+
 struct Mixed {
   int nk = 0, nw = 0, nr = 0;
   int first = 0;                          // position of its first wire in the layout order
@@ -24,8 +26,8 @@ struct Mixed {
   tc::PlaneSet pl{}, tp{}, sp{}, ep{};   // commutator, Toeplitz, sheared, E^T planes
   float* xsh = nullptr;    // exchange sums, un-sheared: 3 x Nw x Nk x Nk complex (FP32)
   void* block = nullptr;   // one allocation for the per-wire vectors below
-  int* ints = nullptr;     // eS, eH, eT, eE, esc, esx, ess, (spare), eO  (9 x nw)
-  unsigned* mx = nullptr;  // Hamiltonian, state, hbar A/B and off-diagonal maxima (4 x nw)
+  int* ints = nullptr;     // eT, eE, esc, esx, ess (5 x nw)
+  unsigned* mx = nullptr;  // the step's maxima (kMaxima x nw)
   unsigned long long* mx64 = nullptr;   // nw: FP64 maxima of the phonon tables
   float* vsf = nullptr;    // 3 x nw x nk screened V by |k1 - k2|
   float2* trf = nullptr;   // 4 x nw x nk traces [2][2nk]
@@ -39,18 +41,19 @@ struct Mixed {
   float2* tpart = nullptr;  // nw x 2 x 32 ceil(2nk/32) x T diagonal partials (T = ceil(nk/32))
   float* cdf = nullptr;     // 4 x nw x nk: hi / lo parts of Re C_kk and Re D_kk (stage state)
   double* xdg = nullptr;    // 2 x nw x nk: Re C_kk, Re D_kk of the stage state in FP64
-  int* eS() { return ints; }
-  int* eH() { return ints + nw; }
-  int* eT() { return ints + 2 * nw; }
-  int* eE() { return ints + 3 * nw; }
-  int* esc() { return ints + 4 * nw; }
-  int* esx() { return ints + 5 * nw; }
-  int* ess() { return ints + 6 * nw; }
-  int* eO() { return ints + 8 * nw; }   // commutator state operands (diagonals of C, D peeled)
-  unsigned* mxH() { return mx; }
-  unsigned* mxS() { return mx + nw; }
-  unsigned* mxAB() { return mx + 2 * nw; }
-  unsigned* mxO() { return mx + 3 * nw; }  // max over P and the off-diagonal C, D
+  int* eT() { return ints; }
+  int* eE() { return ints + nw; }
+  int* esc() { return ints + 2 * nw; }
+  int* esx() { return ints + 3 * nw; }
+  int* ess() { return ints + 4 * nw; }
+  // Maxima, a set of their own for every stage that collects them, so that one memset clears
+  // those of a step: of the states that stages 1 to 4 read (n = 0 .. 3) and of the new one
+  // (n = 4), all elements and P with the off-diagonal C, D; of the stages' Hamiltonians; of the
+  // step's 2 hbar |A|, |B|
+  unsigned* mxS(int n) { return mx + n * nw; }
+  unsigned* mxO(int n) { return mx + (5 + n) * nw; }
+  unsigned* mxH(int n) { return mx + (10 + n) * nw; }
+  unsigned* mxAB() { return mx + 14 * nw; }
 };
 
 struct MixedAll {
@@ -62,10 +65,10 @@ struct MixedAll {
   float* habf = nullptr;     // 2 x tot_mat hbar A, hbar B
   float* epf = nullptr;      // EP, EP^T, HP, HP^T scaled by 2^sP (tot_mat each)
   float *eptf = nullptr, *hpf = nullptr, *hptf = nullptr;
-  float2* ekf = nullptr;     // 3 x tot_r stage field
+  float2* ekf = nullptr;     // 3 x (3 x tot_r) fields at the step's start, middle and end
   float2* ekrf = nullptr;    // tot_kr Expikr
   int* err = nullptr;        // engine error flag (bounded waits that gave up)
-  unsigned* mx = nullptr;    // the buckets' maxima (4 x nw in all)
+  unsigned* mx = nullptr;    // the buckets' maxima
 };
 
 // matrix slots of the commutator plane sets

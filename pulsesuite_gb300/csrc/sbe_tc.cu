@@ -54,39 +54,24 @@ __device__ __forceinline__ void exponents(Blk blk, int nb, const unsigned* mx, i
 }
 SBE_PASS(ExponentsPass, 128, exponents);
 
-// The exponents of one stage in one launch (one thread per wire): eS from the
-// full state maximum, eO from the off-diagonal one, esx = eT + eS (exchange
-// products); with reset set the maxima are cleared for the fused RK4 update of
-// the stage, which collects the next state's maxima in them; mxH is cleared for
-// the stage's Hamiltonian.
-__device__ __forceinline__ void stage_exponents(Blk blk, int nb, unsigned* mxS, unsigned* mxO,
-                                                unsigned* mxH, int* eS, int* eO, const int* eT,
-                                                int* esx, int reset) {
-  const int b = blk.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  const int vs = exponent_of(__uint_as_float(mxS[b]));
-  eS[b] = vs;
-  eO[b] = exponent_of(__uint_as_float(mxO[b]));
-  esx[b] = eT[b] + vs;
-  mxH[b] = 0u;
-  if (reset) {
-    mxS[b] = 0u;
-    mxO[b] = 0u;
-  }
+// The exponent of a matrix: of the larger of two collected maxima (b may be null).  Every block
+// of a pass forms it for itself; a pass that some product's scale depends on leaves it there
+// (sum[b] = exponent + add[b]) from its first block.
+struct ExpOf {
+  const unsigned *a, *b;
+  const int* add;
+  int* sum;
+};
+__device__ __forceinline__ int exponent_of(const ExpOf& x, int b) {
+  float m = __uint_as_float(x.a[b]);
+  if (x.b) m = fmaxf(m, __uint_as_float(x.b[b]));
+  return exponent_of(m);
 }
-SBE_PASS(StageExponentsPass, 128, stage_exponents);
-
-// e[b] from the larger of two maxima (rule of k_exponents) and sum[b] = e[b] + add[b]
-__device__ __forceinline__ void exponents2_sum(Blk blk, int nb, const unsigned* mx1,
-                                               const unsigned* mx2, int* e, const int* add,
-                                               int* sum) {
-  const int b = blk.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  const int v = exponent_of(fmaxf(__uint_as_float(mx1[b]), __uint_as_float(mx2[b])));
-  e[b] = v;
-  sum[b] = v + add[b];
+__device__ __forceinline__ int exponent_of(const ExpOf& x, int b, bool first) {
+  const int e = exponent_of(x, b);
+  if (x.sum && first) x.sum[b] = e + x.add[b];
+  return e;
 }
-SBE_PASS(HamExponentsPass, 128, exponents2_sum);
 
 __device__ __forceinline__ void put_hilo(__half* base, long long plane, float v) {
   const __half h = __float2half_rn(v);
@@ -191,7 +176,7 @@ __device__ __forceinline__ void store_tiles_t(const __half (*hs)[32][40], int np
 // The block (32 x 8 threads) converts its 32 x 32 tile once into shared-memory
 // plane tiles and writes both layouts with 16-byte stores.
 template <typename T>
-__device__ __forceinline__ void planes_nt(Blk blk, const T* X, int nk, const int* e,
+__device__ __forceinline__ void planes_nt(Blk blk, const T* X, int nk, ExpOf e,
                                           tc::PlaneSet dst, int matN, int matT, int nbatch,
                                           float* cdf, const double* dg) {
   __shared__ T tile[32][33];
@@ -214,7 +199,7 @@ __device__ __forceinline__ void planes_nt(Blk blk, const T* X, int nk, const int
     for (int k = 0; k < 4; ++k) tile[threadIdx.y + 8 * k][threadIdx.x] = v[k];
   }
   __syncthreads();
-  const int eb = e[b];
+  const int eb = exponent_of(e, b, blk.x + blk.y + threadIdx.x + threadIdx.y == 0);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int i = threadIdx.y + 8 * k;
@@ -420,7 +405,7 @@ struct Carver {
 static void carve_bucket(Mixed* m, Carver& k) {
   const size_t v = (size_t)m->nw * m->nk;
   const int T = (m->nk + 31) / 32;
-  m->ints = k.take<int>(9 * (size_t)m->nw);
+  m->ints = k.take<int>(5 * (size_t)m->nw);
   m->mx64 = k.take<unsigned long long>((size_t)m->nw);
   m->sP = k.take<int>((size_t)m->nw);
   m->vsf = k.take<float>(3 * v);
@@ -447,10 +432,10 @@ static void carve_all(MixedAll* A, Carver& k, const SbeCtx* c) {
   A->eptf = k.take<float>(tm);
   A->hpf = k.take<float>(tm);
   A->hptf = k.take<float>(tm);
-  A->ekf = k.take<float2>(3 * (size_t)c->tot_r);
+  A->ekf = k.take<float2>(9 * (size_t)c->tot_r);
   A->ekrf = k.take<float2>((size_t)c->tot_kr);
   A->err = k.take<int>(1);
-  A->mx = k.take<unsigned>(4 * (size_t)c->nw);
+  A->mx = k.take<unsigned>(kMaxima * (size_t)c->nw);
 }
 
 static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
@@ -534,8 +519,8 @@ static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
     const int nk = m->nk, nw = m->nw;
     const long long mm = (long long)nk * nk;
     const int T = (nk + 31) / 32;
-    cudaMemsetAsync(m->ints, 0, sizeof(int) * 9 * nw, s);
-    m->mx = A->mx + 4 * (size_t)m->first;
+    cudaMemsetAsync(m->ints, 0, sizeof(int) * 5 * nw, s);
+    m->mx = A->mx + kMaxima * (size_t)m->first;
     // the padding of every plane set stays zero: producers write only inside; the
     // sheared planes are zeroed once, stages write only the in-band part
     cudaMemsetAsync(m->pl.ptr, 0, tc::planeset_bytes(m->pl), s);
@@ -1015,13 +1000,14 @@ SBE_PASS(SrcReducePass, 256, src_reduce_f);
 // dpart[((b * 2 + n - 1) * ndd + dd) * grid x + block x]; the traces of the
 // direct Coulomb terms are their sums over the blocks that exist.
 __device__ __forceinline__ void shear_tiles(Blk blk, int nk, int nw, int ndd, const float2* X0,
-                                            const float2* X1, const float2* X2, const int* e,
+                                            const float2* X1, const float2* X2, ExpOf e,
                                             tc::PlaneSet dst, float2* dpart) {
   __shared__ float2 tile[63][32];
   __shared__ __align__(16) __half hs[2][64][40];   // hi, lo of rows 2 dd0 .. 2 dd0 + 63
   const int n = blk.z / nw, b = blk.z % nw;
   const int t0 = blk.x * 32;
   const int dd0 = (shear_first_block(nk, t0) + blk.y) * 32;
+  const int eb = exponent_of(e, b, n + blk.x + blk.y + threadIdx.x + threadIdx.y == 0);
   if (dd0 >= ndd || !shear_block_live(nk, t0, dd0)) return;
   const float2* X = (n == 0 ? X0 : n == 1 ? X1 : X2) + (long long)b * nk * nk;
   const int rbase = t0 + dd0 - (nk - 1);
@@ -1055,7 +1041,6 @@ __device__ __forceinline__ void shear_tiles(Blk blk, int nk, int nw, int ndd, co
     dpart[(((long long)b * 2 + n - 1) * ndd + dd0 + tx) * blk.gx + blk.x] =
         make_float2(sr, si);
   }
-  const int eb = e[b];
 #pragma unroll
   for (int kd = 0; kd < 4; ++kd) {
     const int ddl = ty + 8 * kd;
@@ -1086,21 +1071,23 @@ __device__ __forceinline__ void shear_tiles(Blk blk, int nk, int nw, int ndd, co
 }
 SBE_PASS(ShearPass, 256, shear_tiles);
 
-// The stage field in FP32.
-
-__global__ void k_field_f(long long n, const double2* ek, const double2* dek, double frac,
-                          float2* ekf) {
+// The field in FP32: at the start, middle and end of the step, Ek0 + frac dEk in FP64 (as the
+// FP64 path's stage field), or Ek0 alone.
+__global__ void k_field_f(long long n, const double2* ek, const double2* dek, float2* ekf) {
   pdl_enter();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double2 a = ek[i];
-  if (dek) {
-    // stage field Ek0 + frac dEk in FP64 (as the FP64 path's stage field)
-    const double2 d = dek[i];
-    a.x += frac * d.x;
-    a.y += frac * d.y;
+  const double2 a = ek[i];
+  if (!dek) {
+    ekf[i] = f64_to_f32(a);
+    return;
   }
-  ekf[i] = f64_to_f32(a);
+  const double2 d = dek[i];
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    const double frac = 0.5 * f;
+    ekf[f * n + i] = f64_to_f32(make_double2(a.x + frac * d.x, a.y + frac * d.y));
+  }
 }
 
 // H = Meh + diagonal energies + direct Coulomb terms + exchange sums
@@ -1208,44 +1195,50 @@ __device__ __forceinline__ void h_build(Blk blk, const WireDev* __restrict__ wir
 }
 SBE_PASS(HBuildPass, 128, h_build);
 
-// Planes of Hee', Hhh' (slots M_EE, M_HH) and of Hee' + i hbar B, Hhh' + i hbar A
-// (slots M_EEX, M_HHX) from the FP32 values.
-__device__ __forceinline__ void hplanes(Blk blk, const float2* hee, const float2* hhh,
-                                        const float* hA, const float* hB, int nk, const int* e,
-                                        tc::PlaneSet dst, int nw) {
+// Planes of Heh and Heh^T (slots M_EH, M_EHT), of Hee', Hhh' (M_EE, M_HH) and of
+// Hee' + i hbar B, Hhh' + i hbar A (M_EEX, M_HHX) from the FP32 values.
+__device__ __forceinline__ void hplanes(Blk blk, const float2* heh, const float2* hee,
+                                        const float2* hhh, const float* hA, const float* hB,
+                                        int nk, ExpOf e, const unsigned* mxo, int* esc,
+                                        tc::PlaneSet dst) {
   // block (32, 8) over a 32 x 32 tile; each slot's planes go through shared memory
   __shared__ __align__(16) __half hs[4][32][40];
   const int b = blk.z;
   const int r0 = blk.y * 32, c0 = blk.x * 32, tx = threadIdx.x, ty = threadIdx.y;
   const long long mm = (long long)nk * nk;
-  const int eb = e[b];
-  float2 a[4], h[4];
+  const int tid = ty * 32 + tx;
+  float2 x[4], a[4], h[4];
   float aa[4], bb[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int r = r0 + ty + 8 * k, c = c0 + tx;
     const bool in = r < nk && c < nk;
     const long long o = (long long)b * mm + (long long)r * nk + c;
+    x[k] = in ? heh[o] : make_float2(0.f, 0.f);
     a[k] = in ? hee[o] : make_float2(0.f, 0.f);
     h[k] = in ? hhh[o] : make_float2(0.f, 0.f);
     bb[k] = in ? hB[o] : 0.f;
     aa[k] = in ? hA[o] : 0.f;
   }
-  const int slot[4] = {M_EE, M_HH, M_EEX, M_HHX};
-  const int tid = ty * 32 + tx;
-  for (int sl = 0; sl < 4; ++sl) {
+  // H exponent: max over the operands and the step's 2 hbar |A|, |B|
+  const int eb = exponent_of(e, b);
+  if (blk.x + blk.y + tid == 0) esc[b] = eb + exponent_of(__uint_as_float(mxo[b]));
+  const int slot[5] = {M_EH, M_EE, M_HH, M_EEX, M_HHX};
+  for (int sl = 0; sl < 5; ++sl) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int i = ty + 8 * k;
-      const float2 v = sl == 0 ? a[k]
-                       : sl == 1 ? h[k]
-                       : sl == 2 ? make_float2(a[k].x, a[k].y + bb[k])
+      const float2 v = sl == 0 ? x[k]
+                       : sl == 1 ? a[k]
+                       : sl == 2 ? h[k]
+                       : sl == 3 ? make_float2(a[k].x, a[k].y + bb[k])
                                  : make_float2(h[k].x, h[k].y + aa[k]);
       hilo4(make_float2(f32_ldexp(v.x, eb), f32_ldexp(v.y, eb)), &hs[0][i][tx], &hs[1][i][tx],
             &hs[2][i][tx], &hs[3][i][tx]);
     }
     __syncthreads();
     store_tiles(hs, 4, dst, slot[sl], b, r0, c0 >> 5, tid, 256);
+    if (sl == 0) store_tiles_t(hs, 4, dst, M_EHT, b, c0, r0 >> 5, tid, 256);
     __syncthreads();
   }
 }
@@ -1691,7 +1684,7 @@ static std::vector<Mixed*> by_size(const MixedAll* A) { return {A->b.rbegin(), A
 static int mixed_prep(SbeCtx* c, const double2* C, const double2* D, cudaStream_t s) {
   MixedAll* A = all_of(c);
   // the maxima that this step's passes collect
-  cudaMemsetAsync(A->mx, 0, sizeof(unsigned) * 4 * c->nw, s);
+  cudaMemsetAsync(A->mx, 0, sizeof(unsigned) * kMaxima * c->nw, s);
   launch_prep_scalar(c, C, D, s);   // occupations, screening (FP64, O(Nk) per wire)
   const std::vector<Mixed*> buckets = by_size(A);
   {
@@ -1749,7 +1742,7 @@ static void mixed_relax(SbeCtx* c, double2* P, double2* C, double2* D, const dou
   launch_mbc_rates(c, -1, s, false, true);
   launch_relax_only(c, P, C, D, Ek, dt, s);
   Batch<DiagMaxPass> pass(256, s);
-  for (Mixed* m : buckets) pass.add(m->nw, m->dw, C, D, m->mxS());
+  for (Mixed* m : buckets) pass.add(m->nw, m->dw, C, D, m->mxS(4));
 }
 
 // Stage-1 state of the mixed path from the FP64 state: FP32 copies (the first
@@ -1765,30 +1758,35 @@ static void mixed_state_in(SbeCtx* c, const double2* P, const double2* C, const 
     const int nk = m->nk, nw = m->nw;
     const long long mm = (long long)nk * nk, vn = (long long)nw * nk, o = m->bm;
     const dim3 grid((unsigned)std::min<long long>((mm + 255) / 256, 128), nw);
-    pass.add(grid, P + o, nk, 0, m->mxS(), m->mxO(), xf + o, nullptr);
-    pass.add(grid, C + o, nk, 1, m->mxS(), m->mxO(), xf + tm + o, m->xdg);
-    pass.add(grid, D + o, nk, 1, m->mxS(), m->mxO(), xf + 2 * tm + o, m->xdg + vn);
+    pass.add(grid, P + o, nk, 0, m->mxS(0), m->mxO(0), xf + o, nullptr);
+    pass.add(grid, C + o, nk, 1, m->mxS(0), m->mxO(0), xf + tm + o, m->xdg);
+    pass.add(grid, D + o, nk, 1, m->mxS(0), m->mxO(0), xf + 2 * tm + o, m->xdg + vn);
   }
+}
+
+// The field of the step's stages in FP32 (all wires): Ek, or with dEk also at the step's middle
+// and end.
+static void mixed_field(SbeCtx* c, const double2* Ek, const double2* dEk, cudaStream_t s) {
+  launch(k_field_f, (int)((3 * c->tot_r + 255) / 256), 256, 0, s, 3 * c->tot_r, Ek, dEk,
+         all_of(c)->ekf);
 }
 
 // One RHS evaluation of the mixed path on the FP32 stage state xs (P, C, D at
 // xs, xs + tot_mat, xs + 2 tot_mat; the FP64 diagonals of C and D in each bucket's
-// xdg; the state maxima already in mxS, mxO) with the wire-k field Ek + frac dEk
-// (dEk may be null).  With stage 1-4 the RK4 update of that stage is fused into the
+// xdg; the state maxima already in the stage's mxS, mxO) with the wire-k field ekf.
+// With stage 1-4 the RK4 update of that stage is fused into the
 // element-wise passes (X64: the FP64 states P, C, D; the next stage state goes to
-// the FP32 stage buffer and its maxima to mxS, mxO); stage 0 stores the RHS in kf.
-static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const double2* dEk,
-                       double frac, int stage, double dt, double2* const* X64, cudaStream_t s) {
+// the FP32 stage buffer and its maxima to the next mxS, mxO); stage 0 stores the RHS in kf.
+static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage, double dt,
+                       double2* const* X64, cudaStream_t s) {
   MixedAll* A = all_of(c);
   const long long tm = c->tot_mat;
   const int have_x = (c->wires[0].flags & SBE_F_EXCITONS) ? 1 : 0;
-  // stage field in FP32 (all wires)
-  launch(k_field_f, (int)((3 * c->tot_r + 255) / 256), 256, 0, s, 3 * c->tot_r, Ek, dEk, frac,
-         A->ekf);
-  // state exponents and planes: P and P^T from one read; C and D need only their own
-  // layout (C^T = conj C and D^T = conj D for the Hermitian C and D).  eS: full state
-  // maximum (sheared exchange operands); eO: maximum over P and the off-diagonal C, D
-  // (commutator operands; the diagonals of C and D are peeled off and applied exactly
+  const int in = stage > 0 ? stage - 1 : 0;   // maxima of the stage's state
+  // state planes: P and P^T from one read; C and D need only their own
+  // layout (C^T = conj C and D^T = conj D for the Hermitian C and D).  The sheared exchange
+  // operands take the exponent of the full state maximum, the commutator operands that over P
+  // and the off-diagonal C, D (the diagonals of C and D are peeled off and applied exactly
   // in the element-wise passes)
   const std::vector<Mixed*> buckets = by_size(A);
   const dim3 tile(32, 8);
@@ -1796,20 +1794,15 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
     return dim3((m->nk + 31) / 32, (m->nk + 31) / 32, m->nw);
   };
   {
-    Batch<StageExponentsPass> pass(128, s);
-    for (Mixed* m : buckets)
-      pass.add((m->nw + 127) / 128, m->nw, m->mxS(), m->mxO(), m->mxH(), m->eS(), m->eO(), m->eT(),
-               m->esx(), stage > 0);
-  }
-  {
     Batch<PlanesPass> pass(tile, s);
     for (Mixed* m : buckets) {
       const int nk = m->nk, nw = m->nw;
       const long long vn = (long long)nw * nk;
       const float2 *P = xs + m->bm, *C = xs + tm + m->bm, *D = xs + 2 * tm + m->bm;
-      pass.add(tiles(m), P, nk, m->eO(), m->pl, M_P, M_PT, nw, nullptr, nullptr);
-      pass.add(tiles(m), C, nk, m->eO(), m->pl, M_C, -1, nw, m->cdf, m->xdg);
-      pass.add(tiles(m), D, nk, m->eO(), m->pl, M_D, -1, nw, m->cdf + 2 * vn, m->xdg + vn);
+      const ExpOf e{m->mxO(in), nullptr, nullptr, nullptr};
+      pass.add(tiles(m), P, nk, e, m->pl, M_P, M_PT, nw, nullptr, nullptr);
+      pass.add(tiles(m), C, nk, e, m->pl, M_C, -1, nw, m->cdf, m->xdg);
+      pass.add(tiles(m), D, nk, e, m->pl, M_D, -1, nw, m->cdf + 2 * vn, m->xdg + vn);
     }
   }
   if (have_x) {
@@ -1827,7 +1820,8 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
         ny = std::max(ny, cnt);
       }
       shear.add(dim3(nbk, ny, 3 * nw), nk, nw, ndd, xs + m->bm, xs + tm + m->bm,
-                xs + 2 * tm + m->bm, m->eS(), m->sp, m->tpart);
+                xs + 2 * tm + m->bm, ExpOf{m->mxS(in), nullptr, m->eT(), m->esx()}, m->sp,
+                m->tpart);
     }
     shear.flush();
     for (Mixed* m : buckets)
@@ -1846,26 +1840,15 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
     Batch<HBuildPass> pass(128, s);
     for (Mixed* m : buckets)
       pass.add(dim3((m->nk + 511) / 512, (m->nk + HB_ROWS - 1) / HB_ROWS, m->nw), m->dw, m->nw,
-               A->ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh),
-               have_x, A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH());
-  }
-  {
-    // H exponent: max over the operands and the step's 2 hbar |A|, |B|
-    Batch<HamExponentsPass> pass(128, s);
-    for (Mixed* m : buckets)
-      pass.add((m->nw + 127) / 128, m->nw, m->mxH(), m->mxAB(), m->eH(), m->eO(), m->esc());
-  }
-  {
-    Batch<PlanesPass> pass(tile, s);
-    for (Mixed* m : buckets)
-      pass.add(tiles(m), A->hf + m->bm, m->nk, m->eH(), m->pl, M_EH, M_EHT, m->nw, nullptr,
-               nullptr);
+               ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh),
+               have_x, A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH(in));
   }
   {
     Batch<HPlanesPass> pass(tile, s);
     for (Mixed* m : buckets)
-      pass.add(tiles(m), A->hf + tm + m->bm, A->hf + 2 * tm + m->bm, A->habf + m->bm,
-               A->habf + tm + m->bm, m->nk, m->eH(), m->pl, m->nw);
+      pass.add(tiles(m), A->hf + m->bm, A->hf + tm + m->bm, A->hf + 2 * tm + m->bm,
+               A->habf + m->bm, A->habf + tm + m->bm, m->nk,
+               ExpOf{m->mxH(in), m->mxAB(), nullptr, nullptr}, m->mxO(in), m->esc(), m->pl);
   }
   // commutator GEMMs: dP and the cross terms of W and V, then the hi*hi products of
   // W and V (the partials of W and V meet in the anti-Hermitian pass)
@@ -1905,8 +1888,8 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const double2* Ek, const dou
       rk[i].acc = A->accf + i * tm + o;
       rk[i].xf = xn + i * tm + o;
       rk[i].dg = i > 0 ? m->xdg + (i - 1) * vn : nullptr;
-      rk[i].mx = m->mxS();
-      rk[i].mo = m->mxO();
+      rk[i].mx = m->mxS(in + 1);
+      rk[i].mo = m->mxO(in + 1);
     }
     dp.add(tiles(m), nk, nw, gp + o, A->hf + o, P, m->dgf, m->gamf, m->cdf, A->kf + o, rk[0]);
     dcd.add(tiles(m), nk, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf, m->dgf + vn, m->cdf,
@@ -1926,17 +1909,13 @@ static int mixed_sources(SbeCtx* c, const double2* P, const double2* C, const do
   MixedAll* A = all_of(c);
   const std::vector<Mixed*> buckets = by_size(A);
   {
-    Batch<ExponentsPass> pass(128, s);
-    for (Mixed* m : buckets)
-      pass.add((m->nw + 127) / 128, m->nw, m->mxS(), m->eS(), m->eE(), m->ess());
-  }
-  {
     Batch<Planes64Pass> pass(dim3(32, 8), s);
     const double2* st[3] = {P, C, D};
     for (Mixed* m : buckets)
       for (int i = 0; i < 3; ++i)
-        pass.add(dim3((m->nk + 31) / 32, (m->nk + 31) / 32, m->nw), st[i] + m->bm, m->nk, m->eS(),
-                 m->pl, 2 * i, -1, m->nw, nullptr, nullptr);
+        pass.add(dim3((m->nk + 31) / 32, (m->nk + 31) / 32, m->nw), st[i] + m->bm, m->nk,
+                 ExpOf{m->mxS(4), nullptr, m->eE(), i ? nullptr : m->ess()}, m->pl, 2 * i, -1,
+                 m->nw, nullptr, nullptr);
   }
   float2* gf = reinterpret_cast<float2*>(c->G);
   {
@@ -1970,8 +1949,8 @@ int rhs_mixed(SbeCtx* c, const double2* P, const double2* C, const double2* D, c
   MixedAll* A = all_of(c);
   const long long n = c->tot_mat;
   mixed_state_in(c, P, C, D, s);
-  rc = mixed_stage(c, reinterpret_cast<const float2*>(c->xs), Ek, nullptr, 0.0, 0, 0.f, nullptr,
-                   s);
+  mixed_field(c, Ek, nullptr, s);
+  rc = mixed_stage(c, reinterpret_cast<const float2*>(c->xs), A->ekf, 0, 0.0, nullptr, s);
   if (rc) return rc;
   const int g = (int)((n + 255) / 256);
   launch(k_f32_to_f64, g, 256, 0, s, n, A->kf, dP);
@@ -1987,16 +1966,18 @@ int rk4_mixed(SbeCtx* c, double2* P, double2* C, double2* D, const double2* Ek0,
   rc = mixed_prep(c, C, D, s);
   if (rc) return rc;
   const long long n = c->tot_mat;
-  const double frac[4] = {0.0, 0.5, 0.5, 1.0};
   // FP32 stage buffers in the FP64 stage-state block (6 tot_mat float2): the
   // step-start state (kept for the RK4 updates), then the stage states of stages 2-4
   float2* x0 = reinterpret_cast<float2*>(c->xs);
   mixed_state_in(c, P, C, D, s);
+  mixed_field(c, Ek0, dEk, s);
+  const MixedAll* A = all_of(c);
   double2* X64[3] = {P, C, D};
   for (int st = 1; st <= 4; ++st) {
     // the RHS of this stage (stage field Ek0 + frac dEk) and its RK4 update (fused
     // into the element-wise passes)
-    rc = mixed_stage(c, st == 1 ? x0 : x0 + 3 * n, Ek0, dEk, frac[st - 1], st, dt, X64, s);
+    const float2* ekf = A->ekf + (dEk ? (st / 2) * 3 * c->tot_r : 0);
+    rc = mixed_stage(c, st == 1 ? x0 : x0 + 3 * n, ekf, st, dt, X64, s);
     if (rc) return rc;
   }
   mixed_relax(c, P, C, D, Ek0, dt, s);   // the new diagonals join the maximum
