@@ -1454,7 +1454,6 @@ __device__ __forceinline__ void antiherm(Blk blk, int nk, const float2* __restri
   }
   if (rk.stage != 0) rk4_block_max(rk, b, mxv, mov);
 }
-SBE_PASS(AntihermPass, 256, antiherm);
 
 // dP of a stage from the FP32 commutator sums G (the engine's scaled products with
 // the off-diagonal C', D'), following dpdt (SBEs.py:1942-1965):
@@ -1542,7 +1541,19 @@ __device__ __forceinline__ void rhs_p(Blk blk, int nk, int nw, const float2* __r
   }
   if (rk.stage != 0) rk4_block_max(rk, b, mxv, mov);
 }
-SBE_PASS(RhsPPass, 256, rhs_p);
+
+// dP, dC and dD of a bucket in one pass: which 0 dP (M0 the sums, M1 Heh, v0 the energies, f0 the
+// rates, f1 the occupations), 1 dC or dD (W, H', energies hi and lo, occupations hi and lo).
+__device__ __forceinline__ void stage_update(Blk blk, int which, int nk, int nw, const float2* M0,
+                                             const float2* M1, const float2* X, const float2* v0,
+                                             const float2* v1, const float* f0, const float* f1,
+                                             float2* out, Rk4Ctl rk) {
+  if (which == 0)
+    rhs_p(blk, nk, nw, M0, M1, X, v0, f0, f1, out, rk);
+  else
+    antiherm(blk, nk, M0, M1, X, v0, v1, f0, f1, out, rk);
+}
+SBE_PASS(StageUpdatePass, 256, stage_update);
 
 __global__ void k_f32_to_f64(long long n, const float2* a, double2* out) {
   pdl_enter();
@@ -1866,8 +1877,7 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage
   // stage buffers (FP32, 3 tot_mat each): the step-start state, then the stage states
   float2* x0 = reinterpret_cast<float2*>(c->xs);
   float2* xn = x0 + 3 * tm;
-  Batch<RhsPPass> dp(tile, s);
-  Batch<AntihermPass> dcd(tile, s);
+  Batch<StageUpdatePass> pass(tile, s);
   for (Mixed* m : buckets) {
     const int nk = m->nk, nw = m->nw;
     const long long vn = (long long)nw * nk, o = m->bm;
@@ -1891,14 +1901,14 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage
       rk[i].mx = m->mxS(in + 1);
       rk[i].mo = m->mxO(in + 1);
     }
-    dp.add(tiles(m), nk, nw, gp + o, A->hf + o, P, m->dgf, m->gamf, m->cdf, A->kf + o, rk[0]);
-    dcd.add(tiles(m), nk, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf, m->dgf + vn, m->cdf,
-            m->cdf + vn, A->kf + tm + o, rk[1]);
-    dcd.add(tiles(m), nk, wf + G_V * tm + o, A->hf + 2 * tm + o, D, m->dgf + 2 * vn,
-            m->dgf + 3 * vn, m->cdf + 2 * vn, m->cdf + 3 * vn, A->kf + 2 * tm + o, rk[2]);
+    pass.add(tiles(m), 0, nk, nw, gp + o, A->hf + o, P, m->dgf, nullptr, m->gamf, m->cdf,
+             A->kf + o, rk[0]);
+    pass.add(tiles(m), 1, nk, nw, wf + G_W * tm + o, A->hf + tm + o, C, m->dgf, m->dgf + vn, m->cdf,
+             m->cdf + vn, A->kf + tm + o, rk[1]);
+    pass.add(tiles(m), 1, nk, nw, wf + G_V * tm + o, A->hf + 2 * tm + o, D, m->dgf + 2 * vn,
+             m->dgf + 3 * vn, m->cdf + 2 * vn, m->cdf + 3 * vn, A->kf + 2 * tm + o, rk[2]);
   }
-  dp.flush();
-  dcd.flush();
+  pass.flush();
   return cuda_check(cudaGetLastError(), "mixed stage");
 }
 
