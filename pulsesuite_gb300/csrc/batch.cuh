@@ -39,7 +39,8 @@ __device__ __forceinline__ void call_part(const Blk& b, const Args<H, T...>& s, 
 }
 
 template <class Body, int N, class... P>
-__global__ void __launch_bounds__(Body::kThreads) k_parts(const __grid_constant__ Parts<N, P...> p) {
+__global__ void __launch_bounds__(Body::kThreads, Body::kBlocks)
+    k_parts(const __grid_constant__ Parts<N, P...> p) {
   pdl_enter();
   const int at = p.same ? blockIdx.z : blockIdx.x;
   int i = 0;   // a constant with one part: its arguments stay where they are
@@ -136,15 +137,17 @@ class Batch<Body, void (*)(Blk, P...)> {
   size_t smem_;
 };
 
-// Names device function f, void(Blk, ...), as the body of a batched pass.
-#define SBE_PASS(Name, threads, f)                            \
-  struct Name {                                               \
-    static constexpr int kThreads = threads;                  \
-    static decltype(&f) signature();                          \
-    template <class... A>                                     \
+// Names a device function, void(Blk, ...), as the body of a batched pass (blocks: per SM at least,
+// 0 for no bound).
+#define SBE_PASS_BLOCKS(Name, threads, blocks, ...)             \
+  struct Name {                                                 \
+    static constexpr int kThreads = threads, kBlocks = blocks;  \
+    static decltype(&__VA_ARGS__) signature();                  \
+    template <class... A>                                       \
     __device__ __forceinline__ static void run(const A&... a) { \
-      f(a...);                                                \
-    }                                                         \
+      __VA_ARGS__(a...);                                        \
+    }                                                           \
   }
+#define SBE_PASS(Name, threads, ...) SBE_PASS_BLOCKS(Name, threads, 0, __VA_ARGS__)
 
 }  // namespace sbe

@@ -2,6 +2,7 @@
 // off-diagonal dephasing, and the Hartree-Fock Hamiltonians (FP64).
 #include "cluster_sum.cuh"
 #include "sbe_ctx.cuh"
+#include "batch.cuh"
 #include "fp_bits.cuh"
 
 namespace sbe {
@@ -226,7 +227,7 @@ void launch_gamma(SbeCtx* c, int w_only, cudaStream_t s) {
 // species "b".  g3 = [gam_eh, gam_e, gam_h]: De uses (g0, g2), Dh uses (g1, g2) (quirk kept).
 //
 // GB300 runs two FP64 operations per clock and SM, so the kernel is written for their
-// count.  On the reference grid the energy differences are integer forms (see k_offdiag_D32,
+// count.  On the reference grid the energy differences are integer forms (see offdiag_D32,
 // which also derives row -q from the sums of row q):
 //   a-a: E = 2 c_a dkr^2 q (k - p + q), tabulated per q: two FMAs per (q, k, p);
 //   a-b: E = q dkr^2 [c_a (2k - 2 j0 + q) + c_b (2p - 2 j0 + q)]: one add, one FMA for
@@ -435,15 +436,13 @@ __device__ inline void split12(double v, float* hi, float* lo) {
 //   sa(-q, k + q) = sb(q, k) [+ the a-a term p = q],  sb(-q, k + q) = sa(q, k) [+ ..]
 // and a block writes D[q][k] and D[-q][k + q] for every k with k + q < Nk, and
 // the zeros of both rows elsewhere; the Lorentzian sums are formed once.
-__global__ void __launch_bounds__(128) k_offdiag_D32(const WireDev* wires, const int* wl,
-                                                     const float* occf,
-                                                     const float* dconst, const float* dpre,
-                                                     double* De, double* Dh) {
-  pdl_enter();
-  const int wi = wl[blockIdx.z >> 1], which = blockIdx.z & 1;   // 0 De, 1 Dh
+__device__ __forceinline__ void offdiag_D32(Blk blk, const WireDev* wires, const int* wl,
+                                            const float* occf, const float* dconst,
+                                            const float* dpre, double* De, double* Dh) {
+  const int wi = wl[blk.z >> 1], which = blk.z & 1;   // 0 De, 1 Dh
   const WireDev& W = wires[wi];
   const int nk = W.nk;
-  const int q = blockIdx.y;   // 0 .. nk; row -q from the same sums
+  const int q = blk.y;   // 0 .. nk; row -q from the same sums
   if (q > nk) return;
   extern __shared__ float sh[];
   float* na = sh;                                        // |n_a|
@@ -485,8 +484,8 @@ __global__ void __launch_bounds__(128) k_offdiag_D32(const WireDev* wires, const
   double* Dm = D + (long long)(nk - q) * nk;   // row -q
   // the a-a term p = q of row -q (absent from row q): L(alpha q k) weights
   const float n0a = na[0], nqa = (q < nk) ? na[q] : 0.f;
-  for (int k0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4; k0 < nk;
-       k0 += gridDim.x * blockDim.x * 4) {
+  for (int k0 = (blk.x * blockDim.x + threadIdx.x) * 4; k0 < nk;
+       k0 += blk.gx * blockDim.x * 4) {
     float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
     if (vaa != 0.f) {
       const int plo = max(q + 1, 0), phi = min(q + nk - 1, nk - 1);
@@ -565,6 +564,7 @@ __global__ void __launch_bounds__(128) k_offdiag_D32(const WireDev* wires, const
     }
   }
 }
+SBE_PASS(Deph1Pass, 128, offdiag_D32);
 
 // The same sums for a group of NW wires that share their Lorentzian factors (same
 // Nk, masses, grid and rates): each Lorentzian is formed once and applied to every
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(128) k_offdiag_D32(const WireDev* wires, const
 // X = (vaa sa + vab ta, vaa sb + vab tb)).  Each thread sums KPT consecutive k for
 // all NW wires, so that every shared-memory weight load (32 p at a time, [p][wire]
 // as float2, read as float4) feeds 2 KPT FMAs; the a-a Lorentzian window slides in
-// registers.  Rows q and -q as in k_offdiag_D32.  grid (Nk / (128 KPT), Nk + 1, species).
+// registers.  Rows q and -q as in offdiag_D32.  grid (Nk / (128 KPT), Nk + 1, species).
 // Packed FP32 pairs (PTX f32x2, sm_100 and later): one fma.rn.f32x2 forms two
 // IEEE FP32 fused multiply-adds (each rounded as fmaf) from one issue slot.
 __device__ __forceinline__ unsigned long long f2_splat(float a) {
@@ -592,16 +592,14 @@ __device__ __forceinline__ float2 f2_unpack(unsigned long long a) {
 }
 
 template <int NW, int KPT>
-__global__ void __launch_bounds__(128, 2) k_offdiag_D32g(const WireDev* wires, const int* wl,
-                                                      int nwl, const float* occf,
-                                                      const float* dconst, const float* dpre,
-                                                      double* De, double* Dh) {
-  pdl_enter();
+__device__ __forceinline__ void offdiag_D32g(Blk blk, const WireDev* wires, const int* wl, int nwl,
+                                             const float* occf, const float* dconst,
+                                             const float* dpre, double* De, double* Dh) {
   constexpr int PC = 32;   // p per shared-memory chunk
-  const int which = blockIdx.z;
+  const int which = blk.z;
   const WireDev& W0 = wires[wl[0]];
   const int nk = W0.nk;
-  const int q = blockIdx.y;
+  const int q = blk.y;
   if (q > nk) return;
   extern __shared__ __align__(16) float sh[];
   float2* ws = reinterpret_cast<float2*>(sh);   // [PC][NW]
@@ -640,7 +638,7 @@ __global__ void __launch_bounds__(128, 2) k_offdiag_D32g(const WireDev* wires, c
     soa[tid] = oa;
     sob[tid] = ob;
   }
-  const int k0 = (blockIdx.x * blockDim.x + tid) * KPT;   // this thread's first k
+  const int k0 = (blk.x * blockDim.x + tid) * KPT;   // this thread's first k
   // sums (x, y) of wire w at k0 + j as one packed FP32 pair; the weights of a
   // wire are the pair (x, y) in shared memory, so one f32x2 FMA updates both
   unsigned long long acc[KPT][NW];
@@ -780,8 +778,10 @@ __global__ void __launch_bounds__(128, 2) k_offdiag_D32g(const WireDev* wires, c
     }
   }
 }
+SBE_PASS_BLOCKS(Deph8Pass, 128, 2, offdiag_D32g<8, 4>);
+SBE_PASS_BLOCKS(Deph16Pass, 128, 2, offdiag_D32g<16, 4>);
 
-// Constants of k_offdiag_D32 (FP64, once per step): per (wire, species)
+// Constants of offdiag_D32 (FP64, once per step): per (wire, species)
 // [2 c_a dkr^2 / b_aa, head/tail of c_a dkr^2 / b_ab, head/tail of c_b dkr^2 / b_ab]
 // and per |q| the prefactors V_aa(q)^2 / (hbar b_aa) and V_ab(q)^2 / (hbar b_ab)
 // (D = (pi/hbar) V^2 Lorentz = V^2 / (hbar b) / (1 + u^2)).
@@ -814,30 +814,25 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
   if (fp32 && w_only < 0 && !g3) {
     launch(k_deph_consts, dim3((c->nk_max + 127) / 128, 2 * c->nw), 128, 0, s, c->d_wires, c->vs,
            c->dconst, c->dpre);
-    // groups of 4 or more wires share the Lorentzian factors (chunks of up to 16
-    // wires); the other wires take the per-wire kernel, one launch each
-    for (const auto& g : c->dgroups) {
-      const int gk = c->wires[c->dwl_host[g.first]].nk;
-      if (g.second < 4) {
-        const size_t sm1 = sizeof(float) * 8 * (size_t)gk;
-        for (int i = 0; i < g.second; ++i)
-          launch(k_offdiag_D32, dim3((gk + 511) / 512, gk + 1, 2), 128, sm1, s, c->d_wires,
-                 c->dwl + g.first + i, c->occf, c->dconst, c->dpre, c->De, c->Dh);
-        continue;
-      }
+    // groups of 4 or more wires share the Lorentzian factors (chunks of up to 16 wires); the
+    // other wires take the per-wire sums.  One launch per kind, the largest Nk first
+    size_t nk = c->nk_max;
+    Batch<Deph16Pass> g16(128, s, sizeof(float) * (2 * 32 * 16 + 2 * nk));
+    Batch<Deph8Pass> g8(128, s, sizeof(float) * (2 * 32 * 8 + 2 * nk));
+    Batch<Deph1Pass> g1(128, s, sizeof(float) * 8 * nk);
+    for (auto g = c->dgroups.rbegin(); g != c->dgroups.rend(); ++g) {
+      const int gk = c->wires[c->dwl_host[g->first]].nk;
       const dim3 grid((gk + 511) / 512, gk + 1, 2);   // 128 threads x 4 k
-      for (int o = 0; o < g.second; o += 16) {
-        const int n = std::min(16, g.second - o);
-        const int* wl = c->dwl + g.first + o;
-        if (n <= 8) {
-          const size_t sm = sizeof(float) * (2 * 32 * 8 + 2 * (size_t)gk);
-          launch(k_offdiag_D32g<8, 4>, grid, 128, sm, s, c->d_wires, wl, n, c->occf, c->dconst,
-                 c->dpre, c->De, c->Dh);
-        } else {
-          const size_t sm = sizeof(float) * (2 * 32 * 16 + 2 * (size_t)gk);
-          launch(k_offdiag_D32g<16, 4>, grid, 128, sm, s, c->d_wires, wl, n, c->occf, c->dconst,
-                 c->dpre, c->De, c->Dh);
-        }
+      for (int o = 0; o < g->second;) {
+        const int n = g->second < 4 ? 1 : std::min(16, g->second - o);
+        const int* wl = c->dwl + g->first + o;
+        o += n;
+        if (g->second < 4)
+          g1.add(grid, c->d_wires, wl, c->occf, c->dconst, c->dpre, c->De, c->Dh);
+        else if (n <= 8)
+          g8.add(grid, c->d_wires, wl, n, c->occf, c->dconst, c->dpre, c->De, c->Dh);
+        else
+          g16.add(grid, c->d_wires, wl, n, c->occf, c->dconst, c->dpre, c->De, c->Dh);
       }
     }
     return;
