@@ -14,48 +14,71 @@ __device__ int g_err;   // a bounded wait gave up
 // ---------------------------------------------------------------------------
 // slicing
 
-// Block: 8 rows of one form of one matrix; warps walk the K blocks, a lane takes 8
-// consecutive k of one row (lane = 4 row + chunk), so a warp stores 512 contiguous bytes
-// per plane and the transposed read covers 128-byte segments.  KB K blocks of a warp stay in
-// registers between the row maximum, the norm and the digits (Nk up to 256 KB); longer rows
-// are read again (from L2).  HBM bound: 16 B read and 32 B written per element.
-template <int KB>
-__global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ SliceArgs a) {
+// Block: 8 rows, or with few K blocks (PACK) as many groups of 8 as its warps can take, of one
+// form of one matrix; a group's warps (SPLIT: pairs of warps, real and imaginary
+// part) walk the K blocks, a lane takes 8 consecutive k of one row (lane = 4 row + chunk), so a
+// warp stores 512 contiguous bytes per plane and the transposed read covers 128-byte segments.  KB
+// K blocks of a warp stay in registers between the row maximum, the norm and the digits (Nk up to
+// 256 KB); longer rows are read again (from L2).  HBM bound: 16 B read and 32 B written per
+// element.  The split halves a thread's chain of digits, which bounds a few small wires (1 x 64
+// 8.9 -> 7.4 us a launch), and its registers, of which two K blocks take too many (2 x 512 75 ->
+// 60); with one K block and many rows its 8-byte reads cost more (8 x 256 62 -> 70), and the warps
+// that two K blocks leave idle take other rows (32 x 64 52 -> 27, 8 x 128 33 -> 28).
+constexpr int kSliceStep = 8;   // K blocks in flight
+
+// log2 of the warps that walk the K blocks of one group of 8 rows (PACK)
+__host__ __device__ inline int slice_lgw(int nkb) { return nkb > 2 ? 2 : nkb - 1; }
+
+template <int KB, bool SPLIT, bool PACK>
+__global__ void __launch_bounds__(32 * kSliceStep * (SPLIT ? 2 : 1))
+    k_f64_slice(const __grid_constant__ SliceArgs a) {
   pdl_enter();
+  constexpr int kWarps = kSliceStep * (SPLIT ? 2 : 1), NC = SPLIT ? 1 : 2;
   const Form& f = a.f[blockIdx.y];
   const int kdim = a.kdim, ld = a.ld, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 8 + (lane >> 2), j = lane & 3;
   const int nkb = k_blocks(kdim), rows_pad = pad_rows(a.rows);
+  const int im = SPLIT ? warp & 1 : 0, w = SPLIT ? warp >> 1 : warp;
+  const int lgw = PACK ? slice_lgw(nkb) : 3, kStep = 1 << lgw, kw = w & (kStep - 1);
+  const int g0 = PACK ? warp - kw : 0, gw = PACK ? kStep : kWarps;   // the group's warps
+  const int r = ((blockIdx.x << (3 - lgw)) + (w >> lgw)) * 8 + (lane >> 2), j = lane & 3;
   const double2* X = f.src + (long long)b * a.src_batch;
   const double2* Y = f.add ? f.add + (long long)b * a.src_batch : nullptr;
-  const bool rok = r < a.rows, held = nkb <= 8 * KB;
-  auto load = [&](int kb, double2* v) {
+  const bool rok = r < a.rows, held = nkb <= kStep * KB;
+  auto load = [&](int kb, double (*v)[8]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = kb * BK + 8 * j + i;
-      v[i] = make_double2(0.0, 0.0);
-      if (rok && k < kdim) {
-        v[i] = f.transpose ? X[(long long)k * ld + r] : X[(long long)r * ld + k];
-        if (Y) v[i].y += a.add_f * Y[(long long)r * ld + k].x;
+      const long long o = f.transpose ? (long long)k * ld + r : (long long)r * ld + k;
+      const bool in = rok && k < kdim;
+      if constexpr (SPLIT) {
+        v[0][i] = in ? reinterpret_cast<const double*>(X)[2 * o + im] : 0.0;
+        if (in && Y && im) v[0][i] += a.add_f * Y[(long long)r * ld + k].x;
+      } else {
+        const double2 z = in ? X[o] : make_double2(0.0, 0.0);
+        v[0][i] = z.x;
+        v[1][i] = z.y;
+        if (in && Y) v[1][i] += a.add_f * Y[(long long)r * ld + k].x;
       }
     }
   };
-  __shared__ unsigned long long red[8][8];
-  __shared__ float reds[8][8];
-  double2 v[KB][8];
+  __shared__ unsigned long long red[kWarps][8];
+  __shared__ float reds[kWarps][8];
+  double v[KB][NC][8];
   unsigned long long m = 0;
-  auto maximum = [&](const double2* x) {
+  auto maximum = [&](const double (*x)[8]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = max(m, max(absbits(x[i].x), absbits(x[i].y)));
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = max(m, absbits(x[c][i]));
   };
   if (held) {
 #pragma unroll
-    for (int u = 0; u < KB; ++u) load(warp + 8 * u, v[u]);   // zeros past the last K block
+    for (int u = 0; u < KB; ++u) load(kw + kStep * u, v[u]);   // zeros past the last K block
 #pragma unroll
     for (int u = 0; u < KB; ++u) maximum(v[u]);
   } else {
-    for (int kb = warp; kb < nkb; kb += 8) {
+    for (int kb = kw; kb < nkb; kb += kStep) {
       load(kb, v[0]);
       maximum(v[0]);
     }
@@ -66,19 +89,22 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
   __syncthreads();
   m = 0;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) m = max(m, red[w][lane >> 2]);
+  for (int i = 0; i < kWarps; ++i)
+    if (i < gw) m = max(m, red[g0 + i][lane >> 2]);
   const int Em = max_exp(m);
   float sq = 0.f;
-  auto squares = [&](const double2* x) {
+  auto squares = [&](const double (*x)[8]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sq += scaled_sq(x[i].x, Em) + scaled_sq(x[i].y, Em);
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sq += scaled_sq(x[c][i], Em);
   };
   if (Em != kBadExp) {
     if (held) {
 #pragma unroll
       for (int u = 0; u < KB; ++u) squares(v[u]);
     } else {
-      for (int kb = warp; kb < nkb; kb += 8) {
+      for (int kb = kw; kb < nkb; kb += kStep) {
         load(kb, v[0]);
         squares(v[0]);
       }
@@ -90,27 +116,27 @@ __global__ void __launch_bounds__(256) k_f64_slice(const __grid_constant__ Slice
   __syncthreads();
   sq = 0.f;
 #pragma unroll
-  for (int w = 0; w < 8; ++w) sq += reds[w][lane >> 2];
+  for (int i = 0; i < kWarps; ++i)
+    if (i < gw) sq += reds[g0 + i][lane >> 2];
   const int E = norm_exp(Em, sq);
-  if (warp == 0 && j == 0 && rok) f.e[(long long)b * a.rows + r] = E;
+  if (kw == 0 && im == 0 && j == 0 && rok) f.e[(long long)b * a.rows + r] = E;
   if (!rok) return;
-  __half* dst = f.dst + (long long)b * a.dst_batch;
-  auto digits = [&](int kb, const double2* x) {
-    long long q[8];
-    __half* d = dst + chunk_off(rows_pad, r, kb, j);
+  __half* dst = f.dst + (long long)b * a.dst_batch + im * NS * a.plane;
+  auto digits = [&](int kb, const double (*x)[8]) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(x[i].x, E);
-    store_digits(q, d, a.plane);
+    for (int c = 0; c < NC; ++c) {
+      long long q[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(x[i].y, E);
-    store_digits(q, d + NS * a.plane, a.plane);
+      for (int i = 0; i < 8; ++i) q[i] = E == kBadExp ? 0 : to_fixed(x[c][i], E);
+      store_digits(q, dst + chunk_off(rows_pad, r, kb, j) + c * NS * a.plane, a.plane);
+    }
   };
   if (held) {
 #pragma unroll
     for (int u = 0; u < KB; ++u)
-      if (warp + 8 * u < nkb) digits(warp + 8 * u, v[u]);
+      if (kw + kStep * u < nkb) digits(kw + kStep * u, v[u]);
   } else {
-    for (int kb = warp; kb < nkb; kb += 8) {
+    for (int kb = kw; kb < nkb; kb += kStep) {
       load(kb, v[0]);
       digits(kb, v[0]);
     }
@@ -537,11 +563,20 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
 }  // namespace f64s
 
 void launch_f64_slice(const f64s::SliceArgs& a, int nforms, cudaStream_t s) {
-  const dim3 grid((a.rows + 7) / 8, nforms, a.batch);
-  if (f64s::k_blocks(a.kdim) <= 8)
-    launch(f64s::k_f64_slice<1>, grid, 256, 0, s, a);
-  else
-    launch(f64s::k_f64_slice<2>, grid, 256, 0, s, a);
+  const int nkb = f64s::k_blocks(a.kdim);
+  dim3 grid((a.rows + 7) / 8, nforms, a.batch);
+  const long long blocks = (long long)grid.x * grid.y * grid.z;
+  if (nkb > f64s::kSliceStep) {
+    launch(f64s::k_f64_slice<2, true, false>, grid, 512, 0, s, a);
+  } else if (blocks < 4 * 152) {
+    launch(f64s::k_f64_slice<1, true, false>, grid, 512, 0, s, a);
+  } else if (nkb > 4) {
+    launch(f64s::k_f64_slice<1, false, false>, grid, 256, 0, s, a);
+  } else {
+    const int per = 8 << (3 - f64s::slice_lgw(nkb));
+    grid.x = (a.rows + per - 1) / per;
+    launch(f64s::k_f64_slice<1, false, true>, grid, 256, 0, s, a);
+  }
 }
 
 static int sm_count() {
