@@ -19,13 +19,14 @@
 //      holds the x lines of all three components of its (ky, kz) columns)
 //   4  y lines, inverse
 //   5  z lines, inverse, 1/N, and out += a c (+ ja J), mask (FP64 out)
-// Every transform is a radix-2 Stockham sequence in shared memory.  The work array
+// Every transform is a Stockham sequence in shared memory (FP64 in radix 4).  The work array
 // W is FP64 or FP32 complex (chosen at creation): with FP32 work the three middle
 // passes move half the bytes and the FP64 field is touched only by passes 1 and 5.
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
+#include "fft64.cuh"
 #include "fp_bits.cuh"
 #include "pstd3d.cuh"
 
@@ -108,6 +109,13 @@ __device__ T* fft_smem(T* a, T* b, int lg, int lgtr, int ps, int cs, bool c_fast
     b = t;
   }
   return a;
+}
+
+// The FP64 transforms run in radix 4 (fft64.cuh).
+template <>
+__device__ double2* fft_smem<double2>(double2* a, double2* b, int lg, int lgtr, int ps, int cs,
+                                      bool c_fast, int dir, const double2* tw, const float2*) {
+  return fft64(a, b, lg, lgtr, ps, cs, c_fast, dir, tw);
 }
 
 __host__ __device__ inline int ilog2i(int v) {
