@@ -223,7 +223,7 @@ __device__ __forceinline__ void planes_nt(Blk blk, const T* X, int nk, ExpOf e,
 SBE_PASS(PlanesPass, 256, planes_nt<float2>);
 SBE_PASS(Planes64Pass, 256, planes_nt<double2>);
 
-// Band of the sheared state planes (k_shear_tiles): the first dd block of the
+// Band of the sheared state planes (shear_tiles): the first dd block of the
 // t' block at t0 whose source rows can reach the matrix, and whether the block
 // (t0, dd0) holds any element of it.
 __host__ __device__ inline int shear_first_block(int nk, int t0) {
@@ -235,7 +235,7 @@ __host__ __device__ inline bool shear_block_live(int nk, int t0, int dd0) {
   return rbase + 62 >= 0 && rbase < nk;
 }
 
-// Traces from the diagonal partials of k_shear_tiles: diagonal dd = k1 - k2 + Nk - 1
+// Traces from the diagonal partials of shear_tiles: diagonal dd = k1 - k2 + Nk - 1
 // of X (row k1, column k2) is trace index d + Nk with d = k2 - k1, summed over the
 // nb column blocks in a fixed order into trf[b][which][d + Nk] (SBEs.py:1094-1103).
 __device__ __forceinline__ void trace_from_shear(Blk blk, int nk, int nb, int ndd,
@@ -1256,7 +1256,7 @@ __device__ __forceinline__ float2 two_sum(float a, float b) {
   return make_float2(s, e);
 }
 
-// RK4 stage update fused into the element-wise RHS passes (k_rhs_p, k_antiherm):
+// RK4 stage update fused into the element-wise RHS passes (rhs_p, antiherm):
 // the stage derivative k of an element is used where it is formed.  The
 // arithmetic is that of the RK4 of the mixed path: FP32 k and sums k1 + 2 k2 +
 // 2 k3; stages 1-3 write the next stage state in FP32 (xf = fp32(X) + f k) and,
