@@ -45,7 +45,7 @@ extern "C" {
 #define SBE_F_LORENTZ    (1 << 11)  /* LorentzDelta of mb.params: Lorentzian broadening of the EHs rates */
 
 /* Precision of the RHS contractions. */
-#define SBE_PREC_FP64  0  /* plain FP64 SIMT (drop-in path and on-device reference) */
+#define SBE_PREC_FP64  0  /* FP64 (drop-in path and on-device reference) */
 #define SBE_PREC_MIXED 1  /* tcgen05 FP16 hi/lo x3, FP32 accumulate, FP64 state    */
 
 /* One wire: grid and material in SI units (qw.params, SBEs.py:4978-5002). */
@@ -92,7 +92,11 @@ int sbe_ctx_layout(const SbeCtx* ctx, long long* out, long long* total_mat, long
  * 11 xe/xh (2*Nk), 12 Expikr (c128 Nk*Nr), 13 scalars (16 doubles).          */
 int sbe_ctx_table(const SbeCtx* ctx, int w, int which, void* dst, long long nbytes, void* stream);
 
-/* ---- reference pure functions, one wire, FP64 ---------------------------- */
+/* ---- reference pure functions, one wire, FP64 ----------------------------
+ * From Nk = 32 on the products run on digit planes in scratch from a stream-ordered
+ * pool of the library's own, which keeps up to 64 MB between calls (no host
+ * synchronisation); without that memory, and inside a stream capture, on plain FP64
+ * kernels that need none.                                                      */
 /* SBEs.py:1839 dpdt (p[kh][ke]).                                               */
 int sbe_dpdt(int nk, const double* C, const double* D, const double* P, const double* Heh,
              const double* Hee, const double* Hhh, const double* GamE, const double* GamH,
@@ -104,9 +108,9 @@ int sbe_dCdt(int nk, const double* C, const double* D, const double* P, const do
 int sbe_dDdt(int nk, const double* C, const double* D, const double* P, const double* Heh,
              const double* Hee, const double* Hhh, double* out, void* stream);
 /* SBEs.py:658 CalcH (VC is Nk*Nk*3 real, [k1][k2][n]; only VC[q][0][n] is read).
- * Having no context, it takes its scratch (3 Nk doubles, 4 Nk complex) from the
- * device's stream-ordered pool (cudaMallocAsync / cudaFreeAsync on stream: no host
- * synchronisation); the batched context path builds H with no allocation.      */
+ * The plain kernels take their scratch (3 Nk doubles, 4 Nk complex) from the
+ * device's stream-ordered pool (cudaMallocAsync / cudaFreeAsync on stream); the
+ * batched context path builds H with no allocation.                             */
 int sbe_calch(int nk, const double* Meh, const double* Wee, const double* Whh, const double* C,
               const double* D, const double* P, const double* VC, const double* Ee,
               const double* Eh, double gap, int excitons, int lf, int freepot, double* Heh,

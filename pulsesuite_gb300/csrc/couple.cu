@@ -536,7 +536,6 @@ int sbe_couple_create(SbeCtx* c, SbePstd* p, const double* wire_x, const SbeCoup
   cudaMemcpyAsync(cp->wx, wire_x, sizeof(double) * c->nw, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(cp->probn, pn.data(), sizeof(int) * pn.size(), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(cp->probl, pl.data(), sizeof(long long) * pl.size(), cudaMemcpyHostToDevice, s);
-  // elimination factors of the grid knots and of each wire's knots (computed once)
   k_twr<<<dim3((c->nr_max + 127) / 128, c->nw), 128, 0, s>>>(c->d_wires, cp->twr, cp->twrf);
   int rc = cuda_check(cudaGetLastError(), "sbe_couple_create");
   if (rc == SBE_OK) rc = cuda_check(cudaStreamSynchronize(s), "sbe_couple_create: tables");

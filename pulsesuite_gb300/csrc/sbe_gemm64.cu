@@ -1,5 +1,5 @@
-// Plain FP64 SIMT complex GEMMs of the SBE right-hand side (the drop-in path and
-// the on-device FP64 reference of the mixed-precision path).
+// Plain FP64 SIMT complex GEMMs of the SBE right-hand side, for wires of Nk < 32 and
+// where the digit-plane products (f64_path.cu) have no workspace, and of DC transport.
 //
 // dpdt/dCdt/dDdt (SBEs.py:1942-1965, 2309-2327, 2607-2625) are sums of four
 // complex matrix products each (p stored [kh][ke]):
