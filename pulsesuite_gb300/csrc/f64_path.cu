@@ -627,9 +627,6 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       const FormSet F{m.pl, m.ef, nk, g, m.sl_m};
       launch(k_f64_diag, dim3((2 * nk - 1 + 3) / 4, 3, g), 128, 0, s, nk, P + o, C + o, D + o,
              c->tr + 4 * vo, m.es);
-      f64s::SliceArgs a = slice_args(F);
-      state_forms(a, F, P + o, C + o, D + o);
-      launch_f64_slice(a, 6, s);
       int rc = SBE_OK;
       if (exc)
         rc = exchange(nk, g, P + o, C + o, D + o, m.tp + w0 * m.sl_m, (long long)m.nw * m.sl_m,
@@ -654,8 +651,11 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       h.Hhh = c->Hhh + o;
       launch(k_f64_hbuild, dim3((nk + 127) / 128, nk, g), 128, 0, s, h);
       const double2* hm[3] = {c->Heh + o, c->Hee + o, c->Hhh + o};
-      a = slice_args(F);
-      int nf = 0, alias[F_N];
+      // the state's forms with the Hamiltonians' in one launch (two: 1 x 64 315 us a step, here
+      // 289; 8 x 256 4.22 ms, 4.14)
+      f64s::SliceArgs a = slice_args(F);
+      state_forms(a, F, P + o, C + o, D + o);
+      int nf = 6, alias[F_N];
       for (int i = 0; i < F_N; ++i) alias[i] = i;
       for (int i = 0; i < 6; ++i)
         a.f[nf++] = f64s::Form{hm[i / 2], nullptr, i & 1, F.plane(F_EH + i), F.exps(F_EH + i)};
