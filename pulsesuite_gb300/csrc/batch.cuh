@@ -100,8 +100,8 @@ class Batch<Body, void (*)(Blk, P...)> {
     const dim3 grid = p_.same ? dim3(p_.gx[0], p_.gy[0], (unsigned)z) : dim3((unsigned)flat);
     if (p_.n == 1)
       start<1>(grid);
-    else if (p_.n <= 3)
-      start<3>(grid);
+    else if (p_.n <= 4)
+      start<4>(grid);
     else
       start<kMax>(grid);
     p_.n = 0;

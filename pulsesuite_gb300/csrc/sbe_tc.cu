@@ -1244,6 +1244,20 @@ __device__ __forceinline__ void hplanes(Blk blk, const float2* heh, const float2
 }
 SBE_PASS(HPlanesPass, 256, hplanes);
 
+// The commutators' operand planes in one pass: which 0 a state matrix (X0), 1 the Hamiltonians.
+__device__ __forceinline__ void operand_planes(Blk blk, int which, const float2* X0,
+                                               const float2* hee, const float2* hhh,
+                                               const float* hA, const float* hB, int nk, ExpOf e,
+                                               const unsigned* mxo, int* esc, tc::PlaneSet dst,
+                                               int matN, int matT, int nbatch, float* cdf,
+                                               const double* dg) {
+  if (which == 0)
+    planes_nt<float2>(blk, X0, nk, e, dst, matN, matT, nbatch, cdf, dg);
+  else
+    hplanes(blk, X0, hee, hhh, hA, hB, nk, e, mxo, esc, dst);
+}
+SBE_PASS(OperandPlanesPass, 256, operand_planes);
+
 // s + e = a + b exactly (Knuth's two-sum in round-to-nearest FP32).  The peeled
 // diagonal energies enter as products with the state every stage; a rounded FP32
 // energy sum would be the same rounding every step, i.e. a frequency bias whose phase
@@ -1804,13 +1818,21 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage
   const auto tiles = [](const Mixed* m) {
     return dim3((m->nk + 31) / 32, (m->nk + 31) / 32, m->nw);
   };
-  {
+  // the state's operand planes are not needed before the commutators: with few tiles they share
+  // the Hamiltonian planes' launch (apart / together: 1 x 64 278 / 267 us a step, 1 x 256 442 /
+  // 429, 32 x 128 767 / 752, 32 x 256 2020 / 2024, 64 wires of 64 to 512 2055 / 2085, 32 x 512
+  // 7708 / 7768: the Hamiltonian pass's registers leave fewer blocks of theirs on an SM)
+  long long blocks = 0;
+  for (Mixed* m : buckets) blocks += 4LL * tiles(m).x * tiles(m).y * m->nw;
+  const bool together = blocks <= 4096;
+  const auto state_exp = [&](Mixed* m) { return ExpOf{m->mxO(in), nullptr, nullptr, nullptr}; };
+  if (!together) {
     Batch<PlanesPass> pass(tile, s);
     for (Mixed* m : buckets) {
       const int nk = m->nk, nw = m->nw;
       const long long vn = (long long)nw * nk;
       const float2 *P = xs + m->bm, *C = xs + tm + m->bm, *D = xs + 2 * tm + m->bm;
-      const ExpOf e{m->mxO(in), nullptr, nullptr, nullptr};
+      const ExpOf e = state_exp(m);
       pass.add(tiles(m), P, nk, e, m->pl, M_P, M_PT, nw, nullptr, nullptr);
       pass.add(tiles(m), C, nk, e, m->pl, M_C, -1, nw, m->cdf, m->xdg);
       pass.add(tiles(m), D, nk, e, m->pl, M_D, -1, nw, m->cdf + 2 * vn, m->xdg + vn);
@@ -1854,12 +1876,29 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage
                ekf, m->vsf, c->Ee, c->Eh, m->trf, reinterpret_cast<const float2*>(m->xsh),
                have_x, A->hf, tm, m->dgE, m->dgH, m->dgf, m->mxH(in));
   }
-  {
+  const auto ham_exp = [&](Mixed* m) { return ExpOf{m->mxH(in), m->mxAB(), nullptr, nullptr}; };
+  if (together) {
+    Batch<OperandPlanesPass> pass(tile, s);
+    for (Mixed* m : buckets) {
+      const int nk = m->nk, nw = m->nw;
+      const long long vn = (long long)nw * nk;
+      const auto state = [&](int i, int matN, int matT, float* cdf, const double* dg) {
+        pass.add(tiles(m), 0, xs + i * tm + m->bm, nullptr, nullptr, nullptr, nullptr, nk,
+                 state_exp(m), nullptr, nullptr, m->pl, matN, matT, nw, cdf, dg);
+      };
+      state(0, M_P, M_PT, nullptr, nullptr);
+      state(1, M_C, -1, m->cdf, m->xdg);
+      state(2, M_D, -1, m->cdf + 2 * vn, m->xdg + vn);
+      pass.add(tiles(m), 1, A->hf + m->bm, A->hf + tm + m->bm, A->hf + 2 * tm + m->bm,
+               A->habf + m->bm, A->habf + tm + m->bm, nk, ham_exp(m), m->mxO(in), m->esc(), m->pl,
+               0, 0, nw, nullptr, nullptr);
+    }
+  } else {
     Batch<HPlanesPass> pass(tile, s);
     for (Mixed* m : buckets)
       pass.add(tiles(m), A->hf + m->bm, A->hf + tm + m->bm, A->hf + 2 * tm + m->bm,
-               A->habf + m->bm, A->habf + tm + m->bm, m->nk,
-               ExpOf{m->mxH(in), m->mxAB(), nullptr, nullptr}, m->mxO(in), m->esc(), m->pl);
+               A->habf + m->bm, A->habf + tm + m->bm, m->nk, ham_exp(m), m->mxO(in), m->esc(),
+               m->pl);
   }
   // commutator GEMMs: dP and the cross terms of W and V, then the hi*hi products of
   // W and V (the partials of W and V meet in the anti-Hermitian pass)
