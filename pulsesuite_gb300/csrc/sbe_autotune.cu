@@ -129,13 +129,14 @@ int save(const char* path, const std::string& key, const std::string& entry) {
 }
 
 // mean time (ms) of reps launches of the job list, after one untimed launch
-int time_jobs(const std::vector<tc::GemmJob>& jobs, cudaStream_t s, int reps, double* ms) {
+int time_jobs(const std::vector<tc::GemmJob>& jobs, int* sched, cudaStream_t s, int reps,
+              double* ms) {
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
-  int rc = launch_jobs(jobs, s);
+  int rc = launch_jobs(jobs, sched, s);
   cudaEventRecord(a, s);
-  for (int i = 0; !rc && i < reps; ++i) rc = launch_jobs(jobs, s);
+  for (int i = 0; !rc && i < reps; ++i) rc = launch_jobs(jobs, sched, s);
   cudaEventRecord(b, s);
   if (!rc) rc = cuda_check(cudaEventSynchronize(b), "sbe_autotune: timing");
   float t = 0.f;
@@ -180,7 +181,7 @@ extern "C" int sbe_autotune(SbeCtx* c, const char* cache_json) {
         m->bn[kind] = kTiles[t];
         std::vector<tc::GemmJob> jobs;
         bucket_jobs(c, m, kind, jobs);
-        rc = time_jobs(jobs, s, 5, &ms[k][t]);
+        rc = time_jobs(jobs, A->sched, s, 5, &ms[k][t]);
       }
       m->bn[kind] = ms[k][1] < ms[k][0] ? 128 : 256;
     }

@@ -68,7 +68,8 @@ struct MixedAll {
   float2* ekf = nullptr;     // 3 x (3 x tot_r) fields at the step's start, middle and end
   float2* ekrf = nullptr;    // tot_kr Expikr
   int* err = nullptr;        // engine error flag (bounded waits that gave up)
-  unsigned* mx = nullptr;    // the buckets' maxima
+  unsigned* mx = nullptr;    // the buckets' maxima, and behind them the engine's counters
+  int* sched = nullptr;      // tile and exit counters of the engine's launches (2)
 };
 
 // matrix slots of the commutator plane sets
@@ -89,6 +90,6 @@ enum JobKind { JK_EXCH = 0, JK_FULL = 1, JK_HH = 2, JK_SRC = 3 };
 void bucket_jobs(SbeCtx* c, Mixed* m, int kind, std::vector<tc::GemmJob>& out);
 // Launch a job list: consecutive jobs of one N tile share a persistent launch
 // (tc::MAX_JOBS per launch).
-int launch_jobs(const std::vector<tc::GemmJob>& jobs, cudaStream_t s);
+int launch_jobs(const std::vector<tc::GemmJob>& jobs, int* sched, cudaStream_t s);
 
 }  // namespace sbe

@@ -435,7 +435,8 @@ static void carve_all(MixedAll* A, Carver& k, const SbeCtx* c) {
   A->ekf = k.take<float2>(9 * (size_t)c->tot_r);
   A->ekrf = k.take<float2>((size_t)c->tot_kr);
   A->err = k.take<int>(1);
-  A->mx = k.take<unsigned>(kMaxima * (size_t)c->nw);
+  A->mx = k.take<unsigned>(kMaxima * (size_t)c->nw + 2);
+  A->sched = A->mx ? reinterpret_cast<int*>(A->mx + kMaxima * (size_t)c->nw) : nullptr;
 }
 
 static int mixed_ensure(SbeCtx* c, cudaStream_t s) {
@@ -1602,11 +1603,11 @@ static tc::GemmJob job(Mixed* m, const tc::PlaneSet& A, const tc::PlaneSet& B, i
 // Launch a job list (built bucket by bucket, largest Nk first, so that the longest
 // tiles start first): consecutive jobs of one N tile share a persistent launch,
 // tc::MAX_JOBS per launch.
-int launch_jobs(const std::vector<tc::GemmJob>& jobs, cudaStream_t s) {
+int launch_jobs(const std::vector<tc::GemmJob>& jobs, int* sched, cudaStream_t s) {
   for (size_t i = 0; i < jobs.size();) {
     size_t j = i + 1;
     while (j < jobs.size() && j - i < (size_t)tc::MAX_JOBS && jobs[j].d.bn == jobs[i].d.bn) ++j;
-    const int rc = tc_gemm_launch(jobs.data() + i, (int)(j - i), s);
+    const int rc = tc_gemm_launch(jobs.data() + i, (int)(j - i), sched, s);
     if (rc) return rc;
     i = j;
   }
@@ -1708,8 +1709,9 @@ static std::vector<Mixed*> by_size(const MixedAll* A) { return {A->b.rbegin(), A
 // dephasing matrices with the FP32 Lorentzian sums) and its FP32 tables.
 static int mixed_prep(SbeCtx* c, const double2* C, const double2* D, cudaStream_t s) {
   MixedAll* A = all_of(c);
-  // the maxima that this step's passes collect
-  cudaMemsetAsync(A->mx, 0, sizeof(unsigned) * kMaxima * c->nw, s);
+  // the maxima that this step's passes collect, and the engine's counters: a count that some
+  // launch should leave behind does not outlast the step
+  cudaMemsetAsync(A->mx, 0, sizeof(unsigned) * (kMaxima * (size_t)c->nw + 2), s);
   launch_prep_scalar(c, C, D, s);   // occupations, screening (FP64, O(Nk) per wire)
   const std::vector<Mixed*> buckets = by_size(A);
   {
@@ -1865,7 +1867,7 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage
   if (have_x) {
     // the three exchange products (eh, ee, hh) of every bucket
     ProfScope ps(c, 1, s);
-    rc = launch_jobs(all_jobs(c, JK_EXCH), s);
+    rc = launch_jobs(all_jobs(c, JK_EXCH), A->sched, s);
     if (rc) return rc;
   }
   // the Hamiltonians: Meh + diagonal + direct + exchange, diagonal peeled; their planes
@@ -1904,12 +1906,12 @@ static int mixed_stage(SbeCtx* c, const float2* xs, const float2* ekf, int stage
   // W and V (the partials of W and V meet in the anti-Hermitian pass)
   {
     ProfScope ps(c, 0, s);
-    rc = launch_jobs(all_jobs(c, JK_FULL), s);
+    rc = launch_jobs(all_jobs(c, JK_FULL), A->sched, s);
     if (rc) return rc;
   }
   {
     ProfScope ps(c, 0, s);
-    rc = launch_jobs(all_jobs(c, JK_HH), s);
+    rc = launch_jobs(all_jobs(c, JK_HH), A->sched, s);
     if (rc) return rc;
   }
   float2* wf = reinterpret_cast<float2*>(c->G);
@@ -1969,7 +1971,7 @@ static int mixed_sources(SbeCtx* c, const double2* P, const double2* C, const do
   float2* gf = reinterpret_cast<float2*>(c->G);
   {
     ProfScope ps(c, 2, s);
-    const int rc = launch_jobs(all_jobs(c, JK_SRC), s);
+    const int rc = launch_jobs(all_jobs(c, JK_SRC), A->sched, s);
     if (rc) return rc;
   }
   {
@@ -2117,7 +2119,7 @@ extern "C" int sbe_tc_selftest(int nk, int nbatch, const double* A, const double
   unsigned* mx = nullptr;
   const size_t pbytes = tc::planeset_bytes(ps);
   if (cudaMallocAsync(&ps.ptr, pbytes, s) != cudaSuccess ||
-      cudaMallocAsync(&ints, sizeof(int) * (3 * nbatch + 1), s) != cudaSuccess ||
+      cudaMallocAsync(&ints, sizeof(int) * (3 * nbatch + 3), s) != cudaSuccess ||
       cudaMallocAsync(&mx, sizeof(unsigned) * nbatch, s) != cudaSuccess)
     return fail(SBE_ERR_OOM, "sbe_tc_selftest: scratch");
   cudaMemsetAsync(ps.ptr, 0, pbytes, s);
@@ -2125,7 +2127,7 @@ extern "C" int sbe_tc_selftest(int nk, int nbatch, const double* A, const double
   int* eB = ints + nbatch;
   int* es = ints + 2 * nbatch;
   int* err = ints + 3 * nbatch;
-  cudaMemsetAsync(err, 0, sizeof(int), s);
+  cudaMemsetAsync(err, 0, sizeof(int) * 3, s);   // and the counters behind it
   const double2* a2 = (const double2*)A;
   const double2* b2 = (const double2*)B;
   launch_exponents(a2, mm, mm, nbatch, mx, eA, nullptr, nullptr, s);
@@ -2150,7 +2152,7 @@ extern "C" int sbe_tc_selftest(int nk, int nbatch, const double* A, const double
   e.out_bstride = mm;
   e.escale = es;
   e.err = err;
-  rc = tc_gemm_launch(d, e, s);
+  rc = tc_gemm_launch(d, e, err + 1, s);
   if (rc) return rc;
   int herr = 0;
   cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s);

@@ -326,9 +326,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       }
       }
     }
-    // the last CTA to have drawn its last tile leaves the slot zeroed for its next launch (a
-    // memset ahead of the launch costs a launch of its own and the overlap with the kernel
-    // before)
+    // the last CTA to have drawn its last tile leaves the counters zeroed for the next launch (a
+    // memset ahead of each launch costs a launch of its own and the overlap with the kernel
+    // before; a context's counters are also cleared once a step)
     if (atomicAdd(L.sched + 1, 1) == (int)gridDim.x - 1) {
       L.sched[0] = 0;
       L.sched[1] = 0;
@@ -570,25 +570,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
 static const int kTcSmem = 1024 + tc::STAGE_AREA + tc::SCR_BYTES + 512;
 
-// per-launch tile and exit counters of the dynamic scheduler (cycled; a launch leaves its
-// pair zeroed)
-static int* g_sched = nullptr;
-static unsigned g_sched_seq = 0;
-constexpr int kSchedSlots = 1024;
-
 int tc_gemm_init() {
   static bool attr = false;
-  if (!g_sched) {
-    int* p = nullptr;
-    if (cudaMalloc(&p, sizeof(int) * 2 * kSchedSlots) != cudaSuccess)
-      return fail(SBE_ERR_OOM, "tc_gemm: scheduler counters");
-    if (cudaMemset(p, 0, sizeof(int) * 2 * kSchedSlots) != cudaSuccess ||
-        cudaStreamSynchronize(0) != cudaSuccess) {
-      cudaFree(p);
-      return cuda_check(cudaGetLastError(), "tc_gemm: scheduler counters");
-    }
-    g_sched = p;
-  }
   if (!attr) {
     using Kernel = void (*)(const tc::GemmLaunch);
     const Kernel kernels[] = {
@@ -712,7 +695,7 @@ static bool splits_parts(const tc::GemmJob* jobs, int njobs, int bnt) {
   return terms > 1 && 2 * tiles <= num_sms();
 }
 
-int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
+int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, int* sched, cudaStream_t s) {
   int rc = tc_gemm_init();
   if (rc) return rc;
   if (njobs < 1 || njobs > tc::MAX_JOBS)
@@ -750,7 +733,7 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s) {
   }
   L.tile_base[njobs] = nt;
   if (nt == 0) return SBE_OK;
-  L.sched = g_sched + 2 * (g_sched_seq++ % kSchedSlots);
+  L.sched = sched;
   const int grid = (int)std::min<long long>(nt, num_sms());
   void (*const kernel)(const tc::GemmLaunch) =
       mode == tc::MODE_HH ? (bnt == 64 ? tc::k_tc_gemm<64, tc::MODE_HH>
@@ -785,9 +768,9 @@ int tc_wait_selftest(int* err, int* gave_up, cudaStream_t s) {
   return cuda_check(cudaGetLastError(), "tc_wait_selftest launch");
 }
 
-int tc_gemm_launch(const tc::GemmDesc& d, const tc::EpiArgs& e, cudaStream_t s) {
+int tc_gemm_launch(const tc::GemmDesc& d, const tc::EpiArgs& e, int* sched, cudaStream_t s) {
   tc::GemmJob j{d, e};
-  return tc_gemm_launch(&j, 1, s);
+  return tc_gemm_launch(&j, 1, sched, s);
 }
 
 }  // namespace sbe

@@ -164,15 +164,17 @@ struct GemmLaunch {
   long long tile_base[MAX_JOBS + 1];
   int njobs;
   int csplit;                 // 1: two tiles per complex output tile, real and imaginary part
-  int* sched;                 // tile and exit counters of this launch (zero; left zero)
+  int* sched;                 // tile and exit counters of the launch (its caller's; zero, left zero)
 };
 static_assert(sizeof(GemmLaunch) <= 32000, "kernel parameter space (32 KB) exceeded");
 
 }  // namespace tc
 
 // Host API of the engine.
-int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, cudaStream_t s);
-int tc_gemm_launch(const tc::GemmDesc& d, const tc::EpiArgs& e, cudaStream_t s);
+// sched: two zeroed ints, owned by the caller and used by launches of one stream order only (a
+// launch leaves them zero)
+int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, int* sched, cudaStream_t s);
+int tc_gemm_launch(const tc::GemmDesc& d, const tc::EpiArgs& e, int* sched, cudaStream_t s);
 // One launch whose bounded wait gives up (~2 s): raises *err, *gave_up = 1.
 int tc_wait_selftest(int* err, int* gave_up, cudaStream_t s);
 int tc_gemm_init();
