@@ -289,7 +289,7 @@ class SBESolver:
         Ek3 = Ek[:3]                                      # the first three rows, contiguous
         ctx.leapfrog_step(self._st[w - 1], Ek3, dt, src)
         ctx.qw2prop(0, RR, src, self.LF, self._dout[0])
-        out = self._fetch(1)[0]
+        out = self._fetch(ctx)[0]
         if self.write_info:
             self._write_info(ctx, w, dt, src, Ek3)
             self._write_maxoffdiag(ctx, 0)
@@ -313,9 +313,15 @@ class SBESolver:
         if self._hin is None or self._hin.shape[2] != n:
             self._hin = torch.empty((nslot, 5, n), dtype=CDTYPE).pin_memory()
             self._din = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
-            self._dout = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
-            self._hout = torch.empty((nslot, 5, n), dtype=CDTYPE).pin_memory()
-            self._hin_np, self._hout_np = self._hin.numpy(), self._hout.numpy()
+            # the resampled sources, and behind them the flag of the products' bounded waits
+            m = nslot * 5 * n
+            self._dres = torch.empty(m + 1, dtype=CDTYPE, device="cuda")
+            self._hres = torch.empty(m + 1, dtype=CDTYPE).pin_memory()
+            self._dout = self._dres[:m].view(nslot, 5, n)
+            self._dflag = torch.view_as_real(self._dres[m:]).view(-1)[:1].view(torch.int32)[:1]
+            self._hin_np, self._hres_np = self._hin.numpy(), self._hres.numpy()
+            self._hout_np = self._hres_np[:m].reshape(nslot, 5, n)
+            self._hflag_np = self._hres_np[m:].view(np.int32)
         elif self._busy:
             torch.cuda.current_stream().synchronize()     # an aborted step's transfers
         h = self._hin_np[w - 1]
@@ -327,11 +333,15 @@ class SBESolver:
         self._busy = not self.batch or w == self.Nw
         return torch.view_as_real(d[4]).reshape(-1)[:n], d[:4]
 
-    def _fetch(self, nslot):
-        """The first nslot blocks of the resampled sources on the host (waits for them)."""
-        self._hout[:nslot].copy_(self._dout[:nslot], non_blocking=True)
+    def _fetch(self, ctx):
+        """The resampled sources of the step of ctx on the host (waits for them); raises if a
+        bounded wait of that step gave up."""
+        ctx.table(0, "wait_flag", self._dflag)
+        self._hres.copy_(self._dres, non_blocking=True)
         torch.cuda.current_stream().synchronize()
         self._busy = False
+        if self._hflag_np[0]:
+            ctx.check()
         return self._hout_np
 
     def _batched(self, w, RR, f4, dt, outs, E3):
@@ -349,7 +359,7 @@ class SBESolver:
         live = [wi for wi in range(self.Nw) if self._outs[wi] is not None]
         for wi in live:
             ctx.qw2prop(wi, RR, ctx.rvec(self._src, wi, 5), self.LF, self._dout[wi])
-        host = self._fetch(self.Nw)
+        host = self._fetch(ctx)
         for wi in live:
             o, out = self._outs[wi], host[wi]
             if self.write_info:

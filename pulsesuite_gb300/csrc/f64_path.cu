@@ -409,7 +409,7 @@ static f64s::Job form_job(const FormSet& F, const TermDef& t, const int* alias) 
 
 // the jobs of outputs [o0, o1) into part
 static int form_products(const FormSet& F, int o0, int o1, const int* alias, int parts, double* part,
-                         cudaStream_t s) {
+                         int* err, cudaStream_t s) {
   std::vector<f64s::Job> jobs;
   const long long cs = (long long)F.nw * F.nk * F.nk;
   for (int o = o0; o < o1; ++o)
@@ -422,12 +422,13 @@ static int form_products(const FormSet& F, int o0, int o1, const int* alias, int
       j.o_batch = (long long)F.nk * F.nk;
       jobs.push_back(j);
     }
-  return launch_f64_gemm(jobs.data(), (int)jobs.size(), s);
+  return launch_f64_gemm(jobs.data(), (int)jobs.size(), err, s);
 }
 
 static int exchange(int nk, int nw, const double2* P, const double2* C, const double2* D,
                     const __half* tp, long long tp_plane, const int* et, long long et_n, __half* sp,
-                    int* es, long long sl_m, long long sl_s, double* xsh, cudaStream_t s) {
+                    int* es, long long sl_m, long long sl_s, double* xsh, int* err,
+                    cudaStream_t s) {
   const int nb = k_blocks(nk);
   int ny = 0;   // dd blocks of the band per t' block
   for (int i = 0; i < nb; ++i) {
@@ -461,7 +462,7 @@ static int exchange(int nk, int nw, const double2* P, const double2* C, const do
     j.o_batch = 2ll * nk * nk;
     j.ldo = 2 * nk;
   }
-  return launch_f64_gemm(jobs, 3, s);
+  return launch_f64_gemm(jobs, 3, err, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -631,7 +632,7 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       if (exc)
         rc = exchange(nk, g, P + o, C + o, D + o, m.tp + w0 * m.sl_m, (long long)m.nw * m.sl_m,
                       m.et + (long long)w0 * nk, (long long)m.nw * nk, m.sp, m.es, m.sl_m, m.sl_s,
-                      m.xsh, s);
+                      m.xsh, c->f64_err, s);
       if (rc) return rc;
       HBuild h{};
       h.nk = nk;
@@ -667,7 +668,7 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
         alias[F_HHX] = F_HH;
       }
       launch_f64_slice(a, nf, s);
-      rc = form_products(F, 0, 3, alias, m.parts, m.part, s);
+      rc = form_products(F, 0, 3, alias, m.parts, m.part, c->f64_err, s);
       if (rc) return rc;
       Finish f{};
       f.nk = nk;
@@ -794,7 +795,7 @@ int f64_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D,
         j.ldo = nr;
       }
       launch_f64_slice(a, 3, s);
-      const int rc = launch_f64_gemm(jobs, 3, s);
+      const int rc = launch_f64_gemm(jobs, 3, c->f64_err, s);
       if (rc) return rc;
       launch(k_f64_src_reduce, dim3((nr + 15) / 16, g), dim3(16, 32), 0, s, m.dw + w0, nk, nr, g,
              m.sparts, c->expikr + ko, m.part, c->window + ro, src + 5 * ro);
@@ -832,7 +833,8 @@ static cudaMemPool_t scratch_pool() {
   return p;
 }
 
-// One block of stream-ordered scratch; null when there is no room or the stream is being
+// One block of stream-ordered scratch (a word of it takes the products' error flag: the calls have
+// no context that could report it, their outputs are NaN then); null when there is no room or the stream is being
 // captured (the callers then take the SIMT kernels).
 struct Scratch {
   char* p = nullptr;
@@ -896,7 +898,7 @@ bool f64_rhs_single(int which, int nk, const double2* C, const double2* D, const
   a.src_batch = mm;
   a.plane = a.dst_batch = sl;
   launch_f64_slice(a, nf, s);
-  *rc = form_products(F, which, which + 1, alias, parts, part, s);
+  *rc = form_products(F, which, which + 1, alias, parts, part, w.take<int>(1), s);
   if (*rc) return true;
   Finish f{};
   f.nk = nk;
@@ -933,7 +935,7 @@ bool f64_calch_single(int nk, const double2* Meh, const double2* Wee, const doub
   cudaMemsetAsync(sp, 0, sizeof(__half) * 3 * NS * ss, s);
   launch(k_f64_diag, dim3((2 * nk - 1 + 3) / 4, 3, 1), 128, 0, s, nk, P, C, D, tr, es);
   launch(k_f64_toeplitz, dim3((nk + 7) / 8, 3, 1), 256, 0, s, nk, 1, vq, tp, et, sl);
-  *rc = exchange(nk, 1, P, C, D, tp, sl, et, nk, sp, es, sl, ss, xsh, s);
+  *rc = exchange(nk, 1, P, C, D, tp, sl, et, nk, sp, es, sl, ss, xsh, w.take<int>(1), s);
   if (*rc) return true;
   HBuild h{};
   h.nk = nk;

@@ -9,8 +9,6 @@
 namespace sbe {
 namespace f64s {
 
-__device__ int g_err;   // a bounded wait gave up
-
 // ---------------------------------------------------------------------------
 // slicing
 
@@ -295,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
   const int nunits = L.base[L.njobs];
-  int* err = &g_err;
+  int* err = L.err;
   if (threadIdx.x == 0) {
     for (int i = 0; i < NA; ++i) {
       mbar_init(&fullA[i], 1);
@@ -327,7 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
     uint32_t pa = 0, pb = 0;   // phases of the ring positions
     long long na = 0, nb = 0;
     bool ok = true;
-    for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
+    for (int u = blockIdx.x; ok && !L.stall && u < nunits; u += gridDim.x) {
       const Unit t = unit_of(L, u);
       if (t.dead) continue;
       const Job& d = L.job[t.job];
@@ -453,8 +451,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const uint32_t ta = tmem + ((uint32_t)(32 * quarter) << 16) + half * 32;
     uint32_t pt = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; ok && u < nunits; u += gridDim.x) {
+    bool ok = true;   // after a wait that gave up the tiles left become NaN
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
       const Unit t = unit_of(L, u);
       if (t.dead) continue;
       const Job& d = L.job[t.job];
@@ -462,7 +460,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
 #pragma unroll
       for (int j = 0; j < 32; ++j) run[j] = 0;
       unsigned long long bias = 0;
-      for (int c0 = t.q0; c0 < t.q1; c0 += CHUNK) {
+      for (int c0 = t.q0; ok && c0 < t.q1; c0 += CHUNK) {
         uint32_t a[16], b[16];
         if (!mbar_wait(&tfull[1], pt, err, abort_flag)) {
           ok = false;
@@ -513,8 +511,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_f64_gemm(const __grid_constant__
         bias += kBias;
       }
       const int m = t.m0 + 32 * quarter + lane;
-      if (!ok || m >= d.M) continue;
-      const int ea = d.ea[(long long)t.b * d.M + m];
+      if (m >= d.M) continue;
+      const int ea = ok ? d.ea[(long long)t.b * d.M + m] : kBadExp;
       const int* eb = d.eb + (long long)t.b * d.N;
       double* o = d.out + t.part * d.o_part + t.comp * d.o_comp + (long long)t.b * d.o_batch;
       const int n0 = t.n0 + 32 * half;
@@ -590,13 +588,15 @@ static int sm_count() {
   return n;
 }
 
-int launch_f64_gemm(const f64s::Job* jobs, int njobs, cudaStream_t s) {
+int launch_f64_gemm(const f64s::Job* jobs, int njobs, int* err, cudaStream_t s, bool stall) {
   if (njobs < 1 || njobs > f64s::MAX_JOBS) return fail(SBE_ERR_ARG, "f64 gemm: 1 to 16 jobs");
   static const cudaError_t attr = cudaFuncSetAttribute(
       f64s::k_f64_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, f64s::SMEM);
   if (attr != cudaSuccess) return fail(SBE_ERR_CUDA, "f64 gemm: cannot raise the shared-memory limit");
   f64s::Launch L{};
   L.njobs = njobs;
+  L.err = err;
+  L.stall = stall;
   long long nt = 0;
   for (int j = 0; j < njobs; ++j) {
     const f64s::Job& d = jobs[j];
@@ -615,13 +615,21 @@ int launch_f64_gemm(const f64s::Job* jobs, int njobs, cudaStream_t s) {
   return cuda_check(cudaGetLastError(), "f64 gemm launch");
 }
 
-int f64_gemm_error(int* flag) {
-  *flag = 0;
-  int rc = cuda_check(cudaMemcpyFromSymbol(flag, f64s::g_err, sizeof(int)), "f64 gemm: read flag");
-  if (!rc && *flag) {
-    const int z = 0;
-    rc = cuda_check(cudaMemcpyToSymbol(f64s::g_err, &z, sizeof(int)), "f64 gemm: clear flag");
-  }
+int f64_wait_selftest(double* out, int* err, cudaStream_t s) {
+  int* e = nullptr;   // row exponents, and the operands that nothing reads
+  if (cudaMallocAsync(&e, 256, s) != cudaSuccess)
+    return fail(SBE_ERR_OOM, "sbe_f64_wait_selftest: scratch allocation failed");
+  cudaMemsetAsync(e, 0, 256, s);
+  f64s::Job j{};
+  j.A = j.B = reinterpret_cast<const __half*>(e);
+  j.a_pad = j.b_pad = 128;
+  j.ea = j.eb = e;
+  j.M = j.N = j.ldo = 64;
+  j.nkb = 2;
+  j.batch = j.parts = 1;
+  j.out = out;
+  const int rc = launch_f64_gemm(&j, 1, err, s, true);
+  cudaFreeAsync(e, s);
   return rc;
 }
 

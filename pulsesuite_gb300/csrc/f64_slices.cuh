@@ -55,6 +55,8 @@ struct Launch {
   Job job[MAX_JOBS];
   int base[MAX_JOBS + 1];
   int njobs;
+  int stall;                        // self-test: no operand arrives, every wait runs out
+  int* err;                         // raised by a wait that gave up
 };
 
 // One operand form of the slicing pass: row r, column k is src[r ld + k], or src[k ld + r]
@@ -154,9 +156,8 @@ __device__ __forceinline__ long long chunk_off(int rows_pad, int r, int kb, int 
 
 // exponents and digit planes of every form's rows
 void launch_f64_slice(const f64s::SliceArgs& a, int nforms, cudaStream_t s);
-// one persistent launch over the jobs' output tiles
-int launch_f64_gemm(const f64s::Job* jobs, int njobs, cudaStream_t s);
-// error flag of the engine's bounded waits: read and cleared (waits for the device)
-int f64_gemm_error(int* flag);
+// One persistent launch over the jobs' output tiles.  A bounded wait that gives up raises *err and
+// leaves NaN in the tiles that its CTA has not finished, so that no call returns stale values.
+int launch_f64_gemm(const f64s::Job* jobs, int njobs, int* err, cudaStream_t s, bool stall = false);
 
 }  // namespace sbe

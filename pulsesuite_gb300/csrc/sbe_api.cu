@@ -222,6 +222,7 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   add((void**)&c->dconst, 4 * 16 * (size_t)n_wires);
   add((void**)&c->dpre, 4 * 4 * ov);
   add((void**)&c->dwl, sizeof(int) * (size_t)n_wires);
+  add((void**)&c->f64_err, sizeof(int));
   size_t total = 0;
   for (auto& p : parts) total += (p.bytes + 255) / 256 * 256;
   if (cudaMalloc(&c->arena, total) != cudaSuccess) {
@@ -344,6 +345,7 @@ int sbe_ctx_table(const SbeCtx* c, int w, int which, void* dst, long long nbytes
                         "sbe_ctx_table");
     }
     case 14: src = c->wk + W.off_r; need = 16 * nr; break;
+    case 15: src = c->f64_err; need = 4; break;
     default: return fail(SBE_ERR_ARG, "sbe_ctx_table: unknown table");
   }
   if (nbytes < need) return fail(SBE_ERR_ARG, "sbe_ctx_table: destination too small");

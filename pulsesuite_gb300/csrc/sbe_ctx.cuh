@@ -72,6 +72,7 @@ struct SbeCtx {
   void* mixed = nullptr;                 // mixed-precision workspace (sbe_tc.cu)
   void* f64 = nullptr;                   // FP64 digit-plane workspace (f64_path.cu)
   int f64_off = 0;                       // no room for it: the FP64 path stays on SIMT
+  int* f64_err = nullptr;                // a wait of the FP64 products gave up
 
   // kernel timing (sbe_ctx_profile): event pairs per category, and a pool
   int prof = 0;
@@ -176,7 +177,7 @@ bool f64_calch_single(int nk, const double2* Meh, const double2* Wee, const doub
                       const double* Ee, const double* Eh, double gap, int excitons, int lf,
                       int freepot, double2* Heh, double2* Hee, double2* Hhh, cudaStream_t s, int* rc);
 void launch_vq_from_vc(int nk, const double* VC, double* vq, cudaStream_t s);
-int f64_gemm_error(int* flag);
+int f64_wait_selftest(double* out, int* err, cudaStream_t s);
 // sbe_step.cu
 void launch_leapfrog(SbeCtx* c, double2* const* st9, const double2* Ek, double dt,
                      cudaStream_t s);

@@ -2066,11 +2066,14 @@ extern "C" int sbe_ctx_check(SbeCtx* c, void* stream) {
   int rc = cuda_check(cudaStreamSynchronize(as_stream(stream)), "sbe_ctx_check");
   if (rc) return rc;
   int f = 0;
-  rc = f64_gemm_error(&f);
+  rc = cuda_check(cudaMemcpy(&f, c->f64_err, sizeof(int), cudaMemcpyDeviceToHost),
+                  "sbe_ctx_check: read FP64 flag");
   if (rc) return rc;
-  if (f)
+  if (f) {
+    cudaMemset(c->f64_err, 0, sizeof(int));
     return fail(SBE_ERR_TIMEOUT, "a pipeline wait of the FP64 products timed out (results of the "
                                  "affected calls are invalid)");
+  }
   MixedAll* A = all_of(c);
   if (!A) return SBE_OK;
   int h = 0;
@@ -2104,6 +2107,11 @@ extern "C" int sbe_wait_selftest(SbeCtx* c, int* gave_up, void* stream) {
   if (!rc) rc = cuda_check(cudaStreamSynchronize(s), "sbe_wait_selftest");
   *gave_up = h;
   return rc;
+}
+
+extern "C" int sbe_f64_wait_selftest(SbeCtx* c, double* out, void* stream) {
+  if (!c || !out) return fail(SBE_ERR_ARG, "sbe_f64_wait_selftest: null argument");
+  return f64_wait_selftest(out, c->f64_err, as_stream(stream));
 }
 
 extern "C" int sbe_tc_selftest(int nk, int nbatch, const double* A, const double* B, int opA,

@@ -96,7 +96,7 @@ class RK4Graph:
 
 
 TABLES = dict(kr=0, r=1, Ee=2, Eh=3, V0=4, Chi1D=5, qeqh=6, EP=7, HP=8, window=9, maps=10,
-              xexh=11, Expikr=12, scalars=13, window_k=14)
+              xexh=11, Expikr=12, scalars=13, window_k=14, wait_flag=15)
 
 
 class WireContext:
@@ -174,18 +174,22 @@ class WireContext:
         return out
 
     # ---- tables ------------------------------------------------------------
-    def table(self, w, name):
+    def table(self, w, name, out=None):
         which = TABLES[name]
         nk = self.nk[w]
         nr = 2 * nk + 2
         shapes = {0: (nk,), 1: (nr,), 2: (nk,), 3: (nk,), 4: (3, nk), 5: (2, nk), 6: (2, nk),
                   7: (nk, nk), 8: (nk, nk), 9: (nr,), 11: (2, nk), 13: (16,)}
-        if which == 10:
+        if out is not None:
+            t = out
+        elif which == 10:
             t = torch.empty((6, nk, nk), dtype=torch.int32, device=self.device)
         elif which == 12:
             t = torch.empty((nk, nr), dtype=CDTYPE, device=self.device)
         elif which == 14:
             t = torch.empty((nr,), dtype=CDTYPE, device=self.device)
+        elif which == 15:
+            t = torch.empty((1,), dtype=torch.int32, device=self.device)
         else:
             t = torch.empty(shapes[which], dtype=torch.float64, device=self.device)
         _lib.check(self.lib.sbe_ctx_table(self.handle, w, which, _lib.ptr(t),
@@ -373,6 +377,14 @@ class WireContext:
         _lib.check(self.lib.sbe_wait_selftest(self.handle, ctypes.byref(g), _lib.stream_handle()),
                    "sbe_wait_selftest")
         return g.value == 1
+
+    def f64_wait_selftest(self):
+        """The same with a wait of the FP64 products: the (64, 64) tile that it could not
+        form, all NaN.  The next check() then raises; the context stays usable."""
+        out = torch.zeros((64, 64), dtype=torch.float64, device=self.device)
+        _lib.check(self.lib.sbe_f64_wait_selftest(self.handle, _lib.ptr(out),
+                                                  _lib.stream_handle()), "sbe_f64_wait_selftest")
+        return out
 
     def charge(self):
         """(n_wires, 2) carrier numbers sum |C_kk|, sum |D_kk| that the charge
