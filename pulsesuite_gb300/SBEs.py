@@ -226,7 +226,6 @@ class SBESolver:
         # pinned staging of the grid fields and of the resampled sources, for the last
         # grid size seen
         self._hin = None
-        self._busy = False
         if self.OffDiagDph and self.write_info:
             # InitializeDephasing opens (truncates) both files (dephasing.py:537-539)
             os.makedirs("dataQW/Wire/info", exist_ok=True)
@@ -307,8 +306,8 @@ class SBESolver:
 
     def _stage(self, w, rr, fields):
         """Copy a wire's grid and its four fields into pinned host memory and from there, in
-        one transfer on the current stream, to the device: (RR, f4).  The step that reads
-        them is waited for (_fetch) before the buffers are filled again."""
+        one transfer on the current stream, to the device: (RR, f4).  Each wire's transfer is
+        waited for before its host memory is filled again."""
         n, nslot = len(rr), self.Nw if self.batch else 1
         if self._hin is None or self._hin.shape[2] != n:
             self._hin = torch.empty((nslot, 5, n), dtype=CDTYPE).pin_memory()
@@ -319,18 +318,20 @@ class SBESolver:
             self._hres = torch.empty(m + 1, dtype=CDTYPE).pin_memory()
             self._dout = self._dres[:m].view(nslot, 5, n)
             self._dflag = torch.view_as_real(self._dres[m:]).view(-1)[:1].view(torch.int32)[:1]
+            self._sent = [None] * nslot         # events after the transfers
             self._hin_np, self._hres_np = self._hin.numpy(), self._hres.numpy()
             self._hout_np = self._hres_np[:m].reshape(nslot, 5, n)
             self._hflag_np = self._hres_np[m:].view(np.int32)
-        elif self._busy:
-            torch.cuda.current_stream().synchronize()     # an aborted step's transfers
+        if self._sent[w - 1] is not None:
+            self._sent[w - 1].synchronize()
         h = self._hin_np[w - 1]
         for i, f in enumerate(fields):
             h[i] = f
         h[4].view(np.float64)[:n] = rr
         d = self._din[w - 1]
         d.copy_(self._hin[w - 1], non_blocking=True)
-        self._busy = not self.batch or w == self.Nw
+        self._sent[w - 1] = self._sent[w - 1] or torch.cuda.Event()
+        self._sent[w - 1].record()
         return torch.view_as_real(d[4]).reshape(-1)[:n], d[:4]
 
     def _fetch(self, ctx):
@@ -339,7 +340,6 @@ class SBESolver:
         ctx.table(0, "wait_flag", self._dflag)
         self._hres.copy_(self._dres, non_blocking=True)
         torch.cuda.current_stream().synchronize()
-        self._busy = False
         if self._hflag_np[0]:
             ctx.check()
         return self._hout_np
