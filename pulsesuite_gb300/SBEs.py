@@ -140,6 +140,15 @@ def QWChi1(lam, dky, Ee, Eh, area, geh, dcv):
 _LEVELS = ("YY1", "YY2", "YY3", "CC1", "CC2", "CC3", "DD1", "DD2", "DD3")
 
 
+def _pinned(shape):
+    """Host memory for asynchronous transfers; pageable, whose copies wait, where pinning is refused."""
+    t = torch.empty(shape, dtype=CDTYPE)
+    try:
+        return t.pin_memory()
+    except RuntimeError:
+        return t
+
+
 class SBESolver:
     """SBEs.py:4619 SBESolver on the GPU.
 
@@ -310,12 +319,12 @@ class SBESolver:
         waited for before its host memory is filled again."""
         n, nslot = len(rr), self.Nw if self.batch else 1
         if self._hin is None or self._hin.shape[2] != n:
-            self._hin = torch.empty((nslot, 5, n), dtype=CDTYPE).pin_memory()
+            self._hin = _pinned((nslot, 5, n))
             self._din = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
             # the resampled sources, and behind them the flag of the products' bounded waits
             m = nslot * 5 * n
             self._dres = torch.empty(m + 1, dtype=CDTYPE, device="cuda")
-            self._hres = torch.empty(m + 1, dtype=CDTYPE).pin_memory()
+            self._hres = _pinned((m + 1,))
             self._dout = self._dres[:m].view(nslot, 5, n)
             self._dflag = torch.view_as_real(self._dres[m:]).view(-1)[:1].view(torch.int32)[:1]
             self._sent = [None] * nslot         # events after the transfers

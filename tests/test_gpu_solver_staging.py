@@ -55,3 +55,18 @@ def test_wire_staged_again_before_the_last_one():
     ref = torch.as_tensor(np.stack(first))
     for g in got:
         assert torch.equal(g.cpu(), ref)
+
+
+def test_pinned_memory_refused(monkeypatch):
+    """Without pinned memory the solver copies from pageable memory, with the same results."""
+    sv, rr = _solver(300)
+    f = _fields(rr, 2e7)
+    ref = [x.copy() for x in _call(sv, rr, f)]
+
+    def refuse(self, *a, **k):
+        raise RuntimeError("CUDA error: out of memory")
+    sv, rr = _solver(300)
+    monkeypatch.setattr(torch.Tensor, "pin_memory", refuse)
+    for a, b in zip(_call(sv, rr, f), ref):
+        assert np.array_equal(a, b)
+
