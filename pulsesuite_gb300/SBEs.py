@@ -317,7 +317,11 @@ class SBESolver:
         """Copy a wire's grid and its four fields into pinned host memory and from there, in
         one transfer on the current stream, to the device: (RR, f4).  Each wire's transfer is
         waited for before its host memory is filled again."""
-        n, nslot = len(rr), self.Nw if self.batch else 1
+        x = np.asarray(rr, dtype=np.float64).reshape(-1)
+        fields = [np.asarray(f, dtype=complex) for f in fields]
+        n, nslot = x.size, self.Nw if self.batch else 1
+        if any(f.shape != fields[0].shape for f in fields) or fields[0].size != n:
+            raise ValueError("QWCalculator: the fields need one shape, with a value per grid point")
         if self._hin is None or self._hin.shape[2] != n:
             self._hin = _pinned((nslot, 5, n))
             self._din = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
@@ -335,8 +339,8 @@ class SBESolver:
             self._sent[w - 1].synchronize()
         h = self._hin_np[w - 1]
         for i, f in enumerate(fields):
-            h[i] = f
-        h[4].view(np.float64)[:n] = rr
+            h[i] = f.reshape(-1)
+        h[4].view(np.float64)[:n] = x
         d = self._din[w - 1]
         d.copy_(self._hin[w - 1], non_blocking=True)
         self._sent[w - 1] = self._sent[w - 1] or torch.cuda.Event()

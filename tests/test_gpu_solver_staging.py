@@ -70,3 +70,21 @@ def test_pinned_memory_refused(monkeypatch):
     for a, b in zip(_call(sv, rr, f), ref):
         assert np.array_equal(a, b)
 
+
+
+def test_field_shapes():
+    """Fields of shapes of their own are refused, as np.stack refuses them; column vectors and
+    lists serve."""
+    sv, rr = _solver(300)
+    f = _fields(rr, 2e7)
+    ref = _call(sv, rr, f)
+    for bad in (np.zeros(1, complex), np.zeros(299, complex), 0.0):
+        sv, rr = _solver(300)
+        with pytest.raises(ValueError):
+            _call(sv, rr, f[:3] + [bad])
+    sv, rr = _solver(300)
+    for a, b in zip(_call(sv, rr, [x[:, None] for x in f]), ref):
+        assert np.array_equal(a, b)
+    sv, rr = _solver(300)
+    for a, b in zip(_call(sv, list(rr), f[:3] + [list(f[3])]), ref):
+        assert np.array_equal(a, b)
