@@ -25,6 +25,11 @@ using f64s::to_fixed;
 // operand forms (rows as stored, or transposed)
 enum { F_P = 0, F_PT, F_C, F_CT, F_D, F_DT, F_EH, F_EHT, F_EE, F_EET, F_HH, F_HHT, F_EEX, F_HHX, F_N };
 
+// The commutators' forms of C, D, Hee and Hhh leave the diagonal (occupations and band energies)
+// to the finish, which applies it element by element in FP64: a row held in fixed point under a
+// norm that its diagonal element sets would keep a coherence of 1e-8 of it to 1e-9 only.
+static int peeled(int f) { return f != F_P && f != F_PT && f != F_EH && f != F_EHT; }
+
 struct F64Bucket {
   int nk = 0, nw = 0, nr = 0, group = 0;   // group: wires per pass
   long long bm = 0, bv = 0, br = 0, bkr = 0;
@@ -271,28 +276,39 @@ __global__ void __launch_bounds__(128) k_f64_hbuild(const __grid_constant__ HBui
 }
 
 // dP, dC, dD from the partial products (SBEs.py:1942-1965, 2309-2327, 2607-2625): the sum
-// of each output's partials over i hbar, for dP also Heh^T / (i hbar), the rates and OffP;
-// with stage 1-4 the RK4 update of k_rk4_axpy.  Bound by the FP64 pipes (some 30 operations an
-// element); one element a thread, so that a few small wires reach all SMs (four elements a thread: 1 x 64
-// 13.3 us, 2 x 512 93; here 2 x 512 81).
+// of each output's partials and of the terms with a diagonal element of C, D, Hee, Hhh,
+//   dP: P_mn (Hhh_mm + Hee_nn) - Heh_nm (D_mm + C_nn)
+//   dC: Hee_nm (C_mm - C_nn) + C_mn (Hee_nn - Hee_mm),   dD with Hhh and D,
+// over i hbar, for dP also Heh^T / (i hbar), the rates and OffP; with stage 1-4 the RK4 update of
+// k_rk4_axpy.  Bound by the FP64 pipes (some 45 operations an element); one element a thread, so
+// that a few small wires reach all SMs (four elements a thread: 1 x 64 13.3 us, 2 x 512 93; one
+// 2 x 512 81 before it had the diagonals' terms).
 struct Finish {
   int nk, nw, nsum, stage, first;   // first: output of blockIdx.z / nw = 0 (single calls)
   double dt, dt6;                   // the step, and a sixth of it
   const double* part;               // [output][nsum][re, im][wire][Nk x Nk]
-  const double2 *Heh, *P, *offp;
+  const double2 *X0[3], *H[3];      // P, C, D and Heh, Hee, Hhh
+  const double2* offp;
   const double *gamE, *gamH;
   double2 *out[3], *X[3], *acc[3], *xs[3];
 };
 
 __global__ void __launch_bounds__(256) k_f64_finish(const __grid_constant__ Finish a) {
   pdl_enter();
-  __shared__ double2 ht[32][9];
+  __shared__ double2 ht[32][9], dn[2][32], dm[2][8];
   const int nk = a.nk, which = blockIdx.z / a.nw + a.first, b = blockIdx.z % a.nw;
   const int m0 = blockIdx.y * 8, n0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
   const long long mm = (long long)nk * nk, mb = (long long)b * mm;
-  if (which == 0) {
+  {
+    // the output's Hamiltonian transposed, and the diagonals: energies (0) and occupations (1) that
+    // go with column n and with row m (dP: Hee, C and Hhh, D)
     const int t = ty * 32 + tx, n = n0 + (t >> 3), m = m0 + (t & 7);
-    if (n < nk && m < nk) ht[t >> 3][t & 7] = a.Heh[mb + (long long)n * nk + m];
+    if (n < nk && m < nk) ht[t >> 3][t & 7] = a.H[which][mb + (long long)n * nk + m];
+    const int kn = which == 2 ? 2 : 1, km = which == 1 ? 1 : 2;
+    if (ty < 2 && n0 + tx < nk)
+      dn[ty][tx] = (ty ? a.X0 : a.H)[kn][mb + (long long)(n0 + tx) * (nk + 1)];
+    else if (ty < 4 && ty >= 2 && tx < 8 && m0 + tx < nk)
+      dm[ty - 2][tx] = (ty == 3 ? a.X0 : a.H)[km][mb + (long long)(m0 + tx) * (nk + 1)];
     __syncthreads();
   }
   const double ih = 1.0 / kHbar;
@@ -305,24 +321,39 @@ __global__ void __launch_bounds__(256) k_f64_finish(const __grid_constant__ Fini
   double2 x0 = make_double2(0.0, 0.0), s0 = x0;
   if (a.stage > 0) x0 = a.X[which][i];
   if (a.stage > 1) s0 = a.acc[which][i];
+  const double2 x = a.X0[which][i];
   double sx = 0.0, sy = 0.0;
   for (int s = 0; s < a.nsum; s += 4) {   // a multiple of four: eight loads in flight
-    double x[4], y[4];
+    double p[4], q[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      x[u] = part[2 * (s + u) * cs + o];
-      y[u] = part[(2 * (s + u) + 1) * cs + o];
+      p[u] = part[2 * (s + u) * cs + o];
+      q[u] = part[(2 * (s + u) + 1) * cs + o];
     }
-    const double tx4 = (x[0] + x[1]) + (x[2] + x[3]), ty4 = (y[0] + y[1]) + (y[2] + y[3]);
-    sx = s ? sx + tx4 : tx4;
-    sy = s ? sy + ty4 : ty4;
+    const double tp = (p[0] + p[1]) + (p[2] + p[3]), tq = (q[0] + q[1]) + (q[2] + q[3]);
+    sx = s ? sx + tp : tp;
+    sy = s ? sy + tq : tq;
+  }
+  const double2 h = ht[tx][ty];
+  {
+    // x (e_n -+ e_m) + h (w_m -+ w_n), the latter turned round for dP
+    const double2 en = dn[0][tx], wn = dn[1][tx], em = dm[0][ty], wm = dm[1][ty];
+    double2 e, w;
+    if (which == 0) {
+      e = cadd(en, em);
+      w = make_double2(-(wm.x + wn.x), -(wm.y + wn.y));
+    } else {
+      e = csub(en, em);
+      w = csub(wm, wn);
+    }
+    sx += fma(x.x, e.x, -x.y * e.y) + fma(h.x, w.x, -h.y * w.y);
+    sy += fma(x.x, e.y, x.y * e.x) + fma(h.x, w.y, h.y * w.x);
   }
   double2 v = make_double2(sy * ih, -sx * ih);
   if (which == 0) {
-    const double2 h = ht[tx][ty], p = a.P[mb + o];
     const double gam = a.gamE[(long long)b * nk + n] + a.gamH[(long long)b * nk + m];
-    v.x += h.y * ih - gam * p.x;
-    v.y += -h.x * ih - gam * p.y;
+    v.x += h.y * ih - gam * x.x;
+    v.y += -h.x * ih - gam * x.y;
     if (a.offp) {
       const double2 f = a.offp[mb + o];
       v.x += f.y * ih;
@@ -565,7 +596,7 @@ bool f64_prepare(SbeCtx* c, cudaStream_t s) {
       cudaStreamSynchronize(s);   // the host vector goes out of scope
       // E^T planes of the sources: Y[r][k] = Expikr[k][r]
       f64s::SliceArgs a{};
-      a.f[0] = f64s::Form{c->expikr + m.bkr, nullptr, 1, m.ep, m.ee};
+      a.f[0] = f64s::Form{c->expikr + m.bkr, nullptr, 1, 0, m.ep, m.ee};
       a.rows = m.nr;
       a.kdim = nk;
       a.ld = m.nr;
@@ -600,7 +631,7 @@ static void state_forms(f64s::SliceArgs& a, const FormSet& F, const double2* P, 
                         const double2* D) {
   const double2* x[3] = {P, C, D};
   for (int i = 0; i < 6; ++i)
-    a.f[i] = f64s::Form{x[i / 2], nullptr, i & 1, F.plane(i), F.exps(i)};
+    a.f[i] = f64s::Form{x[i / 2], nullptr, i & 1, peeled(i), F.plane(i), F.exps(i)};
 }
 
 static f64s::SliceArgs slice_args(const FormSet& F) {
@@ -659,10 +690,11 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       int nf = 6, alias[F_N];
       for (int i = 0; i < F_N; ++i) alias[i] = i;
       for (int i = 0; i < 6; ++i)
-        a.f[nf++] = f64s::Form{hm[i / 2], nullptr, i & 1, F.plane(F_EH + i), F.exps(F_EH + i)};
+        a.f[nf++] = f64s::Form{hm[i / 2], nullptr, i & 1, peeled(F_EH + i), F.plane(F_EH + i),
+                               F.exps(F_EH + i)};
       if (c->any_offdiag) {
-        a.f[nf++] = f64s::Form{hm[1], c->dB + o, 0, F.plane(F_EEX), F.exps(F_EEX)};
-        a.f[nf++] = f64s::Form{hm[2], c->dA + o, 0, F.plane(F_HHX), F.exps(F_HHX)};
+        a.f[nf++] = f64s::Form{hm[1], c->dB + o, 0, 1, F.plane(F_EEX), F.exps(F_EEX)};
+        a.f[nf++] = f64s::Form{hm[2], c->dA + o, 0, 1, F.plane(F_HHX), F.exps(F_HHX)};
       } else {
         alias[F_EEX] = F_EE;
         alias[F_HHX] = F_HH;
@@ -678,12 +710,13 @@ int f64_rhs(SbeCtx* c, const double2* P, const double2* C, const double2* D, con
       f.dt = dt;
       f.dt6 = dt / 6.0;
       f.part = m.part;
-      f.Heh = c->Heh + o;
-      f.P = P + o;
+      const double2* st[3] = {P + o, C + o, D + o};
       f.gamE = c->gamE + vo;
       f.gamH = c->gamH + vo;
       const long long n = c->tot_mat;
       for (int i = 0; i < 3; ++i) {
+        f.X0[i] = st[i];
+        f.H[i] = hm[i];
         f.out[i] = out ? out[i] + o : nullptr;
         f.X[i] = X ? X[i] + o : nullptr;
         f.acc[i] = c->kacc + i * n + o;
@@ -768,7 +801,7 @@ int f64_sources(SbeCtx* c, const double2* P, const double2* C, const double2* D,
       f64s::Job jobs[3];
       const long long cs = (long long)g * nk * nr;
       for (int i = 0; i < 3; ++i) {
-        a.f[i] = f64s::Form{x[i], nullptr, 0, F.plane(2 * i), F.exps(2 * i)};
+        a.f[i] = f64s::Form{x[i], nullptr, 0, 0, F.plane(2 * i), F.exps(2 * i)};
         f64s::Job& j = jobs[i];
         j = f64s::Job{};
         j.A = F.plane(2 * i);
@@ -879,6 +912,7 @@ bool f64_rhs_single(int which, int nk, const double2* C, const double2* D, const
         slot[g] = nf;
         a.f[nf].src = mats[g / 2];
         a.f[nf].transpose = g & 1;
+        a.f[nf].peel = peeled(g);
         ++nf;
       }
       alias[f] = slot[g];
@@ -906,8 +940,10 @@ bool f64_rhs_single(int which, int nk, const double2* C, const double2* D, const
   f.nsum = 4 * parts;
   f.first = which;
   f.part = part;
-  f.Heh = Heh;
-  f.P = P;
+  for (int i = 0; i < 3; ++i) {
+    f.X0[i] = mats[i];
+    f.H[i] = mats[3 + i];
+  }
   f.offp = offp;
   f.gamE = gamE;
   f.gamH = gamH;

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(32 * kSliceStep * (SPLIT ? 2 : 1))
     for (int i = 0; i < 8; ++i) {
       const int k = kb * BK + 8 * j + i;
       const long long o = f.transpose ? (long long)k * ld + r : (long long)r * ld + k;
-      const bool in = rok && k < kdim;
+      const bool in = rok && k < kdim && (k != r || !f.peel);
       if constexpr (SPLIT) {
         v[0][i] = in ? reinterpret_cast<const double*>(X)[2 * o + im] : 0.0;
         if (in && Y && im) v[0][i] += a.add_f * Y[(long long)r * ld + k].x;

@@ -61,11 +61,12 @@ struct Launch {
 
 // One operand form of the slicing pass: row r, column k is src[r ld + k], or src[k ld + r]
 // when transposed, of a batch of complex matrices; add (real parts of a complex matrix, or
-// null, not transposed) times add_f joins the imaginary part.
+// null, not transposed) times add_f joins the imaginary part; with peel the elements r = k count
+// as zero.
 struct Form {
   const double2* src;
   const double2* add;
-  int transpose;
+  int transpose, peel;
   __half* dst;      // plane 0, batch entry 0
   int* e;           // row exponents (batch stride rows)
 };
