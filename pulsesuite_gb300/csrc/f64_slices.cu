@@ -1,6 +1,7 @@
 // Exact-slice FP64 products on tcgen05 (see f64_slices.cuh).
 #include "f64_slices.cuh"
 #include "fp_bits.cuh"
+#include "per_device.cuh"
 #include "sbe_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -577,22 +578,10 @@ void launch_f64_slice(const f64s::SliceArgs& a, int nforms, cudaStream_t s) {
   }
 }
 
-static int sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-      v = 1;
-    return v;
-  }();
-  return n;
-}
-
 int launch_f64_gemm(const f64s::Job* jobs, int njobs, int* err, cudaStream_t s, bool stall) {
   if (njobs < 1 || njobs > f64s::MAX_JOBS) return fail(SBE_ERR_ARG, "f64 gemm: 1 to 16 jobs");
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      f64s::k_f64_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, f64s::SMEM);
-  if (attr != cudaSuccess) return fail(SBE_ERR_CUDA, "f64 gemm: cannot raise the shared-memory limit");
+  const int rc = cuda_check(raise_smem<f64s::k_f64_gemm>(f64s::SMEM), "f64 gemm: shared-memory limit");
+  if (rc) return rc;
   f64s::Launch L{};
   L.njobs = njobs;
   L.err = err;

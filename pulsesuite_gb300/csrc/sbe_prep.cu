@@ -4,6 +4,7 @@
 #include "sbe_ctx.cuh"
 #include "batch.cuh"
 #include "fp_bits.cuh"
+#include "per_device.cuh"
 
 namespace sbe {
 
@@ -397,11 +398,9 @@ static size_t deph64_smem(int nw, int nk) {
 
 template <int NW>
 static void deph64_launch(const Deph64& a, int nk, cudaStream_t s) {
-  static const bool raised = [] {
-    return cudaFuncSetAttribute(k_offdiag_D64<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)deph64_smem(NW, 4096)) == cudaSuccess;
-  }();
-  (void)raised;
+  // enough for the largest Nk that a context takes; a launch that needs more than the default and
+  // did not get it fails and reports
+  raise_smem<k_offdiag_D64<NW>>((int)deph64_smem(NW, 4096));
   launch(k_offdiag_D64<NW>, dim3((nk + 31) / 32, nk - 1, 2), 256, deph64_smem(NW, nk), s, a);
 }
 

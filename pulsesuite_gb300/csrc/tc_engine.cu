@@ -1,6 +1,7 @@
 // tcgen05 / bulk-copy / TMEM split-precision GEMM engine (see tc_gemm.cuh).
 #include "sbe_ctx.cuh"
 #include "fp_bits.cuh"
+#include "per_device.cuh"
 #include "tc_gemm.cuh"
 #include "tc_ptx.cuh"
 
@@ -571,31 +572,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 static const int kTcSmem = 1024 + tc::STAGE_AREA + tc::SCR_BYTES + 512;
 
 int tc_gemm_init() {
-  static bool attr = false;
-  if (!attr) {
-    using Kernel = void (*)(const tc::GemmLaunch);
-    const Kernel kernels[] = {
-        tc::k_tc_gemm<256, tc::MODE_FULL>, tc::k_tc_gemm<128, tc::MODE_FULL>,
-        tc::k_tc_gemm<64, tc::MODE_FULL>,  tc::k_tc_gemm<128, tc::MODE_HH>,
-        tc::k_tc_gemm<64, tc::MODE_HH>};
-    for (Kernel k : kernels)
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) !=
-          cudaSuccess)
-        return fail(SBE_ERR_CUDA, "tc_gemm: cannot raise the shared-memory limit");
-    attr = true;
-  }
+  const cudaError_t e[] = {raise_smem<tc::k_tc_gemm<256, tc::MODE_FULL>>(kTcSmem),
+                           raise_smem<tc::k_tc_gemm<128, tc::MODE_FULL>>(kTcSmem),
+                           raise_smem<tc::k_tc_gemm<64, tc::MODE_FULL>>(kTcSmem),
+                           raise_smem<tc::k_tc_gemm<128, tc::MODE_HH>>(kTcSmem),
+                           raise_smem<tc::k_tc_gemm<64, tc::MODE_HH>>(kTcSmem)};
+  for (cudaError_t x : e)
+    if (x != cudaSuccess) return cuda_check(x, "tc_gemm: shared-memory limit");
   return SBE_OK;
-}
-
-static int num_sms() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 1;
-  }
-  return n;
 }
 
 // every bulk copy stays inside the plane sets: tiles of the launch grid lie in
@@ -641,7 +625,7 @@ static double launch_cost(const tc::GemmJob* jobs, int njobs, int bnt) {
       total += t * rows * d.batch * ks;
     }
   }
-  return std::max(longest, total / num_sms());
+  return std::max(longest, total / sm_count());
 }
 
 // The N tile of a launch: the jobs' own (256, or 128 where chosen), narrowed where that brings
@@ -663,8 +647,8 @@ static int n_tile(const tc::GemmJob* jobs, int njobs, int mode, int widest) {
     const int n = mode == tc::MODE_HH ? 64 : widest;
     tiles += (long long)((d.N + n - 1) / n) * ((d.M + tc::BM - 1) / tc::BM) * d.batch;
   }
-  if (mode == tc::MODE_HH) return tiles <= num_sms() ? 64 : tc::BN_HH;
-  if (tiles > 4LL * num_sms()) return widest;
+  if (mode == tc::MODE_HH) return tiles <= sm_count() ? 64 : tc::BN_HH;
+  if (tiles > 4LL * sm_count()) return widest;
   int best = widest;
   double cost = launch_cost(jobs, njobs, widest);
   for (int n = widest / 2; n >= 64; n /= 2) {
@@ -692,7 +676,7 @@ static bool splits_parts(const tc::GemmJob* jobs, int njobs, int bnt) {
       return false;
     tiles += (long long)((d.N + bnt - 1) / bnt) * ((d.M + tc::BM - 1) / tc::BM) * d.batch;
   }
-  return terms > 1 && 2 * tiles <= num_sms();
+  return terms > 1 && 2 * tiles <= sm_count();
 }
 
 int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, int* sched, cudaStream_t s) {
@@ -734,7 +718,7 @@ int tc_gemm_launch(const tc::GemmJob* jobs, int njobs, int* sched, cudaStream_t 
   L.tile_base[njobs] = nt;
   if (nt == 0) return SBE_OK;
   L.sched = sched;
-  const int grid = (int)std::min<long long>(nt, num_sms());
+  const int grid = (int)std::min<long long>(nt, sm_count());
   void (*const kernel)(const tc::GemmLaunch) =
       mode == tc::MODE_HH ? (bnt == 64 ? tc::k_tc_gemm<64, tc::MODE_HH>
                                        : tc::k_tc_gemm<tc::BN_HH, tc::MODE_HH>)
