@@ -67,14 +67,17 @@ class Batch;
 template <class Body, class... P>
 class Batch<Body, void (*)(Blk, P...)> {
  public:
-  Batch(dim3 block, cudaStream_t s, size_t smem = 0) : block_(block), s_(s), smem_(smem) {}
+  Batch(dim3 block, cudaStream_t s, size_t smem = 0) : block_(block), s_(s), part_smem_(smem) {}
   ~Batch() { flush(); }
+  // dynamic shared memory of the parts that follow; a launch asks for its own parts' largest
+  void smem(size_t bytes) { part_smem_ = bytes; }
   template <class... A>
   void add(dim3 grid, A&&... a) {
     const long long blocks = (long long)grid.x * grid.y * grid.z;
     if (blocks == 0) return;
     if (p_.n == kMax || blocks_ + blocks > 0x7fffffffLL) flush();
     const int i = p_.n++;
+    smem_ = smem_ > part_smem_ ? smem_ : part_smem_;
     z_[i] = grid.z;
     p_.gx[i] = grid.x;
     p_.gy[i] = grid.y;
@@ -106,6 +109,7 @@ class Batch<Body, void (*)(Blk, P...)> {
       start<kMax>(grid);
     p_.n = 0;
     blocks_ = 0;
+    smem_ = 0;
   }
 
  private:
@@ -134,7 +138,7 @@ class Batch<Body, void (*)(Blk, P...)> {
   int z_[kMax] = {};
   dim3 block_;
   cudaStream_t s_;
-  size_t smem_;
+  size_t smem_ = 0, part_smem_;
 };
 
 // Names a device function, void(Blk, ...), as the body of a batched pass (blocks: per SM at least,

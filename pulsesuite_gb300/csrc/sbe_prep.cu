@@ -814,14 +814,16 @@ void launch_offdiag_D(SbeCtx* c, int w_only, const double* g3, bool fp32, cudaSt
     launch(k_deph_consts, dim3((c->nk_max + 127) / 128, 2 * c->nw), 128, 0, s, c->d_wires, c->vs,
            c->dconst, c->dpre);
     // groups of 4 or more wires share the Lorentzian factors (chunks of up to 16 wires); the
-    // other wires take the per-wire sums.  One launch per kind, the largest Nk first
-    size_t nk = c->nk_max;
-    Batch<Deph16Pass> g16(128, s, sizeof(float) * (2 * 32 * 16 + 2 * nk));
-    Batch<Deph8Pass> g8(128, s, sizeof(float) * (2 * 32 * 8 + 2 * nk));
-    Batch<Deph1Pass> g1(128, s, sizeof(float) * 8 * nk);
+    // other wires take the per-wire sums.  One launch per kind
+    Batch<Deph16Pass> g16(128, s);
+    Batch<Deph8Pass> g8(128, s);
+    Batch<Deph1Pass> g1(128, s);
     for (auto g = c->dgroups.rbegin(); g != c->dgroups.rend(); ++g) {
       const int gk = c->wires[c->dwl_host[g->first]].nk;
       const dim3 grid((gk + 511) / 512, gk + 1, 2);   // 128 threads x 4 k
+      g16.smem(sizeof(float) * (2 * 32 * 16 + 2 * (size_t)gk));
+      g8.smem(sizeof(float) * (2 * 32 * 8 + 2 * (size_t)gk));
+      g1.smem(sizeof(float) * 8 * (size_t)gk);
       for (int o = 0; o < g->second;) {
         const int n = g->second < 4 ? 1 : std::min(16, g->second - o);
         const int* wl = c->dwl + g->first + o;
