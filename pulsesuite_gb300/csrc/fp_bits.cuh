@@ -102,6 +102,13 @@ __device__ __forceinline__ double div_by(double x, double d, double r) {
   return fma(fma(-q, d, x), r, q);
 }
 
+// infinite or NaN, by the exponent
+__device__ __forceinline__ bool not_finite(double x) {
+  return (__double2hiint(x) & 0x7FF00000) == 0x7FF00000;
+}
+
+__device__ __forceinline__ double nan64() { return __longlong_as_double(0x7FF8000000000000ll); }
+
 // |x| as an ordered integer (the bit pattern of a non-negative double grows with
 // its value), for maxima without floating-point instructions
 __device__ __forceinline__ unsigned long long absbits(double x) {

@@ -6,6 +6,7 @@
 #include <string>
 
 #include "sbe_ctx.cuh"
+#include "spline.cuh"
 
 namespace sbe {
 
@@ -211,7 +212,7 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   }
   add((void**)&c->emis, D8 * std::max<size_t>(emis_host.size(), 1));
   add((void**)&c->G, C16 * 3 * okr);
-  add((void**)&c->qscr, C16 * (20 * (size_t)c->nr_max + 1));
+  add((void**)&c->qscr, C16 * (20 * (size_t)c->nr_max + 1 + spl_bad_elems(c->nr_max)));
   add((void**)&c->kacc, C16 * 3 * om);
   add((void**)&c->xs, C16 * 3 * om);
   add((void**)&c->scal, D8 * 16 * n_wires);

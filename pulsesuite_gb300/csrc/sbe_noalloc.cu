@@ -27,12 +27,14 @@
 // device code into it; make that first call before any stream capture.
 
 #include "sbe_ctx.cuh"
+#include "spline.cuh"
 
 namespace {
 
 constexpr int kMaxGrid = SBE_NOALLOC_MAX_GRID;  // propagation-grid points (n_rr)
 constexpr int kMaxNr = SBE_NOALLOC_MAX_NR;      // wire points (Nr = 2 Nk + 2, Nk <= 1024)
-constexpr long long kCoefElems = 12LL * kMaxGrid;  // 4 fields x 3 spline coefficients
+// 4 fields x 3 spline coefficients, and a word for each tile of knots
+constexpr long long kCoefElems = 12LL * kMaxGrid + sbe::spl_bad_elems(kMaxGrid);
 constexpr long long kTmpElems = 4LL * kMaxNr;      // 4 resampled fields on the wire grid
 
 // 1.70 MB of complex128 scratch: spline coefficients, then the windowed fields.

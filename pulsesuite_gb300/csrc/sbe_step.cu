@@ -483,7 +483,7 @@ __global__ void k_spline_coef(int n, const double* x, const double2* y, int nf, 
   fmm_spline(n, x, y + (long long)f * n, b, b + n, b + 2 * n);
 }
 
-static void spline_coefs(int n, const double* x, const double2* y, int nf, double2* coef,
+static void spline_coefs(int n, const double* x, const double2* y, int nf, double2* coef, int* bad,
                          cudaStream_t s) {
   if (n < kSplMin) {
     launch(k_spline_coef, 1, 32, 0, s, n, x, y, nf, coef);
@@ -495,24 +495,31 @@ static void spline_coefs(int n, const double* x, const double2* y, int nf, doubl
   b.coef = coef;
   b.n0 = n;
   b.nf = nf;
+  b.bad = bad;
   launch_splines(b, 1, n, s);
 }
 
 // evaluate nf splines (knots x0, n0) at x1 (n1 points); values outside
 // [min x0, max x0] are 0; optional window multiply and real part.  The block finds the
-// knots' range together.
+// knots' range together.  A part of a field (real, imaginary) with a coefficient that is not finite
+// is NaN everywhere, as a solve from end to end leaves it.
 __global__ void __launch_bounds__(128) k_spline_eval(int n0, const double* x0, const double2* y0,
-                                                     const double2* coef, int n1, const double* x1,
-                                                     int nf, const double* win, int real_part,
-                                                     double2* out) {
+                                                     const double2* coef, const int* bad, int n1,
+                                                     const double* x1, int nf, const double* win,
+                                                     int real_part, double2* out) {
   pdl_enter();
   __shared__ double rlo[4], rhi[4];
+  __shared__ int rbad[4];
   double lo = x0[0], hi = lo;
   for (int i = threadIdx.x; i < n0; i += 128) {
     const double x = x0[i];
     lo = fmin(lo, x);
     hi = fmax(hi, x);
   }
+  int nan = 0;
+  if (n0 >= kSplMin)
+    for (int i = threadIdx.x; i < spl_tiles(n0); i += 128) nan |= bad[i];
+  nan = __reduce_or_sync(0xffffffffu, nan);
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
@@ -520,8 +527,10 @@ __global__ void __launch_bounds__(128) k_spline_eval(int n0, const double* x0, c
   if ((threadIdx.x & 31) == 0) {
     rlo[threadIdx.x >> 5] = lo;
     rhi[threadIdx.x >> 5] = hi;
+    rbad[threadIdx.x >> 5] = nan;
   }
   __syncthreads();
+  nan = rbad[0] | rbad[1] | rbad[2] | rbad[3];
   lo = fmin(fmin(rlo[0], rlo[1]), fmin(rlo[2], rlo[3]));
   hi = fmax(fmax(rhi[0], rhi[1]), fmax(rhi[2], rhi[3]));
   const int j = blockIdx.x * 128 + threadIdx.x;
@@ -533,6 +542,8 @@ __global__ void __launch_bounds__(128) k_spline_eval(int n0, const double* x0, c
   for (int f = 0; f < nf; ++f) {
     double2 v = make_double2(0, 0);
     if (in) v = spl_eval(y0 + (long long)f * n0, coef + (long long)f * 3 * n0, n0, i, dx);
+    if (in && (nan >> 2 * f & 1)) v.x = nan64();
+    if (in && (nan >> 2 * f & 2)) v.y = nan64();
     if (win) v = cscale(v, w);
     if (real_part) v.y = 0.0;
     out[(long long)f * n1 + j] = v;
@@ -590,7 +601,7 @@ __global__ void __launch_bounds__(64) k_fftg(int n, const double2* tw, const dou
 // ordered on its stream, so they share the scratch.
 int launch_prop2qw(SbeCtx* c, int w, const double* RR, int n_rr, const double2* fin,
                    double2* out, cudaStream_t s) {
-  const long long need = 12LL * n_rr;
+  const long long need = 12LL * n_rr + spl_bad_elems(n_rr);
   if (need > c->p2q_cap) {
     if (c->p2q_coef && cudaFree(c->p2q_coef) != cudaSuccess)
       return cuda_check(cudaGetLastError(), "prop2qw: release the smaller scratch");
@@ -604,13 +615,14 @@ int launch_prop2qw(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
 }
 
 // The same three launches as launch_prop2qw on scratch the caller provides:
-// coef holds 12 n_rr and tmp 4 Nr complex values.  Allocates nothing.
+// coef holds 12 n_rr + spl_bad_elems(n_rr) and tmp 4 Nr complex values.  Allocates nothing.
 int launch_prop2qw_scratch(SbeCtx* c, int w, const double* RR, int n_rr, const double2* fin,
                            double2* out, double2* coef, double2* tmp, cudaStream_t s) {
   const WireDev& W = c->wires[w];
-  spline_coefs(n_rr, RR, fin, 4, coef, s);
-  launch(k_spline_eval, (W.nr + 127) / 128, 128, 0, s, n_rr, RR, fin, coef, W.nr, c->r + W.off_r, 4,
-         c->window + W.off_r, 1, tmp);
+  int* bad = reinterpret_cast<int*>(coef + 12LL * n_rr);
+  spline_coefs(n_rr, RR, fin, 4, coef, bad, s);
+  launch(k_spline_eval, (W.nr + 127) / 128, 128, 0, s, n_rr, RR, fin, coef, bad, W.nr,
+         c->r + W.off_r, 4, c->window + W.off_r, 1, tmp);
   launch(k_fftg, (W.nr / 2 + 2) / 2, 64, 0, s, W.nr, c->twd + W.off_r, tmp, out);
   return cuda_check(cudaGetLastError(), "prop2qw (caller scratch)");
 }
@@ -651,13 +663,14 @@ int launch_qw2prop(SbeCtx* c, int w, const double* RR, int n_rr, const double2* 
   double2* coef = c->qscr;
   double2* tmp = coef + 15 * (size_t)c->nr_max;
   double* total = reinterpret_cast<double*>(tmp + 5 * (size_t)c->nr_max);
+  int* bad = reinterpret_cast<int*>(total + 2);
   cudaMemcpyAsync(tmp, src, sizeof(double2) * 5 * (size_t)W.nr, cudaMemcpyDeviceToDevice, s);
   const double* rw = c->r + W.off_r;
   if (plasmonics)
     launch(k_plasmonics, kCluster, 256, 0, s, W.nr, rw, tmp + 3 * W.nr, tmp + 4 * W.nr, total, 0);
-  spline_coefs(W.nr, rw, tmp, 5, coef, s);
-  launch(k_spline_eval, (n_rr + 127) / 128, 128, 0, s, W.nr, rw, tmp, coef, n_rr, RR, 5, nullptr, 0,
-         out);
+  spline_coefs(W.nr, rw, tmp, 5, coef, bad, s);
+  launch(k_spline_eval, (n_rr + 127) / 128, 128, 0, s, W.nr, rw, tmp, coef, bad, n_rr, RR, 5,
+         nullptr, 0, out);
   if (plasmonics)
     launch(k_plasmonics, kCluster, 256, 0, s, n_rr, RR, out + 3 * (size_t)n_rr,
            out + 4 * (size_t)n_rr, total, 1);

@@ -12,6 +12,8 @@
 // the pivots come from the determinants theta_i = b_i theta_{i-1} - d_{i-1}^2 theta_{i-2} (one
 // dependent FMA a point, p_i = theta_i / theta_{i-1} beside it), and a block holds few points
 // (64, all fields of one set of knots) so that the grid spreads them over the SMs.
+// A value that is not finite reaches the coefficients of some 100 points only; a solve from end to
+// end spreads it over all, which the calls that resample one wire keep (bad, k_spline_eval).
 // Mean of the solves of a step (4 fields on 4096 points, 5 on Nr = 230): 17.5 ms with one
 // thread per field, 32 us here; with the pivots' coefficients and reciprocals formed by all
 // threads (3 fields on 8192, 5 on 514: 31 -> 22 us) 22 us.
@@ -21,7 +23,7 @@
 namespace sbe {
 namespace {
 
-constexpr int kTile = 64, kSeg = 8, kWarm = 64, kWarmP = 32, kFields = 5;
+constexpr int kTile = kSplTile, kSeg = 8, kWarm = 64, kWarmP = 32, kFields = 5;
 constexpr int kCap = kTile + 2 * kWarm + kWarmP + 16;   // points a block holds
 constexpr int kThreads = 256;
 
@@ -30,10 +32,12 @@ __device__ __forceinline__ double2 cdivr(double2 a, double d) { return cscale(a,
 
 __global__ void __launch_bounds__(kThreads) k_spline(SplBatch s) {
   pdl_enter();
+  __shared__ int bad;
   __shared__ double2 c1[kFields][kCap], c2[kFields][kCap];
   __shared__ double x[kCap], ip[kCap], id[kCap], tt[kCap], mm[kCap];
   __shared__ double red[2][kThreads / 32];
   const int g = blockIdx.y, tid = threadIdx.x, nf = s.nf;
+  if (tid == 0) bad = 0;
   int n = s.n0;
   long long ko = 0;
   if (s.off) {
@@ -213,6 +217,8 @@ __global__ void __launch_bounds__(kThreads) k_spline(SplBatch s) {
     const double2* gy = s.Y + vo;
     double2 *gb = s.coef + 3 * vo, *gc = gb + n, *gd = gb + 2 * n;
     const double2 c = c1[f][j];
+    if (not_finite(c.x)) atomicOr(&bad, 1 << 2 * f);
+    if (not_finite(c.y)) atomicOr(&bad, 2 << 2 * f);
     gc[i] = cscale(c, 3.0);
     if (i < n - 1) {
       const double2 cn = c1[f][j + 1];
@@ -225,6 +231,10 @@ __global__ void __launch_bounds__(kThreads) k_spline(SplBatch s) {
                    cscale(cadd(cp, cscale(c, 2.0)), x[j] - x[j - 1]));
       gd[i] = cscale(csub(c, cp), id[j - 1]);
     }
+  }
+  if (s.bad) {
+    __syncthreads();
+    if (tid == 0) s.bad[g * gridDim.x + blockIdx.x] = bad;
   }
 }
 

@@ -14,10 +14,17 @@ struct SplBatch {
   const int* n;         // knots per problem (nullptr: n0 for all)
   const long long* off; // per problem: knot and value offset (nullptr: 0 and p * n0)
   int n0, nf;           // nf: 1 to 5
+  int* bad;             // per group and tile (or null): bits 2 f, 2 f + 1 of field f's real and
+                        // imaginary part with a coefficient that is not finite
 };
 
 // every problem needs at least kSplMin knots
 constexpr int kSplMin = 4;
+// points whose coefficients one block stores, and the tiles of n knots
+constexpr int kSplTile = 64;
+__host__ __device__ constexpr int spl_tiles(int n) { return (n + kSplTile - 1) / kSplTile; }
+// complex values that hold the tiles' words of n knots
+__host__ __device__ constexpr int spl_bad_elems(int n) { return (spl_tiles(n) + 3) / 4; }
 void launch_splines(const SplBatch& b, int ngroups, int nmax, cudaStream_t s);
 
 // spliner.py:1137-1167 locate on ascending knots
