@@ -504,6 +504,14 @@ static int exchange(int nk, int nw, const double2* P, const double2* C, const do
 constexpr int kMinNk = 32;
 constexpr size_t kGroupBytes = 3ull << 30;   // pass workspace per bucket
 
+// While another stream is being captured (in the default, global mode from any thread), this thread's
+// allocations would fail and spoil that capture; in relaxed mode they do neither.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 bool f64_prepare(SbeCtx* c, cudaStream_t s) {
   if (c->f64) return true;
   if (c->f64_off) return false;
@@ -515,6 +523,7 @@ bool f64_prepare(SbeCtx* c, cudaStream_t s) {
     cudaGetLastError();
     return false;
   }
+  const RelaxedCapture relaxed;
   F64Work* w = new F64Work();
   c->f64 = w;
   bool ok = true;
@@ -851,6 +860,7 @@ static cudaMemPool_t scratch_pool() {
   std::lock_guard<std::mutex> lock(mu);
   auto it = pools.find(dev);
   if (it != pools.end()) return it->second;
+  const RelaxedCapture relaxed;
   cudaMemPoolProps pr{};
   pr.allocType = cudaMemAllocationTypePinned;
   pr.location.type = cudaMemLocationTypeDevice;
