@@ -90,7 +90,7 @@ int sbe_ctx_layout(const SbeCtx* ctx, long long* out, long long* total_mat, long
  * 4 V0 (3*Nk: eh, ee, hh by k1-k2 >= 0), 5 Chi1D (2*Nk by |k1-k2|), 6 qe/qh (2*Nk),
  * 7 EP (Nk*Nk), 8 HP (Nk*Nk), 9 window (Nr), 10 dephasing maps (6*Nk*Nk int32),
  * 11 xe/xh (2*Nk), 12 Expikr (c128 Nk*Nr), 13 scalars (16 doubles), 14 the window
- * in k space (c128 Nr), 15 the flag of the FP64 products' waits (an int).      */
+ * in k space (c128 Nr).                                                        */
 int sbe_ctx_table(const SbeCtx* ctx, int w, int which, void* dst, long long nbytes, void* stream);
 
 /* ---- reference pure functions, one wire, FP64 ----------------------------
@@ -451,11 +451,16 @@ int sbe_ctx_check(SbeCtx* ctx, void* stream);
  * mixed-precision workspace (any mixed call creates it); waits for the stream.  */
 int sbe_wait_selftest(SbeCtx* ctx, int* gave_up, void* stream);
 /* The same for the FP64 products: one launch of a 64 x 64 product whose operands
- * never arrive.  Its waits give up after ~2 s, the context's flag (sbe_ctx_table
- * 15, an int) is raised and out, 64 * 64 doubles on the device, becomes NaN: what
- * a product could not form is NaN, never an older value.  The functions without a
- * context report by those NaN alone.                                            */
+ * never arrive.  Its waits give up after ~2 s, the context's flag is raised and
+ * out, 64 * 64 doubles on the device, becomes NaN: what a product could not form is
+ * NaN, never an older value.  The functions without a context report by those NaN
+ * alone.                                                                        */
 int sbe_f64_wait_selftest(SbeCtx* ctx, double* out, void* stream);
+/* The FP64 products' flag as the host sees it (nonzero: a wait gave up and no
+ * sbe_ctx_check has reported it yet), for callers that wait for the stream anyway:
+ * *flag stays valid as long as the context, and is null where page-locked memory
+ * was refused (sbe_ctx_check then still reports).                               */
+int sbe_ctx_wait_flag(const SbeCtx* ctx, const int** flag);
 
 /* ---- diagnostics ------------------------------------------------------------ */
 /* Diagnostic entry, no counterpart in the reference: out[b] = op(A[b]) op(B[b])

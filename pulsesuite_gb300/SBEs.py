@@ -198,6 +198,7 @@ class SBESolver:
             self.contexts = [WireContext(specs)]
         else:
             self.contexts = [WireContext([sp]) for sp in specs]
+        self._flags = [ctx.wait_flag() for ctx in self.contexts]
         c0 = self.contexts[0]
         self.kr = c0.table(0, "kr").cpu().numpy()
         self.r = c0.table(0, "r").cpu().numpy()
@@ -267,6 +268,7 @@ class SBESolver:
             for spec in ctx.specs:
                 spec.flags = dict(spec.flags, Optics=False)
         self.contexts = [WireContext(ctx.specs) for ctx in self.contexts]
+        self._flags = [ctx.wait_flag() for ctx in self.contexts]
 
     def QWCalculator(self, Exx, Eyy, Ezz, Vrr, rr, q, dt, w, Pxx, Pyy, Pzz, Rho, DoQWP, DoQWDl):
         """SBEs.py:5826-5985: advance wire w by dt and return its sources in place."""
@@ -297,7 +299,7 @@ class SBESolver:
         Ek3 = Ek[:3]                                      # the first three rows, contiguous
         ctx.leapfrog_step(self._st[w - 1], Ek3, dt, src)
         ctx.qw2prop(0, RR, src, self.LF, self._dout[0])
-        out = self._fetch(ctx)[0]
+        out = self._fetch(ctx, self._flags[w - 1])[0]
         if self.write_info:
             self._write_info(ctx, w, dt, src, Ek3)
             self._write_maxoffdiag(ctx, 0)
@@ -319,22 +321,16 @@ class SBESolver:
         waited for before its host memory is filled again."""
         x = np.asarray(rr, dtype=np.float64).reshape(-1)
         fields = [np.asarray(f, dtype=complex) for f in fields]
-        n, nslot = x.size, self.Nw if self.batch else 1
-        if any(f.shape != fields[0].shape for f in fields) or fields[0].size != n:
+        n, nslot, shape = x.size, self.Nw if self.batch else 1, fields[0].shape
+        if fields[0].size != n or not all([f.shape == shape for f in fields]):
             raise ValueError("QWCalculator: the fields need one shape, with a value per grid point")
         if self._hin is None or self._hin.shape[2] != n:
             self._hin = _pinned((nslot, 5, n))
             self._din = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
-            # the resampled sources, and behind them the flag of the products' bounded waits
-            m = nslot * 5 * n
-            self._dres = torch.empty(m + 1, dtype=CDTYPE, device="cuda")
-            self._hres = _pinned((m + 1,))
-            self._dout = self._dres[:m].view(nslot, 5, n)
-            self._dflag = torch.view_as_real(self._dres[m:]).view(-1)[:1].view(torch.int32)[:1]
-            self._sent = [None] * nslot         # events after the transfers
-            self._hin_np, self._hres_np = self._hin.numpy(), self._hres.numpy()
-            self._hout_np = self._hres_np[:m].reshape(nslot, 5, n)
-            self._hflag_np = self._hres_np[m:].view(np.int32)
+            self._dout = torch.empty((nslot, 5, n), dtype=CDTYPE, device="cuda")
+            self._hout = _pinned((nslot, 5, n))
+            self._hin_np, self._hout_np = self._hin.numpy(), self._hout.numpy()
+            self._sent = [None] * nslot         # streams with a transfer not yet waited for
         if self._sent[w - 1] is not None:
             self._sent[w - 1].synchronize()
         h = self._hin_np[w - 1]
@@ -343,17 +339,17 @@ class SBESolver:
         h[4].view(np.float64)[:n] = x
         d = self._din[w - 1]
         d.copy_(self._hin[w - 1], non_blocking=True)
-        self._sent[w - 1] = self._sent[w - 1] or torch.cuda.Event()
-        self._sent[w - 1].record()
+        self._sent[w - 1] = torch.cuda.current_stream()
         return torch.view_as_real(d[4]).reshape(-1)[:n], d[:4]
 
-    def _fetch(self, ctx):
+    def _fetch(self, ctx, flag):
         """The resampled sources of the step of ctx on the host (waits for them); raises if a
         bounded wait of that step gave up."""
-        ctx.table(0, "wait_flag", self._dflag)
-        self._hres.copy_(self._dres, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
-        if self._hflag_np[0]:
+        self._hout.copy_(self._dout, non_blocking=True)
+        stream = torch.cuda.current_stream()
+        stream.synchronize()
+        self._sent = [None if s == stream else s for s in self._sent]
+        if flag is None or flag.value:
             ctx.check()
         return self._hout_np
 
@@ -372,7 +368,7 @@ class SBESolver:
         live = [wi for wi in range(self.Nw) if self._outs[wi] is not None]
         for wi in live:
             ctx.qw2prop(wi, RR, ctx.rvec(self._src, wi, 5), self.LF, self._dout[wi])
-        host = self._fetch(ctx)
+        host = self._fetch(ctx, self._flags[0])
         for wi in live:
             o, out = self._outs[wi], host[wi]
             if self.write_info:

@@ -223,7 +223,8 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   add((void**)&c->dconst, 4 * 16 * (size_t)n_wires);
   add((void**)&c->dpre, 4 * 4 * ov);
   add((void**)&c->dwl, sizeof(int) * (size_t)n_wires);
-  add((void**)&c->f64_err, sizeof(int));
+  int* flag_dev = nullptr;
+  add((void**)&flag_dev, sizeof(int));
   size_t total = 0;
   for (auto& p : parts) total += (p.bytes + 255) / 256 * 256;
   if (cudaMalloc(&c->arena, total) != cudaSuccess) {
@@ -240,8 +241,19 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   }
   cudaStream_t s = as_stream(stream);
   cudaMemsetAsync(c->arena, 0, total, s);
+  c->f64_err = flag_dev;
+  if (cudaHostAlloc((void**)&c->f64_err_host, sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
+    *c->f64_err_host = 0;
+    if (cudaHostGetDevicePointer((void**)&c->f64_err, c->f64_err_host, 0) != cudaSuccess) {
+      cudaFreeHost(c->f64_err_host);
+      c->f64_err_host = nullptr;
+      c->f64_err = flag_dev;
+    }
+  }
+  cudaGetLastError();   // without page-locked memory the flag is on the device
   if (cudaMalloc(&c->d_wires, sizeof(WireDev) * n_wires) != cudaSuccess) {
     cudaFree(c->arena);
+    cudaFreeHost(c->f64_err_host);
     delete c;
     return fail(SBE_ERR_OOM, "sbe_ctx_create: descriptor allocation failed");
   }
@@ -279,6 +291,7 @@ int sbe_ctx_create(const SbeWireDesc* wires, int n_wires, void* stream, SbeCtx**
   if (rc != SBE_OK) {
     cudaFree(c->d_wires);
     cudaFree(c->arena);
+    cudaFreeHost(c->f64_err_host);
     delete c;
     return rc;
   }
@@ -298,11 +311,18 @@ int sbe_ctx_destroy(SbeCtx* c) {
   if (c->d_wires && cudaFree(c->d_wires) != cudaSuccess) rc = SBE_ERR_CUDA;
   if (c->arena && cudaFree(c->arena) != cudaSuccess) rc = SBE_ERR_CUDA;
   if (c->p2q_coef && cudaFree(c->p2q_coef) != cudaSuccess) rc = SBE_ERR_CUDA;
+  if (c->f64_err_host && cudaFreeHost(c->f64_err_host) != cudaSuccess) rc = SBE_ERR_CUDA;
   sbe::mixed_free(c);
   sbe::f64_free(c);
   delete c;
   if (rc != SBE_OK) set_error("sbe_ctx_destroy: cudaFree failed");
   return rc;
+}
+
+int sbe_ctx_wait_flag(const SbeCtx* c, const int** flag) {
+  if (!c || !flag) return fail(SBE_ERR_ARG, "sbe_ctx_wait_flag: null argument");
+  *flag = c->f64_err_host;
+  return SBE_OK;
 }
 
 int sbe_ctx_layout(const SbeCtx* c, long long* out, long long* total_mat, long long* total_r) {
@@ -346,7 +366,6 @@ int sbe_ctx_table(const SbeCtx* c, int w, int which, void* dst, long long nbytes
                         "sbe_ctx_table");
     }
     case 14: src = c->wk + W.off_r; need = 16 * nr; break;
-    case 15: src = c->f64_err; need = 4; break;
     default: return fail(SBE_ERR_ARG, "sbe_ctx_table: unknown table");
   }
   if (nbytes < need) return fail(SBE_ERR_ARG, "sbe_ctx_table: destination too small");

@@ -72,7 +72,8 @@ struct SbeCtx {
   void* mixed = nullptr;                 // mixed-precision workspace (sbe_tc.cu)
   void* f64 = nullptr;                   // FP64 digit-plane workspace (f64_path.cu)
   int f64_off = 0;                       // no room for it: the FP64 path stays on SIMT
-  int* f64_err = nullptr;                // a wait of the FP64 products gave up
+  // a wait of the FP64 products gave up: page-locked, or (f64_err_host null) on the device
+  int *f64_err = nullptr, *f64_err_host = nullptr;
 
   // kernel timing (sbe_ctx_profile): event pairs per category, and a pool
   int prof = 0;

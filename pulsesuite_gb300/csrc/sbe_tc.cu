@@ -2066,11 +2066,17 @@ extern "C" int sbe_ctx_check(SbeCtx* c, void* stream) {
   int rc = cuda_check(cudaStreamSynchronize(as_stream(stream)), "sbe_ctx_check");
   if (rc) return rc;
   int f = 0;
-  rc = cuda_check(cudaMemcpy(&f, c->f64_err, sizeof(int), cudaMemcpyDeviceToHost),
-                  "sbe_ctx_check: read FP64 flag");
+  if (c->f64_err_host)
+    f = *static_cast<volatile int*>(c->f64_err_host);
+  else
+    rc = cuda_check(cudaMemcpy(&f, c->f64_err, sizeof(int), cudaMemcpyDeviceToHost),
+                    "sbe_ctx_check: read FP64 flag");
   if (rc) return rc;
   if (f) {
-    cudaMemset(c->f64_err, 0, sizeof(int));
+    if (c->f64_err_host)
+      *static_cast<volatile int*>(c->f64_err_host) = 0;
+    else
+      cudaMemset(c->f64_err, 0, sizeof(int));
     return fail(SBE_ERR_TIMEOUT, "a pipeline wait of the FP64 products timed out (results of the "
                                  "affected calls are invalid)");
   }

@@ -96,7 +96,7 @@ class RK4Graph:
 
 
 TABLES = dict(kr=0, r=1, Ee=2, Eh=3, V0=4, Chi1D=5, qeqh=6, EP=7, HP=8, window=9, maps=10,
-              xexh=11, Expikr=12, scalars=13, window_k=14, wait_flag=15)
+              xexh=11, Expikr=12, scalars=13, window_k=14)
 
 
 class WireContext:
@@ -174,22 +174,18 @@ class WireContext:
         return out
 
     # ---- tables ------------------------------------------------------------
-    def table(self, w, name, out=None):
+    def table(self, w, name):
         which = TABLES[name]
         nk = self.nk[w]
         nr = 2 * nk + 2
         shapes = {0: (nk,), 1: (nr,), 2: (nk,), 3: (nk,), 4: (3, nk), 5: (2, nk), 6: (2, nk),
                   7: (nk, nk), 8: (nk, nk), 9: (nr,), 11: (2, nk), 13: (16,)}
-        if out is not None:
-            t = out
-        elif which == 10:
+        if which == 10:
             t = torch.empty((6, nk, nk), dtype=torch.int32, device=self.device)
         elif which == 12:
             t = torch.empty((nk, nr), dtype=CDTYPE, device=self.device)
         elif which == 14:
             t = torch.empty((nr,), dtype=CDTYPE, device=self.device)
-        elif which == 15:
-            t = torch.empty((1,), dtype=torch.int32, device=self.device)
         else:
             t = torch.empty(shapes[which], dtype=torch.float64, device=self.device)
         _lib.check(self.lib.sbe_ctx_table(self.handle, w, which, _lib.ptr(t),
@@ -365,6 +361,13 @@ class WireContext:
         _lib.check(self.lib.sbe_ctx_tiles(self.handle, out, cap, ctypes.byref(nb)),
                    "sbe_ctx_tiles")
         return [tuple(out[6 * i:6 * i + 6]) for i in range(nb.value)]
+
+    def wait_flag(self):
+        """The flag of the FP64 products' bounded waits as a ctypes int (.value nonzero: check()
+        raises), valid while the context is open; None where the host cannot see it."""
+        p = ctypes.POINTER(ctypes.c_int)()
+        _lib.check(self.lib.sbe_ctx_wait_flag(self.handle, ctypes.byref(p)), "sbe_ctx_wait_flag")
+        return p.contents if p else None
 
     def check(self):
         """Wait for the current stream and raise if a device-side bounded wait gave up."""

@@ -23,11 +23,14 @@ def _context():
 def test_flag_of_its_own_context():
     from pulsesuite_gb300 import _lib
     a, b = _context(), _context()
+    flags = a.wait_flag(), b.wait_flag()
     tile = a.f64_wait_selftest()
     b.check()                                   # the failure is not b's
+    assert [f.value != 0 for f in flags] == [True, False]
     with pytest.raises(_lib.SbeError):
         a.check()
     a.check()                                   # reported once
+    assert flags[0].value == 0
     assert bool(torch.isnan(tile).all())
     z = torch.ones((64, 64), dtype=torch.complex128, device="cuda")
     from pulsesuite_gb300 import SBEs
