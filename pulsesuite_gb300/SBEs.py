@@ -319,10 +319,10 @@ class SBESolver:
         """Copy a wire's grid and its four fields into pinned host memory and from there, in
         one transfer on the current stream, to the device: (RR, f4).  Each wire's transfer is
         waited for before its host memory is filled again."""
-        x = np.asarray(rr, dtype=np.float64).reshape(-1)
-        fields = [np.asarray(f, dtype=complex) for f in fields]
-        n, nslot, shape = x.size, self.Nw if self.batch else 1, fields[0].shape
-        if fields[0].size != n or not all([f.shape == shape for f in fields]):
+        x = np.asarray(rr, dtype=np.float64)
+        a, b, c, v = fields = [np.asarray(f, dtype=complex) for f in fields]
+        n, nslot = x.size, self.Nw if self.batch else 1
+        if not (a.shape == b.shape == c.shape == v.shape and a.size == n):
             raise ValueError("QWCalculator: the fields need one shape, with a value per grid point")
         if self._hin is None or self._hin.shape[2] != n:
             self._hin = _pinned((nslot, 5, n))
@@ -335,8 +335,8 @@ class SBESolver:
             self._sent[w - 1].synchronize()
         h = self._hin_np[w - 1]
         for i, f in enumerate(fields):
-            h[i] = f.reshape(-1)
-        h[4].view(np.float64)[:n] = x
+            h[i] = f if f.ndim == 1 else f.reshape(-1)
+        h[4].view(np.float64)[:n] = x if x.ndim == 1 else x.reshape(-1)
         d = self._din[w - 1]
         d.copy_(self._hin[w - 1], non_blocking=True)
         self._sent[w - 1] = torch.cuda.current_stream()
