@@ -277,9 +277,9 @@ __global__ void __launch_bounds__(128) k_f64_hbuild(const __grid_constant__ HBui
 
 // dP, dC, dD from the partial products (SBEs.py:1942-1965, 2309-2327, 2607-2625): the sum
 // of each output's partials and of the terms with a diagonal element of C, D, Hee, Hhh,
-//   dP: P_mn (Hhh_mm + Hee_nn) - Heh_nm (D_mm + C_nn)
+//   dP: P_mn (Hhh_mm + Hee_nn) + Heh_nm (1 - D_mm - C_nn)
 //   dC: Hee_nm (C_mm - C_nn) + C_mn (Hee_nn - Hee_mm),   dD with Hhh and D,
-// over i hbar, for dP also Heh^T / (i hbar), the rates and OffP; with stage 1-4 the RK4 update of
+// over i hbar (dP's with the Heh^T of its own), for dP also the rates and OffP; with stage 1-4 the RK4 update of
 // k_rk4_axpy.  Bound by the FP64 pipes (some 45 operations an element); one element a thread, so
 // that a few small wires reach all SMs (four elements a thread: 1 x 64 13.3 us, 2 x 512 93; one
 // 2 x 512 81 before it had the diagonals' terms).
@@ -336,24 +336,24 @@ __global__ void __launch_bounds__(256) k_f64_finish(const __grid_constant__ Fini
   }
   const double2 h = ht[tx][ty];
   {
-    // x (e_n -+ e_m) + h (w_m -+ w_n), the latter turned round for dP
+    // x (e_n - e_m) + h (w_m - w_n), for dP x (e_n + e_m) + h (1 - w_m - w_n)
     const double2 en = dn[0][tx], wn = dn[1][tx], em = dm[0][ty], wm = dm[1][ty];
     double2 e, w;
     if (which == 0) {
       e = cadd(en, em);
-      w = make_double2(-(wm.x + wn.x), -(wm.y + wn.y));
+      w = make_double2(1.0 - (wm.x + wn.x), -(wm.y + wn.y));
     } else {
       e = csub(en, em);
       w = csub(wm, wn);
     }
-    sx += fma(x.x, e.x, -x.y * e.y) + fma(h.x, w.x, -h.y * w.y);
-    sy += fma(x.x, e.y, x.y * e.x) + fma(h.x, w.y, h.y * w.x);
+    sx = fma(x.x, e.x, fma(-x.y, e.y, fma(h.x, w.x, fma(-h.y, w.y, sx))));
+    sy = fma(x.x, e.y, fma(x.y, e.x, fma(h.x, w.y, fma(h.y, w.x, sy))));
   }
   double2 v = make_double2(sy * ih, -sx * ih);
   if (which == 0) {
     const double gam = a.gamE[(long long)b * nk + n] + a.gamH[(long long)b * nk + m];
-    v.x += h.y * ih - gam * x.x;
-    v.y += -h.x * ih - gam * x.y;
+    v.x -= gam * x.x;
+    v.y -= gam * x.y;
     if (a.offp) {
       const double2 f = a.offp[mb + o];
       v.x += f.y * ih;
