@@ -97,7 +97,10 @@ int sbe_ctx_table(const SbeCtx* ctx, int w, int which, void* dst, long long nbyt
  * From Nk = 32 on the products run on digit planes in scratch from a stream-ordered
  * pool of the library's own, which keeps up to 64 MB between calls (no host
  * synchronisation); without that memory, and inside a stream capture, on plain FP64
- * kernels that need none.                                                      */
+ * kernels that need none.  Accuracy of an element of a product A B there: about 2^-52 of
+ * the norms of the row of A and the column of B that meet in it, the diagonals of
+ * C, D, Hee and Hhh left out of them (their terms are plain FP64); the plain kernels
+ * keep it to the magnitudes of the element's own terms.                         */
 /* SBEs.py:1839 dpdt (p[kh][ke]).                                               */
 int sbe_dpdt(int nk, const double* C, const double* D, const double* P, const double* Heh,
              const double* Hee, const double* Hhh, const double* GamE, const double* GamH,
@@ -221,7 +224,12 @@ int sbe_leapfrog_step(SbeCtx* ctx, double* const* state9, const double* Ek, doub
  * SBE_PREC_FP64 or SBE_PREC_MIXED (SBE_ERR_UNSUPPORTED for a context with
  * SBE_F_DCTRANS: the reference's transport leaves C, D non-Hermitian; the mixed
  * path also needs one flag set over the context and every Nk a multiple of 8; the
- * Nk may differ between wires).                                                */
+ * Nk may differ between wires).
+ * The FP64 steps (this, sbe_leapfrog_step, sbe_rhs) run their products on digit planes
+ * as the pure functions do, in a workspace that the first of them allocates.  A
+ * context takes plain FP64 kernels instead, 25 to 60 times slower, if one of its wires
+ * has Nk < 32, if that allocation fails (for the context's life), or while the first
+ * step of all is itself being captured: make one step before a capture of your own.  */
 int sbe_rk4_step(SbeCtx* ctx, double* P, double* C, double* D, const double* Ek0,
                  const double* dEk, double dt, int precision, double* src_out, void* stream);
 /* A local field uniform along every wire (the local-field drivers of the reference,

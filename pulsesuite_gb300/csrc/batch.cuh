@@ -59,8 +59,8 @@ __global__ void __launch_bounds__(Body::kThreads, Body::kBlocks)
 }
 
 // Collects the parts of one pass and launches them, kMax a launch; a pass of few parts takes a
-// small parameter block.  A sweep of 64 wires in seven buckets: 548 launches a step, 83 so, and
-// 3.87 -> 2.27 ms (one launch per part left the SMs between a few small blocks and the launch
+// small parameter block.  A sweep of 64 wires in seven buckets: 548 launches a step, 83 so (57 with
+// the passes joined since), and 3.87 -> 2.27 ms (one launch per part left the SMs between a few small blocks and the launch
 // gap); 1 x 64 (P, C, D together) 403 -> 334 us.
 template <class Body, class F = decltype(Body::signature())>
 class Batch;

@@ -281,8 +281,9 @@ __global__ void __launch_bounds__(128) k_f64_hbuild(const __grid_constant__ HBui
 //   dC: Hee_nm (C_mm - C_nn) + C_mn (Hee_nn - Hee_mm),   dD with Hhh and D,
 // over i hbar (dP's with the Heh^T of its own), for dP also the rates and OffP; with stage 1-4 the RK4 update of
 // k_rk4_axpy.  Bound by the FP64 pipes (some 45 operations an element); one element a thread, so
-// that a few small wires reach all SMs (four elements a thread: 1 x 64 13.3 us, 2 x 512 93; one
-// 2 x 512 81 before it had the diagonals' terms).
+// that a few small wires reach all SMs (four elements a thread: 1 x 64 13.3 us, 2 x 512 93; one: 4.7
+// and 81).  The diagonals' terms take it from 81 to 112 us at 2 x 512, 56 to 87 at 8 x 256, 4.7 to
+// 5.2 at 1 x 64.
 struct Finish {
   int nk, nw, nsum, stage, first;   // first: output of blockIdx.z / nw = 0 (single calls)
   double dt, dt6;                   // the step, and a sixth of it
@@ -389,9 +390,12 @@ static const TermDef kTerms[3][4] = {
     // D Hhh^T - Hhh^T D + conj(P) Heh - Heh^H P^T
     {{F_D, F_HH, 0, 0, 0}, {F_HHT, F_DT, 0, 0, 1}, {F_P, F_EHT, 1, 0, 0}, {F_EHT, F_P, 1, 0, 1}}};
 
-// Cuts of a product's K sequence (2 nkb K blocks): the fewest K-block times over the waves of
-// 152 CTAs, a tile's fixed cost being about 1.2 of them and a further part's sums and traffic
-// 0.15 (sources, whose reduction is as large as the products' output: 2) (1 x 512, 768 tiles: 340 us uncut, 322 in two; 8 x 256, 1536 tiles: 326 uncut, 331).
+// Into how many parts a product's K sequence (2 nkb K blocks) is cut, each a tile of its own whose
+// partial result the finish adds.  Cost of p parts, in times of one K block: the waves of 152 CTAs
+// (an SM each) times what a tile takes, its K blocks and 1.2 for its start and end; and for every
+// part after the first the memory traffic and additions of its partial result, 0.15 for commutators
+// and 2 for sources, whose reduction reads as much as the products write.  Measured: 1 x 512 (768
+// tiles) 340 us uncut, 322 in two; 8 x 256 (1536 tiles) 326 uncut, 331 in two.
 static int product_parts(long long units, int nkb, double part_cost = 0.15) {
   const int n = 2 * nkb;
   int best = 1;

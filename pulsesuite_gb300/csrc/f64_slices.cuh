@@ -11,6 +11,9 @@
 // The planes with i + j > 7 are left out: they add about 2^-57 of the rows' norms at K =
 // 1024.  By Cauchy-Schwarz the whole sum over K stays below 2^124, so the epilogue adds the
 // accumulators modulo 2^64 in units of 2^62 and rounds once to FP64.
+// The error of an element is therefore measured by the norms of the two rows that meet in it, not
+// by its own terms: an operand whose rows hold a few large elements beside small ones that matter
+// gives those to the caller's FP64 (f64_path.cu: the diagonals of C, D, Hee, Hhh).
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

@@ -4,7 +4,7 @@
 
 namespace sbe {
 
-// 2^lgtr transforms of length 2^lg (at least 4): element p of transform c at a[p ps + c cs];
+// 2^lgtr transforms of length 2^lg (2 points take the opening stage alone): element p of transform c at a[p ps + c cs];
 // consecutive threads walk c (c_fast) or p.  dir -1: exp(-i ...), +1: exp(+i ...);
 // tw[j] = exp(-2 pi i j / 2^lg).  Returns the buffer, a or b, that holds the result in natural
 // order.  Radix 4 (an odd log length opens with a radix-2 stage): the two-wide FP64 pipe bounds

@@ -14,9 +14,9 @@
 // (64, all fields of one set of knots) so that the grid spreads them over the SMs.
 // A value that is not finite reaches the coefficients of some 100 points only; a solve from end to
 // end spreads it over all, which the calls that resample one wire keep (bad, k_spline_eval).
-// Mean of the solves of a step (4 fields on 4096 points, 5 on Nr = 230): 17.5 ms with one
-// thread per field, 32 us here; with the pivots' coefficients and reciprocals formed by all
-// threads (3 fields on 8192, 5 on 514: 31 -> 22 us) 22 us.
+// Mean of the solves of a step (4 fields on 4096 points, 5 on Nr = 230): 17.5 ms with one thread
+// per field, 32 us with the chains in threads of their own, 22 us with the pivots' coefficients and
+// reciprocals formed by all threads (3 fields on 8192, 5 on 514: 31 -> 22 us).
 #include "spline.cuh"
 #include "fp_bits.cuh"
 
